@@ -1194,7 +1194,8 @@ void batch_run(lvg_ctx* c, const BatchInput& in, int32_t* part_out, double* q_ou
     double* gm = a.lo_n<double>(G);
     LVG_CUDA(cudaMemcpyAsync(vbase_d, L.vbase.data(), sizeof(int32_t) * (G + 1), cudaMemcpyHostToDevice, s));
     batch_vgid(vbase_d, G, V, vgid, s);
-    batch_m(lsrc_d, lw_d, E, vgid, gm, G, s);
+    int64_t* ecnt_d = a.lo_n<int64_t>(G);
+    batch_m(lsrc_d, lw_d, E, vgid, gm, ecnt_d, G, s);
     g.gm = gm;
     g.vgid = vgid;
     build_level(g, c->tune, a, s);
@@ -1305,8 +1306,6 @@ void batch_run(lvg_ctx* c, const BatchInput& in, int32_t* part_out, double* q_ou
     gather_u32(pos, vbase_d, G + 1, cbase_d, s);
     std::vector<int32_t> cbase(G + 1);
     LVG_CUDA(cudaMemcpyAsync(cbase.data(), cbase_d, sizeof(int32_t) * (G + 1), cudaMemcpyDeviceToHost, s));
-    int64_t* ecnt_d = a.hi_n<int64_t>(G);
-    batch_count(lsrc_d, E, vgid, ecnt_d, G, s);
     std::vector<int64_t> ecnt(G);
     LVG_CUDA(cudaMemcpyAsync(ecnt.data(), ecnt_d, sizeof(int64_t) * G, cudaMemcpyDeviceToHost, s));
     std::vector<int32_t> lidx(G0, -1);

@@ -270,7 +270,8 @@ void batch_globalize(const int32_t* const* psrc, const int32_t* const* pdst, con
 void batch_vgid(const int32_t* vbase, int32_t G, int32_t V, int32_t* vgid, cudaStream_t s);
 // local[i] = i - voff[gid[i]]
 void batch_local_ids(const int32_t* gid, const int32_t* voff, int32_t V, int32_t* local, cudaStream_t s);
-void batch_m(const int32_t* src, const float* w, int64_t E, const int32_t* vgid, double* gm, int32_t G,
+// m and entry count of every graph (each graph's entries are one range of the list)
+void batch_m(const int32_t* src, const float* w, int64_t E, const int32_t* vgid, double* gm, int64_t* cnt, int32_t G,
              cudaStream_t s);
 void batch_init(const LevelGraph& g, CommState& st, cudaStream_t s);
 // mode: 0 init (Q only), 1 pass (per-graph ΔQ test + commit), 2 force commit
@@ -290,8 +291,6 @@ int64_t batch_induce(const LevelGraph& g, const int32_t* part, const int32_t* vg
                      cudaStream_t s);
 // out[j] = pos[idx[j]]
 void gather_u32(const uint32_t* pos, const int32_t* idx, int32_t n, int32_t* out, cudaStream_t s);
-// entries of the list per graph
-void batch_count(const int32_t* src, int64_t E, const int32_t* vgid, int64_t* cnt, int32_t G, cudaStream_t s);
 void batch_compose(int32_t* local0, const int32_t* gid0, int64_t n, const int32_t* lidx, const int32_t* vbase,
                    const int32_t* cbase, const int32_t* part, cudaStream_t s);
 // FP64 Newman modularity of every graph: community ids coff[g] + local0[v]
