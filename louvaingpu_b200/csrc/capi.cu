@@ -360,44 +360,10 @@ int32_t renumber_level(lvg_ctx* c) {
 
 // Coarsen into the next level and build it.
 void induce_level(lvg_ctx* c) {
-  int32_t *os = nullptr, *od = nullptr;
-  float* ow = nullptr;
   c->arena.hi = c->run_hi;
   LVG_CUDA(cudaEventRecord(c->pev[4], c->stream));
-  PreCsr hi_csr;
-  int64_t n = induce(c->g, c->d_part_cur, c->C_cur, &os, &od, &ow, c->arena, c->stream, &hi_csr, c->tune.coarsen);
-  // the next level's list (and its CSR, when the coarsening wrote it) moves
-  // down to the start of the level region
-  c->arena.lo = c->base_lo;
-  int32_t* ns = c->arena.lo_n<int32_t>(n);
-  int32_t* nd = c->arena.lo_n<int32_t>(n);
-  float* nw = c->arena.lo_n<float>(n);
-  auto down = [&](void* dst, const void* src, size_t bytes) {
-    if (bytes) LVG_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, c->stream));
-  };
-  down(ns, os, sizeof(int32_t) * n);
-  down(nd, od, sizeof(int32_t) * n);
-  down(nw, ow, sizeof(float) * n);
-  const int32_t C1 = c->C_cur;
-  c->pre_next = PreCsr();
-  if (hi_csr.valid) {
-    PreCsr& p = c->pre_next;
-    p.off = c->arena.lo_n<int64_t>((int64_t)C1 + 1);
-    p.col = c->arena.lo_n<int32_t>(hi_csr.nnz);
-    p.cw = c->arena.lo_n<float>(hi_csr.nnz);
-    p.k = c->arena.lo_n<double>(C1);
-    p.loopw = c->arena.lo_n<float>(C1);
-    p.has_loop = c->arena.lo_n<uint8_t>(C1);
-    down(p.off, hi_csr.off, sizeof(int64_t) * ((size_t)C1 + 1));
-    down(p.col, hi_csr.col, sizeof(int32_t) * hi_csr.nnz);
-    down(p.cw, hi_csr.cw, sizeof(float) * hi_csr.nnz);
-    down(p.k, hi_csr.k, sizeof(double) * C1);
-    down(p.loopw, hi_csr.loopw, sizeof(float) * C1);
-    down(p.has_loop, hi_csr.has_loop, C1);
-    p.m = hi_csr.m;
-    p.nnz = hi_csr.nnz;
-    p.valid = true;
-  }
+  CoarseList L;
+  induce(c->g, c->d_part_cur, c->C_cur, c->base_lo, L, c->pre_next, c->arena, c->stream, c->tune.coarsen);
   LVG_CUDA(cudaEventRecord(c->pev[5], c->stream));
   sync(c);
   if (!c->levels.empty()) {
@@ -408,10 +374,10 @@ void induce_level(lvg_ctx* c) {
   int32_t C = c->C_cur;
   c->g = LevelGraph();
   c->g.V = C;
-  c->g.E = n;
-  c->g.src = ns;
-  c->g.dst = nd;
-  c->g.w = nw;
+  c->g.E = L.n;
+  c->g.src = L.src;
+  c->g.dst = L.dst;
+  c->g.w = L.w;
   c->g.pre = &c->pre_next;
   c->level += 1;
   prepare_level(c);
@@ -1188,6 +1154,7 @@ void batch_run(lvg_ctx* c, const BatchInput& in, int32_t* part_out, double* q_ou
     g.src = lsrc_d;
     g.dst = ldst_d;
     g.w = lw_d;
+    g.pre = level > 0 ? &c->pre_next : nullptr;
     // per-level graph arrays
     int32_t* vbase_d = a.lo_n<int32_t>(G + 1);
     int32_t* vgid = a.lo_n<int32_t>(V);
@@ -1346,24 +1313,14 @@ void batch_run(lvg_ctx* c, const BatchInput& in, int32_t* part_out, double* q_ou
     }
     int32_t* shift_d = a.hi_n<int32_t>(G);
     LVG_CUDA(cudaMemcpyAsync(shift_d, shift.data(), sizeof(int32_t) * G, cudaMemcpyHostToDevice, s));
-    int32_t *os = nullptr, *od = nullptr;
-    float* ow = nullptr;
-    int64_t n = batch_induce(g, part, vgid, shift_d, N.vbase.back(), E_keep, &os, &od, &ow, a, s);
-    a.lo = base_lo;
-    int32_t* ns = a.lo_n<int32_t>(n);
-    int32_t* nd = a.lo_n<int32_t>(n);
-    float* nw = a.lo_n<float>(n);
-    if (n > 0) {
-      LVG_CUDA(cudaMemcpyAsync(ns, os, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, s));
-      LVG_CUDA(cudaMemcpyAsync(nd, od, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, s));
-      LVG_CUDA(cudaMemcpyAsync(nw, ow, sizeof(float) * n, cudaMemcpyDeviceToDevice, s));
-    }
+    CoarseList next;
+    batch_induce(g, part, vgid, shift_d, N.vbase.back(), E_keep, base_lo, next, c->pre_next, a, s, c->tune.coarsen);
     sync(c);
     a.hi = run_hi;
-    lsrc_d = ns;
-    ldst_d = nd;
-    lw_d = nw;
-    E = n;
+    lsrc_d = next.src;
+    ldst_d = next.dst;
+    lw_d = next.w;
+    E = next.n;
     L = std::move(N);
   }
   // per-graph FP64 Newman modularity of the final partitions

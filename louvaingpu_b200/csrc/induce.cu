@@ -71,13 +71,15 @@ unsigned ic_grid(int64_t n) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (n); i += (int64_t)gridDim.x * blockDim.x)
 
 // ------------------------------------------------------------------ members
-// Sort key of a vertex: its community, or C for a vertex without entries
-// (those sort after every member and take no list positions).
+// Sort key of a vertex: its community, or C for a vertex without entries or
+// without a community (part < 0: its graph has finished, in a batched run);
+// those sort after every member and take no list positions.
 __global__ void ic_member_keys_kernel(int32_t V, const int64_t* off, const uint8_t* has_loop, const int32_t* part,
                                       int32_t C, uint64_t* key, float* val, uint32_t* loops) {
   IC_FOR(i, V) {
     const int64_t rl = off[i + 1] - off[i] + has_loop[i];
-    key[i] = rl > 0 ? (uint64_t)(uint32_t)part[i] : (uint64_t)(uint32_t)C;
+    const int32_t p = part[i];
+    key[i] = rl > 0 && p >= 0 ? (uint64_t)(uint32_t)p : (uint64_t)(uint32_t)C;
     val[i] = __int_as_float((int32_t)i);
     loops[i] = has_loop[i];
   }
@@ -1127,11 +1129,12 @@ __global__ void tx_dense_kernel(int32_t nz, const int32_t* mcomm, const uint32_t
   }
 }
 
-// Dense community id of every vertex with entries (the only vertices that
-// appear as a neighbour); 0 for the others, which are never read.
+// Dense community id of every vertex with entries and a community (the only
+// vertices that appear as a neighbour in the rows laid out); 0 for the
+// others, which are never read.
 __global__ void tx_vdense_kernel(int32_t V, const int32_t* part, const int64_t* off, const uint8_t* has_loop,
                                  const int32_t* dn, int32_t* pd) {
-  IC_FOR(v, V) pd[v] = (off[v + 1] > off[v] || has_loop[v]) ? dn[part[v]] : 0;
+  IC_FOR(v, V) pd[v] = (off[v + 1] > off[v] || has_loop[v]) && part[v] >= 0 ? dn[part[v]] : 0;
 }
 
 void tx_attributes() {
@@ -1163,14 +1166,12 @@ size_t induce_transposed_scratch(int64_t V, int64_t E, int64_t C) {
   return b + ((size_t)64 << 10) * 32;                                              // alignment slack
 }
 
-bool induce_transposed(const LevelGraph& g, const int32_t* part, int32_t C, int32_t* osrc, int32_t* odst, float* ow,
-                       int64_t* count, PreCsr* next, Arena& a, cudaStream_t s) {
+bool induce_transposed(const LevelGraph& g, const int32_t* part, int32_t C, int64_t E, size_t base_lo,
+                       CoarseList& out, PreCsr& next, Arena& a, cudaStream_t s) {
   const int32_t V = g.V;
-  const int64_t E = g.E;
-  if (!g.sorted_symmetric || V <= 0 || C <= 0) return false;
+  if (!g.sorted_symmetric || V <= 0 || C <= 0 || E <= 0) return false;
   if (E + 2 * (int64_t)kIcChunk >= ((int64_t)1 << 32)) return false;   // heads and positions are 32-bit
   if (a.hi < a.lo || a.hi - a.lo < induce_transposed_scratch(V, E, C)) return false;
-  if (E == 0) { *count = 0; return true; }
   HiScope hs(a);
   const int64_t nchunks = (E + kIcChunk - 1) / kIcChunk;
   // members in community order (stable: vertex order inside a community)
@@ -1243,7 +1244,40 @@ bool induce_transposed(const LevelGraph& g, const int32_t* part, int32_t C, int3
   LVG_CUDA(cudaMemcpyAsync(&h_frac, flags, sizeof h_frac, cudaMemcpyDeviceToHost, s));
   LVG_CUDA(cudaStreamSynchronize(s));   // both values with one wait
   const int64_t cnt = (int64_t)((uint64_t)h_tot & 0xffffffffull);
-  const bool int_weights = h_frac == 0u;
+  // The CSR is written only for integral weights: then every sum is exact,
+  // so the coarse list is exactly symmetric, as the CSR written from one
+  // direction assumes.
+  const bool csr = h_frac == 0u;
+  // The coarse list and CSR go straight to their place at the start of the
+  // level region: their sizes are known (each run is one entry, each
+  // self-loop run no CSR entry), and what is there -- this level's list, CSR
+  // and state -- has been read for the last time by the layout.  The region
+  // never grows past the room checked on entry.  Writing them to scratch and
+  // copying them down cost 5.8 ms of a 151 ms R-MAT scale 24 run.
+  const size_t old_lo = a.lo;
+  a.lo = base_lo;
+  IcCsrOut O{};
+  try {
+    out.src = a.lo_n<int32_t>(cnt);
+    out.dst = a.lo_n<int32_t>(cnt);
+    out.w = a.lo_n<float>(cnt);
+    if (csr) {
+      next.nnz = cnt - (int64_t)((uint64_t)h_tot >> 32);
+      next.off = a.lo_n<int64_t>((int64_t)C + 1);
+      next.col = a.lo_n<int32_t>(next.nnz);
+      next.cw = a.lo_n<float>(next.nnz);
+      next.k = a.lo_n<double>(C);
+      next.loopw = a.lo_n<float>(C);
+      next.has_loop = a.lo_n<uint8_t>(C);
+    }
+  } catch (...) {   // the level stays as it is
+    a.lo = old_lo;
+    next = PreCsr();
+    throw;
+  }
+  out.n = cnt;
+  int32_t *osrc = out.src, *odst = out.dst;
+  float* ow = out.w;
   double* opensum = a.hi_n<double>(nchunks);
   uint32_t* openflag = a.hi_n<uint32_t>(nchunks);
   uint32_t* hl = a.hi_n<uint32_t>((int64_t)C + 1);
@@ -1252,16 +1286,11 @@ bool induce_transposed(const LevelGraph& g, const int32_t* part, int32_t C, int3
   LVG_CUDA(cudaMemsetAsync(openflag, 0, sizeof(uint32_t) * (size_t)nchunks, s));
   LVG_CUDA(cudaMemsetAsync(hl, 0, sizeof(uint32_t) * ((size_t)C + 1), s));
   LVG_CUDA(cudaMemsetAsync(dcount, 0, sizeof(uint32_t) * ((size_t)C + 1), s));
-  // The CSR is written only for integral weights: then every sum is exact,
-  // so the coarse list is exactly symmetric, as the CSR written from one
-  // direction assumes.
-  IcCsrOut O{};
-  const bool csr = next && next->col && int_weights;
   if (csr) {
-    LVG_CUDA(cudaMemsetAsync(next->k, 0, sizeof(double) * (size_t)C, s));
-    LVG_CUDA(cudaMemsetAsync(next->loopw, 0, sizeof(float) * (size_t)C, s));
-    LVG_CUDA(cudaMemsetAsync(next->has_loop, 0, (size_t)C, s));
-    O = IcCsrOut{next->col, next->cw, next->k, next->loopw, next->has_loop, hl, nullptr};
+    LVG_CUDA(cudaMemsetAsync(next.k, 0, sizeof(double) * (size_t)C, s));
+    LVG_CUDA(cudaMemsetAsync(next.loopw, 0, sizeof(float) * (size_t)C, s));
+    LVG_CUDA(cudaMemsetAsync(next.has_loop, 0, (size_t)C, s));
+    O = IcCsrOut{next.col, next.cw, next.k, next.loopw, next.has_loop, hl, nullptr};
   }
   tx_emit_kernel<<<(unsigned)nchunks, kTxThreads, sizeof(TxEmitSmem), s>>>(keys, vals, E, Bb, tscan, und, osrc,
                                                                            odst, ow, opensum, openflag, hl, dcount,
@@ -1274,17 +1303,14 @@ bool induce_transposed(const LevelGraph& g, const int32_t* part, int32_t C, int3
     uint32_t* loopx = a.hi_n<uint32_t>((int64_t)C + 1);
     scan_u32(dcount, segoff, C, a, s);
     scan_u32(hl, loopx, C, a, s);
-    ic_csr_off_kernel<<<ic_grid((int64_t)C + 1), kIcFlat, 0, s>>>(C, segoff, loopx, next->off);
+    ic_csr_off_kernel<<<ic_grid((int64_t)C + 1), kIcFlat, 0, s>>>(C, segoff, loopx, next.off);
     LVG_LAUNCH();
     double* d_m = a.hi_n<double>(1);
     tree_sum_f32(ow, cnt, d_m, a, s);   // as build_level's m over the list (NeighbourCompute.cu:46)
-    LVG_CUDA(cudaMemcpyAsync(&next->m, d_m, sizeof(double), cudaMemcpyDeviceToHost, s));
-    const int64_t loops = read_back(loopx + C, s);
-    next->nnz = cnt - loops;
-    next->valid = true;
+    LVG_CUDA(cudaMemcpyAsync(&next.m, d_m, sizeof(double), cudaMemcpyDeviceToHost, s));
+    next.valid = true;
   }
   LVG_CUDA(cudaStreamSynchronize(s));
-  *count = cnt;
   return true;
 }
 

@@ -2747,38 +2747,76 @@ int32_t renumber(const LevelGraph& g, const int32_t* comm, int32_t* part, Arena&
   return (int32_t)C;
 }
 
-int64_t induce(const LevelGraph& g, const int32_t* part, int32_t C, int32_t** out_src, int32_t** out_dst,
-               float** out_w, Arena& a, cudaStream_t s, PreCsr* next, int32_t mode) {
+// A coarse list (and CSR) written to scratch at the arena's high end, moved to
+// the start of the level region.
+static void move_down(const CoarseList& hi, const PreCsr& hi_csr, int32_t C, size_t base_lo, CoarseList& out,
+                      PreCsr& next, Arena& a, cudaStream_t s) {
+  a.lo = base_lo;
+  const int64_t n = hi.n;
+  out.src = a.lo_n<int32_t>(n);
+  out.dst = a.lo_n<int32_t>(n);
+  out.w = a.lo_n<float>(n);
+  out.n = n;
+  auto down = [&](void* dst, const void* src, size_t bytes) {
+    if (bytes) LVG_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, s));
+  };
+  down(out.src, hi.src, sizeof(int32_t) * n);
+  down(out.dst, hi.dst, sizeof(int32_t) * n);
+  down(out.w, hi.w, sizeof(float) * n);
+  next = PreCsr();
+  if (!hi_csr.valid) return;
+  next.off = a.lo_n<int64_t>((int64_t)C + 1);
+  next.col = a.lo_n<int32_t>(hi_csr.nnz);
+  next.cw = a.lo_n<float>(hi_csr.nnz);
+  next.k = a.lo_n<double>(C);
+  next.loopw = a.lo_n<float>(C);
+  next.has_loop = a.lo_n<uint8_t>(C);
+  down(next.off, hi_csr.off, sizeof(int64_t) * ((size_t)C + 1));
+  down(next.col, hi_csr.col, sizeof(int32_t) * hi_csr.nnz);
+  down(next.cw, hi_csr.cw, sizeof(float) * hi_csr.nnz);
+  down(next.k, hi_csr.k, sizeof(double) * C);
+  down(next.loopw, hi_csr.loopw, sizeof(float) * C);
+  down(next.has_loop, hi_csr.has_loop, C);
+  next.m = hi_csr.m;
+  next.nnz = hi_csr.nnz;
+  next.valid = true;
+}
+
+void induce(const LevelGraph& g, const int32_t* part, int32_t C, size_t base_lo, CoarseList& out, PreCsr& next,
+            Arena& a, cudaStream_t s, int32_t mode) {
   const int64_t E = g.E;
   if (E >= ((int64_t)1 << 32)) throw Error(LVG_ERR_CAPACITY, "level edge list exceeds 2^32-1 entries");
-  // the output stays in high scratch for the caller; temporaries are released below it
-  int32_t* osrc = a.hi_n<int32_t>(E);
-  int32_t* odst = a.hi_n<int32_t>(E);
-  float* ow = a.hi_n<float>(E);
-  int64_t cnt = 0;
-  if (next) {
-    *next = PreCsr();
-    if (g.sorted_symmetric) {
-      next->off = a.hi_n<int64_t>((int64_t)C + 1);
-      next->col = a.hi_n<int32_t>(E);
-      next->cw = a.hi_n<float>(E);
-      next->k = a.hi_n<double>(C);
-      next->loopw = a.hi_n<float>(C);
-      next->has_loop = a.hi_n<uint8_t>(C);
-    }
-  }
+  out = CoarseList();
+  next = PreCsr();
   // automatic: by transposition (measured on one B200, R-MAT scale 25: level 0
   // 1.05 G -> 0.68 G entries 156 -> 106 ms; level 1, where most entries merge,
   // 46 -> 48 ms; the LFR n = 2^20 levels 2.2 -> 1.9 and 1.7 -> 1.5 ms)
   // (a sort-free method that lacks arena room declines, and the next one is tried)
   const bool by_tx = mode == kCoarsenTransposed || mode == kCoarsenAuto;
-  if ((by_tx && induce_transposed(g, part, C, osrc, odst, ow, &cnt, next, a, s)) ||
-      (mode != kCoarsenSort && induce_sorted(g, part, C, osrc, odst, ow, &cnt, next, a, s))) {
-    *out_src = osrc;
-    *out_dst = odst;
-    *out_w = ow;
-    return cnt;
+  if (by_tx && induce_transposed(g, part, C, E, base_lo, out, next, a, s)) return;
+  HiScope outer(a);
+  CoarseList hi;
+  PreCsr hi_csr;
+  hi.src = a.hi_n<int32_t>(E);
+  hi.dst = a.hi_n<int32_t>(E);
+  hi.w = a.hi_n<float>(E);
+  if (g.sorted_symmetric) {
+    hi_csr.off = a.hi_n<int64_t>((int64_t)C + 1);
+    hi_csr.col = a.hi_n<int32_t>(E);
+    hi_csr.cw = a.hi_n<float>(E);
+    hi_csr.k = a.hi_n<double>(C);
+    hi_csr.loopw = a.hi_n<float>(C);
+    hi_csr.has_loop = a.hi_n<uint8_t>(C);
   }
+  if (mode != kCoarsenSort && induce_sorted(g, part, C, hi.src, hi.dst, hi.w, &hi.n, &hi_csr, a, s)) {
+    move_down(hi, hi_csr, C, base_lo, out, next, a, s);
+    LVG_CUDA(cudaStreamSynchronize(s));
+    return;
+  }
+  hi_csr = PreCsr();
+  int32_t *osrc = hi.src, *odst = hi.dst;
+  float* ow = hi.w;
+  int64_t cnt = 0;
   {
     HiScope hs(a);
     const int B = std::max(1, bits_for(C));
@@ -2816,10 +2854,9 @@ int64_t induce(const LevelGraph& g, const int32_t* part, int32_t C, int32_t** ou
     }
     LVG_CUDA(cudaStreamSynchronize(s));
   }
-  *out_src = osrc;
-  *out_dst = odst;
-  *out_w = ow;
-  return cnt;
+  hi.n = cnt;
+  move_down(hi, hi_csr, C, base_lo, out, next, a, s);
+  LVG_CUDA(cudaStreamSynchronize(s));
 }
 
 // Kc and Ain of a list known to be symmetric (every (u, v, w) has its
@@ -3200,6 +3237,15 @@ __global__ void batch_keys_kernel(const int32_t* src, const int32_t* dst, const 
   }
 }
 
+// Community of the next level's numbering; -1 where the graph has finished.
+__global__ void batch_part_kernel(int32_t V, const int32_t* part, const int32_t* vgid, const int32_t* shift,
+                                  int32_t* out) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < V; i += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t sh = shift[vgid[i]];
+    out[i] = sh == INT_MIN ? -1 : part[i] + sh;
+  }
+}
+
 __global__ void gather_u32_kernel(const uint32_t* pos, const int32_t* idx, int32_t n, int32_t* out) {
   for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x)
     out[j] = (int32_t)pos[idx[j]];
@@ -3361,14 +3407,33 @@ int32_t renumber_pos(const LevelGraph& g, const int32_t* comm, int32_t* part, ui
   return (int32_t)C;
 }
 
-int64_t batch_induce(const LevelGraph& g, const int32_t* part, const int32_t* vgid, const int32_t* shift,
-                     int32_t C_next, int64_t E_keep, int32_t** out_src, int32_t** out_dst, float** out_w, Arena& a,
-                     cudaStream_t s) {
+void batch_induce(const LevelGraph& g, const int32_t* part, const int32_t* vgid, const int32_t* shift, int32_t C_next,
+                  int64_t E_keep, size_t base_lo, CoarseList& out, PreCsr& next, Arena& a, cudaStream_t s,
+                  int32_t mode) {
   const int64_t E = g.E;
   if (E >= ((int64_t)1 << 32)) throw Error(LVG_ERR_CAPACITY, "level edge list exceeds 2^32-1 entries");
-  int32_t* osrc = a.hi_n<int32_t>(E_keep);
-  int32_t* odst = a.hi_n<int32_t>(E_keep);
-  float* ow = a.hi_n<float>(E_keep);
+  out = CoarseList();
+  next = PreCsr();
+  HiScope outer(a);
+  // The union of sorted symmetric lists is one, and finished graphs leave it
+  // row by row, so the batch coarsens as a single graph does: one stable sort
+  // by the width of a dense community id instead of a sort by both ids, and
+  // the next level's CSR with it (128 graphs of up to 200,000 vertices: 69.8
+  // -> 51.3 ms a run).
+  if (mode == kCoarsenTransposed || mode == kCoarsenAuto) {
+    int32_t* pshift = a.hi_n<int32_t>(g.V);
+    if (g.V > 0) {
+      batch_part_kernel<<<sm_grid(g.V, kThreads), kThreads, 0, s>>>(g.V, part, vgid, shift, pshift);
+      LVG_LAUNCH();
+    }
+    if (induce_transposed(g, pshift, C_next, E_keep, base_lo, out, next, a, s)) return;
+  }
+  CoarseList hi;
+  hi.src = a.hi_n<int32_t>(E_keep);
+  hi.dst = a.hi_n<int32_t>(E_keep);
+  hi.w = a.hi_n<float>(E_keep);
+  int32_t *osrc = hi.src, *odst = hi.dst;
+  float* ow = hi.w;
   int64_t cnt = 0;
   {
     HiScope hs(a);
@@ -3408,10 +3473,9 @@ int64_t batch_induce(const LevelGraph& g, const int32_t* part, const int32_t* vg
     }
     LVG_CUDA(cudaStreamSynchronize(s));
   }
-  *out_src = osrc;
-  *out_dst = odst;
-  *out_w = ow;
-  return cnt;
+  hi.n = cnt;
+  move_down(hi, PreCsr(), C_next, base_lo, out, next, a, s);
+  LVG_CUDA(cudaStreamSynchronize(s));
 }
 
 void gather_u32(const uint32_t* pos, const int32_t* idx, int32_t n, int32_t* out, cudaStream_t s) {

@@ -199,8 +199,14 @@ void reset_ctl(CommState& st, double lower, double pass_min, int32_t max_passes,
 // member index; returns the community count (synchronises).
 int32_t renumber(const LevelGraph& g, const int32_t* comm, int32_t* part, Arena& a, cudaStream_t s);
 
-// Coarsen (InducedGraphKernel.cu:50-113): writes the next level input list to
-// high-end scratch and returns its size; out_* point into that scratch.
+// A coarse list: one entry per distinct (cu, cv) key, in key order.
+struct CoarseList {
+  int32_t* src = nullptr;
+  int32_t* dst = nullptr;
+  float* w = nullptr;
+  int64_t n = 0;
+};
+
 // Coarsening of a strictly sorted, symmetric level list without a device-wide
 // sort of all its entries (induce.cu).  Writes the same list as the
 // sort-based path into osrc/odst/ow (capacity E) and its length into *count;
@@ -210,16 +216,21 @@ int32_t renumber(const LevelGraph& g, const int32_t* comm, int32_t* part, Arena&
 // and marks it valid.
 bool induce_sorted(const LevelGraph& g, const int32_t* part, int32_t C, int32_t* osrc, int32_t* odst, float* ow,
                    int64_t* count, PreCsr* next, Arena& a, cudaStream_t s);
-// The same list (and CSR) by transposition (induce.cu): the keys listed in
-// segment order of the second community, then one stable sort by the first.
-// Same preconditions and return value as induce_sorted.
-bool induce_transposed(const LevelGraph& g, const int32_t* part, int32_t C, int32_t* osrc, int32_t* odst,
-                       float* ow, int64_t* count, PreCsr* next, Arena& a, cudaStream_t s);
-// Coarse list of the level under `part` (C communities), left at the arena's
-// high end.  With `next`: when the sort-free path runs, also the next level's
-// CSR (high end, next->valid set); otherwise next->valid stays false.
-int64_t induce(const LevelGraph& g, const int32_t* part, int32_t C, int32_t** out_src, int32_t** out_dst,
-               float** out_w, Arena& a, cudaStream_t s, PreCsr* next = nullptr, int32_t mode = kCoarsenAuto);
+// The same list (and CSR, for integral weights) by transposition (induce.cu):
+// the keys listed in segment order of the second community, then one stable
+// sort by the first.  Vertices with part < 0 and their rows are left out;
+// E: entries of the rows that stay (a row and all its neighbours' rows stay
+// or go together).  Returns false, having done nothing, when the list is not
+// in that form or the arena lacks room; otherwise list and CSR are at the
+// arena's low end from base_lo (the level's own arrays there are overwritten)
+// and a.lo is past them.
+bool induce_transposed(const LevelGraph& g, const int32_t* part, int32_t C, int64_t E, size_t base_lo,
+                       CoarseList& out, PreCsr& next, Arena& a, cudaStream_t s);
+// Coarsen (InducedGraphKernel.cu:50-113): the next level's list, and its CSR
+// when a sort-free path writes one (next.valid), at the arena's low end from
+// base_lo in place of the level's own arrays; a.lo is left past them.
+void induce(const LevelGraph& g, const int32_t* part, int32_t C, size_t base_lo, CoarseList& out, PreCsr& next,
+            Arena& a, cudaStream_t s, int32_t mode);
 
 // FP64 Newman modularity of part[] (values < C) over an input list (device).
 // symmetric: the list is known to hold (v, u, w) for every (u, v, w) (its
@@ -286,9 +297,10 @@ void launch_merge_deltas(const LevelGraph& g, CommState& st, cudaStream_t s);
 int32_t renumber_pos(const LevelGraph& g, const int32_t* comm, int32_t* part, uint32_t* pos, Arena& a,
                      cudaStream_t s);
 // Coarsen the graphs still running: part[v] + shift[graph] (INT_MIN: dropped).
-int64_t batch_induce(const LevelGraph& g, const int32_t* part, const int32_t* vgid, const int32_t* shift,
-                     int32_t C_next, int64_t E_keep, int32_t** out_src, int32_t** out_dst, float** out_w, Arena& a,
-                     cudaStream_t s);
+// E_keep: entries of the graphs that stay.  List and CSR as induce() leaves them.
+void batch_induce(const LevelGraph& g, const int32_t* part, const int32_t* vgid, const int32_t* shift, int32_t C_next,
+                  int64_t E_keep, size_t base_lo, CoarseList& out, PreCsr& next, Arena& a, cudaStream_t s,
+                  int32_t mode);
 // out[j] = pos[idx[j]]
 void gather_u32(const uint32_t* pos, const int32_t* idx, int32_t n, int32_t* out, cudaStream_t s);
 void batch_compose(int32_t* local0, const int32_t* gid0, int64_t n, const int32_t* lidx, const int32_t* vbase,
