@@ -20,6 +20,7 @@
 
 #include "louvain.cuh"
 #include "prims.cuh"
+#include "small.cuh"
 
 using namespace lvg;
 
@@ -62,6 +63,11 @@ struct lvg_ctx {
   CommState st;
   bool have_state = false;
   bool renumbered = false;
+  bool built = false;            // the level's CSR and state exist (c->g, c->st); else only its list
+  bool small0 = false;           // level 0 is a list small_run takes
+  bool replay = false;           // not built because small_run finished the run on this level:
+  double replay_lower = 0.0;     //   its state is that of a one-level phase with this floor
+  bool timed = false;            // the last level's renumbering is between pev[2] and pev[3]
   bool pristine = false;         // level 0 as loaded: no pass, state change or renumbering since
   bool symmetric0 = false;       // the level-0 list was found sorted and symmetric at load
   int32_t* d_part_cur = nullptr;
@@ -170,11 +176,18 @@ void prepare_level(lvg_ctx* c) {
   init_state(c->g, c->st, 0.0, c->cfg.pass_min_gain, c->cfg.max_passes, c->arena, c->stream);
   LVG_CUDA(cudaEventRecord(c->pev[1], c->stream));   // read once the stream has synchronised
   c->have_state = true;
+  c->built = true;
   c->renumbered = false;
 }
 
+// Largest list one launch runs to the end (small_run), and its cluster.
+constexpr int64_t kSmallRunEntries = 256 * 1024;
+constexpr int kSmallRunBlocks = 16;
+
+// `ready`: the list is sorted and symmetric, small, and has room for its level
+// build, which then waits until a call needs it.
 void load_common(lvg_ctx* c, const int32_t* d_src, const int32_t* d_dst, const float* d_w, int64_t E,
-                 int32_t V) {
+                 int32_t V, bool ready) {
   c->V0 = V;
   c->E0 = E;
   c->src0 = d_src;
@@ -193,20 +206,26 @@ void load_common(lvg_ctx* c, const int32_t* d_src, const int32_t* d_dst, const f
   c->g.dst = d_dst;
   c->g.w = d_w;
   c->g.pre = &c->pre0;
-  prepare_level(c);
-  c->symmetric0 = c->g.sorted_symmetric;
+  c->small0 = ready;
+  c->replay = false;
+  c->built = false;
+  if (ready) {
+    c->have_state = true;
+    c->renumbered = false;
+    c->symmetric0 = true;
+  } else {
+    prepare_level(c);
+    c->symmetric0 = c->g.sorted_symmetric;
+  }
   c->loaded = true;
   c->pristine = true;
 }
 
-void reset_to_level0(lvg_ctx* c) {
+void reset_to_level0(lvg_ctx* c, bool build = true) {
   // rebuild level 0 from the loaded list (used by lvg_run after partial steps)
   c->arena.lo = c->base_lo;
   c->arena.hi = c->run_hi = c->arena.cap;
-  std::vector<int32_t> iota(c->V0);
-  for (int32_t i = 0; i < c->V0; ++i) iota[i] = i;
-  LVG_CUDA(cudaMemcpyAsync(c->composed, iota.data(), sizeof(int32_t) * c->V0, cudaMemcpyHostToDevice, c->stream));
-  sync(c);
+  iota(c->composed, c->V0, c->stream);
   c->levels.clear();
   c->level = 0;
   c->g = LevelGraph();
@@ -216,7 +235,10 @@ void reset_to_level0(lvg_ctx* c) {
   c->g.dst = c->dst0;
   c->g.w = c->w0;
   c->g.pre = &c->pre0;
-  prepare_level(c);
+  c->replay = false;
+  c->built = false;
+  c->renumbered = false;
+  if (build) prepare_level(c);
   c->pristine = true;
 }
 
@@ -345,6 +367,7 @@ int32_t renumber_level(lvg_ctx* c) {
   c->d_part_cur = part;
   c->C_cur = C;
   c->renumbered = true;
+  c->timed = true;
   LevelRec r;
   std::memset(&r.info, 0, sizeof r.info);
   r.d_part = part;
@@ -367,7 +390,7 @@ void induce_level(lvg_ctx* c) {
   LVG_CUDA(cudaEventRecord(c->pev[5], c->stream));
   sync(c);
   if (!c->levels.empty()) {
-    c->levels.back().info.ms_renumber = elapsed(c->pev[2], c->pev[3]);
+    if (c->timed) c->levels.back().info.ms_renumber = elapsed(c->pev[2], c->pev[3]);
     c->levels.back().info.ms_induce = elapsed(c->pev[4], c->pev[5]);
   }
   c->arena.hi = c->run_hi;
@@ -380,7 +403,170 @@ void induce_level(lvg_ctx* c) {
   c->g.w = L.w;
   c->g.pre = &c->pre_next;
   c->level += 1;
+  c->built = false;
+  c->replay = false;
+  c->renumbered = false;
+}
+
+// The level's CSR and state, where a call needs them and only the list exists.
+void ensure_built(lvg_ctx* c) {
+  if (c->built) return;
+  const bool renumbered = c->renumbered, pristine = c->pristine;
   prepare_level(c);
+  if (c->replay) {
+    const std::vector<float> ms = c->pass_ms, move_ms = c->move_pass_ms;
+    const double total = c->move_ms;
+    const int64_t passes = c->move_passes;
+    one_level(c, c->replay_lower, nullptr, nullptr, nullptr, nullptr);
+    c->pass_ms = ms;
+    c->move_pass_ms = move_ms;
+    c->move_ms = total;
+    c->move_passes = passes;
+    c->replay = false;
+  }
+  c->renumbered = renumbered;
+  c->pristine = pristine;
+}
+
+struct RunState {
+  double mod = 0.0;
+  int64_t pass_entries = 0;
+  int32_t status = 0;
+  double q_final = 0.0;
+  bool have_q = false;   // q_final is set
+  bool no_small = false; // a list was found not to be in small_run's form
+};
+
+// Runs the levels from the current one (a list, not built) on in one launch.
+// Returns true when that finished the run.  Otherwise the context stands at
+// the level it left open (perhaps the same one), still only a list.
+bool run_small(lvg_ctx* c, RunState& R) {
+  const int32_t V = c->g.V;
+  const int64_t E = c->g.E;
+  if (R.no_small || !small_fits(V, E, kSmallRunEntries)) return false;
+  Arena& a = c->arena;
+  cudaStream_t s = c->stream;
+  a.hi = c->run_hi;
+  constexpr int kRoomLevels = 12;
+  const int64_t parts_cap = 2 * (int64_t)kRoomLevels * V;
+  const size_t need = small_list_bytes(E) + small_work_bytes(V, E) + sizeof(int32_t) * ((size_t)parts_cap + V) +
+                      sizeof(SmallOut) + sizeof(SmallJob) + 16 * Arena::kAlign;
+  if (a.hi < a.lo || a.hi - a.lo < need) return false;
+  c->pristine = false;
+  const size_t lo0 = a.lo, hi0 = a.hi;
+  SmallJob J{};
+  J.src = c->g.src;
+  J.dst = c->g.dst;
+  J.w = c->g.w;
+  J.E = E;
+  J.V = V;
+  J.level0 = c->level;
+  J.mod = R.mod;
+  J.lists = (char*)a.alloc_lo(small_list_bytes(E));
+  J.parts = a.hi_n<int32_t>(parts_cap);
+  J.parts_cap = parts_cap;
+  const size_t run_hi = a.hi;
+  // level 0: checked at load; later lists are symmetric when their CSR was written
+  J.check = c->level == 0 || c->pre_next.valid ? 0 : 1;
+  J.want_q = c->level == 0 ? 1 : 0;
+  SmallOut o;
+  {
+    HiScope hs(a);
+    J.work = (char*)a.alloc_hi(small_work_bytes(V, E));
+    J.comp = c->level == 0 ? c->composed : a.hi_n<int32_t>(V);
+    SmallOut* d_out = a.hi_n<SmallOut>(1);
+    J.res = &d_out->res;
+    J.lv = d_out->lv;
+    SmallJob* d_job = a.hi_n<SmallJob>(1);
+    LVG_CUDA(cudaMemcpyAsync(d_job, &J, sizeof J, cudaMemcpyHostToDevice, s));
+    const SmallCfg cfg{c->cfg.pass_min_gain, c->cfg.level_min_gain, c->cfg.max_passes, c->cfg.max_levels};
+    small_run(d_job, 1, kSmallRunBlocks, cfg, s);
+    LVG_CUDA(cudaMemcpyAsync(&o, d_out, sizeof o, cudaMemcpyDeviceToHost, s));
+    if (c->level > 0) {   // a launch that finishes no level leaves no composition
+      sync(c);
+      if (o.res.n_levels > 0) compose(c->composed, J.comp, c->V0, s);
+    }
+    sync(c);
+  }
+  if (o.res.n_levels == 0) {
+    a.lo = lo0;
+    a.hi = hi0;
+    R.no_small = true;
+    if (c->level == 0) iota(c->composed, c->V0, s);
+    return false;
+  }
+  c->run_hi = run_hi;
+  for (int32_t l = 0; l < o.res.n_levels; ++l) {
+    const SmallLevel& x = o.lv[l];
+    LevelRec r;
+    std::memset(&r.info, 0, sizeof r.info);
+    r.d_part = J.parts + x.part_off;
+    r.d_labels = r.d_part + x.V;
+    r.info.n_vertices = x.V;
+    r.info.n_entries = x.E;
+    r.info.nnz = x.nnz;
+    r.info.n_comms = x.C;
+    r.info.passes = x.passes;
+    r.info.q_start = x.q_start;
+    r.info.q_level = x.q_level;
+    r.info.ms_build = x.ms[0];
+    r.info.ms_passes = x.ms[1];
+    r.info.ms_renumber = x.ms[2];
+    r.info.ms_induce = x.ms[3];
+    c->levels.push_back(r);
+    R.pass_entries += x.nnz * (int64_t)x.passes;
+  }
+  c->timed = false;
+  const SmallLevel& z = o.lv[o.res.n_levels - 1];
+  c->d_part_cur = c->levels.back().d_part;
+  c->C_cur = z.C;
+  c->pass_ms.assign(1, z.ms[1]);
+  c->move_pass_ms.assign(z.pass_ms, z.pass_ms + std::min(z.passes, 2));
+  c->move_passes = z.passes;
+  c->move_ms = 0.0;
+  for (float ms : c->move_pass_ms) c->move_ms += ms;
+  R.mod = o.res.mod;
+  // the level the context now stands at: the last one, or the one left open
+  c->level += o.res.n_levels - (o.res.open ? 0 : 1);
+  c->g = LevelGraph();
+  c->g.V = o.res.V;
+  c->g.E = o.res.E;
+  if (o.res.buf < 0) {
+    c->g.src = J.src;
+    c->g.dst = J.dst;
+    c->g.w = J.w;
+  } else {
+    int32_t *ls = nullptr, *ld = nullptr;
+    float* lw = nullptr;
+    small_list(J.lists, E, o.res.buf, &ls, &ld, &lw);
+    c->g.src = ls;
+    c->g.dst = ld;
+    c->g.w = lw;
+  }
+  c->pre_next = PreCsr();
+  c->g.pre = nullptr;
+  c->renumbered = !o.res.open;
+  c->replay = !o.res.open;
+  c->replay_lower = o.res.lower;
+  if (o.res.open) {
+    R.no_small = true;
+    return false;
+  }
+  R.status = o.res.status;
+  R.q_final = o.res.q_final;
+  R.have_q = J.want_q != 0;
+  return true;
+}
+
+// The entry checks of a load; *ready when the list is one small_run takes and
+// the arena could hold its level build (so that what a load refuses for lack
+// of memory does not depend on the list's order).
+bool check_small(lvg_ctx* c, const int32_t* src, const int32_t* dst, const float* w, int64_t E, int32_t V, bool copied,
+                 bool* ready) {
+  *ready = false;
+  if (!small_fits(V, E, kSmallRunEntries) || c->arena.cap < arena_estimate(V, E, copied))
+    return validate_edges(src, dst, w, E, V, c->arena, c->stream);
+  return check_edges(src, dst, w, E, V, ready, c->arena, c->stream);
 }
 
 void check_ctx(lvg_ctx* c) {
@@ -518,7 +704,7 @@ lvg_status lvg_load_edges(lvg_ctx* c, const int32_t* src, const int32_t* dst, co
     float* ww = c->arena.lo_n<float>(E);
     int64_t chunk = c->cfg.load_chunk_entries > 0 ? c->cfg.load_chunk_entries : ((int64_t)1 << 25);
     chunk = (chunk + 2047) / 2048 * 2048;
-    bool ok;
+    bool ok, ready = false;
     if (E >= 2 * chunk) {   // copy in chunks, checking and building level 0 as they arrive
       if (!c->copy_stream) LVG_CUDA(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
       ok = stream_load_level0(src, dst, w, s, d, ww, E, V, chunk, c->pre0, c->load_ev, c->arena, c->stream,
@@ -529,10 +715,10 @@ lvg_status lvg_load_edges(lvg_ctx* c, const int32_t* src, const int32_t* dst, co
         LVG_CUDA(cudaMemcpyAsync(d, dst, sizeof(int32_t) * E, cudaMemcpyHostToDevice, c->stream));
         LVG_CUDA(cudaMemcpyAsync(ww, w, sizeof(float) * E, cudaMemcpyHostToDevice, c->stream));
       }
-      ok = validate_edges(s, d, ww, E, V, c->arena, c->stream);
+      ok = check_small(c, s, d, ww, E, V, true, &ready);
     }
     require(ok, LVG_ERR_INVALID_ARG, "edge list has a vertex id out of range or a negative / non-finite weight");
-    load_common(c, s, d, ww, E, V);
+    load_common(c, s, d, ww, E, V, ready);
   });
 }
 
@@ -546,9 +732,10 @@ lvg_status lvg_load_edges_device(lvg_ctx* c, const int32_t* src, const int32_t* 
     c->pre0 = PreCsr();
     size_t need = c->cfg.arena_bytes > 0 ? (size_t)c->cfg.arena_bytes : arena_estimate(V, E, false);
     c->arena.reserve(need);
-    require(validate_edges(src, dst, w, E, V, c->arena, c->stream), LVG_ERR_INVALID_ARG,
+    bool ready = false;
+    require(check_small(c, src, dst, w, E, V, false, &ready), LVG_ERR_INVALID_ARG,
             "edge list has a vertex id out of range or a negative / non-finite weight");
-    load_common(c, src, dst, w, E, V);
+    load_common(c, src, dst, w, E, V, ready);
   });
 }
 
@@ -557,6 +744,7 @@ lvg_status lvg_modularity(lvg_ctx* c, double* q) {
     check_ctx(c);
     require(c->loaded && c->have_state, LVG_ERR_STATE, "no graph loaded");
     require(q != nullptr, LVG_ERR_INVALID_ARG, "null output");
+    ensure_built(c);
     *q = read_q(c);
   });
 }
@@ -566,6 +754,7 @@ lvg_status lvg_one_level(lvg_ctx* c, double lower, double* q, int32_t* passes) {
   lvg_status s = guarded(c, [&] {
     check_ctx(c);
     require(c->loaded && c->have_state, LVG_ERR_STATE, "no graph loaded");
+    ensure_built(c);
     one_level(c, lower, q, passes, &status, nullptr);
   });
   if (s == LVG_OK && status != 0) return fail(c, (lvg_status)status, "pass cap reached before convergence");
@@ -576,6 +765,7 @@ lvg_status lvg_renumber(lvg_ctx* c, int32_t* comm_out, int32_t* n_comms) {
   return guarded(c, [&] {
     check_ctx(c);
     require(c->loaded && c->have_state, LVG_ERR_STATE, "no graph loaded");
+    ensure_built(c);
     int32_t C = renumber_level(c);
     if (comm_out && c->g.V > 0)
       LVG_CUDA(cudaMemcpyAsync(comm_out, c->d_part_cur, sizeof(int32_t) * c->g.V, cudaMemcpyDeviceToHost,
@@ -589,7 +779,9 @@ lvg_status lvg_induce(lvg_ctx* c) {
   return guarded(c, [&] {
     check_ctx(c);
     require(c->loaded && c->renumbered, LVG_ERR_STATE, "lvg_induce needs lvg_renumber first");
+    ensure_built(c);
     induce_level(c);
+    prepare_level(c);
   });
 }
 
@@ -598,7 +790,9 @@ lvg_status lvg_run(lvg_ctx* c, lvg_result* res) {
   lvg_status s = guarded(c, [&] {
     check_ctx(c);
     require(c->loaded, LVG_ERR_STATE, "no graph loaded");
-    if (!c->pristine) reset_to_level0(c);   // a run starts from level 0 as loaded
+    // a run starts from level 0 as loaded
+    if (c->small0) reset_to_level0(c, false);
+    else if (!c->pristine) reset_to_level0(c);
     if (res) std::memset(res, 0, sizeof *res);
     if (c->E0 == 0) {
       // LouvainCPP.cpp:211-230: an empty edge list yields one identity partition
@@ -607,11 +801,15 @@ lvg_status lvg_run(lvg_ctx* c, lvg_result* res) {
       if (res) { res->n_levels = 1; res->n_comms = c->V0; res->q_final = 0.0; }
       return;
     }
-    double mod = 0.0;
-    int64_t pass_entries = 0;
+    RunState R;
+    bool finished = false;   // by small_run
     for (;;) {
+      if (!c->built) {
+        if (run_small(c, R)) { finished = true; break; }
+        ensure_built(c);
+      }
       double q0 = read_q(c);                      // modularityCUDA (LouvainCPP.cpp:356)
-      double lower = c->level == 0 ? q0 : mod;
+      double lower = c->level == 0 ? q0 : R.mod;
       double ql = 0.0;
       int32_t passes = 0, st = 0;
       one_level(c, lower, &ql, &passes, &st, nullptr);
@@ -622,23 +820,25 @@ lvg_status lvg_run(lvg_ctx* c, lvg_result* res) {
       r.info.q_start = q0;
       r.info.q_level = ql;
       r.info.ms_passes = ms_passes;
-      pass_entries += c->g.nnz * (int64_t)passes;
-      if (st != 0) { run_status = st; break; }
-      if (c->level > 0 && (ql - mod) < c->cfg.level_min_gain) break;   // LouvainCPP.cpp:466
-      if (c->cfg.max_levels >= 0 && c->level + 1 >= c->cfg.max_levels) { run_status = LVG_ERR_NOT_CONVERGED; break; }
-      mod = ql;
+      R.pass_entries += c->g.nnz * (int64_t)passes;
+      if (st != 0) { R.status = st; break; }
+      if (c->level > 0 && (ql - R.mod) < c->cfg.level_min_gain) break;   // LouvainCPP.cpp:466
+      if (c->cfg.max_levels >= 0 && c->level + 1 >= c->cfg.max_levels) { R.status = LVG_ERR_NOT_CONVERGED; break; }
+      R.mod = ql;
       induce_level(c);
     }
+    run_status = R.status;
     if (res) {
       res->n_levels = (int32_t)c->levels.size();
       res->n_comms = c->C_cur;
-      res->pass_entries = pass_entries;
+      res->pass_entries = R.pass_entries;
       res->status = run_status;
-      res->q_final = modularity_fp64(c->src0, c->dst0, c->w0, c->E0, std::max(c->C_cur, 1), c->composed,
-                                     c->arena, c->stream, c->symmetric0);
+      res->q_final = R.have_q ? R.q_final
+                              : modularity_fp64(c->src0, c->dst0, c->w0, c->E0, std::max(c->C_cur, 1), c->composed,
+                                                c->arena, c->stream, c->symmetric0);
     }
     sync(c);
-    if (!c->levels.empty()) c->levels.back().info.ms_renumber = elapsed(c->pev[2], c->pev[3]);
+    if (!finished && !c->levels.empty()) c->levels.back().info.ms_renumber = elapsed(c->pev[2], c->pev[3]);
   });
   if (s == LVG_OK && run_status != 0) return fail(c, (lvg_status)run_status, "cap reached before convergence");
   return s;
@@ -742,6 +942,7 @@ lvg_status lvg_get_csr(const lvg_ctx* cc, int32_t* n_vertices, int64_t* nnz, dou
   return guarded(c, [&] {
     check_ctx(c);
     require(c->loaded && c->have_state, LVG_ERR_STATE, "no graph loaded");
+    ensure_built(c);
     const LevelGraph& g = c->g;
     if (n_vertices) *n_vertices = g.V;
     if (nnz) *nnz = g.nnz;
@@ -776,6 +977,7 @@ lvg_status lvg_set_communities(lvg_ctx* c, const int32_t* comm) {
   return guarded(c, [&] {
     check_ctx(c);
     require(c->loaded && c->have_state, LVG_ERR_STATE, "no graph loaded");
+    ensure_built(c);
     require(comm != nullptr, LVG_ERR_INVALID_ARG, "null communities");
     const int32_t V = c->g.V;
     for (int32_t i = 0; i < V; ++i)
@@ -793,6 +995,7 @@ lvg_status lvg_move_decide(lvg_ctx* c, int32_t* next, int32_t* cand) {
   return guarded(c, [&] {
     check_ctx(c);
     require(c->loaded && c->have_state, LVG_ERR_STATE, "no graph loaded");
+    ensure_built(c);
     const int32_t V = c->g.V;
     cudaStream_t s = c->stream;
     reset_ctl(c->st, 0.0, c->cfg.pass_min_gain, -1, s);
@@ -938,6 +1141,7 @@ extern "C" lvg_status lvg_autotune(lvg_ctx* c, const lvg_tune_space* sp, lvg_tun
     if (n_points) *n_points = 0;
     const int32_t pref_tile = c->tune.warp_max, pref_block = c->tune.block_max;
     if (!c->pristine) reset_to_level0(c);   // tune from level 0 as loaded
+    ensure_built(c);
     if (c->E0 == 0 || c->g.nnz == 0) {   // no move pass to time (lvg_run runs none either)
       if (best) *best = lvg_tune_point{pref_tile, pref_block, -1.0f, -1.0f};
       return;
@@ -1053,28 +1257,17 @@ struct BatchInput {
   bool host = false;
 };
 
-void batch_run(lvg_ctx* c, const BatchInput& in, int32_t* part_out, double* q_out, int32_t* levels_out,
-               int32_t* comms_out, int32_t* status_out) {
+// Every level of the graphs of `in` (device lists) in shared launches over
+// their disjoint union.  Results per graph of `in`; with `scatter`, the
+// partitions go to scatter + scatter_off[g] on the device instead of part_out.
+void batch_union(lvg_ctx* c, const BatchInput& in, int32_t* part_out, double* q_out, int32_t* levels_out,
+                 int32_t* comms_out, int32_t* status_out, int32_t* scatter, const int32_t* scatter_off) {
   cudaStream_t s = c->stream;
   const int32_t G0 = in.G;
   const int64_t* eoff = in.eoff;
   const int32_t* voff = in.voff;
   const int64_t E0 = eoff[G0];
   const int32_t V0 = voff[G0];
-  for (int32_t g = 0; g < G0; ++g) {
-    require(eoff[g + 1] >= eoff[g] && voff[g + 1] >= voff[g], LVG_ERR_INVALID_ARG, "offsets must not decrease");
-    require((int64_t)(voff[g + 1] - voff[g]) <= (int64_t)kGroup * kGroup, LVG_ERR_CAPACITY,
-            "a batched graph may have at most 2048*2048 vertices");
-    require(eoff[g + 1] == eoff[g] || (in.src[g] && in.dst[g] && in.w[g]), LVG_ERR_INVALID_ARG, "null edge array");
-  }
-  require(E0 < ((int64_t)1 << 31), LVG_ERR_CAPACITY, "a batch may hold at most 2^31-1 entries");
-  drop_graphs(c);
-  c->pre0 = PreCsr();   // the batch reuses the arena
-  c->loaded = false;
-  c->have_state = false;
-  size_t need = c->cfg.arena_bytes > 0 ? (size_t)c->cfg.arena_bytes
-                                       : arena_estimate(V0, E0, true) + 256 * (size_t)G0 + 8 * (size_t)V0;
-  c->arena.reserve(need);
   Arena& a = c->arena;
   // level-0 union list with global vertex ids
   int32_t* src0 = a.lo_n<int32_t>(E0);
@@ -1085,36 +1278,10 @@ void batch_run(lvg_ctx* c, const BatchInput& in, int32_t* part_out, double* q_ou
   {
     HiScope hs(a);
     std::vector<const void*> ptrs(3 * (size_t)G0);
-    if (in.host) {
-      // stage the host lists (graph by graph, in entry order) and point into the copy
-      int32_t* ss = a.hi_n<int32_t>(E0);
-      int32_t* sd = a.hi_n<int32_t>(E0);
-      float* sw = a.hi_n<float>(E0);
-      bool packed = G0 > 0 && in.src[0] && in.dst[0] && in.w[0];
-      for (int32_t g = 0; packed && g < G0; ++g)
-        packed = in.src[g] == in.src[0] + eoff[g] && in.dst[g] == in.dst[0] + eoff[g] && in.w[g] == in.w[0] + eoff[g];
-      if (packed && E0 > 0) {   // one copy per array
-        LVG_CUDA(cudaMemcpyAsync(ss, in.src[0], sizeof(int32_t) * E0, cudaMemcpyHostToDevice, s));
-        LVG_CUDA(cudaMemcpyAsync(sd, in.dst[0], sizeof(int32_t) * E0, cudaMemcpyHostToDevice, s));
-        LVG_CUDA(cudaMemcpyAsync(sw, in.w[0], sizeof(float) * E0, cudaMemcpyHostToDevice, s));
-      }
-      for (int32_t g = 0; g < G0; ++g) {
-        const int64_t e0 = eoff[g], n = eoff[g + 1] - eoff[g];
-        if (n > 0 && !packed) {
-          LVG_CUDA(cudaMemcpyAsync(ss + e0, in.src[g], sizeof(int32_t) * n, cudaMemcpyHostToDevice, s));
-          LVG_CUDA(cudaMemcpyAsync(sd + e0, in.dst[g], sizeof(int32_t) * n, cudaMemcpyHostToDevice, s));
-          LVG_CUDA(cudaMemcpyAsync(sw + e0, in.w[g], sizeof(float) * n, cudaMemcpyHostToDevice, s));
-        }
-        ptrs[g] = ss + e0;
-        ptrs[G0 + g] = sd + e0;
-        ptrs[2 * G0 + g] = sw + e0;
-      }
-    } else {
-      for (int32_t g = 0; g < G0; ++g) {
-        ptrs[g] = in.src[g];
-        ptrs[G0 + g] = in.dst[g];
-        ptrs[2 * G0 + g] = in.w[g];
-      }
+    for (int32_t g = 0; g < G0; ++g) {
+      ptrs[g] = in.src[g];
+      ptrs[G0 + g] = in.dst[g];
+      ptrs[2 * G0 + g] = in.w[g];
     }
     const void** dptrs = a.hi_n<const void*>(3 * (int64_t)G0);
     int64_t* deoff = a.hi_n<int64_t>(G0 + 1);
@@ -1360,13 +1527,206 @@ void batch_run(lvg_ctx* c, const BatchInput& in, int32_t* part_out, double* q_ou
     cp.gblk0 = gb_d;
     batch_modularity(src0, dst0, w0, E0, gid0, local0, cp, cg_d, Ctot, G0, q_d, a, s);
     if (q_out) LVG_CUDA(cudaMemcpyAsync(q_out, q_d, sizeof(double) * G0, cudaMemcpyDeviceToHost, s));
-    if (part_out && V0 > 0)
+    if (scatter) {
+      int32_t* from_d = a.hi_n<int32_t>(G0 + 1);
+      int32_t* to_d = a.hi_n<int32_t>(G0);
+      LVG_CUDA(cudaMemcpyAsync(from_d, voff, sizeof(int32_t) * (G0 + 1), cudaMemcpyHostToDevice, s));
+      LVG_CUDA(cudaMemcpyAsync(to_d, scatter_off, sizeof(int32_t) * G0, cudaMemcpyHostToDevice, s));
+      batch_scatter(local0, gid0, from_d, to_d, V0, scatter, s);
+    } else if (part_out && V0 > 0) {
       LVG_CUDA(cudaMemcpyAsync(part_out, local0, sizeof(int32_t) * V0, cudaMemcpyDeviceToHost, s));
+    }
     sync(c);
   }
   if (levels_out) std::copy(levels.begin(), levels.end(), levels_out);
   if (comms_out) std::copy(comms.begin(), comms.end(), comms_out);
   if (status_out) std::copy(status.begin(), status.end(), status_out);
+  c->g = LevelGraph();
+  c->st = CommState();
+}
+
+// Largest list of a batch that small_run takes, and the blocks of its cluster.
+constexpr int64_t kSmallBatchEntries = 256 * 1024;
+int small_blocks(int64_t E) {
+  return E <= 16 * 1024 ? 1 : E <= 48 * 1024 ? 2 : E <= 128 * 1024 ? 4 : 8;
+}
+
+// Runs the small graphs of a batch, each by its own cluster; marks the graphs
+// that are finished, their partitions at part_d + voff[g].  Leaves the arena
+// as it was.  A graph whose list is not in the form small_run takes stays
+// unmarked.
+void batch_small(lvg_ctx* c, const BatchInput& in, int32_t* part_d, std::vector<char>& done, double* q_out,
+                 int32_t* levels_out, int32_t* comms_out, int32_t* status_out) {
+  Arena& a = c->arena;
+  cudaStream_t s = c->stream;
+  std::vector<int32_t> which;
+  for (int32_t g = 0; g < in.G; ++g)
+    if (small_fits(in.voff[g + 1] - in.voff[g], in.eoff[g + 1] - in.eoff[g], kSmallBatchEntries)) which.push_back(g);
+  if (which.empty()) return;
+  auto entries = [&](int32_t g) { return in.eoff[g + 1] - in.eoff[g]; };
+  std::sort(which.begin(), which.end(), [&](int32_t x, int32_t y) {   // longest first
+    return entries(x) != entries(y) ? entries(x) > entries(y) : x < y;
+  });
+  const int64_t n = (int64_t)which.size();
+  size_t lists = 0, work = 0;
+  for (int32_t g : which) {
+    lists += Arena::up(small_list_bytes(entries(g)));
+    work += Arena::up(small_work_bytes(in.voff[g + 1] - in.voff[g], entries(g)));
+  }
+  const size_t need = lists + work + n * (sizeof(SmallJob) + sizeof(SmallResult)) + 8 * Arena::kAlign;
+  if (a.hi < a.lo || a.hi - a.lo < need) return;   // the union path takes them all
+  HiScope hs(a);
+  char* lp = (char*)a.alloc_hi(lists);
+  char* wp = (char*)a.alloc_hi(work);
+  SmallResult* res = a.hi_n<SmallResult>(n);
+  SmallJob* jobs_d = a.hi_n<SmallJob>(n);
+  std::vector<SmallJob> jobs((size_t)n);
+  for (int64_t k = 0; k < n; ++k) {
+    const int32_t g = which[k];
+    SmallJob& J = jobs[k];
+    J = SmallJob{};
+    J.src = in.src[g];
+    J.dst = in.dst[g];
+    J.w = in.w[g];
+    J.E = entries(g);
+    J.V = in.voff[g + 1] - in.voff[g];
+    J.lists = lp;
+    J.work = wp;
+    lp += Arena::up(small_list_bytes(J.E));
+    wp += Arena::up(small_work_bytes(J.V, J.E));
+    J.comp = part_d + in.voff[g];
+    J.res = res + k;
+    J.check = 1;
+    J.want_q = 1;
+  }
+  LVG_CUDA(cudaMemcpyAsync(jobs_d, jobs.data(), sizeof(SmallJob) * n, cudaMemcpyHostToDevice, s));
+  const SmallCfg cfg{c->cfg.pass_min_gain, c->cfg.level_min_gain, c->cfg.max_passes, c->cfg.max_levels};
+  // one launch per cluster size, side by side
+  LVG_CUDA(cudaEventRecord(c->side.fork, s));
+  for (int k = 0; k < 3; ++k) LVG_CUDA(cudaStreamWaitEvent(c->side.side[k], c->side.fork, 0));
+  const cudaStream_t streams[4] = {s, c->side.side[0], c->side.side[1], c->side.side[2]};
+  int slot = 0;
+  for (int64_t k0 = 0; k0 < n;) {
+    const int K = small_blocks(jobs[k0].E);
+    int64_t k1 = k0;
+    while (k1 < n && small_blocks(jobs[k1].E) == K) ++k1;
+    small_run(jobs_d + k0, (int)(k1 - k0), K, cfg, streams[slot++ & 3]);
+    k0 = k1;
+  }
+  for (int k = 0; k < 3; ++k) {
+    LVG_CUDA(cudaEventRecord(c->side.join[k], c->side.side[k]));
+    LVG_CUDA(cudaStreamWaitEvent(s, c->side.join[k], 0));
+  }
+  std::vector<SmallResult> o((size_t)n);
+  LVG_CUDA(cudaMemcpyAsync(o.data(), res, sizeof(SmallResult) * n, cudaMemcpyDeviceToHost, s));
+  sync(c);
+  for (int64_t k = 0; k < n; ++k) {
+    const int32_t g = which[k];
+    require(!o[k].bad, LVG_ERR_INVALID_ARG,
+            "edge list has a vertex id out of its graph or a negative / non-finite weight");
+    if (o[k].open) continue;
+    done[g] = 1;
+    if (q_out) q_out[g] = o[k].q_final;
+    if (levels_out) levels_out[g] = o[k].n_levels;
+    if (comms_out) comms_out[g] = o[k].n_comms;
+    if (status_out) status_out[g] = o[k].status;
+  }
+}
+
+void batch_run(lvg_ctx* c, const BatchInput& given, int32_t* part_out, double* q_out, int32_t* levels_out,
+               int32_t* comms_out, int32_t* status_out) {
+  cudaStream_t s = c->stream;
+  const int32_t G0 = given.G;
+  const int64_t* eoff = given.eoff;
+  const int32_t* voff = given.voff;
+  const int64_t E0 = eoff[G0];
+  const int32_t V0 = voff[G0];
+  for (int32_t g = 0; g < G0; ++g) {
+    require(eoff[g + 1] >= eoff[g] && voff[g + 1] >= voff[g], LVG_ERR_INVALID_ARG, "offsets must not decrease");
+    require((int64_t)(voff[g + 1] - voff[g]) <= (int64_t)kGroup * kGroup, LVG_ERR_CAPACITY,
+            "a batched graph may have at most 2048*2048 vertices");
+    require(eoff[g + 1] == eoff[g] || (given.src[g] && given.dst[g] && given.w[g]), LVG_ERR_INVALID_ARG,
+            "null edge array");
+  }
+  require(E0 < ((int64_t)1 << 31), LVG_ERR_CAPACITY, "a batch may hold at most 2^31-1 entries");
+  drop_graphs(c);
+  c->pre0 = PreCsr();   // the batch reuses the arena
+  c->loaded = false;
+  c->have_state = false;
+  size_t need = c->cfg.arena_bytes > 0 ? (size_t)c->cfg.arena_bytes
+                                       : arena_estimate(V0, E0, true) + 256 * (size_t)G0 + 8 * (size_t)V0;
+  c->arena.reserve(need);
+  Arena& a = c->arena;
+  BatchInput in = given;
+  HiScope hs(a);
+  if (given.host) {
+    // stage the host lists (graph by graph, in entry order) and point into the copy
+    int32_t* ss = a.hi_n<int32_t>(E0);
+    int32_t* sd = a.hi_n<int32_t>(E0);
+    float* sw = a.hi_n<float>(E0);
+    bool packed = G0 > 0 && in.src[0] && in.dst[0] && in.w[0];
+    for (int32_t g = 0; packed && g < G0; ++g)
+      packed = in.src[g] == in.src[0] + eoff[g] && in.dst[g] == in.dst[0] + eoff[g] && in.w[g] == in.w[0] + eoff[g];
+    if (packed && E0 > 0) {   // one copy per array
+      LVG_CUDA(cudaMemcpyAsync(ss, in.src[0], sizeof(int32_t) * E0, cudaMemcpyHostToDevice, s));
+      LVG_CUDA(cudaMemcpyAsync(sd, in.dst[0], sizeof(int32_t) * E0, cudaMemcpyHostToDevice, s));
+      LVG_CUDA(cudaMemcpyAsync(sw, in.w[0], sizeof(float) * E0, cudaMemcpyHostToDevice, s));
+    }
+    for (int32_t g = 0; g < G0; ++g) {
+      const int64_t e0 = eoff[g], n = eoff[g + 1] - eoff[g];
+      if (n > 0 && !packed) {
+        LVG_CUDA(cudaMemcpyAsync(ss + e0, in.src[g], sizeof(int32_t) * n, cudaMemcpyHostToDevice, s));
+        LVG_CUDA(cudaMemcpyAsync(sd + e0, in.dst[g], sizeof(int32_t) * n, cudaMemcpyHostToDevice, s));
+        LVG_CUDA(cudaMemcpyAsync(sw + e0, in.w[g], sizeof(float) * n, cudaMemcpyHostToDevice, s));
+      }
+      in.src[g] = ss + e0;
+      in.dst[g] = sd + e0;
+      in.w[g] = sw + e0;
+    }
+    in.host = false;
+  }
+  const size_t lo0 = a.lo;
+  int32_t* part_d = a.lo_n<int32_t>(V0);
+  std::vector<char> done((size_t)G0, 0);
+  batch_small(c, in, part_d, done, q_out, levels_out, comms_out, status_out);
+  const int64_t ndone = std::count(done.begin(), done.end(), (char)1);
+  if (ndone == 0) {
+    a.lo = lo0;
+    batch_union(c, in, part_out, q_out, levels_out, comms_out, status_out, nullptr, nullptr);
+    return;
+  }
+  if (ndone < G0) {   // the other graphs, as a batch of their own
+    std::vector<int32_t> rest, rvoff(1, 0), to;
+    std::vector<int64_t> reoff(1, 0);
+    BatchInput sub;
+    for (int32_t g = 0; g < G0; ++g) {
+      if (done[g]) continue;
+      rest.push_back(g);
+      to.push_back(voff[g]);
+      rvoff.push_back(rvoff.back() + voff[g + 1] - voff[g]);
+      reoff.push_back(reoff.back() + eoff[g + 1] - eoff[g]);
+      sub.src.push_back(in.src[g]);
+      sub.dst.push_back(in.dst[g]);
+      sub.w.push_back(in.w[g]);
+    }
+    sub.G = (int32_t)rest.size();
+    sub.eoff = reoff.data();
+    sub.voff = rvoff.data();
+    std::vector<double> q(rest.size());
+    std::vector<int32_t> lev(rest.size()), com(rest.size()), stat(rest.size());
+    batch_union(c, sub, nullptr, q.data(), lev.data(), com.data(), stat.data(), part_d, to.data());
+    for (size_t k = 0; k < rest.size(); ++k) {
+      const int32_t g = rest[k];
+      if (q_out) q_out[g] = q[k];
+      if (levels_out) levels_out[g] = lev[k];
+      if (comms_out) comms_out[g] = com[k];
+      if (status_out) status_out[g] = stat[k];
+    }
+  }
+  if (part_out && V0 > 0)
+    LVG_CUDA(cudaMemcpyAsync(part_out, part_d, sizeof(int32_t) * V0, cudaMemcpyDeviceToHost, s));
+  sync(c);
+  c->levels.clear();
   c->g = LevelGraph();
   c->st = CommState();
 }

@@ -17,6 +17,7 @@
 
 #include "louvain.cuh"
 #include "prims.cuh"
+#include "rules.cuh"
 
 namespace lvg {
 
@@ -36,25 +37,8 @@ struct VInfo {
 
 namespace {
 
-__device__ __forceinline__ void delta_clear(Delta& d) {
-  d.tot = 0.0; d.in = 0.0; d.size = 0; d.out = 0; d.iw_out = 0.0;
-}
-
-// Commit of one community's pass deltas (communitySetKernel,
-// OneLevelKernel.cu:93-107): tot/in/size move by the deltas, and a vertex
-// that left its singleton community takes its degree and weight out of it.
-__device__ __forceinline__ void delta_commit(Delta& d, double kc, double& tot, double& in, int32_t& size) {
-  double t = tot, x = in;
-  if (d.out) { t = __dsub_rn(t, kc); x = __dsub_rn(x, d.iw_out); }
-  tot = __dadd_rn(t, d.tot);
-  in = __dadd_rn(x, d.in);
-  size += d.size - d.out;
-  delta_clear(d);
-}
-
 constexpr int kThreads = 256;
 constexpr int kHubChunk = 4096;
-constexpr int kNone = INT_MAX;
 
 // ------------------------------------------------------------------ validate
 __global__ void validate_kernel(const int32_t* src, const int32_t* dst, const float* w, int64_t E,
@@ -79,29 +63,6 @@ __global__ void make_keys_kernel(const int32_t* src, const int32_t* dst, const f
     keys[E + e] = (b << B) | a;
     vals[E + e] = x;
   }
-}
-
-// Segmented inclusive warp sum over contiguous runs of equal `seg`.
-template <typename K>
-__device__ __forceinline__ double seg_warp_sum(double v, K seg) {
-  const unsigned full = 0xffffffffu;
-  int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    double u = __shfl_up_sync(full, v, o);
-    K t = __shfl_up_sync(full, seg, o);
-    if (lane >= o && t == seg) v = __dadd_rn(v, u);
-  }
-  return v;
-}
-
-template <typename K>
-__device__ __forceinline__ bool seg_warp_last(K seg, bool valid) {
-  const unsigned full = 0xffffffffu;
-  int lane = threadIdx.x & 31;
-  K nx = __shfl_down_sync(full, seg, 1);
-  bool nvalid = __shfl_down_sync(full, valid, 1);
-  return valid && (lane == 31 || !nvalid || nx != seg);
 }
 
 // Per sorted entry: CSR heads, row counts, degree (InitKernel.cu:154-179:
@@ -165,17 +126,15 @@ enum : uint32_t { kNotSorted = 1u, kNotSymmetric = 2u, kBadEntry = 4u };
 // entries against the same sums of (dst, src, weight bits).  A strictly sorted
 // list has no repeated entry, so the sums agree when the list equals its
 // transpose; a list that is not symmetric passes only on a 128-bit collision.
-__device__ __forceinline__ uint64_t edge_hash(uint32_t u, uint32_t v, uint32_t wb, uint64_t key) {
-  return mix64(mix64((((uint64_t)u << 32) | v) ^ key) + (uint64_t)wb * 0x9E3779B97F4A7C15ull + key);
-}
-
-__global__ void list_check_kernel(const int32_t* src, const int32_t* dst, const float* w, int64_t E,
+// Ids out of [0, V) and bad weights are reported as kBadEntry.
+__global__ void list_check_kernel(const int32_t* src, const int32_t* dst, const float* w, int64_t E, int32_t V,
                                   uint32_t* flags, unsigned long long* sums) {
   const uint64_t K1 = 0x243F6A8885A308D3ull, K2 = 0x13198A2E03707344ull;
   uint64_t d1 = 0, d2 = 0;
-  bool unsorted = false;
+  bool unsorted = false, bad = false;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E; e += (int64_t)gridDim.x * blockDim.x) {
     const int32_t u = src[e], v = dst[e];
+    bad |= !entry_ok(u, v, w[e], V);
     if (e + 1 < E) {
       const int32_t u2 = src[e + 1], v2 = dst[e + 1];
       if (!(u2 > u || (u2 == u && v2 > v))) unsorted = true;
@@ -192,11 +151,12 @@ __global__ void list_check_kernel(const int32_t* src, const int32_t* dst, const 
     d1 += __shfl_down_sync(full, d1, o);
     d2 += __shfl_down_sync(full, d2, o);
   }
-  const bool any_unsorted = __any_sync(full, unsorted);
+  const bool any_unsorted = __any_sync(full, unsorted), any_bad = __any_sync(full, bad);
   if ((threadIdx.x & 31) == 0) {
     if (d1) atomicAdd(&sums[0], (unsigned long long)d1);
     if (d2) atomicAdd(&sums[1], (unsigned long long)d2);
     if (any_unsorted) atomicOr(flags, kNotSorted);
+    if (any_bad) atomicOr(flags, kBadEntry);
   }
 }
 
@@ -232,10 +192,6 @@ __global__ void csr_fast_emit_kernel(const int32_t* src, const int32_t* dst, con
 // chunk, each chunk processed while later ones are still being copied.  The
 // CSR is the one build_csr_fast makes; it is kept only if the whole list
 // turns out strictly sorted and symmetric.
-
-__device__ __forceinline__ bool entry_ok(int32_t u, int32_t v, float x, int32_t V) {
-  return u >= 0 && u < V && v >= 0 && v < V && x >= 0.0f && !isinf(x);   // as validate_kernel
-}
 
 // One chunk [b, e_end): range/weight check, strict order against the previous
 // entry, the symmetry fingerprints of list_check_kernel, per-row counts of
@@ -466,13 +422,6 @@ __device__ __forceinline__ int64_t work_advance(unsigned long long* q, int64_t i
   return item + 1 < w.end ? item + 1 : work_take(q, w);
 }
 
-// Candidate order: higher gain first, then lower community id
-// (OneLevelKernel.cu:330,358).  Only strictly positive gains are candidates.
-__device__ __forceinline__ bool better(double g2, int32_t c2, double g1, int32_t c1) {
-  return g2 > g1 || (g2 == g1 && c2 < c1);
-}
-
-
 __device__ __forceinline__ void warp_best(double& bg, int32_t& bc, double& bw) {
   const unsigned full = 0xffffffffu;
 #pragma unroll
@@ -482,24 +431,6 @@ __device__ __forceinline__ void warp_best(double& bg, int32_t& bc, double& bw) {
     double w = __shfl_xor_sync(full, bw, o);
     if (better(g, c, bg, bc)) { bg = g; bc = c; bw = w; }
   }
-}
-
-// remove/insert (OneLevelKernel.cu:52-78) of a vertex of degree ki moving
-// with weight iw from community own to best.  SINGLETON: own holds only this
-// vertex, so its side is two plain stores the commit applies.
-template <bool SINGLETON>
-__device__ __forceinline__ void move_deltas(Delta* d, int32_t own, int32_t best, double ki, double iw) {
-  if (SINGLETON) {
-    d[own].out = 1;
-    d[own].iw_out = iw;
-  } else {
-    atomicAdd(&d[own].tot, -ki);
-    atomicAdd(&d[own].in, -iw);
-    atomicAdd(&d[own].size, -1);
-  }
-  atomicAdd(&d[best].tot, ki);
-  atomicAdd(&d[best].in, iw);
-  atomicAdd(&d[best].size, 1);
 }
 
 // The decision for one vertex from its best candidate: singleton-pair rule
@@ -1658,14 +1589,6 @@ __global__ void hub_decide_kernel(MoveArgs P, HubArgs H, int64_t nhub) {
 }
 
 // ------------------------------------------------------------------ commit + Q
-// term_c = in_c/m - (tot_c/2m)^2 (OneLevelKernel.cu:447-448), zero when m <= 0.
-__device__ __forceinline__ double q_term(double in, double tot, double m, double twom) {
-  if (!(m > 0.0)) return 0.0;
-  double a = __ddiv_rn(in, m);
-  double b = __ddiv_rn(tot, twom);
-  return __dsub_rn(a, __dmul_rn(b, b));
-}
-
 enum { kCommitInit = 0, kCommitPass = 1, kCommitForce = 2 };
 
 // kCommitPass: the ΔQ test of the pass (OneLevelKernel.cu:889-896), then
@@ -2038,6 +1961,22 @@ bool validate_edges(const int32_t* src, const int32_t* dst, const float* w, int6
   return h == 0;
 }
 
+bool check_edges(const int32_t* src, const int32_t* dst, const float* w, int64_t E, int32_t V, bool* sorted_symmetric,
+                 Arena& a, cudaStream_t s) {
+  *sorted_symmetric = false;
+  if (E == 0) return true;
+  HiScope hs(a);
+  unsigned long long* chk = a.hi_n<unsigned long long>(3);   // flags, two fingerprint sums
+  LVG_CUDA(cudaMemsetAsync(chk, 0, 3 * sizeof(unsigned long long), s));
+  list_check_kernel<<<sm_grid(E, kThreads), kThreads, 0, s>>>(src, dst, w, E, V, (uint32_t*)chk, chk + 1);
+  LVG_LAUNCH();
+  unsigned long long h[3] = {0, 0, 0};
+  LVG_CUDA(cudaMemcpyAsync(h, chk, sizeof h, cudaMemcpyDeviceToHost, s));
+  LVG_CUDA(cudaStreamSynchronize(s));
+  *sorted_symmetric = h[0] == 0 && h[1] == 0 && h[2] == 0;
+  return (h[0] & kBadEntry) == 0;
+}
+
 bool stream_load_level0(const int32_t* hsrc, const int32_t* hdst, const float* hw, int32_t* src, int32_t* dst,
                         float* w, int64_t E, int32_t V, int64_t chunk, PreCsr& pre, std::vector<cudaEvent_t>& evs,
                         Arena& a, cudaStream_t s, cudaStream_t copy) {
@@ -2135,7 +2074,7 @@ static bool build_csr_fast(LevelGraph& g, Arena& a, cudaStream_t s) {
   int64_t* rowstart = a.hi_n<int64_t>(V + 1);
   unsigned long long* chk = a.hi_n<unsigned long long>(3);   // flags, two fingerprint sums
   LVG_CUDA(cudaMemsetAsync(chk, 0, 3 * sizeof(unsigned long long), s));
-  list_check_kernel<<<sm_grid(E, kThreads), kThreads, 0, s>>>(g.src, g.dst, g.w, E, (uint32_t*)chk, chk + 1);
+  list_check_kernel<<<sm_grid(E, kThreads), kThreads, 0, s>>>(g.src, g.dst, g.w, E, V, (uint32_t*)chk, chk + 1);
   LVG_LAUNCH();
   unsigned long long h[3] = {0, 0, 0};
   LVG_CUDA(cudaMemcpyAsync(h, chk, sizeof h, cudaMemcpyDeviceToHost, s));
@@ -3259,6 +3198,14 @@ __global__ void batch_compose_kernel(int32_t* local0, const int32_t* gid0, int64
   }
 }
 
+__global__ void batch_scatter_kernel(const int32_t* local, const int32_t* gid, const int32_t* from, const int32_t* to,
+                                     int32_t V, int32_t* out) {
+  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V; v += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t g = gid[v];
+    out[to[g] + (v - from[g])] = local[v];
+  }
+}
+
 // Newman modularity per graph over its level-0 entries (global community
 // ids coff[g] + local id).
 __global__ void batch_nm_accum_kernel(const int32_t* src, const int32_t* dst, const float* w, int64_t E,
@@ -3488,6 +3435,13 @@ void batch_compose(int32_t* local0, const int32_t* gid0, int64_t n, const int32_
                    const int32_t* cbase, const int32_t* part, cudaStream_t s) {
   if (n == 0) return;
   batch_compose_kernel<<<sm_grid(n, kThreads), kThreads, 0, s>>>(local0, gid0, n, lidx, vbase, cbase, part);
+  LVG_LAUNCH();
+}
+
+void batch_scatter(const int32_t* local, const int32_t* gid, const int32_t* from_off, const int32_t* to_off, int32_t V,
+                   int32_t* out, cudaStream_t s) {
+  if (V <= 0) return;
+  batch_scatter_kernel<<<sm_grid(V, kThreads), kThreads, 0, s>>>(local, gid, from_off, to_off, V, out);
   LVG_LAUNCH();
 }
 

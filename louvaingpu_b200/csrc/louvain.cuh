@@ -151,6 +151,11 @@ enum : int32_t { kCoarsenAuto = 0, kCoarsenChunks = 1, kCoarsenTransposed = 2, k
 bool validate_edges(const int32_t* src, const int32_t* dst, const float* w, int64_t E, int32_t V,
                     Arena& a, cudaStream_t s);
 
+// The same check with the list's form: *sorted_symmetric when it is strictly
+// sorted by (src, dst) and symmetric with bitwise-equal weights.
+bool check_edges(const int32_t* src, const int32_t* dst, const float* w, int64_t E, int32_t V, bool* sorted_symmetric,
+                 Arena& a, cudaStream_t s);
+
 // Build the level CSR, degrees, loops and buckets (NeighbourCompute.cu:42-117,
 // InitKernel.cu:245-339).  Level arrays go to the arena's low end.
 void build_level(LevelGraph& g, const Tuning& t, Arena& a, cudaStream_t s);
@@ -311,6 +316,10 @@ void batch_compose(int32_t* local0, const int32_t* gid0, int64_t n, const int32_
 void batch_modularity(const int32_t* src, const int32_t* dst, const float* w, int64_t E, const int32_t* gid0,
                       const int32_t* local0, const BatchPlan& cp, const int32_t* cg, int32_t Ctot, int32_t G,
                       double* q, Arena& a, cudaStream_t s);
+
+// out[to_off[g] + i] = local[from_off[g] + i] for the vertices i of graph gid = g.
+void batch_scatter(const int32_t* local, const int32_t* gid, const int32_t* from_off, const int32_t* to_off, int32_t V,
+                   int32_t* out, cudaStream_t s);
 
 // Largest row of the level CSR (synchronises).
 int64_t max_degree(const LevelGraph& g, Arena& a, cudaStream_t s);

@@ -1,0 +1,75 @@
+// Whole dendrograms of small graphs in one launch (small.cu).
+#pragma once
+#include "louvain.cuh"
+
+namespace lvg {
+
+constexpr int32_t kSmallMaxV = 1 << 16;     // a coarse key (two community ids) fits 32 bits
+constexpr int32_t kSmallLevels = 48;        // levels one launch may record
+constexpr int32_t kSmallPassCap = 4096;     // passes of a level before it is left to the caller
+constexpr int kSmallPhases = 4;             // build, passes, renumbering, coarsening
+
+struct SmallLevel {
+  int32_t V, C, passes, pad;
+  int64_t E, nnz;
+  double q_start, q_level;
+  float ms[kSmallPhases];
+  float pass_ms[2];         // move kernels of the first two passes
+  int64_t part_off;         // partition at parts + part_off, labels V later
+};
+
+struct SmallResult {
+  int32_t n_levels;         // levels finished
+  int32_t n_comms;          // communities of the last finished level
+  int32_t open;             // 1: the next level was left to the caller, its list as below
+  int32_t status;           // lvg_status of the run
+  int32_t bad;              // an entry out of range or with a bad weight
+  int32_t V;                // list of the last level (or of the open one)
+  int32_t buf;              // -1: the job's own list, else coarse list buffer 0 or 1
+  int32_t pad;
+  int64_t E;
+  double mod;               // Q of the last finished level
+  double lower;             // floor of the last finished level's pass loop
+  double q_final;           // FP64 modularity of comp over the job's list (want_q)
+};
+
+struct SmallOut {
+  SmallResult res;
+  SmallLevel lv[kSmallLevels];
+};
+
+// One graph (or the rest of a run from a coarse level on).
+struct SmallJob {
+  const int32_t* src;
+  const int32_t* dst;
+  const float* w;
+  int64_t E;
+  int32_t V;
+  int32_t level0;           // level of the given list in its run
+  double mod;               // Q of the level before (level0 > 0)
+  char* lists;              // two coarse list buffers of E entries each
+  char* work;               // small_work_bytes(V, E)
+  int32_t* parts;           // per-level partitions and labels, or nullptr
+  int64_t parts_cap;        // ints
+  int32_t* comp;            // [V] composition of the levels' partitions
+  SmallResult* res;
+  SmallLevel* lv;           // [kSmallLevels], or nullptr
+  int32_t check;            // 1: ids, weights, order and symmetry not checked yet
+  int32_t want_q;
+};
+
+struct SmallCfg {
+  double pass_min, level_min;
+  int32_t max_passes, max_levels;
+};
+
+size_t small_list_bytes(int64_t E);           // both coarse list buffers
+size_t small_work_bytes(int32_t V, int64_t E);
+// Coarse list buffer `buf` of a job's lists.
+void small_list(char* lists, int64_t E, int buf, int32_t** src, int32_t** dst, float** w);
+// True when the sizes are ones this path takes.
+bool small_fits(int64_t V, int64_t E, int64_t max_entries);
+// Runs n jobs (device array), each by a cluster of K blocks.
+void small_run(const SmallJob* d_jobs, int n, int K, const SmallCfg& cfg, cudaStream_t s);
+
+}  // namespace lvg
