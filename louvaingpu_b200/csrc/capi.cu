@@ -180,8 +180,10 @@ void prepare_level(lvg_ctx* c) {
   c->renumbered = false;
 }
 
-// Largest list one launch runs to the end (small_run), and its cluster.
-constexpr int64_t kSmallRunEntries = 256 * 1024;
+// Largest list one launch runs to the end: by a cluster of 16 blocks up to
+// kClusterEntries entries, above by a cooperative grid of the whole chip.
+constexpr int64_t kSmallRunEntries = 2 * 1024 * 1024;
+constexpr int64_t kClusterEntries = 64 * 1024;
 constexpr int kSmallRunBlocks = 16;
 
 // `ready`: the list is sorted and symmetric, small, and has room for its level
@@ -480,15 +482,17 @@ bool run_small(lvg_ctx* c, RunState& R) {
     SmallJob* d_job = a.hi_n<SmallJob>(1);
     LVG_CUDA(cudaMemcpyAsync(d_job, &J, sizeof J, cudaMemcpyHostToDevice, s));
     const SmallCfg cfg{c->cfg.pass_min_gain, c->cfg.level_min_gain, c->cfg.max_passes, c->cfg.max_levels};
-    small_run(d_job, 1, kSmallRunBlocks, cfg, s);
+    LVG_CUDA(cudaMemsetAsync(J.res, 0, sizeof(SmallResult), s));
+    if (E <= kClusterEntries) small_run(d_job, 1, kSmallRunBlocks, cfg, s);
+    else small_run_grid(d_job, J.work, small_grid_blocks(), cfg, s);
     LVG_CUDA(cudaMemcpyAsync(&o, d_out, sizeof o, cudaMemcpyDeviceToHost, s));
     if (c->level > 0) {   // a launch that finishes no level leaves no composition
       sync(c);
-      if (o.res.n_levels > 0) compose(c->composed, J.comp, c->V0, s);
+      if (o.res.finished && o.res.n_levels > 0) compose(c->composed, J.comp, c->V0, s);
     }
     sync(c);
   }
-  if (o.res.n_levels == 0) {
+  if (!o.res.finished || o.res.n_levels == 0) {
     a.lo = lo0;
     a.hi = hi0;
     R.no_small = true;
@@ -509,10 +513,11 @@ bool run_small(lvg_ctx* c, RunState& R) {
     r.info.passes = x.passes;
     r.info.q_start = x.q_start;
     r.info.q_level = x.q_level;
-    r.info.ms_build = x.ms[0];
-    r.info.ms_passes = x.ms[1];
-    r.info.ms_renumber = x.ms[2];
-    r.info.ms_induce = x.ms[3];
+    const double tick = o.res.ms_per_tick;
+    r.info.ms_build = x.ticks[0] * tick;
+    r.info.ms_passes = x.ticks[1] * tick;
+    r.info.ms_renumber = x.ticks[2] * tick;
+    r.info.ms_induce = x.ticks[3] * tick;
     c->levels.push_back(r);
     R.pass_entries += x.nnz * (int64_t)x.passes;
   }
@@ -520,8 +525,9 @@ bool run_small(lvg_ctx* c, RunState& R) {
   const SmallLevel& z = o.lv[o.res.n_levels - 1];
   c->d_part_cur = c->levels.back().d_part;
   c->C_cur = z.C;
-  c->pass_ms.assign(1, z.ms[1]);
-  c->move_pass_ms.assign(z.pass_ms, z.pass_ms + std::min(z.passes, 2));
+  c->pass_ms.assign(1, (float)(z.ticks[1] * o.res.ms_per_tick));
+  c->move_pass_ms.clear();
+  for (int p = 0; p < std::min(z.passes, 2); ++p) c->move_pass_ms.push_back((float)(z.pass_ticks[p] * o.res.ms_per_tick));
   c->move_passes = z.passes;
   c->move_ms = 0.0;
   for (float ms : c->move_pass_ms) c->move_ms += ms;
@@ -1600,6 +1606,7 @@ void batch_small(lvg_ctx* c, const BatchInput& in, int32_t* part_d, std::vector<
     J.want_q = 1;
   }
   LVG_CUDA(cudaMemcpyAsync(jobs_d, jobs.data(), sizeof(SmallJob) * n, cudaMemcpyHostToDevice, s));
+  LVG_CUDA(cudaMemsetAsync(res, 0, sizeof(SmallResult) * n, s));
   const SmallCfg cfg{c->cfg.pass_min_gain, c->cfg.level_min_gain, c->cfg.max_passes, c->cfg.max_levels};
   // one launch per cluster size, side by side
   LVG_CUDA(cudaEventRecord(c->side.fork, s));
@@ -1624,7 +1631,7 @@ void batch_small(lvg_ctx* c, const BatchInput& in, int32_t* part_d, std::vector<
     const int32_t g = which[k];
     require(!o[k].bad, LVG_ERR_INVALID_ARG,
             "edge list has a vertex id out of its graph or a negative / non-finite weight");
-    if (o[k].open) continue;
+    if (o[k].open || !o[k].finished) continue;
     done[g] = 1;
     if (q_out) q_out[g] = o[k].q_final;
     if (levels_out) levels_out[g] = o[k].n_levels;

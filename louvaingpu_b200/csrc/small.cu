@@ -27,6 +27,7 @@
 #include <algorithm>
 #include <cooperative_groups.h>
 #include <mutex>
+#include <type_traits>
 
 #include "prims.cuh"
 #include "rules.cuh"
@@ -37,33 +38,62 @@ namespace {
 
 namespace cg = cooperative_groups;
 
-constexpr int kTileInt = 4096;             // entries of a tile, packed slots
-constexpr int kSlots = 2 * kTileInt;       // 64 KB of slots, at most half full
-constexpr int kTileF64 = kTileInt / 2;     // key + sum take two slots
-constexpr int kTileRows = 1024;            // rows of a tile (10 bits of a packed key)
-constexpr int kCommBits = 16;              // community bits of a packed key
+constexpr int kItems = 4;                  // entries of a tile per thread
+// Tile of a block of NT threads: entries, slots (16 or 8 bytes an entry, at
+// most half full), and rows (10 bits of a packed key).
+template <int NT>
+struct Tile {
+  static constexpr int kInt = kItems * NT;       // entries, packed slots
+  static constexpr int kSlots = 2 * kInt;
+  static constexpr int kF64 = kInt / 2;          // entries, key and sum in two slots
+  static constexpr int kRows = NT;
+  static constexpr int kLog = NT == 1024 ? 13 : 12;
+  static_assert(kSlots == 1 << kLog && kRows <= 1 << 10, "tile sizes");
+};
+constexpr int kCommBits = 18;              // community bits of a packed key
 constexpr int kDigits = 256;
+constexpr int64_t kGridEntries = 4096;     // grid mode: entries a block, at least
+constexpr int kResThreads = 512;
+constexpr int kResV = 512, kResE = 6144;   // a level this small lives in one block's shared memory
+constexpr unsigned long long kWaitNs = 4000000000ull;   // limit of a grid barrier's wait
 constexpr unsigned long long kEmpty = ~0ull;
-static_assert(kSmallMaxV <= (1 << kCommBits), "packed keys hold 16-bit communities");
-static_assert(kTileRows <= (1 << 10) && kTileInt < (1 << 14), "packed key or claimed slot too wide");
+static_assert(kSmallMaxV <= (1 << kCommBits), "packed keys hold 18-bit communities");
 
 enum : uint32_t { fNotInt = 1u, fUnfit = 2u, fBad = 4u, fUnsorted = 8u };
+enum : int32_t { kPhaseNone = 0, kPhaseTail = 1, kPhaseEnd = 2 };
+enum : int32_t { kCompDone = 0, kCompTail = 1, kCompTailAll = 2 };
 
-// Shared control words of a job (device memory).
+// Control words of a level's blocks.
 struct Ctl {
   uint32_t flags, flags2, check, loops;
   unsigned long long sums[2];
-  uint32_t count[2][16];
+  uint32_t count[2][kSmallMaxBlocks];
+  unsigned long long arrived;   // grid barrier: arrivals so far
+  uint32_t dead;                // grid barrier: a wait ran out
+};
+
+// Where the levels of a job stand between its launches.
+struct Between {
+  int32_t phase;             // kPhase*
+  int32_t nlev, buf, symmetric;
+  int32_t V, ncomms, open, bad, status;
+  int32_t comp;              // kComp*: what the composition still needs
+  int64_t E, part_off;
+  double mod, lower;
+  double ms_per_tick;
 };
 
 struct Work {
   Ctl* ctl;
+  Between* bt;
   double *k, *kfrac, *tot, *in, *qpart, *mpart;
   Delta* delta;
-  int32_t *roff, *comm, *next, *cand, *size, *minidx, *newid, *part;
+  int32_t *roff, *comm, *next, *cand, *size, *minidx, *newid;
   float* loopw;
   int32_t* hasl;
-  uint32_t *key[2], *ghist;
+  uint64_t* key[2];
+  uint32_t* ghist;
+  int32_t* rc;               // composition of the resident levels
   float* val[2];
   double* wsum;
 };
@@ -78,6 +108,7 @@ __host__ __device__ inline size_t carve(char* base, int64_t V, int64_t E, Work& 
     return p;
   };
   W.ctl = (Ctl*)take(sizeof(Ctl));
+  W.bt = (Between*)take(sizeof(Between));
   W.k = (double*)take(8 * V);
   W.kfrac = (double*)take(8 * V);
   W.tot = (double*)take(8 * V);
@@ -92,15 +123,15 @@ __host__ __device__ inline size_t carve(char* base, int64_t V, int64_t E, Work& 
   W.size = (int32_t*)take(4 * V);
   W.minidx = (int32_t*)take(4 * V);
   W.newid = (int32_t*)take(4 * V);
-  W.part = (int32_t*)take(4 * V);
   W.loopw = (float*)take(4 * V);
   W.hasl = (int32_t*)take(4 * V);
-  W.key[0] = (uint32_t*)take(4 * E);
-  W.key[1] = (uint32_t*)take(4 * E);
+  W.key[0] = (uint64_t*)take(8 * E);
+  W.key[1] = (uint64_t*)take(8 * E);
   W.val[0] = (float*)take(4 * E);
   W.val[1] = (float*)take(4 * E);
   W.wsum = (double*)take(8 * E);
-  W.ghist = (uint32_t*)take(4 * kDigits * 16);
+  W.ghist = (uint32_t*)take(4 * kDigits * kSmallMaxBlocks);
+  W.rc = (int32_t*)take(4 * kResV);
   return o;
 }
 
@@ -111,13 +142,36 @@ __host__ __device__ inline void list_of(char* lists, int64_t E, int buf, int32_t
   *w = (float*)(p + 2 * up256(4 * E));
 }
 
-template <int NT>
-struct Smem {
+// A resident level: its list and per-vertex arrays in shared memory, under
+// the names Work gives their device-memory counterparts.
+struct Resident {
+  int32_t src[kResE], dst[kResE];
+  float w[kResE];
+  Delta delta[kResV];
+  double k[kResV], kfrac[kResV], tot[kResV], in[kResV], qpart[1], mpart[kResE / kGroup + 1];
+  int32_t roff[kResV + 1], comm[kResV], next[kResV], cand[kResV], size[kResV], minidx[kResV], newid[kResV],
+      hasl[kResV], comp[kResV];
+  float loopw[kResV];
+  Ctl ctl[1];
+  uint64_t* key[2];          // device memory (levels of more communities than `cell` holds pairs for)
+  uint32_t* ghist;
+  float* val[2];
+  double* wsum;
+};
+static_assert(kResV < kGroup, "one group of communities");
+
+// Working space of a block of NT threads.
+template <int NT, int CELLS>
+struct Space {
+  static constexpr int kSlots = Tile<NT>::kSlots, kTileRows = Tile<NT>::kRows, kTileInt = Tile<NT>::kInt;
   union {
     unsigned long long slot[kSlots];
     uint32_t wc[NT / 32][kDigits + 1];
+    uint32_t part[2][NT / kDigits][kDigits];
+    double stage[kGroup];
+    double cell[CELLS];        // sums of a coarse graph of few communities
   } u;
-  unsigned long long bestg[kTileRows];
+  uint32_t besth[kTileRows], bestl[kTileRows];   // best gain, upper and lower half
   double bestw[kTileRows];
   double kf[kTileRows];
   int32_t bestc[kTileRows];
@@ -126,90 +180,184 @@ struct Smem {
   uint16_t claimed[kTileInt];
   uint32_t hist[kDigits];
   uint32_t dbase[kDigits];
-  double ws[NT / 256][8];
+  double ws[8];
   double bcast;
   uint32_t wtot[NT / 32];
-  int32_t nclaimed;
+  int32_t nclaimed, row0, row1;
+  unsigned long long goal;   // grid barrier: arrivals awaited
+  int32_t alive;
+  SmallJob J;
 };
 
-// ------------------------------------------------------------------ the cluster
-template <int NT>
-struct Team {
-  int K, rank, tid;
-  __device__ int gt() const { return rank * NT + tid; }
-  __device__ int stride() const { return K * NT; }
-  // Barrier of the job's threads; global writes before it are seen after it.
-  __device__ void sync() const {
-    if (K == 1) {
-      __syncthreads();
-    } else {
-      __threadfence();
-      cg::this_cluster().sync();
+extern __shared__ __align__(16) unsigned char smem_raw[];
+
+// A job's levels by several blocks, or one, over device memory.
+template <int NT_>
+struct Multi {
+  static constexpr int NT = NT_;
+  static constexpr bool kResident = false;
+  static constexpr int kCells = 1;
+  struct Smem {
+    Space<NT, kCells> s;
+    Work w;                  // read from here, not held in registers
+  };
+  static __device__ __forceinline__ Smem& mem() { return *reinterpret_cast<Smem*>(smem_raw); }
+  static __device__ __forceinline__ Space<NT, kCells>& S() { return mem().s; }
+  static __device__ __forceinline__ Work& W() { return mem().w; }
+};
+
+// The last levels of a job by one block over its shared memory.
+struct Tail {
+  static constexpr int NT = kResThreads;
+  static constexpr bool kResident = true;
+  static constexpr int kCells = 8192;   // 90 communities
+  struct Smem {
+    Space<NT, kCells> s;
+    Resident w;
+  };
+  static __device__ __forceinline__ Smem& mem() { return *reinterpret_cast<Smem*>(smem_raw); }
+  static __device__ __forceinline__ Space<NT, kCells>& S() { return mem().s; }
+  static __device__ __forceinline__ Resident& W() { return mem().w; }
+};
+
+enum { kModeCluster = 0, kModeGrid = 1 };
+
+__device__ __forceinline__ unsigned long long now_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+
+// Waits until *p reaches `goal`; false when the wait's limit has passed.
+__device__ __forceinline__ bool wait_for(unsigned long long* p, unsigned long long goal, uint32_t* dead) {
+  unsigned long long t0 = 0ull;
+  for (unsigned spin = 0;; ++spin) {
+    if (*reinterpret_cast<volatile unsigned long long*>(p) >= goal) return true;
+    if ((spin & 1023u) != 1023u) continue;
+    if (t0 == 0ull) t0 = now_ns();
+    if (*reinterpret_cast<volatile uint32_t*>(dead) || now_ns() - t0 > kWaitNs) {
+      atomicOr(dead, 1u);
+      return false;
     }
+  }
+}
+
+// The blocks working on a level: K of the job's, this one `rank`.
+template <typename X>
+struct Team {
+  int K_, rank_, mode;
+  __device__ __forceinline__ int K() const { return X::kResident ? 1 : K_; }
+  __device__ __forceinline__ int rank() const { return X::kResident ? 0 : rank_; }
+  __device__ __forceinline__ int gt() const { return rank() * X::NT + (int)threadIdx.x; }
+  __device__ __forceinline__ int stride() const { return K() * X::NT; }
+  __device__ __forceinline__ bool lead() const { return rank() == 0 && threadIdx.x == 0; }
+  // Barrier of the team's threads; global writes before it are seen after it.
+  // A cluster uses the hardware barrier (release and acquire at cluster
+  // scope).  A cooperative grid counts arrivals in device memory; its wait is
+  // bounded, and false (in every thread of the block) ends the kernel.
+  __device__ __forceinline__ bool sync() const {
+    if (K() == 1) {
+      __syncthreads();
+      return true;
+    }
+    if (mode == kModeCluster) {
+      cg::this_cluster().sync();
+      return true;
+    }
+    return grid_sync(K_);
+  }
+  static __device__ __noinline__ bool grid_sync(int K) {
+    __syncthreads();
+    if constexpr (!X::kResident) {
+      if (threadIdx.x == 0) {
+        Ctl* c = X::W().ctl;
+        X::S().goal += (unsigned long long)K;
+        __threadfence();
+        atomicAdd(&c->arrived, 1ull);
+        X::S().alive = wait_for(&c->arrived, X::S().goal, &c->dead) ? 1 : 0;
+        __threadfence();
+      }
+    }
+    __syncthreads();
+    return X::S().alive != 0;
   }
 };
 
-template <int NT>
-__device__ __forceinline__ uint32_t block_excl(uint32_t v, uint32_t* wtot, uint32_t* total) {
+template <typename X>
+__device__ __forceinline__ uint32_t block_excl(uint32_t v, uint32_t* total) {
+  uint32_t* wtot = X::S().wtot;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const uint32_t inc = warp_inclusive_scan(v);
   if (lane == 31) wtot[w] = inc;
   __syncthreads();
   if (w == 0) {
-    uint32_t x = lane < NT / 32 ? wtot[lane] : 0u;
+    uint32_t x = lane < X::NT / 32 ? wtot[lane] : 0u;
     x = warp_inclusive_scan(x);
-    if (lane < NT / 32) wtot[lane] = x;
+    if (lane < X::NT / 32) wtot[lane] = x;
   }
   __syncthreads();
   const uint32_t base = w > 0 ? wtot[w - 1] : 0u;
-  *total = wtot[NT / 32 - 1];
+  *total = wtot[X::NT / 32 - 1];
   __syncthreads();
   return base + inc - v;
 }
 
-// block_tree256 of each 256-thread quarter; the result in its first thread.
-template <int NT>
-__device__ __forceinline__ double quarter_tree(double s, Smem<NT>& S) {
+// block_tree256 of the block's first 256 threads; the result in thread 0.
+template <typename X>
+__device__ __forceinline__ double first_tree(double s) {
   const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31, w = (threadIdx.x & 255) >> 5, q = threadIdx.x >> 8;
-  for (int o = 16; o >= 1; o >>= 1) s = __dadd_rn(s, __shfl_down_sync(full, s, o));
-  if (lane == 0) S.ws[q][w] = s;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (w < 8) {
+    for (int o = 16; o >= 1; o >>= 1) s = __dadd_rn(s, __shfl_down_sync(full, s, o));
+    if (lane == 0) X::S().ws[w] = s;
+  }
   __syncthreads();
   double r = 0.0;
   if (w == 0) {
-    double v = lane < 8 ? S.ws[q][lane] : 0.0;
-    for (int o = 16; o >= 1; o >>= 1) v = __dadd_rn(v, __shfl_down_sync(full, v, o));
-    r = v;
+    r = lane < 8 ? X::S().ws[lane] : 0.0;
+    for (int o = 16; o >= 1; o >>= 1) r = __dadd_rn(r, __shfl_down_sync(full, r, o));
   }
   __syncthreads();
   return r;
 }
 
-// Group partials of the fixed-tree sum of val(i), i < n (groups of 2048, a
-// quarter block each); val is called once per index.
-template <int NT, typename F>
-__device__ __forceinline__ void group_partials(const Team<NT>& T, Smem<NT>& S, int64_t n, double* partials, F val) {
+// Group partials of the fixed-tree sum of val(load(i)), i < n (groups of
+// 2048, a block each).  Both are called once per index, the loads of two
+// indices before the first val, which may write.
+template <typename X, typename G, typename F>
+__device__ __forceinline__ void group_partials(const Team<X> T, int64_t n, double* partials, G load, F val) {
+  constexpr int kPer = kGroup / X::NT;
+  const int tid = threadIdx.x;
+  double* stage = X::S().u.stage;
   const int64_t ng = max((int64_t)1, (n + kGroup - 1) / kGroup);
-  const int nq = NT / 256, q = T.tid >> 8, t = T.tid & 255;
-  for (int64_t g0 = (int64_t)T.rank * nq; g0 < ng; g0 += (int64_t)T.K * nq) {
-    const int64_t g = g0 + q;
-    double s = 0.0;
-    if (g < ng) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int64_t i = g * kGroup + j * 256 + t;
-        if (i < n) s = __dadd_rn(s, val(i));
-      }
+#pragma unroll 1
+  for (int64_t g = T.rank(); g < ng; g += T.K()) {
+    const int64_t i0 = g * kGroup + tid;
+#pragma unroll 1
+    for (int j = 0; j < kPer; j += 2) {
+      const int64_t ia = i0 + j * X::NT, ib = ia + X::NT;
+      decltype(load(ia)) xa, xb;
+      if (ia < n) xa = load(ia);
+      if (ib < n) xb = load(ib);
+      stage[j * X::NT + tid] = ia < n ? val(ia, xa) : 0.0;
+      stage[(j + 1) * X::NT + tid] = ib < n ? val(ib, xb) : 0.0;
     }
-    const double r = quarter_tree<NT>(s, S);
-    if (t == 0 && g < ng) partials[g] = r;
+    __syncthreads();
+    double s = 0.0;
+    if (tid < 256) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s = __dadd_rn(s, stage[j * 256 + tid]);
+    }
+    s = first_tree<X>(s);
+    if (tid == 0) partials[g] = s;
   }
 }
 
 // Sum of the partials of n values, in every thread (at most 2048 partials).
-template <int NT>
-__device__ __forceinline__ double finish_sum(Smem<NT>& S, const double* partials, int64_t n) {
-  const int64_t np = max((int64_t)1, (n + kGroup - 1) / kGroup);
+template <typename X>
+__device__ __forceinline__ double finish_sum(const double* partials, int64_t n) {
+  if (n <= kGroup) return partials[0];   // the tree of one value
+  const int64_t np = (n + kGroup - 1) / kGroup;
   double s = 0.0;
   if (threadIdx.x < 256) {
 #pragma unroll
@@ -218,47 +366,59 @@ __device__ __forceinline__ double finish_sum(Smem<NT>& S, const double* partials
       if (i < np) s = __dadd_rn(s, partials[i]);
     }
   }
-  const double r = quarter_tree<NT>(s, S);
-  if (threadIdx.x == 0) S.bcast = r;
+  s = first_tree<X>(s);
+  if (threadIdx.x == 0) X::S().bcast = s;
   __syncthreads();
-  const double x = S.bcast;
+  const double x = X::S().bcast;
   __syncthreads();
   return x;
 }
 
-// First v in [0, V] with roff[v] >= x.
-__device__ __forceinline__ int32_t row_at(const int32_t* roff, int32_t V, int64_t x) {
-  int32_t lo = 0, hi = V;
-  while (lo < hi) {
-    const int32_t mid = (lo + hi) >> 1;
-    if (roff[mid] >= x) hi = mid; else lo = mid + 1;
+// The block's share of the rows: those starting in its share of the list.
+// row0 and row1 become the first rows starting at or after the share's ends.
+template <typename X>
+__device__ __forceinline__ void find_rows(const Team<X> T, int32_t V, int64_t E) {
+  auto& S = X::S();
+  const int64_t x0 = E * T.rank() / T.K(), x1 = E * (T.rank() + 1) / T.K();
+  if (threadIdx.x == 0) {   // a share that starts or ends at entry 0 does so at row 0
+    S.row0 = 0;
+    S.row1 = T.rank() == T.K() - 1 ? V : 0;
   }
-  return lo;
+  __syncthreads();
+  if (T.K() > 1) {
+    const int32_t* roff = X::W().roff;
+#pragma unroll 2
+    for (int32_t v = 1 + (int)threadIdx.x; v <= V; v += X::NT) {
+      const int32_t a = roff[v - 1], b = roff[v];
+      if (T.rank() > 0 && a < x0 && b >= x0) S.row0 = v;
+      if (T.rank() < T.K() - 1 && a < x1 && b >= x1) S.row1 = v;
+    }
+    __syncthreads();
+  }
 }
 
 // The decision for one vertex (apply_decision_kl of the level kernels).
-template <bool SINGLETON>
-__device__ __forceinline__ void decide(const Work& W, int32_t i, int32_t own, int32_t bc, double bw, int32_t nseg) {
+// `last`: the pass ends the level, whose totals then stay as they are.
+template <typename X, bool SINGLETON>
+__device__ __forceinline__ void decide(int32_t i, int32_t own, int32_t bc, double bw, int32_t nseg, bool last) {
+  auto& W = X::W();
   const int32_t raw = bc == kNone ? own : bc;
   const int32_t so = SINGLETON ? 1 : W.size[own], sb = SINGLETON ? 1 : W.size[raw];
   int32_t best = raw;
   if (so == 1 && sb == 1 && raw > own) best = own;
   W.next[i] = best;
   W.cand[i] = (so == 1 && nseg == 1 && raw != own && own < raw) ? raw : -1;
-  if (best != own) move_deltas<SINGLETON>(W.delta, own, best, W.k[i], __dadd_rn(bw, (double)W.loopw[i]));
+  if (best != own && !last) move_deltas<SINGLETON>(W.delta, own, best, W.k[i], __dadd_rn(bw, (double)W.loopw[i]));
 }
 
-// Rows [v0, v0 + return value) of the next tile: at most `cap` entries and
-// kTileRows rows.  Uniform over the block.
-template <int NT>
+// Rows [v0, v0 + return value) of the next tile: at most `cap` entries and a
+// row a thread.  Uniform over the block.
+template <typename X>
 __device__ __forceinline__ int tile_rows(const int32_t* roff, int32_t v0, int32_t vend, int cap) {
+  static_assert(Tile<X::NT>::kRows == X::NT, "a thread a row");
   const int32_t base = roff[v0];
-  int nv = 0;
-  for (int x = threadIdx.x; x < kTileRows; x += NT) {
-    const int32_t v = v0 + 1 + x;
-    nv += __syncthreads_count(v <= vend && roff[v] - base <= cap);
-  }
-  return nv;
+  const int32_t v = v0 + 1 + (int)threadIdx.x;
+  return __syncthreads_count(v <= vend && roff[v] - base <= cap);
 }
 
 struct List {
@@ -269,28 +429,48 @@ struct List {
 
 __device__ __forceinline__ double merged_w(float w) { return (double)__double2float_rn(__dadd_rn((double)w, (double)w)); }
 
-// First pass of a level: every neighbour is its own candidate.
-template <int NT>
-__device__ void moves_first(const Team<NT>& T, Smem<NT>& S, const Work& W, const List& L, int32_t v, int32_t vend) {
-  constexpr int kItems = kTileInt / NT;
+// Runs of equal `seg` in a warp (lanes hold consecutive list entries): the
+// lane's distance from its run's first lane, and whether it is the run's last.
+// Two votes and a shuffle, where a scan that shuffles `seg` along needs one a
+// step: the shuffles are what bounds the scans below.
+__device__ __forceinline__ int run_depth(int32_t seg, bool& last) {
   const unsigned full = 0xffffffffu;
-  const int lane = T.tid & 31;
+  const int lane = threadIdx.x & 31;
+  const int32_t before = __shfl_up_sync(full, seg, 1);
+  const unsigned heads = __ballot_sync(full, lane == 0 || before != seg);
+  last = lane == 31 || ((heads >> (lane + 1)) & 1u);
+  return lane - (31 - __clz(heads & (0xffffffffu >> (31 - lane))));
+}
+
+// Halves of a positive double, whose bits order as its value does.
+__device__ __forceinline__ uint32_t hi32(double x) { return (uint32_t)__double2hiint(x); }
+__device__ __forceinline__ uint32_t lo32(double x) { return (uint32_t)__double2loint(x); }
+
+// First pass of a level: every neighbour is its own candidate.
+template <typename X>
+__device__ __forceinline__ void moves_first_body(const List L, int32_t v, int32_t vend, bool last_pass) {
+  constexpr int NT = X::NT;
+  auto& S = X::S();
+  auto& W = X::W();
+  const unsigned full = 0xffffffffu;
+  const int tid = threadIdx.x, lane = tid & 31;
+#pragma unroll 1
   while (v < vend) {
-    const int nv = tile_rows<NT>(W.roff, v, vend, kTileInt);
+    const int nv = tile_rows<X>(W.roff, v, vend, Tile<NT>::kInt);
     if (nv == 0) return;   // cannot happen: rows longer than a tile leave the level open
     const int32_t base = W.roff[v];
     const int n = W.roff[v + nv] - base;
     if (n > 0) {
-      for (int j = T.tid; j < nv; j += NT) {
-        S.kf[j] = W.kfrac[v + j];
-        S.bestg[j] = 0ull;
-        S.bestc[j] = kNone;
+      if (tid < nv) {
+        S.kf[tid] = W.kfrac[v + tid];
+        S.besth[tid] = S.bestl[tid] = 0u;
+        S.bestc[tid] = kNone;
       }
       int jj[kItems], cc[kItems];
       double gg[kItems], wd[kItems];
 #pragma unroll
       for (int q = 0; q < kItems; ++q) {
-        const int x = q * NT + T.tid;
+        const int x = q * NT + tid;
         jj[q] = -1;
         cc[q] = 0;
         wd[q] = 0.0;
@@ -304,47 +484,57 @@ __device__ void moves_first(const Team<NT>& T, Smem<NT>& S, const Work& W, const
       for (int q = 0; q < kItems; ++q) gg[q] = jj[q] >= 0 ? W.k[cc[q]] : 0.0;   // singleton tot = k
       __syncthreads();
       unsigned last = 0;
+      double pg[kItems];
+      int32_t pc[kItems];
 #pragma unroll
       for (int q = 0; q < kItems; ++q) {
+        pg[q] = 0.0;
+        pc[q] = kNone;
+        if (q * NT + (tid & ~31) >= n) continue;   // whole warps
         const int j = jj[q];
-        double g = 0.0, w = wd[q];
+        double g = 0.0;
         int32_t c = kNone;
-        if (j >= 0 && cc[q] != v + j && w != 0.0) {                        // OneLevelKernel.cu:303
-          const double t = __dsub_rn(w, __dmul_rn(gg[q], S.kf[j]));        // OneLevelKernel.cu:307-313
+        if (j >= 0 && cc[q] != v + j && wd[q] != 0.0) {                    // OneLevelKernel.cu:303
+          const double t = __dsub_rn(wd[q], __dmul_rn(gg[q], S.kf[j]));    // OneLevelKernel.cu:307-313
           if (t > 0.0) { g = t; c = cc[q]; }
         }
+        gg[q] = g;
+        bool run_last;
+        const int depth = run_depth(j, run_last);
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {   // best candidate of the lane's row piece so far
-          const double g2 = __shfl_up_sync(full, g, o), w2 = __shfl_up_sync(full, w, o);
-          const int32_t c2 = __shfl_up_sync(full, c, o), j2 = __shfl_up_sync(full, j, o);
-          if (lane >= o && j2 == j && better(g2, c2, g, c)) { g = g2; c = c2; w = w2; }
+          const double g2 = __shfl_up_sync(full, g, o);
+          const int32_t c2 = __shfl_up_sync(full, c, o);
+          if (o <= depth && better(g2, c2, g, c)) { g = g2; c = c2; }
         }
-        const int32_t jn = __shfl_down_sync(full, j, 1);
-        if (j >= 0 && c != kNone && (lane == 31 || jn != j)) {
+        if (j >= 0 && c != kNone && run_last) {
           last |= 1u << q;
-          atomicMax(&S.bestg[j], (unsigned long long)__double_as_longlong(g));
+          atomicMax(&S.besth[j], hi32(g));
         }
-        gg[q] = g;
-        cc[q] = c;
-        wd[q] = w;
+        pg[q] = g;
+        pc[q] = c;
       }
       __syncthreads();
 #pragma unroll
       for (int q = 0; q < kItems; ++q)
         if ((last >> q) & 1u) {
-          if ((unsigned long long)__double_as_longlong(gg[q]) == S.bestg[jj[q]]) atomicMin(&S.bestc[jj[q]], cc[q]);
+          if (hi32(pg[q]) == S.besth[jj[q]]) atomicMax(&S.bestl[jj[q]], lo32(pg[q]));
           else last &= ~(1u << q);
         }
       __syncthreads();
 #pragma unroll
       for (int q = 0; q < kItems; ++q)
-        if (((last >> q) & 1u) && cc[q] == S.bestc[jj[q]]) S.bestw[jj[q]] = wd[q];
+        if (((last >> q) & 1u) && lo32(pg[q]) == S.bestl[jj[q]]) atomicMin(&S.bestc[jj[q]], pc[q]);
       __syncthreads();
-      for (int j = T.tid; j < nv; j += NT) {
-        const int32_t i = v + j, len = W.roff[i + 1] - W.roff[i];
-        const int32_t c = S.bestc[j];
+#pragma unroll
+      for (int q = 0; q < kItems; ++q)   // the winner's own entry
+        if (jj[q] >= 0 && gg[q] > 0.0 && cc[q] == S.bestc[jj[q]]) S.bestw[jj[q]] = wd[q];
+      __syncthreads();
+      if (tid < nv) {
+        const int32_t i = v + tid, len = W.roff[i + 1] - W.roff[i];
+        const int32_t c = S.bestc[tid];
         // distinct candidates: one per neighbour, and the own community with a self loop
-        if (len > 0) decide<true>(W, i, i, c, c == kNone ? 0.0 : S.bestw[j], len);
+        if (len > 0) decide<X, true>(i, i, c, c == kNone ? 0.0 : S.bestw[tid], len, last_pass);
       }
       __syncthreads();
     }
@@ -352,51 +542,61 @@ __device__ void moves_first(const Team<NT>& T, Smem<NT>& S, const Work& W, const
   }
 }
 
-// (row, community) tables.  Packed: row << 16 | community in the high half,
-// integer sum in the low half; all ones when empty.
-template <bool INT>
-struct Table;
-
-template <>
-struct Table<true> {
-  static constexpr int kTile = kTileInt;
-  static __device__ __forceinline__ uint32_t hash(uint32_t key) {
-    return (uint32_t)(((unsigned long long)key * 0x9E3779B97F4A7C15ull) >> (64 - 13));
+// (row, community) tables.  Integral weights: a 32-bit key (row << 18 |
+// community, all ones when empty) and a 32-bit sum, both with the atomics
+// shared memory has in hardware (64-bit adds and maxima are compare-and-swap
+// loops there, which contend on the rows' favourite communities).
+template <int NT, bool INT>
+struct Table {
+  static constexpr int kSlots = Tile<NT>::kSlots;
+  static constexpr int kUsed = kSlots;
+  static constexpr int kTile = Tile<NT>::kInt;
+  static constexpr uint32_t kNoKey = 0xffffffffu;
+  static __device__ __forceinline__ uint32_t* key_of(unsigned long long* slot) {
+    return reinterpret_cast<uint32_t*>(slot);
   }
+  static __device__ __forceinline__ uint32_t* sum_of(unsigned long long* slot) { return key_of(slot) + kSlots; }
   static __device__ __forceinline__ void insert(unsigned long long* slot, int32_t* ncl, uint16_t* claimed, int j,
                                                 int32_t c, double w) {
-    const uint32_t key = ((uint32_t)j << kCommBits) | (uint32_t)c, wi = (uint32_t)w;
-    uint32_t h = hash(key);
+    uint32_t *keys = key_of(slot), *sums = sum_of(slot);
+    const uint32_t key = ((uint32_t)j << kCommBits) | (uint32_t)c;
+    uint32_t h = (uint32_t)(((unsigned long long)key * 0x9E3779B97F4A7C15ull) >> (64 - Tile<NT>::kLog));
     for (int p = 0; p < kSlots; ++p) {   // at most half the slots are ever taken
-      const unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(&slot[h]);
-      if ((uint32_t)(cur >> 32) == key) { atomicAdd(&slot[h], (unsigned long long)wi); return; }
-      if (cur == kEmpty) {
-        const unsigned long long prev = atomicCAS(&slot[h], kEmpty, ((unsigned long long)key << 32) | wi);
-        if (prev == kEmpty) { claimed[atomicAdd(ncl, 1)] = (uint16_t)h; return; }
-        if ((uint32_t)(prev >> 32) == key) { atomicAdd(&slot[h], (unsigned long long)wi); return; }
+      uint32_t cur = *reinterpret_cast<volatile uint32_t*>(&keys[h]);
+      if (cur == kNoKey) {
+        cur = atomicCAS(&keys[h], kNoKey, key);
+        if (cur == kNoKey) {
+          claimed[atomicAdd(ncl, 1)] = (uint16_t)h;
+          cur = key;
+        }
       }
+      if (cur == key) { atomicAdd(&sums[h], (uint32_t)w); return; }
       h = (h + 1) & (kSlots - 1);
     }
   }
-  static __device__ __forceinline__ void get(const unsigned long long* slot, int s, int& j, int32_t& c, double& w) {
-    const unsigned long long x = slot[s];
-    const uint32_t key = (uint32_t)(x >> 32);
+  static __device__ __forceinline__ void get(unsigned long long* slot, int s, int& j, int32_t& c, double& w) {
+    const uint32_t key = key_of(slot)[s];
     j = (int)(key >> kCommBits);
     c = (int32_t)(key & ((1u << kCommBits) - 1u));
-    w = (double)(uint32_t)x;
+    w = (double)sum_of(slot)[s];
   }
-  static __device__ __forceinline__ void clear(unsigned long long* slot, int s) { slot[s] = kEmpty; }
+  static __device__ __forceinline__ void clear(unsigned long long* slot, int s) {
+    key_of(slot)[s] = kNoKey;
+    sum_of(slot)[s] = 0u;
+  }
 };
+static_assert(kCommBits + 10 < 32, "no key is all ones");
 
-template <>
-struct Table<false> {
-  static constexpr int kTile = kTileF64;
-  static constexpr int kHalf = kSlots / 2;   // keys below, FP64 sums above
+template <int NT>
+struct Table<NT, false> {
+  static constexpr int kTile = Tile<NT>::kF64;
+  static constexpr int kHalf = Tile<NT>::kSlots / 2;   // keys below, FP64 sums above
+  static constexpr int kUsed = kHalf;
   static __device__ __forceinline__ void insert(unsigned long long* slot, int32_t* ncl, uint16_t* claimed, int j,
                                                 int32_t c, double w) {
     const unsigned long long key = ((unsigned long long)j << 32) | (uint32_t)c;
     double* sum = reinterpret_cast<double*>(slot + kHalf);
-    uint32_t h = (uint32_t)((key * 0x9E3779B97F4A7C15ull) >> (64 - 12));
+    uint32_t h = (uint32_t)((key * 0x9E3779B97F4A7C15ull) >> (64 - Tile<NT>::kLog + 1));
     for (int p = 0; p < kHalf; ++p) {
       const unsigned long long prev = atomicCAS(&slot[h], kEmpty, key);
       if (prev == kEmpty) claimed[atomicAdd(ncl, 1)] = (uint16_t)h;
@@ -404,7 +604,7 @@ struct Table<false> {
       h = (h + 1) & (kHalf - 1);
     }
   }
-  static __device__ __forceinline__ void get(const unsigned long long* slot, int s, int& j, int32_t& c, double& w) {
+  static __device__ __forceinline__ void get(unsigned long long* slot, int s, int& j, int32_t& c, double& w) {
     const unsigned long long key = slot[s];
     j = (int)(key >> 32);
     c = (int32_t)(uint32_t)key;
@@ -417,34 +617,39 @@ struct Table<false> {
 };
 
 // A later pass: rows hashed tile by tile.
-template <int NT, bool INT>
-__device__ void moves_hash(const Team<NT>& T, Smem<NT>& S, const Work& W, const List& L, int32_t v, int32_t vend) {
-  using Tab = Table<INT>;
+template <typename X, bool INT>
+__device__ __forceinline__ void moves_hash_body(const List L, int32_t v, int32_t vend, bool last_pass) {
+  constexpr int NT = X::NT;
+  using Tab = Table<NT, INT>;
   constexpr int kItems = Tab::kTile / NT;
-  constexpr int kTabSlots = INT ? kSlots : kSlots / 2;
+  auto& S = X::S();
+  auto& W = X::W();
+  const int tid = threadIdx.x;
   unsigned long long* slot = S.u.slot;
-  for (int s = T.tid; s < kTabSlots; s += NT) Tab::clear(slot, s);
-  if (T.tid == 0) S.nclaimed = 0;
+#pragma unroll 2
+  for (int s = tid; s < Tab::kUsed; s += NT) Tab::clear(slot, s);
+  if (tid == 0) S.nclaimed = 0;
   __syncthreads();
+#pragma unroll 1
   while (v < vend) {
-    const int nv = tile_rows<NT>(W.roff, v, vend, Tab::kTile);
+    const int nv = tile_rows<X>(W.roff, v, vend, Tab::kTile);
     if (nv == 0) return;   // cannot happen, as above
     const int32_t base = W.roff[v];
     const int n = W.roff[v + nv] - base;
     if (n > 0) {
-      for (int j = T.tid; j < nv; j += NT) {
-        S.own[j] = W.comm[v + j];
-        S.kf[j] = W.kfrac[v + j];
-        S.bestg[j] = 0ull;
-        S.bestc[j] = kNone;
-        S.nseg[j] = 0;
+      if (tid < nv) {
+        S.own[tid] = W.comm[v + tid];
+        S.kf[tid] = W.kfrac[v + tid];
+        S.besth[tid] = S.bestl[tid] = 0u;
+        S.bestc[tid] = kNone;
+        S.nseg[tid] = 0;
       }
       int jj[kItems];
       int32_t cc[kItems];
       double wd[kItems];
 #pragma unroll
       for (int q = 0; q < kItems; ++q) {
-        const int x = q * NT + T.tid;
+        const int x = q * NT + tid;
         jj[q] = -1;
         cc[q] = 0;
         wd[q] = 0.0;
@@ -471,34 +676,49 @@ __device__ void moves_hash(const Team<NT>& T, Smem<NT>& S, const Work& W, const 
       double gg[kItems];
 #pragma unroll
       for (int q = 0; q < kItems; ++q) {       // count, best gain bits
-        const int x = q * NT + T.tid;
+        const int x = q * NT + tid;
         gg[q] = 0.0;
         jj[q] = -1;
         if (x < nc) {
-          Tab::get(slot, S.claimed[x], jj[q], cc[q], wd[q]);
+          const int sl = S.claimed[x];
+          Tab::get(slot, sl, jj[q], cc[q], wd[q]);
+          Tab::clear(slot, sl);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < kItems; ++q)
+        if (jj[q] >= 0 && wd[q] != 0.0) gg[q] = W.tot[cc[q]];
+#pragma unroll
+      for (int q = 0; q < kItems; ++q) {
+        if (jj[q] >= 0) {
           atomicAdd(&S.nseg[jj[q]], 1);
-          if (wd[q] != 0.0) gg[q] = __dsub_rn(wd[q], __dmul_rn(W.tot[cc[q]], S.kf[jj[q]]));
-          if (gg[q] > 0.0) atomicMax(&S.bestg[jj[q]], (unsigned long long)__double_as_longlong(gg[q]));
-          Tab::clear(slot, S.claimed[x]);
+          if (wd[q] != 0.0) gg[q] = __dsub_rn(wd[q], __dmul_rn(gg[q], S.kf[jj[q]]));
+          if (gg[q] > 0.0) atomicMax(&S.besth[jj[q]], hi32(gg[q]));
         }
       }
       __syncthreads();
 #pragma unroll
+      for (int q = 0; q < kItems; ++q)
+        if (jj[q] >= 0 && gg[q] > 0.0) {
+          if (hi32(gg[q]) == S.besth[jj[q]]) atomicMax(&S.bestl[jj[q]], lo32(gg[q]));
+          else gg[q] = 0.0;
+        }
+      __syncthreads();
+#pragma unroll
       for (int q = 0; q < kItems; ++q)         // smallest community among the best gains
-        if (jj[q] >= 0 && gg[q] > 0.0 && (unsigned long long)__double_as_longlong(gg[q]) == S.bestg[jj[q]])
-          atomicMin(&S.bestc[jj[q]], cc[q]);
+        if (jj[q] >= 0 && gg[q] > 0.0 && lo32(gg[q]) == S.bestl[jj[q]]) atomicMin(&S.bestc[jj[q]], cc[q]);
       __syncthreads();
 #pragma unroll
       for (int q = 0; q < kItems; ++q)
         if (jj[q] >= 0 && cc[q] == S.bestc[jj[q]]) S.bestw[jj[q]] = wd[q];
-      if (T.tid == 0) S.nclaimed = 0;
+      if (tid == 0) S.nclaimed = 0;
       __syncthreads();
-      for (int j = T.tid; j < nv; j += NT) {
-        const int32_t i = v + j;
+      if (tid < nv) {
+        const int32_t i = v + tid;
         if (W.roff[i + 1] > W.roff[i]) {
-          const int32_t c = S.bestc[j], s = S.nseg[j];
+          const int32_t c = S.bestc[tid], s = S.nseg[tid];
           const int32_t nseg = (s & ((1 << 30) - 1)) + ((W.hasl[i] && !(s >> 30)) ? 1 : 0);
-          decide<false>(W, i, S.own[j], c, c == kNone ? 0.0 : S.bestw[j], nseg);
+          decide<X, false>(i, S.own[tid], c, c == kNone ? 0.0 : S.bestw[tid], nseg, last_pass);
         }
       }
       __syncthreads();
@@ -507,36 +727,58 @@ __device__ void moves_hash(const Team<NT>& T, Smem<NT>& S, const Work& W, const 
   }
 }
 
-// Commit of a pass (communitySetKernel) with the Q partials of the new state.
-template <int NT>
-__device__ __forceinline__ void commit(const Team<NT>& T, Smem<NT>& S, const Work& W, int32_t V, double m) {
-  const double twom = __dmul_rn(2.0, m);
-  group_partials<NT>(T, S, V, W.qpart, [&](int64_t c) {
-    double t = W.tot[c], x = W.in[c];
-    int32_t sz = W.size[c];
-    delta_commit(W.delta[c], W.k[c], t, x, sz);
-    W.tot[c] = t;
-    W.in[c] = x;
-    W.size[c] = sz;
-    W.comm[c] = W.next[c];
-    return q_term(x, t, m, twom);
-  });
+// Out of line over device memory, where registers are short.
+template <typename X>
+__device__ __noinline__ void moves_first_call(const List L, int32_t v, int32_t vend, bool last) {
+  moves_first_body<X>(L, v, vend, last);
+}
+template <typename X, bool INT>
+__device__ __noinline__ void moves_hash_call(const List L, int32_t v, int32_t vend, bool last) {
+  moves_hash_body<X, INT>(L, v, vend, last);
 }
 
-__device__ __forceinline__ unsigned long long now_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
+struct Committed {
+  Delta d;
+  double tot, in, k;
+  int32_t size, next;
+};
+
+// Commit of a pass (communitySetKernel) with the Q partials of the new state.
+// FINAL: the level's last commit, which also takes every community's smallest
+// member.
+template <typename X, bool FINAL>
+__device__ __forceinline__ void commit(const Team<X> T, int32_t V, double m) {
+  auto& W = X::W();
+  const double twom = __dmul_rn(2.0, m);
+  group_partials<X>(
+      T, V, W.qpart,
+      [&](int64_t c) {
+        return Committed{W.delta[c], W.tot[c], W.in[c], W.k[c], W.size[c], W.next[c]};
+      },
+      [&](int64_t c, Committed& x) {
+        delta_commit(x.d, x.k, x.tot, x.in, x.size);
+        W.comm[c] = x.next;
+        if (FINAL) {
+          atomicMin(&W.minidx[x.next], (int32_t)c);
+        } else {
+          W.delta[c] = x.d;
+          W.tot[c] = x.tot;
+          W.in[c] = x.in;
+          W.size[c] = x.size;
+        }
+        return q_term(x.in, x.tot, m, twom);
+      });
 }
 
 // Entries of the list checked: ids and weights, strict order, and symmetry by
 // the fingerprints of list_check_kernel.
-template <int NT>
-__device__ void check_list(const Team<NT>& T, const Work& W, const List& L, int64_t E, int32_t V) {
+template <typename X>
+__device__ __noinline__ void check_list(const Team<X> T, const List L, int64_t E, int32_t V) {
   const uint64_t K1 = 0x243F6A8885A308D3ull, K2 = 0x13198A2E03707344ull;
   const unsigned full = 0xffffffffu;
   uint64_t d1 = 0, d2 = 0;
   uint32_t f = 0;
+#pragma unroll 1
   for (int64_t e = T.gt(); e < E; e += T.stride()) {
     const int32_t u = L.src[e], v = L.dst[e];
     const float x = L.w[e];
@@ -557,72 +799,156 @@ __device__ void check_list(const Team<NT>& T, const Work& W, const List& L, int6
     d2 += __shfl_down_sync(full, d2, o);
   }
   f = __reduce_or_sync(full, f);
-  if ((T.tid & 31) == 0) {
-    if (d1) atomicAdd(&W.ctl->sums[0], (unsigned long long)d1);
-    if (d2) atomicAdd(&W.ctl->sums[1], (unsigned long long)d2);
-    if (f) atomicOr(&W.ctl->check, f);
+  if ((threadIdx.x & 31) == 0) {
+    Ctl* c = X::W().ctl;
+    if (d1) atomicAdd(&c->sums[0], (unsigned long long)d1);
+    if (d2) atomicAdd(&c->sums[1], (unsigned long long)d2);
+    if (f) atomicOr(&c->check, f);
   }
 }
 
-// The coarse list of the level under W.part (C communities) into (osrc, odst,
-// ow); returns its length.  Stable LSD sort of the entries' keys over the
-// cluster: block r owns the r-th share of the positions, counts its digits,
-// and places its keys after those of all blocks before it.
-template <int NT>
-__device__ int64_t coarsen(const Team<NT>& T, Smem<NT>& S, const Work& W, const List& L, int64_t E, int32_t C,
-                           int32_t* osrc, int32_t* odst, float* ow) {
-  constexpr int kIt = 4;
+// A resident level's coarse list is summed pair by pair in shared memory.
+template <typename X>
+__device__ __forceinline__ bool cells_fit(int32_t C) {
+  return X::kResident && C <= 1024 && C * C <= X::kCells;
+}
+
+// The coarse list of a level of C communities (new ids W.newid of the labels
+// W.comm) into (osrc, odst, ow); returns its length (-1: a barrier's wait ran
+// out).  Stable LSD sort of the entries' keys over the team: block r owns the
+// r-th share of the positions, counts its digits, and places its keys after
+// those of all blocks before it.
+template <typename X, typename Key>
+__device__ __noinline__ int64_t coarsen(const Team<X> T, const List L, int64_t E, int32_t C, bool integral,
+                                        int32_t* osrc, int32_t* odst, float* ow) {
+  constexpr int NT = X::NT, kIt = 4, kQ = NT / kDigits;
+  auto& S = X::S();
+  auto& W = X::W();
   const unsigned full = 0xffffffffu;
-  const int lane = T.tid & 31, wid = T.tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const unsigned lt = (1u << lane) - 1u;
-  int b = 1;
-  while (b < kCommBits && (1 << b) < C) ++b;
-  const int bits = 2 * b, np = (bits + 7) / 8, width = (bits + np - 1) / np;
-  const uint32_t dmask = (1u << width) - 1u;
-  const int64_t s0 = E * T.rank / T.K, s1 = E * (T.rank + 1) / T.K;
-  int cur = 0;
-  for (int p = 0; p < np; ++p) {
-    for (int x = T.tid; x < kDigits; x += NT) S.hist[x] = 0;
+  if (cells_fit<X>(C)) {
+    // few communities, one block: a sum for every pair of them, the pairs met
+    // (sums are positive: weight 0 counts 1) written in order, to the resident
+    // list as well
+    const int cells = C * C;
+#pragma unroll 1
+    for (int x = tid; x < cells; x += NT) S.u.cell[x] = 0.0;
     __syncthreads();
-    for (int64_t e = s0 + T.tid; e < s1; e += NT) {
-      uint32_t key;
-      if (p == 0) {
-        key = ((uint32_t)W.part[L.src[e]] << b) | (uint32_t)W.part[L.dst[e]];
-        const float x = L.w[e];
-        W.key[0][e] = key;
-        W.val[0][e] = x == 0.0f ? 1.0f : x;       // InducedGraphKernel.cu:38-39
-        W.wsum[e] = 0.0;
-      } else {
-        key = W.key[cur][e];
-      }
-      atomicAdd(&S.hist[(key >> (p * width)) & dmask], 1u);
+#pragma unroll 4
+    for (int64_t e = tid; e < E; e += NT) {
+      const float x = L.w[e];
+      const int cell = W.newid[W.comm[L.src[e]]] * C + W.newid[W.comm[L.dst[e]]];
+      // integral weights add as integers (shared memory adds those in place)
+      if (integral) atomicAdd(reinterpret_cast<unsigned long long*>(&S.u.cell[cell]),
+                              x == 0.0f ? 1ull : (unsigned long long)x);       // InducedGraphKernel.cu:38-39
+      else atomicAdd(&S.u.cell[cell], x == 0.0f ? 1.0 : (double)x);
     }
     __syncthreads();
-    for (int x = T.tid; x < kDigits; x += NT) W.ghist[x * T.K + T.rank] = S.hist[x];
-    T.sync();
+    // a run of consecutive cells a thread
+    const int per = (cells + NT - 1) / NT, x0 = min(tid * per, cells), x1 = min(x0 + per, cells);
+    uint32_t met = 0;
+#pragma unroll 4
+    for (int x = x0; x < x1; ++x) met += S.u.cell[x] != 0.0 ? 1u : 0u;   // (an integer's bits are 0 for 0 alone)
+    uint32_t all;
+    uint32_t r = block_excl<X>(met, &all);
+    int row = x0 / C, column = x0 % C;
+    if constexpr (X::kResident) {
+#pragma unroll 1
+      for (int x = x0; x < x1; ++x) {
+        const double sum = S.u.cell[x];
+        if (sum != 0.0) {
+          const float w = __double2float_rn(integral ? (double)__double_as_longlong(sum) : sum);
+          W.src[r] = osrc[r] = row;
+          W.dst[r] = odst[r] = column;
+          W.w[r] = ow[r] = w;
+          ++r;
+        }
+        if (++column == C) {
+          column = 0;
+          ++row;
+        }
+      }
+    }
+    __syncthreads();
+    return (int64_t)all;
+  }
+  int b = 1;
+  while ((1 << b) < C) ++b;
+  Key* const keys[2] = {(Key*)W.key[0], (Key*)W.key[1]};
+  const int bits = 2 * b, np = (bits + 7) / 8, width = (bits + np - 1) / np;
+  const uint32_t dmask = (1u << width) - 1u;
+  const int64_t s0 = E * T.rank() / T.K(), s1 = E * (T.rank() + 1) / T.K();
+  int cur = 0;
+#pragma unroll 1
+  for (int p = 0; p < np; ++p) {
+    if (tid < kDigits) S.hist[tid] = 0;
+    __syncthreads();
+    if (p == 0) {
+      const int32_t *comm = W.comm, *newid = W.newid;
+      double* wsum = W.wsum;
+      float* val = W.val[0];
+#pragma unroll 2
+      for (int64_t e = s0 + tid; e < s1; e += NT) {
+        const Key key = ((Key)newid[comm[L.src[e]]] << b) | (Key)newid[comm[L.dst[e]]];
+        const float x = L.w[e];
+        keys[0][e] = key;
+        val[e] = x == 0.0f ? 1.0f : x;       // InducedGraphKernel.cu:38-39
+        wsum[e] = 0.0;
+        atomicAdd(&S.hist[(uint32_t)key & dmask], 1u);
+      }
+    } else {
+#pragma unroll 4
+      for (int64_t e = s0 + tid; e < s1; e += NT)
+        atomicAdd(&S.hist[(uint32_t)(keys[cur][e] >> (p * width)) & dmask], 1u);
+    }
+    __syncthreads();
     uint32_t tot = 0, pre = 0;
-    if (T.tid < kDigits)
-      for (int r = 0; r < T.K; ++r) {
-        const uint32_t c = W.ghist[T.tid * T.K + r];
-        if (r < T.rank) pre += c;
+    if (T.K() > 1) {
+      // digit counts of all blocks: kQ threads a digit, then their sums
+      if (tid < kDigits) W.ghist[T.rank() * kDigits + tid] = S.hist[tid];
+      if (!T.sync()) return -1;
+      const int d = tid & (kDigits - 1), q = tid / kDigits;
+      const int r0 = T.K() * q / kQ, r1 = T.K() * (q + 1) / kQ;
+#pragma unroll 8
+      for (int r = r0; r < r1; ++r) {
+        const uint32_t c = W.ghist[r * kDigits + d];
+        if (r < T.rank()) pre += c;
         tot += c;
       }
-    uint32_t all;
-    const uint32_t ex = block_excl<NT>(tot, S.wtot, &all);
-    if (T.tid < kDigits) S.dbase[T.tid] = ex + pre;
-    for (int64_t t0 = s0; t0 < s1; t0 += NT * kIt) {
-      for (int x = T.tid; x < (NT / 32) * (kDigits + 1); x += NT) (&S.u.wc[0][0])[x] = 0;
+      S.u.part[0][q][d] = tot;
+      S.u.part[1][q][d] = pre;
       __syncthreads();
-      uint32_t key[kIt], rank[kIt], dg[kIt];
+      tot = pre = 0;
+      if (tid < kDigits) {
+#pragma unroll
+        for (int k = 0; k < kQ; ++k) {
+          tot += S.u.part[0][k][tid];
+          pre += S.u.part[1][k][tid];
+        }
+      }
+    } else if (tid < kDigits) {
+      tot = S.hist[tid];
+    }
+    uint32_t all;
+    const uint32_t ex = block_excl<X>(tot, &all);
+    if (tid < kDigits) S.dbase[tid] = ex + pre;
+#pragma unroll 1
+    for (int64_t t0 = s0; t0 < s1; t0 += NT * kIt) {
+#pragma unroll 2
+      for (int x = tid; x < (NT / 32) * (kDigits + 1); x += NT) (&S.u.wc[0][0])[x] = 0;
+      Key key[kIt];
+      uint32_t rank[kIt], dg[kIt];
       float val[kIt];
       const int64_t base = t0 + (int64_t)wid * 32 * kIt;
 #pragma unroll
       for (int j = 0; j < kIt; ++j) {
         const int64_t i = base + j * 32 + lane;
-        key[j] = i < s1 ? W.key[cur][i] : 0u;
+        key[j] = i < s1 ? keys[cur][i] : Key(0);
         val[j] = i < s1 ? W.val[cur][i] : 0.0f;
-        dg[j] = i < s1 ? (key[j] >> (p * width)) & dmask : (uint32_t)kDigits;
+        dg[j] = i < s1 ? (uint32_t)(key[j] >> (p * width)) & dmask : (uint32_t)kDigits;
       }
+      __syncthreads();
 #pragma unroll
       for (int j = 0; j < kIt; ++j) {
         const unsigned peers = __match_any_sync(full, dg[j]);
@@ -633,56 +959,65 @@ __device__ int64_t coarsen(const Team<NT>& T, Smem<NT>& S, const Work& W, const 
         __syncwarp();
       }
       __syncthreads();
-      if (T.tid < kDigits) {
-        uint32_t run = S.dbase[T.tid];
+      if (tid < kDigits) {
+        uint32_t run = S.dbase[tid];
+#pragma unroll 8
         for (int w = 0; w < NT / 32; ++w) {
-          const uint32_t c = S.u.wc[w][T.tid];
-          S.u.wc[w][T.tid] = run;
+          const uint32_t c = S.u.wc[w][tid];
+          S.u.wc[w][tid] = run;
           run += c;
         }
-        S.dbase[T.tid] = run;
+        S.dbase[tid] = run;
       }
       __syncthreads();
 #pragma unroll
       for (int j = 0; j < kIt; ++j)
         if (dg[j] < (uint32_t)kDigits) {
           const uint32_t o = S.u.wc[wid][dg[j]] + rank[j];
-          W.key[cur ^ 1][o] = key[j];
+          keys[cur ^ 1][o] = key[j];
           W.val[cur ^ 1][o] = val[j];
         }
       __syncthreads();
     }
-    T.sync();
+    if (!T.sync()) return -1;
     cur ^= 1;
   }
   // runs of equal keys: heads counted per block, then each run's pieces added
-  const uint32_t* key = W.key[cur];
+  const Key* key = keys[cur];
   const float* val = W.val[cur];
+  double* wsum = W.wsum;
   uint32_t heads = 0;
+#pragma unroll 1
   for (int64_t i0 = s0; i0 < s1; i0 += NT) {
-    const int64_t i = i0 + T.tid;
+    const int64_t i = i0 + tid;
     heads += __syncthreads_count(i < s1 && (i == 0 || key[i] != key[i - 1]));
   }
-  if (T.tid == 0) W.ctl->count[1][T.rank] = heads;
-  T.sync();
-  uint32_t run = 0, cnt = 0;
-  for (int r = 0; r < T.K; ++r) {
-    const uint32_t c = W.ctl->count[1][r];
-    if (r < T.rank) run += c;
-    cnt += c;
+  uint32_t run = 0, cnt = heads;
+  if (T.K() > 1) {
+    if (tid == 0) W.ctl->count[1][T.rank()] = heads;
+    if (!T.sync()) return -1;
+    cnt = 0;
+#pragma unroll 4
+    for (int r = 0; r < T.K(); ++r) {
+      const uint32_t c = W.ctl->count[1][r];
+      if (r < T.rank()) run += c;
+      cnt += c;
+    }
   }
-  const uint32_t cmask = (1u << b) - 1u;
+  const Key cmask = (Key(1) << b) - 1;
+#pragma unroll 1
   for (int64_t t0 = s0; t0 < s1; t0 += NT * kIt) {
-    const int64_t i0 = t0 + (int64_t)T.tid * kIt;
-    uint32_t k[kIt + 1], hm = 0;
-    k[0] = i0 > 0 && i0 < s1 ? key[i0 - 1] : 0u;
+    const int64_t i0 = t0 + (int64_t)tid * kIt;
+    Key k[kIt + 1];
+    uint32_t hm = 0;
+    k[0] = i0 > 0 && i0 < s1 ? key[i0 - 1] : Key(0);
 #pragma unroll
     for (int j = 0; j < kIt; ++j) {
-      k[j + 1] = i0 + j < s1 ? key[i0 + j] : 0u;
+      k[j + 1] = i0 + j < s1 ? key[i0 + j] : Key(0);
       if (i0 + j < s1 && (i0 + j == 0 || k[j + 1] != k[j])) hm |= 1u << j;
     }
     uint32_t all;
-    uint32_t r = run + block_excl<NT>((uint32_t)__popc(hm), S.wtot, &all);   // runs started before the thread
+    uint32_t r = run + block_excl<X>((uint32_t)__popc(hm), &all);   // runs started before the thread
     run += all;
     double s = 0.0;
     bool any = false;
@@ -690,7 +1025,7 @@ __device__ int64_t coarsen(const Team<NT>& T, Smem<NT>& S, const Work& W, const 
     for (int j = 0; j < kIt; ++j) {
       if (i0 + j < s1) {
         if ((hm >> j) & 1u) {
-          if (any) atomicAdd(&W.wsum[r - 1], s);
+          if (any) atomicAdd(&wsum[r - 1], s);
           s = 0.0;
           osrc[r] = (int32_t)(k[j + 1] >> b);
           odst[r] = (int32_t)(k[j + 1] & cmask);
@@ -700,35 +1035,85 @@ __device__ int64_t coarsen(const Team<NT>& T, Smem<NT>& S, const Work& W, const 
         any = true;
       }
     }
-    if (any) atomicAdd(&W.wsum[r - 1], s);
+    if (any) atomicAdd(&wsum[r - 1], s);
   }
-  T.sync();
-  for (int64_t i = T.gt(); i < cnt; i += T.stride()) ow[i] = __double2float_rn(W.wsum[i]);
+  if (!T.sync()) return -1;
+#pragma unroll 2
+  for (int64_t i = T.gt(); i < cnt; i += T.stride()) ow[i] = __double2float_rn(wsum[i]);
+  if (!T.sync()) return -1;   // the next level's team may be smaller
   return (int64_t)cnt;
 }
 
-template <int NT>
-__global__ void __launch_bounds__(NT) small_kernel(const SmallJob* jobs, int K, SmallCfg cfg) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Smem<NT>& S = *reinterpret_cast<Smem<NT>*>(smem_raw);
-  const SmallJob J = jobs[blockIdx.x / K];
-  const Team<NT> T{K, (int)(blockIdx.x % K), (int)threadIdx.x};
-  Work W;
-  carve(J.work, J.V, J.E, W);
-  const bool lead = T.rank == 0 && T.tid == 0;
-  List L{J.src, J.dst, J.w};
-  int32_t V = J.V;
-  int64_t E = J.E;
+// Where a job's levels stand, the same in every thread of its team.
+struct At {
+  int32_t V;
+  int64_t E;
   int32_t ncomms = 0;
   int buf = -1, nlev = 0, status = LVG_OK;
-  bool open = false, symmetric = J.check == 0, bad = false;
-  double mod = J.mod, lower = 0.0;
+  bool open = false, symmetric = true, bad = false, tail = false;
+  double mod = 0.0, lower = 0.0;
   int64_t part_off = 0;
+};
+
+struct Row {
+  double k;
+  float loopw;
+  int32_t len;
+};
+
+// The level loop from `at` on, until the run has ended, a level is left open,
+// or (not resident) a level fits one block's shared memory.  False: a
+// barrier's wait ran out.
+template <typename X>
+__device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& at) {
+  constexpr int NT = X::NT;
+  auto& S = X::S();
+  auto& W = X::W();
+  const SmallJob& J = S.J;
+  const bool lead = T.lead();
+  List L{J.src, J.dst, J.w};
+  if (at.buf >= 0) {
+    int32_t *ls, *ld;
+    float* lw;
+    list_of(J.lists, J.E, at.buf, &ls, &ld, &lw);
+    L = List{ls, ld, lw};
+  }
+  int64_t res_v = 0;
+  bool list_here = false;   // the resident list is already this level's
   for (;;) {
-    unsigned long long t0 = lead ? now_ns() : 0ull;
-    const int level = J.level0 + nlev;
-    if (nlev >= kSmallLevels || (J.parts && part_off + 2 * (int64_t)V > J.parts_cap)) { open = true; break; }
+    const long long t0 = clock64();
+    const int level = J.level0 + at.nlev;
+    const int32_t V = at.V;
+    const int64_t E = at.E;
+    if (at.nlev >= kSmallLevels || (J.parts && at.part_off + 2 * (int64_t)V > J.parts_cap)) { at.open = true; return true; }
+    if (!X::kResident) {
+      if (V <= kResV && E <= kResE) { at.tail = true; return true; }
+      // few entries for so many blocks: the last ones leave
+      if (T.mode == kModeGrid && T.K_ > 1) {
+        T.K_ = (int)min((int64_t)T.K_, (E + kGridEntries - 1) / kGridEntries);
+        if (T.rank_ >= T.K_) return true;
+      }
+    }
     // ---- build
+    if constexpr (X::kResident) {
+      __syncthreads();   // the list is this block's own work
+      if (res_v == 0) {
+        res_v = V;
+        for (int32_t i = threadIdx.x; i < V; i += NT) W.comp[i] = i;
+      }
+      if (!list_here) {
+#pragma unroll 4
+        for (int64_t e = threadIdx.x; e < E; e += NT) {
+          const int32_t u = L.src[e], d = L.dst[e];
+          const float x = L.w[e];
+          W.src[e] = u;
+          W.dst[e] = d;
+          W.w[e] = x;
+        }
+      }
+      L = List{W.src, W.dst, W.w};
+    }
+#pragma unroll 1
     for (int32_t i = T.gt(); i < V; i += T.stride()) {
       W.k[i] = 0.0;
       W.loopw[i] = 0.0f;
@@ -738,105 +1123,128 @@ __global__ void __launch_bounds__(NT) small_kernel(const SmallJob* jobs, int K, 
       W.ctl->flags = W.ctl->flags2 = W.ctl->check = W.ctl->loops = 0u;
       W.ctl->sums[0] = W.ctl->sums[1] = 0ull;
     }
-    T.sync();
-    if (!symmetric) {
-      check_list<NT>(T, W, L, E, V);
-      T.sync();
+    if (!T.sync()) return false;
+    if (!at.symmetric) {
+      check_list<X>(T, L, E, V);
+      if (!T.sync()) return false;
       const uint32_t f = W.ctl->check;
-      if (f & fBad) { bad = true; break; }
-      if (f != 0u || W.ctl->sums[0] != 0ull || W.ctl->sums[1] != 0ull) { open = true; break; }
+      if (f & fBad) { at.bad = true; return true; }
+      if (f != 0u || W.ctl->sums[0] != 0ull || W.ctl->sums[1] != 0ull) { at.open = true; return true; }
     }
     {
       uint32_t f = 0, nl = 0;
-      for (int64_t e0 = (int64_t)T.rank * NT; e0 < E; e0 += T.stride()) {
-        const int64_t e = e0 + T.tid;
+#pragma unroll 1
+      for (int64_t e0 = (int64_t)T.rank() * NT; e0 < E; e0 += T.stride()) {
+        const int64_t e = e0 + threadIdx.x;
+        if (e0 + (threadIdx.x & ~31) >= E) break;   // whole warps
         const bool in = e < E;
         const int32_t u = in ? L.src[e] : -1, d = in ? L.dst[e] : -2;
+        const int32_t up = in && e > 0 ? L.src[e - 1] : -1;
         const float x = in ? L.w[e] : 0.0f;
         if (in) {
-          const int32_t up = e > 0 ? L.src[e - 1] : -1;
+#pragma unroll 1
           for (int32_t r = up + 1; r <= u; ++r) W.roff[r] = (int32_t)e;
-          if (e == E - 1)
+          if (e == E - 1) {
+#pragma unroll 1
             for (int32_t r = u + 1; r <= V; ++r) W.roff[r] = (int32_t)E;
+          }
           if (x != truncf(x)) f |= fNotInt;
           if (u == d) { W.loopw[u] = x; W.hasl[u] = 1; ++nl; }
         }
         float g = x == 0.0f ? 1.0f : x;             // InitKernel.cu:165-170, both copies of the entry
         if (u == d) g *= 2.0f;
-        const double s = seg_warp_sum<int32_t>(in ? __dadd_rn((double)g, (double)g) : 0.0, u);
-        if (seg_warp_last<int32_t>(u, in)) atomicAdd(&W.k[u], s);
+        bool run_last;
+        const int depth = run_depth(u, run_last);
+        double s = in ? __dadd_rn((double)g, (double)g) : 0.0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const double t = __shfl_up_sync(0xffffffffu, s, o);
+          if (o <= depth) s = __dadd_rn(s, t);
+        }
+        if (in && run_last) atomicAdd(&W.k[u], s);
       }
       f = __reduce_or_sync(0xffffffffu, f);
       nl = __reduce_add_sync(0xffffffffu, nl);
-      if ((T.tid & 31) == 0) {
+      if ((threadIdx.x & 31) == 0) {
         if (f) atomicOr(&W.ctl->flags, f);
         if (nl) atomicAdd(&W.ctl->loops, nl);
       }
-      group_partials<NT>(T, S, E, W.mpart, [&](int64_t e) { return (double)L.w[e]; });   // NeighbourCompute.cu:46
+      group_partials<X>(   // NeighbourCompute.cu:46
+          T, E, W.mpart, [&](int64_t e) { return L.w[e]; }, [&](int64_t, float x) { return (double)x; });
     }
-    T.sync();
+    if (!T.sync()) return false;
     const bool integral = !(W.ctl->flags & fNotInt);
-    symmetric = integral;   // of the next list: exact sums round alike in both directions
+    at.symmetric = integral;   // of the next list: exact sums round alike in both directions
     const int64_t nnz = E - (int64_t)W.ctl->loops;
-    const double m = finish_sum<NT>(S, W.mpart, E);
+    const double m = finish_sum<X>(W.mpart, E);
     const double twom = __dmul_rn(2.0, m);
     {
-      const int32_t longest = integral ? kTileInt : kTileF64;
+      const int32_t longest = integral ? Tile<NT>::kInt : Tile<NT>::kF64;
       uint32_t f = 0;
-      group_partials<NT>(T, S, V, W.qpart, [&](int64_t i) {
-        const double k = W.k[i], x = (double)W.loopw[i];
-        W.comm[i] = (int32_t)i;                 // InitKernel.cu:213-215
-        W.next[i] = (int32_t)i;
-        W.tot[i] = k;                           // InitKernel.cu:236
-        W.in[i] = x;                            // InitKernel.cu:242
-        W.size[i] = 1;                          // OneLevelKernel.cu:87
-        delta_clear(W.delta[i]);
-        W.cand[i] = -1;
-        W.kfrac[i] = m > 0.0 ? __ddiv_rn(k, twom) : 0.0;   // OneLevelKernel.cu:307
-        W.minidx[i] = kNone;
-        if (W.roff[i + 1] - W.roff[i] > longest) f |= fUnfit;
-        if (!(k < 1073741824.0)) f |= fNotInt;
-        return q_term(x, k, m, twom);
-      });
+      group_partials<X>(
+          T, V, W.qpart, [&](int64_t i) { return Row{W.k[i], W.loopw[i], W.roff[i + 1] - W.roff[i]}; },
+          [&](int64_t i, const Row& r) {
+            const double x = (double)r.loopw;
+            W.comm[i] = (int32_t)i;                 // InitKernel.cu:213-215
+            W.next[i] = (int32_t)i;
+            W.tot[i] = r.k;                         // InitKernel.cu:236
+            W.in[i] = x;                            // InitKernel.cu:242
+            W.size[i] = 1;                          // OneLevelKernel.cu:87
+            delta_clear(W.delta[i]);
+            W.cand[i] = -1;
+            W.kfrac[i] = m > 0.0 ? __ddiv_rn(r.k, twom) : 0.0;   // OneLevelKernel.cu:307
+            W.minidx[i] = kNone;
+            if (r.len > longest) f |= fUnfit;
+            if (!(r.k < 1073741824.0)) f |= fNotInt;
+            return q_term(x, r.k, m, twom);
+          });
       if (f) atomicOr(&W.ctl->flags2, f);
     }
-    T.sync();
+    if (!T.sync()) return false;
     const uint32_t f2 = W.ctl->flags2;
     const bool packed = integral && !(f2 & fNotInt);
     // sums beyond 32 bits take the FP64 tiles, whose rows are shorter
-    if ((f2 & fUnfit) || (integral && !packed)) { open = true; break; }
-    const double q0 = finish_sum<NT>(S, W.qpart, V);
-    lower = level == 0 ? q0 : mod;              // LouvainCPP.cpp:356,446
-    const int32_t v0 = row_at(W.roff, V, E * T.rank / T.K);
-    const int32_t v1 = T.rank == T.K - 1 ? V : row_at(W.roff, V, E * (T.rank + 1) / T.K);
-    unsigned long long t1 = lead ? now_ns() : 0ull;
+    if ((f2 & fUnfit) || (integral && !packed)) { at.open = true; return true; }
+    const double q0 = finish_sum<X>(W.qpart, V);
+    at.lower = level == 0 ? q0 : at.mod;        // LouvainCPP.cpp:356,446
+    find_rows<X>(T, V, E);
+    const int32_t v0 = S.row0, v1 = S.row1;
+    const long long t1 = clock64();
     // ---- passes
     double q_prev = q0, floor_q = -1.0;         // curMod = -1 (OneLevelKernel.cu:528)
     int pass = 1, st = LVG_OK;
-    float pass_ms[2] = {0.0f, 0.0f};
+    float pass_ticks[2] = {0.0f, 0.0f};
+#pragma unroll 1
     for (;; ++pass) {
-      const unsigned long long p0 = lead ? now_ns() : 0ull;
-      if (pass == 1) moves_first<NT>(T, S, W, L, v0, v1);
-      else if (packed) moves_hash<NT, true>(T, S, W, L, v0, v1);
-      else moves_hash<NT, false>(T, S, W, L, v0, v1);
-      T.sync();
-      if (lead && pass <= 2) pass_ms[pass - 1] = (float)(now_ns() - p0) * 1e-6f;
-      const bool stop = __dsub_rn(q_prev, floor_q) < cfg.pass_min;             // OneLevelKernel.cu:889-896
+      const long long p0 = clock64();
+      // the pass's test uses the Q of the state before it, so it is known here
+      // (OneLevelKernel.cu:889-896): the pass that ends the level keeps its
+      // decisions but not their totals
+      const bool stop = __dsub_rn(q_prev, floor_q) < cfg.pass_min;
       const bool capped = cfg.max_passes >= 0 && pass >= cfg.max_passes;
+      if (pass == 1) {
+        if constexpr (X::kResident) moves_first_body<X>(L, v0, v1, stop || capped);
+        else moves_first_call<X>(L, v0, v1, stop || capped);
+      } else if (packed) {
+        if constexpr (X::kResident) moves_hash_body<X, true>(L, v0, v1, stop || capped);
+        else moves_hash_call<X, true>(L, v0, v1, stop || capped);
+      } else {
+        moves_hash_call<X, false>(L, v0, v1, stop || capped);
+      }
+      if (!T.sync()) return false;
+      if (pass <= 2) pass_ticks[pass - 1] = (float)(clock64() - p0);
       if (stop || capped) {
-        for (int32_t i = T.gt(); i < V; i += T.stride()) delta_clear(W.delta[i]);
         st = stop ? LVG_OK : LVG_ERR_NOT_CONVERGED;
         break;
       }
-      commit<NT>(T, S, W, V, m);
-      T.sync();
-      const double q = finish_sum<NT>(S, W.qpart, V);
-      floor_q = q_prev < lower ? lower : q_prev;
+      commit<X, false>(T, V, m);
+      if (!T.sync()) return false;
+      const double q = finish_sum<X>(W.qpart, V);
+      floor_q = q_prev < at.lower ? at.lower : q_prev;
       q_prev = q;
-      if (pass >= kSmallPassCap) { open = true; break; }
+      if (pass >= kSmallPassCap) { at.open = true; return true; }
     }
-    if (open) break;
-    T.sync();
+#pragma unroll 1
     for (int32_t i = T.gt(); i < V; i += T.stride()) {      // isolated merge (OneLevelKernel.cu:138-171)
       const int32_t c = W.cand[i];
       if (c >= 0) {
@@ -844,65 +1252,78 @@ __global__ void __launch_bounds__(NT) small_kernel(const SmallJob* jobs, int K, 
         move_deltas<false>(W.delta, W.comm[i], c, W.k[i], __dadd_rn(0.0, (double)W.loopw[i]));
       }
     }
-    T.sync();
-    commit<NT>(T, S, W, V, m);
-    T.sync();
-    const double ql = finish_sum<NT>(S, W.qpart, V);
-    unsigned long long t2 = lead ? now_ns() : 0ull;
+    if (!T.sync()) return false;
+    commit<X, true>(T, V, m);
+    if (!T.sync()) return false;
+    const double ql = finish_sum<X>(W.qpart, V);
+    const long long t2 = clock64();
     // ---- renumber by smallest member (RenumberKernel.cu:121-133)
-    for (int32_t i = T.gt(); i < V; i += T.stride()) atomicMin(&W.minidx[W.comm[i]], i);
-    T.sync();
-    const int32_t i0 = (int32_t)((int64_t)V * T.rank / T.K), i1 = (int32_t)((int64_t)V * (T.rank + 1) / T.K);
-    uint32_t heads = 0;
-    for (int32_t b0 = i0; b0 < i1; b0 += NT) {
-      const int32_t i = b0 + T.tid;
-      heads += __syncthreads_count(i < i1 && W.minidx[W.comm[i < i1 ? i : i0]] == i);
-    }
-    if (T.tid == 0) W.ctl->count[0][T.rank] = heads;
-    T.sync();
+    const int32_t i0 = (int32_t)((int64_t)V * T.rank() / T.K()), i1 = (int32_t)((int64_t)V * (T.rank() + 1) / T.K());
     uint32_t run = 0, C = 0;
-    for (int r = 0; r < T.K; ++r) {
-      const uint32_t c = W.ctl->count[0][r];
-      if (r < T.rank) run += c;
-      C += c;
-    }
-    for (int32_t b0 = i0; b0 < i1; b0 += NT) {
-      const int32_t i = b0 + T.tid;
-      const int32_t c = i < i1 ? W.comm[i] : 0;
-      const bool h = i < i1 && W.minidx[c] == i;
-      uint32_t all;
-      const uint32_t ex = block_excl<NT>(h ? 1u : 0u, S.wtot, &all);
-      if (h) W.newid[c] = (int32_t)(run + ex);
-      run += all;
-    }
-    T.sync();
-    for (int32_t i = T.gt(); i < V; i += T.stride()) {
-      const int32_t c = W.comm[i], id = W.newid[c];
-      W.part[i] = id;
-      if (J.parts) {
-        J.parts[part_off + i] = id;
-        J.parts[part_off + V + i] = c;
+    if (T.K() > 1) {
+      uint32_t heads = 0;
+#pragma unroll 1
+      for (int32_t b0 = i0; b0 < i1; b0 += NT) {
+        const int32_t i = b0 + threadIdx.x;
+        heads += __syncthreads_count(i < i1 && W.minidx[W.comm[i < i1 ? i : i0]] == i);
+      }
+      if (threadIdx.x == 0) W.ctl->count[0][T.rank()] = heads;
+      if (!T.sync()) return false;
+#pragma unroll 4
+      for (int r = 0; r < T.K(); ++r) {
+        const uint32_t c = W.ctl->count[0][r];
+        if (r < T.rank()) run += c;
+        C += c;
       }
     }
-    for (int32_t i = T.gt(); i < J.V; i += T.stride())       // partitionAtLevel (LouvainCPP.cpp:82-106)
-      J.comp[i] = W.newid[W.comm[nlev == 0 ? i : J.comp[i]]];
-    T.sync();
-    unsigned long long t3 = lead ? now_ns() : 0ull;
+    {
+      uint32_t at_run = run;
+#pragma unroll 1
+      for (int32_t b0 = i0; b0 < i1; b0 += NT) {
+        const int32_t i = b0 + threadIdx.x;
+        const int32_t c = i < i1 ? W.comm[i] : 0;
+        const bool h = i < i1 && W.minidx[c] == i;
+        uint32_t all;
+        const uint32_t ex = block_excl<X>(h ? 1u : 0u, &all);
+        if (h) W.newid[c] = (int32_t)(at_run + ex);
+        at_run += all;
+      }
+      if (T.K() == 1) C = at_run;
+    }
+    if (!T.sync()) return false;
+    if (J.parts) {
+#pragma unroll 1
+      for (int32_t i = T.gt(); i < V; i += T.stride()) {
+        const int32_t c = W.comm[i];
+        J.parts[at.part_off + i] = W.newid[c];
+        J.parts[at.part_off + V + i] = c;
+      }
+    }
+    if constexpr (X::kResident) {
+      for (int32_t i = threadIdx.x; i < res_v; i += NT) W.comp[i] = W.newid[W.comm[W.comp[i]]];
+    } else {
+#pragma unroll 2
+      for (int32_t i = T.gt(); i < J.V; i += T.stride())     // partitionAtLevel (LouvainCPP.cpp:82-106)
+        J.comp[i] = W.newid[W.comm[at.nlev == 0 ? i : J.comp[i]]];
+    }
+    const long long t3 = clock64();
     // ---- level break (LouvainCPP.cpp:466)
     bool last = false;
-    if (st != LVG_OK) { status = st; last = true; }
-    else if (level > 0 && (ql - mod) < cfg.level_min) last = true;
-    else if (cfg.max_levels >= 0 && level + 1 >= cfg.max_levels) { status = LVG_ERR_NOT_CONVERGED; last = true; }
-    mod = ql;
+    if (st != LVG_OK) { at.status = st; last = true; }
+    else if (level > 0 && (ql - at.mod) < cfg.level_min) last = true;
+    else if (cfg.max_levels >= 0 && level + 1 >= cfg.max_levels) { at.status = LVG_ERR_NOT_CONVERGED; last = true; }
+    at.mod = ql;
     int64_t E1 = 0;
     int32_t *ns = nullptr, *nd = nullptr;
     float* nw = nullptr;
     if (!last) {
-      list_of(J.lists, J.E, nlev & 1, &ns, &nd, &nw);
-      E1 = coarsen<NT>(T, S, W, L, E, (int32_t)C, ns, nd, nw);
+      list_of(J.lists, J.E, at.nlev & 1, &ns, &nd, &nw);
+      if (X::kResident || C <= (1u << 16)) E1 = coarsen<X, uint32_t>(T, L, E, (int32_t)C, integral, ns, nd, nw);
+      else E1 = coarsen<X, uint64_t>(T, L, E, (int32_t)C, integral, ns, nd, nw);
+      if (E1 < 0) return false;
     }
     if (lead && J.lv) {
-      SmallLevel& R = J.lv[nlev];
+      SmallLevel& R = J.lv[at.nlev];
       R.V = V;
       R.C = (int32_t)C;
       R.passes = pass;
@@ -910,71 +1331,236 @@ __global__ void __launch_bounds__(NT) small_kernel(const SmallJob* jobs, int K, 
       R.nnz = nnz;
       R.q_start = q0;
       R.q_level = ql;
-      R.ms[0] = (float)(t1 - t0) * 1e-6f;
-      R.ms[1] = (float)(t2 - t1) * 1e-6f;
-      R.ms[2] = (float)(t3 - t2) * 1e-6f;
-      R.ms[3] = last ? 0.0f : (float)(now_ns() - t3) * 1e-6f;
-      R.pass_ms[0] = pass_ms[0];
-      R.pass_ms[1] = pass_ms[1];
-      R.part_off = part_off;
+      R.ticks[0] = (float)(t1 - t0);
+      R.ticks[1] = (float)(t2 - t1);
+      R.ticks[2] = (float)(t3 - t2);
+      R.ticks[3] = last ? 0.0f : (float)(clock64() - t3);
+      R.pass_ticks[0] = pass_ticks[0];
+      R.pass_ticks[1] = pass_ticks[1];
+      R.part_off = at.part_off;
     }
-    part_off += 2 * (int64_t)V;
-    ncomms = (int32_t)C;
-    ++nlev;
-    if (last) break;
-    buf = (nlev - 1) & 1;
+    at.part_off += 2 * (int64_t)V;
+    at.ncomms = (int32_t)C;
+    ++at.nlev;
+    if (last) return true;
+    at.buf = (at.nlev - 1) & 1;
     L = List{ns, nd, nw};
-    V = (int32_t)C;
-    E = E1;
-  }
-  double q_final = 0.0;
-  if (J.want_q && !open && !bad) {
-    // Newman modularity of comp over the job's list, as nm_accum_sym_kernel:
-    // the list is symmetric, so each entry adds 2w to its source's community
-    const int64_t C = ncomms;
-    for (int64_t i = T.gt(); i < C; i += T.stride()) W.tot[i] = W.in[i] = 0.0;
-    T.sync();
-    for (int64_t e0 = (int64_t)T.rank * NT; e0 < J.E; e0 += T.stride()) {
-      const int64_t e = e0 + T.tid;
-      const bool in = e < J.E;
-      const int32_t u = in ? J.src[e] : -1;
-      const double x = in ? 2.0 * (double)J.w[e] : 0.0;
-      const int32_t a = in ? J.comp[u] : -1, b = in ? J.comp[J.dst[e]] : -1;
-      const double kin = seg_warp_sum<int32_t>(x, u);
-      const double ain = seg_warp_sum<int32_t>(a == b ? x : 0.0, u);
-      if (seg_warp_last<int32_t>(u, in)) {
-        atomicAdd(&W.tot[a], kin);
-        if (ain != 0.0) atomicAdd(&W.in[a], ain);
-      }
-    }
-    T.sync();
-    group_partials<NT>(T, S, C, W.mpart, [&](int64_t c) { return W.tot[c]; });
-    T.sync();
-    const double tw = finish_sum<NT>(S, W.mpart, C);
-    group_partials<NT>(T, S, C, W.qpart, [&](int64_t c) {
-      const double f = __ddiv_rn(W.tot[c], tw);
-      return tw > 0.0 ? __dsub_rn(__ddiv_rn(W.in[c], tw), __dmul_rn(f, f)) : 0.0;
-    });
-    T.sync();
-    q_final = finish_sum<NT>(S, W.qpart, C);
-  }
-  if (lead) {
-    SmallResult& O = *J.res;
-    O.n_levels = nlev;
-    O.n_comms = ncomms;
-    O.open = open ? 1 : 0;
-    O.status = status;
-    O.bad = bad ? 1 : 0;
-    O.V = V;
-    O.buf = buf;
-    O.E = E;
-    O.mod = mod;
-    O.lower = lower;
-    O.q_final = q_final;
+    list_here = cells_fit<X>((int32_t)C);
+    at.V = (int32_t)C;
+    at.E = E1;
   }
 }
 
+template <typename X>
+__device__ __forceinline__ void load_job(const SmallJob* job) {
+  static_assert(sizeof(SmallJob) % 4 == 0 && sizeof(SmallJob) / 4 <= X::NT, "a word a thread");
+  if (threadIdx.x < sizeof(SmallJob) / 4)
+    reinterpret_cast<uint32_t*>(&X::S().J)[threadIdx.x] = reinterpret_cast<const uint32_t*>(job)[threadIdx.x];
+  __syncthreads();
+}
+
+__device__ __forceinline__ void store_between(Between& B, const At& at) {
+  B.nlev = at.nlev;
+  B.buf = at.buf;
+  B.symmetric = at.symmetric ? 1 : 0;
+  B.V = at.V;
+  B.ncomms = at.ncomms;
+  B.open = at.open ? 1 : 0;
+  B.bad = at.bad ? 1 : 0;
+  B.status = at.status;
+  B.E = at.E;
+  B.part_off = at.part_off;
+  B.mod = at.mod;
+  B.lower = at.lower;
+}
+
+// First launch: the levels until one fits a block's shared memory.
 template <int NT>
+__global__ void __launch_bounds__(NT, 1024 / NT) small_kernel(const SmallJob* jobs, int K, int mode, SmallCfg cfg) {
+  using X = Multi<NT>;
+  load_job<X>(jobs + blockIdx.x / K);
+  const SmallJob& J = X::S().J;
+  if (threadIdx.x == 0) {
+    carve(J.work, J.V, J.E, X::W());
+    X::S().goal = 0ull;
+  }
+  __syncthreads();
+  Team<X> T{K, (int)(blockIdx.x % K), mode};
+  const unsigned long long ns0 = now_ns();
+  const long long c0 = clock64();
+  At at;
+  at.V = J.V;
+  at.E = J.E;
+  at.symmetric = J.check == 0;
+  at.mod = J.mod;
+  if (!run_levels<X>(T, cfg, at)) return;
+  if (T.lead()) {
+    Between& B = *X::W().bt;
+    store_between(B, at);
+    const long long ticks = clock64() - c0;
+    B.ms_per_tick = ticks > 0 ? 1e-6 * (double)(now_ns() - ns0) / (double)ticks : 0.0;
+    B.comp = kCompDone;
+    B.phase = at.tail ? kPhaseTail : kPhaseEnd;
+  }
+}
+
+// Second launch, a block per job: the levels that fit its shared memory, and
+// the sums of the modularity cleared.
+__global__ void __launch_bounds__(kResThreads, 1) small_tail_kernel(const SmallJob* jobs, SmallCfg cfg) {
+  using X = Tail;
+  load_job<X>(jobs + blockIdx.x);
+  const SmallJob& J = X::S().J;
+  Work g;
+  carve(J.work, J.V, J.E, g);
+  Between& B = *g.bt;
+  const int32_t phase = B.phase;
+  int32_t ncomms = B.ncomms;
+  if (phase == kPhaseTail) {
+    if (threadIdx.x == 0) {
+      Resident& W = X::W();
+      W.key[0] = g.key[0];
+      W.key[1] = g.key[1];
+      W.val[0] = g.val[0];
+      W.val[1] = g.val[1];
+      W.wsum = g.wsum;
+      W.ghist = g.ghist;
+    }
+    At at;
+    at.V = B.V;
+    at.E = B.E;
+    at.ncomms = ncomms;
+    at.buf = B.buf;
+    at.nlev = B.nlev;
+    at.symmetric = B.symmetric != 0;
+    at.mod = B.mod;
+    at.lower = B.lower;
+    at.part_off = B.part_off;
+    const bool first = at.nlev == 0;
+    const int32_t nlev0 = at.nlev, v0 = at.V;
+    __syncthreads();
+    Team<X> T{1, 0, kModeCluster};
+    run_levels<X>(T, cfg, at);
+    ncomms = at.ncomms;
+    const bool any = at.nlev > nlev0;
+    if (any)
+      for (int32_t i = threadIdx.x; i < v0; i += kResThreads) g.rc[i] = X::W().comp[i];
+    if (threadIdx.x == 0) {
+      store_between(B, at);
+      B.comp = !any ? kCompDone : (first ? kCompTailAll : kCompTail);
+      B.phase = kPhaseEnd;
+    }
+  }
+  if (J.want_q)
+    for (int32_t i = threadIdx.x; i < ncomms; i += kResThreads) g.tot[i] = g.in[i] = 0.0;
+}
+
+__device__ __forceinline__ int32_t final_comm(const SmallJob& J, const Work& g, int32_t how, int32_t i) {
+  return how == kCompDone ? J.comp[i] : g.rc[how == kCompTailAll ? i : J.comp[i]];
+}
+
+__device__ __forceinline__ bool wants_q(const SmallJob& J, const Between& B) {
+  return J.want_q && B.phase == kPhaseEnd && !B.open && !B.bad;
+}
+
+constexpr int kQThreads = 512;
+
+// Third launch (K blocks a job): community strengths and internal weights of
+// the final communities over the job's list, as nm_accum_sym_kernel: the list
+// is symmetric, so each entry adds 2w to its source's community.
+__global__ void __launch_bounds__(kQThreads) small_sum_kernel(const SmallJob* jobs, int K) {
+  const SmallJob& J = jobs[blockIdx.x / K];
+  Work g;
+  carve(J.work, J.V, J.E, g);
+  const Between& B = *g.bt;
+  if (!wants_q(J, B)) return;
+  const int32_t how = B.comp;
+  const int64_t stride = (int64_t)K * kQThreads;
+#pragma unroll 2
+  for (int64_t e0 = (int64_t)(blockIdx.x % K) * kQThreads; e0 < J.E; e0 += stride) {
+    const int64_t e = e0 + threadIdx.x;
+    const bool in = e < J.E;
+    const int32_t u = in ? J.src[e] : -1;
+    const double x = in ? 2.0 * (double)J.w[e] : 0.0;
+    const int32_t a = in ? final_comm(J, g, how, u) : -1, b = in ? final_comm(J, g, how, J.dst[e]) : -1;
+    bool run_last;
+    const int depth = run_depth(u, run_last);
+    double kin = x, ain = a == b ? x : 0.0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double t1 = __shfl_up_sync(0xffffffffu, kin, o), t2 = __shfl_up_sync(0xffffffffu, ain, o);
+      if (o <= depth) {
+        kin = __dadd_rn(kin, t1);
+        ain = __dadd_rn(ain, t2);
+      }
+    }
+    if (in && run_last) {
+      atomicAdd(&g.tot[a], kin);
+      if (ain != 0.0) atomicAdd(&g.in[a], ain);
+    }
+  }
+}
+
+struct QSpace {
+  static constexpr int NT = kQThreads;
+  static constexpr bool kResident = true;
+  struct Smem {
+    union {
+      double stage[kGroup];
+    } u;
+    double ws[8];
+    double bcast;
+  };
+  static __device__ __forceinline__ Smem& S() { return *reinterpret_cast<Smem*>(smem_raw); }
+};
+
+// Fourth launch (K blocks a job): the composition of the tail's levels; the
+// job's first block takes the modularity and writes the result.
+__global__ void __launch_bounds__(kQThreads) small_end_kernel(const SmallJob* jobs, int K) {
+  const SmallJob& J = jobs[blockIdx.x / K];
+  Work g;
+  carve(J.work, J.V, J.E, g);
+  const Between& B = *g.bt;
+  if (B.phase != kPhaseEnd) return;   // a barrier's wait ran out: no result
+  const int32_t how = B.comp;
+  if (how != kCompDone)
+    for (int64_t i = (int64_t)(blockIdx.x % K) * kQThreads + threadIdx.x; i < J.V; i += (int64_t)K * kQThreads)
+      J.comp[i] = final_comm(J, g, how, (int32_t)i);
+  if (blockIdx.x % K != 0) return;
+  double q = 0.0;
+  if (wants_q(J, B)) {
+    const Team<QSpace> T{1, 0, kModeCluster};
+    const int64_t C = B.ncomms;
+    group_partials<QSpace>(
+        T, C, g.mpart, [&](int64_t c) { return g.tot[c]; }, [&](int64_t, double x) { return x; });
+    __syncthreads();
+    const double tw = finish_sum<QSpace>(g.mpart, C);
+    group_partials<QSpace>(
+        T, C, g.qpart, [&](int64_t c) { return make_double2(g.tot[c], g.in[c]); },
+        [&](int64_t, const double2& x) {
+          const double f = __ddiv_rn(x.x, tw);
+          return tw > 0.0 ? __dsub_rn(__ddiv_rn(x.y, tw), __dmul_rn(f, f)) : 0.0;
+        });
+    __syncthreads();
+    q = finish_sum<QSpace>(g.qpart, C);
+  }
+  if (threadIdx.x == 0) {
+    SmallResult& O = *J.res;
+    O.n_levels = B.nlev;
+    O.n_comms = B.ncomms;
+    O.open = B.open;
+    O.status = B.status;
+    O.bad = B.bad;
+    O.V = B.V;
+    O.buf = B.buf;
+    O.E = B.E;
+    O.ms_per_tick = B.ms_per_tick;
+    O.mod = B.mod;
+    O.lower = B.lower;
+    O.q_final = q;
+    O.finished = 1;
+  }
+}
+
 void set_attributes() {
   constexpr int kDevs = 64;
   static std::mutex mu;
@@ -983,28 +1569,42 @@ void set_attributes() {
   LVG_CUDA(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lock(mu);
   if (dev >= 0 && dev < kDevs && done[dev]) return;
-  LVG_CUDA(cudaFuncSetAttribute(small_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem<NT>)));
-  LVG_CUDA(cudaFuncSetAttribute(small_kernel<NT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  constexpr auto kSmem = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  LVG_CUDA(cudaFuncSetAttribute(small_kernel<512>, kSmem, (int)sizeof(Multi<512>::Smem)));
+  LVG_CUDA(cudaFuncSetAttribute(small_kernel<1024>, kSmem, (int)sizeof(Multi<1024>::Smem)));
+  LVG_CUDA(cudaFuncSetAttribute(small_kernel<1024>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  LVG_CUDA(cudaFuncSetAttribute(small_tail_kernel, kSmem, (int)sizeof(Tail::Smem)));
   if (dev >= 0 && dev < kDevs) done[dev] = true;
 }
 
 template <int NT>
-void launch(const SmallJob* jobs, int n, int K, const SmallCfg& cfg, cudaStream_t s) {
-  set_attributes<NT>();
+void launch(const SmallJob* jobs, int n, int K, int mode, const SmallCfg& cfg, cudaStream_t s) {
+  set_attributes();
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3((unsigned)(n * K));
   lc.blockDim = dim3(NT);
-  lc.dynamicSmemBytes = sizeof(Smem<NT>);
+  lc.dynamicSmemBytes = sizeof(typename Multi<NT>::Smem);
   lc.stream = s;
   cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = (unsigned)K;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
+  if (mode == kModeGrid) {
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+  } else {
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)K;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+  }
   lc.attrs = at;
-  lc.numAttrs = K > 1 ? 1 : 0;
-  LVG_CUDA(cudaLaunchKernelEx(&lc, small_kernel<NT>, jobs, K, cfg));
+  lc.numAttrs = mode == kModeGrid || K > 1 ? 1 : 0;
+  LVG_CUDA(cudaLaunchKernelEx(&lc, small_kernel<NT>, jobs, K, mode, cfg));
   count_launch();
+  small_tail_kernel<<<(unsigned)n, kResThreads, sizeof(Tail::Smem), s>>>(jobs, cfg);
+  LVG_LAUNCH();
+  small_sum_kernel<<<(unsigned)(n * K), kQThreads, 0, s>>>(jobs, K);
+  LVG_LAUNCH();
+  small_end_kernel<<<(unsigned)(n * K), kQThreads, sizeof(QSpace::Smem), s>>>(jobs, K);
+  LVG_LAUNCH();
 }
 
 }  // namespace
@@ -1026,8 +1626,31 @@ bool small_fits(int64_t V, int64_t E, int64_t max_entries) {
 
 void small_run(const SmallJob* d_jobs, int n, int K, const SmallCfg& cfg, cudaStream_t s) {
   if (n <= 0) return;
-  if (K >= 8) launch<1024>(d_jobs, n, K, cfg, s);
-  else launch<512>(d_jobs, n, K, cfg, s);
+  if (K >= 8) launch<1024>(d_jobs, n, K, kModeCluster, cfg, s);
+  else launch<512>(d_jobs, n, K, kModeCluster, cfg, s);
+}
+
+int small_grid_blocks() {
+  constexpr int kDevs = 64;
+  static std::mutex mu;
+  static int blocks[kDevs] = {};
+  set_attributes();
+  int dev = 0;
+  LVG_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lock(mu);
+  if (dev >= 0 && dev < kDevs && blocks[dev] > 0) return blocks[dev];
+  int sms = 0, per = 0;
+  LVG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  LVG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, small_kernel<1024>, 1024, sizeof(Multi<1024>::Smem)));
+  const int n = std::min(sms * std::min(per, 1), kSmallMaxBlocks);
+  if (dev >= 0 && dev < kDevs) blocks[dev] = n;
+  return n;
+}
+
+void small_run_grid(const SmallJob* d_job, void* work, int K, const SmallCfg& cfg, cudaStream_t s) {
+  // the barrier's words, and the phase, should a wait run out
+  LVG_CUDA(cudaMemsetAsync(work, 0, up256(sizeof(Ctl)) + up256(sizeof(Between)), s));
+  launch<1024>(d_job, 1, K, kModeGrid, cfg, s);
 }
 
 }  // namespace lvg

@@ -4,7 +4,8 @@
 
 namespace lvg {
 
-constexpr int32_t kSmallMaxV = 1 << 16;     // a coarse key (two community ids) fits 32 bits
+constexpr int32_t kSmallMaxV = 1 << 18;     // communities of a packed table slot
+constexpr int kSmallMaxBlocks = 160;
 constexpr int32_t kSmallLevels = 48;        // levels one launch may record
 constexpr int32_t kSmallPassCap = 4096;     // passes of a level before it is left to the caller
 constexpr int kSmallPhases = 4;             // build, passes, renumbering, coarsening
@@ -13,8 +14,8 @@ struct SmallLevel {
   int32_t V, C, passes, pad;
   int64_t E, nnz;
   double q_start, q_level;
-  float ms[kSmallPhases];
-  float pass_ms[2];         // move kernels of the first two passes
+  float ticks[kSmallPhases];
+  float pass_ticks[2];      // the moves of the first two passes
   int64_t part_off;         // partition at parts + part_off, labels V later
 };
 
@@ -26,8 +27,9 @@ struct SmallResult {
   int32_t bad;              // an entry out of range or with a bad weight
   int32_t V;                // list of the last level (or of the open one)
   int32_t buf;              // -1: the job's own list, else coarse list buffer 0 or 1
-  int32_t pad;
+  int32_t finished;         // 1: the launch came to its end (0: a barrier's wait ran out)
   int64_t E;
+  double ms_per_tick;
   double mod;               // Q of the last finished level
   double lower;             // floor of the last finished level's pass loop
   double q_final;           // FP64 modularity of comp over the job's list (want_q)
@@ -69,7 +71,12 @@ size_t small_work_bytes(int32_t V, int64_t E);
 void small_list(char* lists, int64_t E, int buf, int32_t** src, int32_t** dst, float** w);
 // True when the sizes are ones this path takes.
 bool small_fits(int64_t V, int64_t E, int64_t max_entries);
-// Runs n jobs (device array), each by a cluster of K blocks.
+// Runs n jobs (device array), each by a cluster of K blocks.  The caller has
+// cleared the results (finished == 0).
 void small_run(const SmallJob* d_jobs, int n, int K, const SmallCfg& cfg, cudaStream_t s);
+// Runs one job (work: its work area) by a cooperative grid of
+// K <= small_grid_blocks() blocks.
+void small_run_grid(const SmallJob* d_job, void* work, int K, const SmallCfg& cfg, cudaStream_t s);
+int small_grid_blocks();
 
 }  // namespace lvg
