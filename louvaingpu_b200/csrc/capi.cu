@@ -172,6 +172,7 @@ void prepare_level(lvg_ctx* c) {
   build_level(c->g, c->tune, c->arena, c->stream);
   c->st.gid = nullptr;     // one graph (a batch that failed part-way may have left its maps)
   c->st.gdone = nullptr;
+  c->st.glast = nullptr;
   alloc_state(c->g, c->st, c->arena);
   init_state(c->g, c->st, 0.0, c->cfg.pass_min_gain, c->cfg.max_passes, c->arena, c->stream);
   LVG_CUDA(cudaEventRecord(c->pev[1], c->stream));   // read once the stream has synchronised
@@ -1377,11 +1378,13 @@ void batch_union(lvg_ctx* c, const BatchInput& in, int32_t* part_out, double* q_
     C.done = ints + 2 * G;
     C.status = ints + 3 * G;
     C.passes = ints + 4 * G;
+    C.last = ints + 5 * G;
     C.ndone = ints + 6 * G;
     C.pass_min = c->cfg.pass_min_gain;
     C.max_passes = c->cfg.max_passes;
     st.gid = vgid;
     st.gdone = C.done;
+    st.glast = C.last;
     batch_init(g, st, s);
     reset_ctl(st, 0.0, c->cfg.pass_min_gain, -1, s);
     batch_commit(0, bp, gm, g.k, st, C, s);

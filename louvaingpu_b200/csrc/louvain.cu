@@ -391,6 +391,7 @@ struct MoveArgs {
   const int32_t* k32;    // degrees as int32 (integral weights), else nullptr: the singleton tot
   const int32_t* gid;    // batched runs: graph of each vertex (nullptr for one graph)
   const int32_t* gdone;  // batched runs: 1 once a graph's level loop has stopped
+  const int32_t* glast;  // batched runs: 1 when a graph's pass in progress ends its level
   unsigned long long* queue;   // batched runs: work counter of this launch (nullptr: grid-stride)
 };
 
@@ -439,6 +440,14 @@ __device__ __forceinline__ void warp_best(double& bg, int32_t& bc, double& bw) {
 // (OneLevelKernel.cu:142-169).
 // SINGLETON: the state is the level's initial one (every community a single
 // vertex), so both sizes are 1 without reading them.
+// A pass that ends the level keeps its decisions but not their totals
+// (OneLevelKernel.cu:921,934-937), and which pass that is is known before it
+// starts: it makes no delta updates (six scattered atomics a moved vertex;
+// with the commit that cleared them, 0.9 ms of an R-MAT scale 24 run).
+__device__ __forceinline__ bool pass_is_last(const MoveArgs& P, int32_t i) {
+  return P.glast ? P.glast[P.gid[i]] != 0 : P.ctl->last != 0;
+}
+
 template <bool SINGLETON = false>
 __device__ __forceinline__ void apply_decision_kl(const MoveArgs& P, int32_t i, int32_t own, int32_t bc, double bw,
                                                   int32_t nseg, double ki, float loopw) {
@@ -449,7 +458,8 @@ __device__ __forceinline__ void apply_decision_kl(const MoveArgs& P, int32_t i, 
   if (so == 1 && sb == 1 && raw > own) best = own;
   P.next[i] = best;
   P.cand[i] = (so == 1 && nseg == 1 && raw != own && own < raw) ? raw : -1;
-  if (best != own) move_deltas<SINGLETON>(P.delta, own, best, ki, __dadd_rn(bw, (double)loopw));
+  if (best != own && (SINGLETON || !pass_is_last(P, i)))
+    move_deltas<SINGLETON>(P.delta, own, best, ki, __dadd_rn(bw, (double)loopw));
 }
 
 template <bool SINGLETON = false>
@@ -462,12 +472,9 @@ __device__ __forceinline__ void apply_decision(const MoveArgs& P, int32_t i, int
   if (so == 1 && sb == 1 && raw > own) best = own;
   P.next[i] = best;
   P.cand[i] = (so == 1 && nseg == 1 && raw != own && own < raw) ? raw : -1;
-  if (best != own) move_deltas<SINGLETON>(P.delta, own, best, P.k[i], __dadd_rn(bw, (double)P.loopw[i]));
+  if (best != own && (SINGLETON || !pass_is_last(P, i)))
+    move_deltas<SINGLETON>(P.delta, own, best, P.k[i], __dadd_rn(bw, (double)P.loopw[i]));
 }
-
-// Packed (community << 32 | integer sum) slots are all ones when empty; the
-// add of an integral weight cannot carry into the key (sums stay below 2^30).
-constexpr unsigned long long kPackedEmpty = ~0ull;
 
 __device__ __forceinline__ uint32_t hash_c(int32_t c, int logT) {
   return (uint32_t)(((uint64_t)(uint32_t)c * 0x9E3779B97F4A7C15ull) >> (64 - logT));
@@ -483,8 +490,12 @@ __device__ __forceinline__ bool table_insert(int32_t* keys, Acc* vals, int logT,
   uint32_t T = 1u << logT;
   uint32_t h = hash_c(c, logT);
   for (uint32_t p = 0; p < T; ++p) {
-    int32_t prev = atomicCAS(&keys[h], -1, c);
-    if (prev == -1 || prev == c) { atomicAdd(&vals[h], w); return true; }
+    int32_t cur = *reinterpret_cast<volatile int32_t*>(&keys[h]);   // most entries meet their community's slot
+    if (cur == -1) {
+      cur = atomicCAS(&keys[h], -1, c);
+      if (cur == -1) cur = c;
+    }
+    if (cur == c) { atomicAdd(&vals[h], w); return true; }
     h = (h + 1) & (T - 1);
   }
   return false;
@@ -881,6 +892,7 @@ static_assert(kTileVtx >= kTileCost / 37 + 1, "tile vertex arrays too small");
 static_assert(kTileCost + kTileMaxDeg + 4 <= (1 << 11) + 8, "tile table load above one half");
 static_assert(kTileCost + kTileMaxDeg + 4 <= 256 * 9, "tile row ids: 9 entries per thread");
 static_assert(kTileVtx < 256, "tile row ids are bytes");
+constexpr int kTileClaims = kThreads * 9;   // >= the entries of a tile
 
 template <typename Acc>
 struct TileSmem {
@@ -890,7 +902,7 @@ struct TileSmem {
   int64_t beg[kTileVtx];
   double kf[kTileVtx];
   double bestw[kTileVtx];
-  unsigned long long bestg[kTileVtx];
+  uint32_t besth[kTileVtx], bestl[kTileVtx];   // best gain, upper and lower half
   int32_t vid[kTileVtx];
   int32_t own[kTileVtx];
   int32_t rowbeg[kTileVtx + 1];
@@ -943,7 +955,7 @@ __global__ void __launch_bounds__(kThreads) move_tile_kernel(MoveArgs P, const i
       S.own[threadIdx.x] = P.comm[i];
       S.kf[threadIdx.x] = P.kfrac[i];
       S.flags[threadIdx.x] = P.has_loop[i] ? 2 : 0;
-      S.bestg[threadIdx.x] = 0ull;
+      S.besth[threadIdx.x] = S.bestl[threadIdx.x] = 0u;
       S.bestc[threadIdx.x] = kNone;
       S.nseg[threadIdx.x] = 0;
     }
@@ -995,28 +1007,37 @@ __global__ void __launch_bounds__(kThreads) move_tile_kernel(MoveArgs P, const i
     }
     __syncthreads();
     const int nc = S.nclaimed;
-    for (int x = threadIdx.x; x < nc; x += kThreads) {       // count, best gain bits
-      int sl = S.claimed[x];
-      unsigned long long k = S.key[sl];
-      int j = (int)(k >> 32);
-      int32_t c = (int32_t)(uint32_t)k;
-      atomicAdd(&S.nseg[j], 1);
-      double W = (double)S.val[sl];
-      if (W != 0.0) {
-        double g = __dsub_rn(W, __dmul_rn(P.tot[c], S.kf[j]));
-        if (g > 0.0) atomicMax(&S.bestg[j], (unsigned long long)__double_as_longlong(g));
+    double rg[kTileClaims / kThreads];
+#pragma unroll
+    for (int q = 0; q < kTileClaims / kThreads; ++q) {       // count, best gain
+      const int x = q * kThreads + threadIdx.x;
+      rg[q] = 0.0;
+      if (x < nc) {
+        const int sl = S.claimed[x];
+        const unsigned long long k = S.key[sl];
+        const int j = (int)(k >> 32);
+        const double W = (double)S.val[sl];
+        if (W != 0.0) rg[q] = __dsub_rn(W, __dmul_rn(P.tot[(int32_t)(uint32_t)k], S.kf[j]));
+        atomicAdd(&S.nseg[j], 1);
+        if (rg[q] > 0.0) atomicMax(&S.besth[j], gain_hi(rg[q]));
       }
     }
     __syncthreads();
-    for (int x = threadIdx.x; x < nc; x += kThreads) {       // smallest community among the best gains
-      int sl = S.claimed[x];
-      unsigned long long k = S.key[sl];
-      int j = (int)(k >> 32);
-      int32_t c = (int32_t)(uint32_t)k;
-      double W = (double)S.val[sl];
-      if (W != 0.0 && S.bestg[j] != 0ull) {
-        double g = __dsub_rn(W, __dmul_rn(P.tot[c], S.kf[j]));
-        if ((unsigned long long)__double_as_longlong(g) == S.bestg[j]) atomicMin(&S.bestc[j], c);
+#pragma unroll
+    for (int q = 0; q < kTileClaims / kThreads; ++q) {
+      if (rg[q] > 0.0) {
+        const int j = (int)(S.key[S.claimed[q * kThreads + threadIdx.x]] >> 32);
+        if (gain_hi(rg[q]) == S.besth[j]) atomicMax(&S.bestl[j], gain_lo(rg[q]));
+        else rg[q] = 0.0;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kTileClaims / kThreads; ++q) {       // smallest community among the best gains
+      if (rg[q] > 0.0) {
+        const unsigned long long k = S.key[S.claimed[q * kThreads + threadIdx.x]];
+        const int j = (int)(k >> 32);
+        if (gain_lo(rg[q]) == S.bestl[j]) atomicMin(&S.bestc[j], (int32_t)(uint32_t)k);
       }
     }
     __syncthreads();
@@ -1044,12 +1065,13 @@ __global__ void __launch_bounds__(kThreads) move_tile_kernel(MoveArgs P, const i
 }
 
 struct TilePackedSmem {
-  unsigned long long slot[kTileSlots];
-  uint16_t claimed[kTileSlots];
+  uint32_t key[kTileSlots];       // tile row << 26 | community, all ones when empty
+  uint32_t sum[kTileSlots];
+  uint16_t claimed[kTileClaims];
   int64_t beg[kTileVtx];
   double kf[kTileVtx];
   double bestw[kTileVtx];
-  unsigned long long bestg[kTileVtx];
+  uint32_t besth[kTileVtx], bestl[kTileVtx];   // best gain, upper and lower half
   int32_t vid[kTileVtx];
   int32_t own[kTileVtx];
   int32_t rowbeg[kTileVtx + 1];
@@ -1057,34 +1079,45 @@ struct TilePackedSmem {
   int32_t nseg[kTileVtx];
   int32_t flags[kTileVtx];
   int32_t nclaimed;
-  uint8_t rowid[kThreads * 9];
+  uint8_t rowid[kTileClaims];
 };
 constexpr int kTilePackedMaxComm = 1 << 26;
+
+constexpr uint32_t kTileNoKey = 0xffffffffu, kTileCommMask = (1u << 26) - 1u;
 
 __device__ __forceinline__ void tile_packed_insert(TilePackedSmem& S, uint32_t key, uint32_t w, bool& overflow) {
   uint32_t h = (uint32_t)(((unsigned long long)key * 0x9E3779B97F4A7C15ull) >> (64 - kTileSlotsLog));
   for (int p = 0; p < kTileSlots; ++p) {
-    const unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(&S.slot[h]);
-    if ((uint32_t)(cur >> 32) == key) { atomicAdd(&S.slot[h], (unsigned long long)w); return; }
-    if (cur == kPackedEmpty) {
-      const unsigned long long prev = atomicCAS(&S.slot[h], kPackedEmpty, ((unsigned long long)key << 32) | w);
-      if (prev == kPackedEmpty) { S.claimed[atomicAdd(&S.nclaimed, 1)] = (uint16_t)h; return; }
-      if ((uint32_t)(prev >> 32) == key) { atomicAdd(&S.slot[h], (unsigned long long)w); return; }
+    uint32_t cur = *reinterpret_cast<volatile uint32_t*>(&S.key[h]);
+    if (cur == kTileNoKey) {
+      cur = atomicCAS(&S.key[h], kTileNoKey, key);
+      if (cur == kTileNoKey) {
+        S.claimed[atomicAdd(&S.nclaimed, 1)] = (uint16_t)h;
+        cur = key;
+      }
     }
+    if (cur == key) { atomicAdd(&S.sum[h], w); return; }
     h = (h + 1) & (kTileSlots - 1);
   }
   overflow = true;
 }
 
-// The tile kernel with packed slots ((j << 26 | c) << 32 | integer sum, all
-// ones when empty; j < 48, so no key is all ones): one shared atomic per
-// entry and a smaller table.  Integral weights, community ids below 2^26.
-__global__ void __launch_bounds__(kThreads) move_tile_packed_kernel(MoveArgs P, const int32_t* tile_start,
+// The tile kernel for integral weights and community ids below 2^26 (rows of
+// a tile below 48, so no key is all ones).  Bound by the shared-memory tables:
+// keys, sums and the best gains (upper, then lower half) are 32-bit words, for
+// which shared memory has atomics -- a 64-bit add or maximum is a
+// compare-and-swap loop there -- and the claimed slots' gains stay in
+// registers through the three rounds of the argmax, so each slot's community
+// total is gathered once.  R-MAT scale 24, four levels: 10.5 -> 5.7 ms.
+__global__ void __launch_bounds__(kThreads, 5) move_tile_packed_kernel(MoveArgs P, const int32_t* tile_start,
                                                                     int64_t ntiles) {
   extern __shared__ __align__(16) unsigned char smem[];
   TilePackedSmem& S = *reinterpret_cast<TilePackedSmem*>(smem);
   if (P.ctl->done) return;
-  for (int sl = threadIdx.x; sl < kTileSlots; sl += kThreads) S.slot[sl] = kPackedEmpty;
+  for (int sl = threadIdx.x; sl < kTileSlots; sl += kThreads) {
+    S.key[sl] = kTileNoKey;
+    S.sum[sl] = 0u;
+  }
   if (threadIdx.x == 0) S.nclaimed = 0;
   bool overflow = false;
   __shared__ WorkQueue wq;
@@ -1101,7 +1134,7 @@ __global__ void __launch_bounds__(kThreads) move_tile_packed_kernel(MoveArgs P, 
       S.own[threadIdx.x] = P.comm[i];
       S.kf[threadIdx.x] = P.kfrac[i];
       S.flags[threadIdx.x] = P.has_loop[i] ? 2 : 0;
-      S.bestg[threadIdx.x] = 0ull;
+      S.besth[threadIdx.x] = S.bestl[threadIdx.x] = 0u;
       S.bestc[threadIdx.x] = kNone;
       S.nseg[threadIdx.x] = 0;
     }
@@ -1152,41 +1185,47 @@ __global__ void __launch_bounds__(kThreads) move_tile_packed_kernel(MoveArgs P, 
     }
     __syncthreads();
     const int nc = S.nclaimed;
-    for (int x = threadIdx.x; x < nc; x += kThreads) {       // count, best gain bits
-      int sl = S.claimed[x];
-      const unsigned long long sv = S.slot[sl];
-      const uint32_t key = (uint32_t)(sv >> 32);
-      int j = (int)(key >> 26);
-      int32_t c = (int32_t)(key & ((1u << 26) - 1u));
-      atomicAdd(&S.nseg[j], 1);
-      double W = (double)(uint32_t)sv;
-      if (W != 0.0) {
-        double g = __dsub_rn(W, __dmul_rn(P.tot[c], S.kf[j]));
-        if (g > 0.0) atomicMax(&S.bestg[j], (unsigned long long)__double_as_longlong(g));
+    double rg[kTileClaims / kThreads];
+#pragma unroll
+    for (int q = 0; q < kTileClaims / kThreads; ++q) {       // count, best gain
+      const int x = q * kThreads + threadIdx.x;
+      rg[q] = 0.0;
+      if (x < nc) {
+        const int sl = S.claimed[x];
+        const uint32_t key = S.key[sl], w = S.sum[sl];
+        if (w != 0u) rg[q] = __dsub_rn((double)w, __dmul_rn(P.tot[key & kTileCommMask], S.kf[key >> 26]));
+        atomicAdd(&S.nseg[key >> 26], 1);
+        if (rg[q] > 0.0) atomicMax(&S.besth[key >> 26], gain_hi(rg[q]));
       }
     }
     __syncthreads();
-    for (int x = threadIdx.x; x < nc; x += kThreads) {       // smallest community among the best gains
-      int sl = S.claimed[x];
-      const unsigned long long sv = S.slot[sl];
-      const uint32_t key = (uint32_t)(sv >> 32);
-      int j = (int)(key >> 26);
-      int32_t c = (int32_t)(key & ((1u << 26) - 1u));
-      double W = (double)(uint32_t)sv;
-      if (W != 0.0 && S.bestg[j] != 0ull) {
-        double g = __dsub_rn(W, __dmul_rn(P.tot[c], S.kf[j]));
-        if ((unsigned long long)__double_as_longlong(g) == S.bestg[j]) atomicMin(&S.bestc[j], c);
+#pragma unroll
+    for (int q = 0; q < kTileClaims / kThreads; ++q) {
+      if (rg[q] > 0.0) {
+        const int j = (int)(S.key[S.claimed[q * kThreads + threadIdx.x]] >> 26);
+        if (gain_hi(rg[q]) == S.besth[j]) atomicMax(&S.bestl[j], gain_lo(rg[q]));
+        else rg[q] = 0.0;
       }
     }
     __syncthreads();
-    for (int x = threadIdx.x; x < nc; x += kThreads) {       // weight to the winner; clear the table
-      int sl = S.claimed[x];
-      const unsigned long long sv = S.slot[sl];
-      const uint32_t key = (uint32_t)(sv >> 32);
-      int j = (int)(key >> 26);
-      int32_t c = (int32_t)(key & ((1u << 26) - 1u));
-      if (c == S.bestc[j]) S.bestw[j] = (double)(uint32_t)sv;
-      S.slot[sl] = kPackedEmpty;
+#pragma unroll
+    for (int q = 0; q < kTileClaims / kThreads; ++q) {       // smallest community among the best gains
+      if (rg[q] > 0.0) {
+        const uint32_t key = S.key[S.claimed[q * kThreads + threadIdx.x]];
+        if (gain_lo(rg[q]) == S.bestl[key >> 26]) atomicMin(&S.bestc[key >> 26], (int32_t)(key & kTileCommMask));
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kTileClaims / kThreads; ++q) {       // weight to the winner; clear the table
+      const int x = q * kThreads + threadIdx.x;
+      if (x < nc) {
+        const int sl = S.claimed[x];
+        const uint32_t key = S.key[sl];
+        if ((int32_t)(key & kTileCommMask) == S.bestc[key >> 26]) S.bestw[key >> 26] = (double)S.sum[sl];
+        S.key[sl] = kTileNoKey;
+        S.sum[sl] = 0u;
+      }
     }
     __syncthreads();
     if (threadIdx.x < nv) {
@@ -1345,27 +1384,30 @@ __global__ void __launch_bounds__(kHubPartThreads) hub_part_kernel(MoveArgs P, H
   if (__syncthreads_or(sawown) && threadIdx.x == 0) atomicOr(&H.sawown[h], 1u);
 }
 
-// Shared-memory tables of hub_agg_kernel.  Packed (integral weights):
-// community << 32 | integer sum, all ones when empty, one atomic per entry.
+// Shared-memory tables of hub_agg_kernel.  PACKED (integral weights): 32-bit
+// keys and sums, which shared memory adds in place (a 64-bit add is a
+// compare-and-swap loop there, and a hub's entries meet a few communities
+// over and over): R-MAT scale 24, three levels, 13.1 -> 6.6 ms.
 template <bool PACKED>
 struct AggTable {
-  unsigned long long slot[kAggSlots];
-  __device__ __forceinline__ void clear(int s) { slot[s] = kPackedEmpty; }
-  __device__ __forceinline__ void get(int s, int32_t& c, double& W) const {
-    c = (int32_t)(uint32_t)(slot[s] >> 32);
-    W = (double)(uint32_t)slot[s];
-  }
+  int32_t key[kAggSlots];
+  uint32_t sum[kAggSlots];
+  __device__ __forceinline__ void clear(int s) { key[s] = -1; sum[s] = 0u; }
+  __device__ __forceinline__ void get(int s, int32_t& c, double& W) const { c = key[s]; W = (double)sum[s]; }
   // 1: added to an existing community, 2: claimed a slot, 0: table full
   __device__ __forceinline__ int insert(int32_t c, float w, uint32_t& where) {
-    const uint32_t wi = (uint32_t)w;
     uint32_t h = agg_slot(c);
     for (int p = 0; p < kAggSlots; ++p) {
-      const unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(&slot[h]);
-      if ((uint32_t)(cur >> 32) == (uint32_t)c) { atomicAdd(&slot[h], (unsigned long long)wi); return 1; }
-      if (cur == kPackedEmpty) {
-        const unsigned long long prev = atomicCAS(&slot[h], kPackedEmpty, ((unsigned long long)(uint32_t)c << 32) | wi);
-        if (prev == kPackedEmpty) { where = h; return 2; }
-        if ((uint32_t)(prev >> 32) == (uint32_t)c) { atomicAdd(&slot[h], (unsigned long long)wi); return 1; }
+      int32_t cur = *reinterpret_cast<volatile int32_t*>(&key[h]);
+      int r = 1;
+      if (cur == -1) {
+        cur = atomicCAS(&key[h], -1, c);
+        if (cur == -1) { cur = c; r = 2; }
+      }
+      if (cur == c) {
+        atomicAdd(&sum[h], (uint32_t)w);
+        where = h;
+        return r;
       }
       h = (h + 1) & (kAggSlots - 1);
     }
@@ -1606,9 +1648,11 @@ __global__ void __launch_bounds__(kRedThreads) commit_kernel(int32_t V, double m
     bool stop = __dsub_rn(ctl->q_prev, ctl->cur) < ctl->pass_min;
     bool capped = ctl->max_passes >= 0 && ctl->pass >= ctl->max_passes;
     if (stop || capped) {
-      for (int j = 0; j < 8; ++j) {
-        int64_t c = base + (int64_t)j * 256;
-        if (c < V) delta_clear(delta[c]);
+      if (!ctl->last) {   // the pass did make delta updates
+        for (int j = 0; j < 8; ++j) {
+          int64_t c = base + (int64_t)j * 256;
+          if (c < V) delta_clear(delta[c]);
+        }
       }
       if (blockIdx.x == 0 && threadIdx.x == 0) ctl->stop_now = stop ? 1 : 2;
       return;
@@ -1673,6 +1717,8 @@ __global__ void __launch_bounds__(kRedThreads) ctl_pass_kernel(const double* par
     ctl->cur = cur;
     ctl->q_prev = q;
     ctl->pass += 1;
+    // the next pass's test (commit_kernel)
+    ctl->last = (__dsub_rn(q, cur) < ctl->pass_min || (ctl->max_passes >= 0 && ctl->pass >= ctl->max_passes)) ? 1 : 0;
   }
 }
 
@@ -1694,6 +1740,7 @@ __global__ void ctl_init_kernel(PassCtl* ctl, double lower, double pass_min, int
   ctl->status = 0;
   ctl->passes = 0;
   ctl->err = 0;
+  ctl->last = 0;
 }
 
 // Isolated-vertex merge (OneLevelKernel.cu:138-171) from the candidates of
@@ -1939,6 +1986,7 @@ MoveArgs move_args(const LevelGraph& g, CommState& st) {
   P.k32 = g.k32;
   P.gid = st.gid;
   P.gdone = st.gdone;
+  P.glast = st.glast;
   P.queue = nullptr;
   return P;
 }
@@ -3084,9 +3132,11 @@ __global__ void __launch_bounds__(kRedThreads) batch_commit_kernel(
     bool stop = __dsub_rn(C.q_prev[g], C.cur[g]) < C.pass_min;
     bool capped = C.max_passes >= 0 && C.pass[g] >= C.max_passes;
     if (stop || capped) {
-      for (int j = 0; j < 8; ++j) {
-        int64_t c = base + (int64_t)j * 256;
-        if (c < cend) delta_clear(delta[c]);
+      if (!C.last[g]) {
+        for (int j = 0; j < 8; ++j) {
+          int64_t c = base + (int64_t)j * 256;
+          if (c < cend) delta_clear(delta[c]);
+        }
       }
       if (c0 == vbase[g] && threadIdx.x == 0) C.stop_now[g] = stop ? 1 : 2;
       return;
@@ -3149,6 +3199,7 @@ __global__ void __launch_bounds__(kRedThreads) batch_ctl_kernel(const int32_t* g
       C.cur[g] = cur;
       C.q_prev[g] = q;
       C.pass[g] += 1;
+      C.last[g] = (__dsub_rn(q, cur) < C.pass_min || (C.max_passes >= 0 && C.pass[g] >= C.max_passes)) ? 1 : 0;
     } else if (MODE == kBatchCtlInit) {
       C.q_prev[g] = q;
     } else {

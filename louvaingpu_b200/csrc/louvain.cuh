@@ -22,7 +22,7 @@ struct PassCtl {
   int32_t status;    // LVG_OK or LVG_ERR_NOT_CONVERGED
   int32_t passes;    // passes executed
   uint32_t err;      // device-side error bits
-  int32_t pad;
+  int32_t last;      // 1: the pass in progress ends the level (its test uses the Q before it)
 };
 
 enum : uint32_t { kErrProbe = 1u };
@@ -134,6 +134,7 @@ struct CommState {
   size_t hot_bytes = 0;           // tot | comm | size, contiguous from tot
   const int32_t* gid = nullptr;   // batched runs: graph of each vertex
   int32_t* gdone = nullptr;       // batched runs: per-graph stop flags
+  const int32_t* glast = nullptr; // batched runs: 1 when a graph's pass in progress ends its level
   unsigned long long* queue = nullptr;   // work counters of the persistent move kernels (batched runs)
 };
 constexpr int kQueueSlots = 8;    // hub buckets, tiles, up to six block-class degree bands
@@ -263,6 +264,7 @@ struct BatchCtl {
   int32_t* done;
   int32_t* status;
   int32_t* passes;
+  int32_t* last;
   int32_t* ndone;
   double pass_min;
   int32_t max_passes;

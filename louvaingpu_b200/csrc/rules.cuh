@@ -58,6 +58,10 @@ __device__ __forceinline__ bool better(double g2, int32_t c2, double g1, int32_t
   return g2 > g1 || (g2 == g1 && c2 < c1);
 }
 
+// Halves of a positive double, whose bits order as its value does.
+__device__ __forceinline__ uint32_t gain_hi(double x) { return (uint32_t)__double2hiint(x); }
+__device__ __forceinline__ uint32_t gain_lo(double x) { return (uint32_t)__double2loint(x); }
+
 // remove/insert (OneLevelKernel.cu:52-78) of a vertex of degree ki moving
 // with weight iw from community own to best.  SINGLETON: own holds only this
 // vertex, so its side is two plain stores the commit applies.

@@ -442,10 +442,6 @@ __device__ __forceinline__ int run_depth(int32_t seg, bool& last) {
   return lane - (31 - __clz(heads & (0xffffffffu >> (31 - lane))));
 }
 
-// Halves of a positive double, whose bits order as its value does.
-__device__ __forceinline__ uint32_t hi32(double x) { return (uint32_t)__double2hiint(x); }
-__device__ __forceinline__ uint32_t lo32(double x) { return (uint32_t)__double2loint(x); }
-
 // First pass of a level: every neighbour is its own candidate.
 template <typename X>
 __device__ __forceinline__ void moves_first_body(const List L, int32_t v, int32_t vend, bool last_pass) {
@@ -509,7 +505,7 @@ __device__ __forceinline__ void moves_first_body(const List L, int32_t v, int32_
         }
         if (j >= 0 && c != kNone && run_last) {
           last |= 1u << q;
-          atomicMax(&S.besth[j], hi32(g));
+          atomicMax(&S.besth[j], gain_hi(g));
         }
         pg[q] = g;
         pc[q] = c;
@@ -518,13 +514,13 @@ __device__ __forceinline__ void moves_first_body(const List L, int32_t v, int32_
 #pragma unroll
       for (int q = 0; q < kItems; ++q)
         if ((last >> q) & 1u) {
-          if (hi32(pg[q]) == S.besth[jj[q]]) atomicMax(&S.bestl[jj[q]], lo32(pg[q]));
+          if (gain_hi(pg[q]) == S.besth[jj[q]]) atomicMax(&S.bestl[jj[q]], gain_lo(pg[q]));
           else last &= ~(1u << q);
         }
       __syncthreads();
 #pragma unroll
       for (int q = 0; q < kItems; ++q)
-        if (((last >> q) & 1u) && lo32(pg[q]) == S.bestl[jj[q]]) atomicMin(&S.bestc[jj[q]], pc[q]);
+        if (((last >> q) & 1u) && gain_lo(pg[q]) == S.bestl[jj[q]]) atomicMin(&S.bestc[jj[q]], pc[q]);
       __syncthreads();
 #pragma unroll
       for (int q = 0; q < kItems; ++q)   // the winner's own entry
@@ -693,20 +689,20 @@ __device__ __forceinline__ void moves_hash_body(const List L, int32_t v, int32_t
         if (jj[q] >= 0) {
           atomicAdd(&S.nseg[jj[q]], 1);
           if (wd[q] != 0.0) gg[q] = __dsub_rn(wd[q], __dmul_rn(gg[q], S.kf[jj[q]]));
-          if (gg[q] > 0.0) atomicMax(&S.besth[jj[q]], hi32(gg[q]));
+          if (gg[q] > 0.0) atomicMax(&S.besth[jj[q]], gain_hi(gg[q]));
         }
       }
       __syncthreads();
 #pragma unroll
       for (int q = 0; q < kItems; ++q)
         if (jj[q] >= 0 && gg[q] > 0.0) {
-          if (hi32(gg[q]) == S.besth[jj[q]]) atomicMax(&S.bestl[jj[q]], lo32(gg[q]));
+          if (gain_hi(gg[q]) == S.besth[jj[q]]) atomicMax(&S.bestl[jj[q]], gain_lo(gg[q]));
           else gg[q] = 0.0;
         }
       __syncthreads();
 #pragma unroll
       for (int q = 0; q < kItems; ++q)         // smallest community among the best gains
-        if (jj[q] >= 0 && gg[q] > 0.0 && lo32(gg[q]) == S.bestl[jj[q]]) atomicMin(&S.bestc[jj[q]], cc[q]);
+        if (jj[q] >= 0 && gg[q] > 0.0 && gain_lo(gg[q]) == S.bestl[jj[q]]) atomicMin(&S.bestc[jj[q]], cc[q]);
       __syncthreads();
 #pragma unroll
       for (int q = 0; q < kItems; ++q)
