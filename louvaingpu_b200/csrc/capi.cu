@@ -166,10 +166,10 @@ void ensure_graphs(lvg_ctx* c) {
   cudaGraphDestroy(gr);
 }
 
-void prepare_level(lvg_ctx* c) {
+void prepare_level(lvg_ctx* c, const ListFacts* facts = nullptr) {
   drop_graphs(c);
   LVG_CUDA(cudaEventRecord(c->pev[0], c->stream));
-  build_level(c->g, c->tune, c->arena, c->stream);
+  build_level(c->g, c->tune, c->arena, c->stream, facts);
   c->st.gid = nullptr;     // one graph (a batch that failed part-way may have left its maps)
   c->st.gdone = nullptr;
   c->st.glast = nullptr;
@@ -187,10 +187,16 @@ constexpr int64_t kSmallRunEntries = 2 * 1024 * 1024;
 constexpr int64_t kClusterEntries = 64 * 1024;
 constexpr int kSmallRunBlocks = 16;
 
-// `ready`: the list is sorted and symmetric, small, and has room for its level
-// build, which then waits until a call needs it.
+// `copied`: the list lies in the arena.  facts: of the list, unless it was
+// built while it streamed in.
 void load_common(lvg_ctx* c, const int32_t* d_src, const int32_t* d_dst, const float* d_w, int64_t E,
-                 int32_t V, bool ready) {
+                 int32_t V, bool copied, const ListFacts* facts) {
+  // A sorted and symmetric list that one launch can run waits with its level
+  // build until a call needs it -- if the arena has room for any list's build,
+  // so that what a load refuses for lack of memory does not depend on the
+  // list's order.
+  const bool ready = facts && facts->sorted_symmetric && small_fits(V, E, kSmallRunEntries) &&
+                     c->arena.cap >= arena_estimate(V, E, copied);
   c->V0 = V;
   c->E0 = E;
   c->src0 = d_src;
@@ -217,7 +223,7 @@ void load_common(lvg_ctx* c, const int32_t* d_src, const int32_t* d_dst, const f
     c->renumbered = false;
     c->symmetric0 = true;
   } else {
-    prepare_level(c);
+    prepare_level(c, facts);
     c->symmetric0 = c->g.sorted_symmetric;
   }
   c->loaded = true;
@@ -565,17 +571,6 @@ bool run_small(lvg_ctx* c, RunState& R) {
   return true;
 }
 
-// The entry checks of a load; *ready when the list is one small_run takes and
-// the arena could hold its level build (so that what a load refuses for lack
-// of memory does not depend on the list's order).
-bool check_small(lvg_ctx* c, const int32_t* src, const int32_t* dst, const float* w, int64_t E, int32_t V, bool copied,
-                 bool* ready) {
-  *ready = false;
-  if (!small_fits(V, E, kSmallRunEntries) || c->arena.cap < arena_estimate(V, E, copied))
-    return validate_edges(src, dst, w, E, V, c->arena, c->stream);
-  return check_edges(src, dst, w, E, V, ready, c->arena, c->stream);
-}
-
 void check_ctx(lvg_ctx* c) {
   require(c != nullptr, LVG_ERR_INVALID_ARG, "null context");
   LVG_CUDA(cudaSetDevice(c->device));
@@ -667,7 +662,7 @@ lvg_status lvg_destroy(lvg_ctx* c) {
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
   drop_graphs(c);
-  c->arena.release();
+  c->arena.destroy();
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
   for (auto& e : c->pev)
@@ -711,8 +706,11 @@ lvg_status lvg_load_edges(lvg_ctx* c, const int32_t* src, const int32_t* dst, co
     float* ww = c->arena.lo_n<float>(E);
     int64_t chunk = c->cfg.load_chunk_entries > 0 ? c->cfg.load_chunk_entries : ((int64_t)1 << 25);
     chunk = (chunk + 2047) / 2048 * 2048;
-    bool ok, ready = false;
-    if (E >= 2 * chunk) {   // copy in chunks, checking and building level 0 as they arrive
+    bool ok;
+    HiScope hs(c->arena);
+    ListFacts facts;
+    const bool chunked = E >= 2 * chunk;
+    if (chunked) {   // copy in chunks, checking and building level 0 as they arrive
       if (!c->copy_stream) LVG_CUDA(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
       ok = stream_load_level0(src, dst, w, s, d, ww, E, V, chunk, c->pre0, c->load_ev, c->arena, c->stream,
                               c->copy_stream);
@@ -722,10 +720,11 @@ lvg_status lvg_load_edges(lvg_ctx* c, const int32_t* src, const int32_t* dst, co
         LVG_CUDA(cudaMemcpyAsync(d, dst, sizeof(int32_t) * E, cudaMemcpyHostToDevice, c->stream));
         LVG_CUDA(cudaMemcpyAsync(ww, w, sizeof(float) * E, cudaMemcpyHostToDevice, c->stream));
       }
-      ok = check_small(c, s, d, ww, E, V, true, &ready);
+      facts = list_facts(s, d, ww, E, V, c->arena, c->stream);
+      ok = facts.ok;
     }
     require(ok, LVG_ERR_INVALID_ARG, "edge list has a vertex id out of range or a negative / non-finite weight");
-    load_common(c, s, d, ww, E, V, ready);
+    load_common(c, s, d, ww, E, V, true, chunked ? nullptr : &facts);
   });
 }
 
@@ -739,10 +738,11 @@ lvg_status lvg_load_edges_device(lvg_ctx* c, const int32_t* src, const int32_t* 
     c->pre0 = PreCsr();
     size_t need = c->cfg.arena_bytes > 0 ? (size_t)c->cfg.arena_bytes : arena_estimate(V, E, false);
     c->arena.reserve(need);
-    bool ready = false;
-    require(check_small(c, src, dst, w, E, V, false, &ready), LVG_ERR_INVALID_ARG,
+    HiScope hs(c->arena);
+    const ListFacts facts = list_facts(src, dst, w, E, V, c->arena, c->stream);
+    require(facts.ok, LVG_ERR_INVALID_ARG,
             "edge list has a vertex id out of range or a negative / non-finite weight");
-    load_common(c, src, dst, w, E, V, ready);
+    load_common(c, src, dst, w, E, V, false, &facts);
   });
 }
 

@@ -259,7 +259,7 @@ struct Scratch {
   }
   ~Scratch() {
     for (void* p : bufs) cudaFree(p);
-    for (Arena* a : arenas) { a->release(); delete a; }
+    for (Arena* a : arenas) { a->destroy(); delete a; }
   }
 };
 

@@ -1308,6 +1308,7 @@ bool induce_transposed(const LevelGraph& g, const int32_t* part, int32_t C, int6
     double* d_m = a.hi_n<double>(1);
     tree_sum_f32(ow, cnt, d_m, a, s);   // as build_level's m over the list (NeighbourCompute.cu:46)
     LVG_CUDA(cudaMemcpyAsync(&next.m, d_m, sizeof(double), cudaMemcpyDeviceToHost, s));
+    next.integral = true;
     next.valid = true;
   }
   LVG_CUDA(cudaStreamSynchronize(s));
@@ -1443,6 +1444,7 @@ bool induce_sorted(const LevelGraph& g, const int32_t* part, int32_t C, int32_t*
     LVG_CUDA(cudaMemcpyAsync(&next->m, d_m, sizeof(double), cudaMemcpyDeviceToHost, s));
     const int64_t loops = read_back(loopx + C, s);
     next->nnz = cnt - loops;
+    next->integral = true;
     next->valid = true;
   }
   LVG_CUDA(cudaStreamSynchronize(s));

@@ -40,16 +40,6 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kHubChunk = 4096;
 
-// ------------------------------------------------------------------ validate
-__global__ void validate_kernel(const int32_t* src, const int32_t* dst, const float* w, int64_t E,
-                                int32_t V, uint32_t* bad) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E; e += (int64_t)gridDim.x * blockDim.x) {
-    int32_t a = src[e], b = dst[e];
-    float x = w[e];
-    if (a < 0 || a >= V || b < 0 || b >= V || !(x >= 0.0f) || isinf(x)) atomicOr(bad, 1u);
-  }
-}
-
 // ------------------------------------------------------------------ CSR build
 // Doubled list D = input ++ reversed(input) (NeighbourCompute.cu:66-68) as
 // 64-bit keys (src << B | dst) with the weight as payload.
@@ -107,180 +97,162 @@ __global__ void csr_emit_kernel(const uint64_t* keys, const float* vals, int64_t
 
 // Sort-free build: a level list that is strictly sorted by (src, dst) and
 // symmetric with bitwise-equal weights doubles into each entry twice, so the
-// merged CSR row of u is its list row without the self loop, weights 2w.
-// Entries per row; runs of equal rows inside a warp add once.  Grid covers E
-// in whole warps.
-__global__ void row_count_kernel(const int32_t* src, int64_t E, int64_t* rowcnt) {
-  int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  bool valid = e < E;
-  int64_t u = valid ? src[e] : -1;
-  double n = seg_warp_sum<int64_t>(valid ? 1.0 : 0.0, u);
-  if (seg_warp_last<int64_t>(u, valid)) atomicAdd((unsigned long long*)&rowcnt[u], (unsigned long long)n);
-}
+// merged CSR row of u is its list row without the self loop, weights 2w.  Two
+// passes over the list, a block per 2048 entries with all its loads issued
+// before any is used: list_facts_kernel checks the list, sums m and counts
+// the non-loop entries; csr_emit_kernel writes the CSR from the counts' scan.
+// (Seven passes before -- checks, m, order and symmetry, row counts, loop
+// flags and their scan, the CSR, integral weights: 20.1 ms of an R-MAT scale
+// 24 load, 520 M entries; BUILDFIG now.)
+enum : uint32_t { kNotSorted = 1u, kBadEntry = 4u, kNotIntegral = 8u };
+constexpr int kListItems = kGroup / kThreads;   // entries per thread
 
-enum : uint32_t { kNotSorted = 1u, kNotSymmetric = 2u, kBadEntry = 4u };
-
-// Sortedness (exact) and symmetry of the list in one coalesced pass.  The
-// symmetry test compares order-free fingerprints: the sums mod 2^64 of two
-// independent 64-bit hashes of (src, dst, weight bits) over the non-loop
-// entries against the same sums of (dst, src, weight bits).  A strictly sorted
-// list has no repeated entry, so the sums agree when the list equals its
-// transpose; a list that is not symmetric passes only on a 128-bit collision.
-// Ids out of [0, V) and bad weights are reported as kBadEntry.
-__global__ void list_check_kernel(const int32_t* src, const int32_t* dst, const float* w, int64_t E, int32_t V,
-                                  uint32_t* flags, unsigned long long* sums) {
+// Order (exact), symmetry, ids and weights, m's group sums, and the non-loop
+// entries of every group, over entries [b, e_end) (b a multiple of 2048; the
+// entry before b has been read before).  The symmetry test compares order-free
+// fingerprints: two 64-bit hashes of (smaller id, larger id, weight bits),
+// summed mod 2^64 with the sign of dst - src.  A strictly sorted list has no
+// repeated entry, so the sums vanish when its upper half equals the transpose
+// of its lower half; another list passes only on a 128-bit collision.
+__global__ void __launch_bounds__(kThreads) list_facts_kernel(const int32_t* src, const int32_t* dst, const float* w,
+                                                              int64_t b, int64_t e_end, int32_t V, uint32_t* flags,
+                                                              unsigned long long* sums, uint32_t* cnt,
+                                                              double* gpart) {
   const uint64_t K1 = 0x243F6A8885A308D3ull, K2 = 0x13198A2E03707344ull;
-  uint64_t d1 = 0, d2 = 0;
-  bool unsorted = false, bad = false;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E; e += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t u = src[e], v = dst[e];
-    bad |= !entry_ok(u, v, w[e], V);
-    if (e + 1 < E) {
-      const int32_t u2 = src[e + 1], v2 = dst[e + 1];
-      if (!(u2 > u || (u2 == u && v2 > v))) unsorted = true;
-    }
-    if (u != v) {
-      const uint32_t wb = __float_as_uint(w[e]);
-      d1 += edge_hash((uint32_t)u, (uint32_t)v, wb, K1) - edge_hash((uint32_t)v, (uint32_t)u, wb, K1);
-      d2 += edge_hash((uint32_t)u, (uint32_t)v, wb, K2) - edge_hash((uint32_t)v, (uint32_t)u, wb, K2);
-    }
-  }
+  __shared__ double ws[8];
+  __shared__ uint32_t wc[kThreads / 32];
   const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  uint64_t d1 = 0, d2 = 0;
+  uint32_t f = 0;
+  const int64_t ngroups = (e_end - b + kGroup - 1) / kGroup;
+  for (int64_t g = blockIdx.x; g < ngroups; g += gridDim.x) {
+    const int64_t e0 = b + g * kGroup + threadIdx.x;
+    int32_t u[kListItems], v[kListItems];
+    float x[kListItems];
+#pragma unroll
+    for (int j = 0; j < kListItems; ++j) {
+      const int64_t e = e0 + j * kThreads;
+      const bool in = e < e_end;
+      u[j] = in ? src[e] : 0;
+      v[j] = in ? dst[e] : 0;
+      x[j] = in ? w[e] : 0.0f;
+    }
+    uint32_t n = 0;
+    double s = 0.0;
+#pragma unroll
+    for (int j = 0; j < kListItems; ++j) {
+      const int64_t e = e0 + j * kThreads;
+      const bool in = e < e_end;
+      int32_t up = __shfl_up_sync(full, u[j], 1), vp = __shfl_up_sync(full, v[j], 1);
+      if (lane == 0 && in && e > 0) {
+        up = src[e - 1];
+        vp = dst[e - 1];
+      }
+      const bool ok = in && entry_ok(u[j], v[j], x[j], V);
+      if (in && !ok) f |= kBadEntry;
+      if (in && e > 0 && !(u[j] > up || (u[j] == up && v[j] > vp))) f |= kNotSorted;
+      const float x2 = __fadd_rn(x[j], x[j]);
+      if (in && x2 != truncf(x2)) f |= kNotIntegral;
+      if (ok && u[j] != v[j]) {
+        const uint64_t key = ((uint64_t)(uint32_t)min(u[j], v[j]) << 32) | (uint32_t)max(u[j], v[j]);
+        const uint64_t h1 = mix64((key ^ K1) + (uint64_t)__float_as_uint(x[j]) * 0x9E3779B97F4A7C15ull);
+        const uint64_t h2 = mix64(h1 ^ key ^ K2);
+        d1 += u[j] < v[j] ? h1 : 0ull - h1;
+        d2 += u[j] < v[j] ? h2 : 0ull - h2;
+      }
+      n += __popc(__ballot_sync(full, ok && u[j] != v[j]));
+      if (in) s = __dadd_rn(s, (double)x[j]);
+    }
+    if (lane == 0) wc[wid] = n;
+    const double r = block_tree256(s, ws);   // (its barriers order wc too)
+    if (threadIdx.x == 0) {
+      uint32_t t = 0;
+      for (int k = 0; k < kThreads / 32; ++k) t += wc[k];
+      cnt[g] = t;
+      gpart[g] = r;
+    }
+    __syncthreads();
+  }
 #pragma unroll
   for (int o = 16; o >= 1; o >>= 1) {
     d1 += __shfl_down_sync(full, d1, o);
     d2 += __shfl_down_sync(full, d2, o);
   }
-  const bool any_unsorted = __any_sync(full, unsorted), any_bad = __any_sync(full, bad);
-  if ((threadIdx.x & 31) == 0) {
+  f = __reduce_or_sync(full, f);
+  if (lane == 0) {
     if (d1) atomicAdd(&sums[0], (unsigned long long)d1);
     if (d2) atomicAdd(&sums[1], (unsigned long long)d2);
-    if (any_unsorted) atomicOr(flags, kNotSorted);
-    if (any_bad) atomicOr(flags, kBadEntry);
+    if (f) atomicOr(flags, f);
   }
 }
 
-__global__ void nonloop_flag_kernel(const int32_t* src, const int32_t* dst, int64_t E, uint32_t* flag) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E; e += (int64_t)gridDim.x * blockDim.x)
-    flag[e] = src[e] != dst[e] ? 1u : 0u;
-}
-
-__global__ void csr_fast_emit_kernel(const int32_t* src, const int32_t* dst, const float* w, int64_t E,
-                                     const uint32_t* pos, int32_t* col, float* cw, double* k, float* loopw,
-                                     uint8_t* has_loop) {
-  int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  bool valid = e < E;
-  int64_t u = valid ? src[e] : -1;
-  int32_t v = valid ? dst[e] : -1;
-  float x = valid ? w[e] : 0.0f;
-  bool loop = valid && u == v;
-  if (valid && !loop) {
-    uint32_t p = pos[e];
-    col[p] = v;
-    cw[p] = __double2float_rn(__dadd_rn((double)x, (double)x));
-  }
-  if (loop) { loopw[u] = x; has_loop[u] = 1; }
-  float f = x == 0.0f ? 1.0f : x;             // InitKernel.cu:165-170, both copies of the entry
-  if (loop) f *= 2.0f;
-  double dv = valid ? __dadd_rn((double)f, (double)f) : 0.0;
-  double sum = seg_warp_sum<int64_t>(dv, u);
-  if (seg_warp_last<int64_t>(u, valid)) atomicAdd(&k[u], sum);
-}
-
-// ---------------------------------------------------------- streamed level-0 build
-// The checks and CSR build of a list that arrives from the host chunk by
-// chunk, each chunk processed while later ones are still being copied.  The
-// CSR is the one build_csr_fast makes; it is kept only if the whole list
-// turns out strictly sorted and symmetric.
-
-// One chunk [b, e_end): range/weight check, strict order against the previous
-// entry, the symmetry fingerprints of list_check_kernel, per-row counts of
-// non-loop entries (into cnt) and the chunk's non-loop flags (pos[b..e_end),
-// scanned next).  Grid covers the chunk in whole warps.
-__global__ void pre_chunk_kernel(const int32_t* src, const int32_t* dst, const float* w, int64_t b, int64_t e_end,
-                                 int32_t V, uint32_t* flags, unsigned long long* sums, unsigned long long* cnt,
-                                 uint32_t* pos) {
-  const uint64_t K1 = 0x243F6A8885A308D3ull, K2 = 0x13198A2E03707344ull;   // as list_check_kernel
+// CSR entries, degrees, self loops and row ends of entries [b, e_end): pos[g]
+// = non-loop entries before group g, plus *carry.  end[u] becomes the CSR
+// position behind row u (of the row's part so far); off is their running
+// maximum.  Entries that fail the checks are skipped (the list is rejected).
+__global__ void __launch_bounds__(kThreads) csr_emit_rows_kernel(const int32_t* src, const int32_t* dst,
+                                                                 const float* w, int64_t b, int64_t e_end, int32_t V,
+                                                                 const uint32_t* pos, const uint32_t* carry,
+                                                                 int32_t* col, float* cw, double* k, float* loopw,
+                                                                 uint8_t* has_loop, int64_t* end) {
+  __shared__ uint32_t wc[kListItems * (kThreads / 32)];
   const unsigned full = 0xffffffffu;
-  const int64_t e = b + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const bool in = e < e_end;
-  const int32_t u = in ? src[e] : 0, v = in ? dst[e] : 0;
-  const float x = in ? w[e] : 0.0f;
-  const bool ok = in && entry_ok(u, v, x, V);
-  bool unsorted = false;
-  if (in && e > 0) {
-    const int32_t u0 = src[e - 1], v0 = dst[e - 1];
-    unsorted = !(u > u0 || (u == u0 && v > v0));
-  }
-  uint64_t d1 = 0, d2 = 0;
-  if (ok && u != v) {
-    const uint32_t wb = __float_as_uint(x);
-    d1 = edge_hash((uint32_t)u, (uint32_t)v, wb, K1) - edge_hash((uint32_t)v, (uint32_t)u, wb, K1);
-    d2 = edge_hash((uint32_t)u, (uint32_t)v, wb, K2) - edge_hash((uint32_t)v, (uint32_t)u, wb, K2);
-  }
-  if (in) pos[e] = (ok && u != v) ? 1u : 0u;
-  const int64_t key = ok ? (int64_t)u : -1;
-  const double n = seg_warp_sum<int64_t>((ok && u != v) ? 1.0 : 0.0, key);
-  if (seg_warp_last<int64_t>(key, ok) && n > 0.0) atomicAdd(&cnt[u], (unsigned long long)n);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int64_t e0 = b + blockIdx.x * (int64_t)kGroup + threadIdx.x;
+  int32_t u[kListItems], v[kListItems];
+  float x[kListItems];
 #pragma unroll
-  for (int o = 16; o >= 1; o >>= 1) {
-    d1 += __shfl_down_sync(full, d1, o);
-    d2 += __shfl_down_sync(full, d2, o);
+  for (int j = 0; j < kListItems; ++j) {
+    const int64_t e = e0 + j * kThreads;
+    const bool in = e < e_end;
+    u[j] = in ? src[e] : -1;
+    v[j] = in ? dst[e] : -1;
+    x[j] = in ? w[e] : 0.0f;
+    if (!in || !entry_ok(u[j], v[j], x[j], V)) u[j] = -1;
   }
-  const bool any_bad = __any_sync(full, in && !ok), any_unsorted = __any_sync(full, unsorted);
-  if ((threadIdx.x & 31) == 0) {
-    if (d1) atomicAdd(&sums[0], (unsigned long long)d1);
-    if (d2) atomicAdd(&sums[1], (unsigned long long)d2);
-    if (any_unsorted) atomicOr(flags, kNotSorted);
-    if (any_bad) atomicOr(flags, kBadEntry);
+  unsigned nl[kListItems];
+#pragma unroll
+  for (int j = 0; j < kListItems; ++j) {
+    nl[j] = __ballot_sync(full, u[j] >= 0 && u[j] != v[j]);
+    if (lane == 0) wc[j * (kThreads / 32) + wid] = __popc(nl[j]);
+  }
+  __syncthreads();
+  if (wid == 0) {   // entry order: item, then warp, then lane
+    static_assert(kListItems * (kThreads / 32) == 64, "two counts a lane");
+    const uint32_t c0 = wc[2 * lane], c1 = wc[2 * lane + 1];
+    const uint32_t ex = warp_inclusive_scan(c0 + c1) - (c0 + c1);
+    wc[2 * lane] = ex;
+    wc[2 * lane + 1] = ex + c0;
+  }
+  __syncthreads();
+  const uint32_t base = pos[blockIdx.x] + (carry ? *carry : 0u);
+#pragma unroll
+  for (int j = 0; j < kListItems; ++j) {
+    const bool ok = u[j] >= 0, loop = ok && u[j] == v[j];
+    const uint32_t p = base + wc[j * (kThreads / 32) + wid] + __popc(nl[j] & ((1u << lane) - 1u));
+    if (ok && !loop) {
+      col[p] = v[j];
+      cw[p] = __double2float_rn(__dadd_rn((double)x[j], (double)x[j]));
+    }
+    if (loop) { loopw[u[j]] = x[j]; has_loop[u[j]] = 1; }
+    float f = x[j] == 0.0f ? 1.0f : x[j];             // InitKernel.cu:165-170, both copies of the entry
+    if (loop) f *= 2.0f;
+    bool last;
+    const int depth = run_depth(u[j], last);
+    const double sum = run_sum(ok ? __dadd_rn((double)f, (double)f) : 0.0, depth);
+    if (ok && last) {
+      atomicAdd(&k[u[j]], sum);
+      // a row's last piece lies in the last block and item that holds the row:
+      // the plain store of an earlier piece must not come after it
+      atomicMax((unsigned long long*)&end[u[j]], (unsigned long long)(p + (loop ? 0u : 1u)));
+    }
   }
 }
 
 // carry[i + 1] = carry[i] + (non-loop entries of chunk i)
 __global__ void pre_carry_kernel(uint32_t* carry, int64_t i, const uint32_t* chunk_total) {
   carry[i + 1] = carry[i] + *chunk_total;
-}
-
-// The chunk's CSR entries, degrees and self loops, as csr_fast_emit_kernel
-// does for the whole list (positions: chunk scan + carry).  Entries that
-// failed the checks are skipped.  Grid covers the chunk in whole warps.
-__global__ void pre_emit_kernel(const int32_t* src, const int32_t* dst, const float* w, int64_t b, int64_t e_end,
-                                int32_t V, const uint32_t* pos, const uint32_t* carry, int32_t* col, float* cw,
-                                double* k, float* loopw, uint8_t* has_loop) {
-  const int64_t e = b + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const bool in = e < e_end;
-  const int32_t u = in ? src[e] : 0, v = in ? dst[e] : 0;
-  const float x = in ? w[e] : 0.0f;
-  const bool ok = in && entry_ok(u, v, x, V);
-  const bool loop = ok && u == v;
-  if (ok && !loop) {
-    const uint32_t p = pos[e] + *carry;
-    col[p] = v;
-    cw[p] = __double2float_rn(__dadd_rn((double)x, (double)x));
-  }
-  if (loop) { loopw[u] = x; has_loop[u] = 1; }
-  float f = x == 0.0f ? 1.0f : x;             // InitKernel.cu:165-170, both copies of the entry
-  if (loop) f *= 2.0f;
-  const double dv = ok ? __dadd_rn((double)f, (double)f) : 0.0;
-  const int64_t key = ok ? (int64_t)u : -1;
-  const double sum = seg_warp_sum<int64_t>(dv, key);
-  if (seg_warp_last<int64_t>(key, ok)) atomicAdd(&k[u], sum);
-}
-
-// Group partials of the fixed-tree sum of the weights (as tree_sum_f32's
-// first round; group b of the chunk starting at x).
-__global__ void __launch_bounds__(kRedThreads) pre_group_kernel(const float* x, int64_t n, double* out) {
-  __shared__ double ws[8];
-  const int64_t b = blockIdx.x;
-  int64_t len = n - b * kGroup;
-  if (len > kGroup) len = kGroup;
-  const double r = group_sum_block<float>(x + b * kGroup, len, ws);
-  if (threadIdx.x == 0) out[b] = r;
-}
-
-__global__ void row_off_kernel(const int64_t* rowstart, const uint32_t* pos, int32_t V, int64_t* off) {
-  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u <= V; u += (int64_t)gridDim.x * blockDim.x)
-    off[u] = pos[rowstart[u]];
 }
 
 __global__ void to_float_kernel(const double* x, float* y, int64_t n) {
@@ -305,16 +277,19 @@ __device__ __forceinline__ int bucket_of(int32_t i, const int64_t* off, const do
 
 __global__ void __launch_bounds__(kThreads) bucket_count_kernel(int32_t V, const int64_t* off, const double* k,
                                                                 int32_t tmax, int32_t bmax, uint32_t* cnt,
-                                                                int64_t nblk) {
+                                                                int64_t nblk, uint32_t* big) {
   uint32_t c[kNumBuckets] = {};
   int64_t base = (int64_t)blockIdx.x * 2048 + (int64_t)threadIdx.x * 8;
+  bool large = false;   // a degree that 32-bit sums cannot hold
   for (int j = 0; j < 8; ++j) {
     int64_t i = base + j;
     if (i < V) {
       int b = bucket_of((int32_t)i, off, k, tmax, bmax);
       if (b < kNumBuckets) c[b]++;
+      large |= !(k[i] < 1073741824.0);
     }
   }
+  if (large) atomicOr(big, 1u);
   for (int b = 0; b < kNumBuckets; ++b) {
     uint32_t tot;
     block_exclusive_scan256<uint32_t>(c[b], &tot);
@@ -343,6 +318,12 @@ __global__ void __launch_bounds__(kThreads) bucket_scatter_kernel(int32_t V, con
     int b = bid[j];
     if (b < kNumBuckets) list[pre[b]++] = (int32_t)(base + j);
   }
+}
+
+// First item of every class (and their total): the counts' scan at each
+// class's first block.
+__global__ void bucket_starts_kernel(const uint32_t* cnt, int64_t nblk, uint32_t* starts) {
+  if (threadIdx.x <= kNumBuckets) starts[threadIdx.x] = cnt[threadIdx.x * nblk];
 }
 
 __global__ void hub_info_kernel(const int32_t* hubs, int64_t nhub, const int64_t* off, int64_t* beg_end) {
@@ -1259,15 +1240,16 @@ __global__ void tile_start_kernel(const int64_t* cum, int64_t n, int32_t* tile_s
   }
 }
 
-// Integral weights with small degrees allow an exact int32 accumulator.
-__global__ void int_weights_kernel(const float* cw, int64_t nnz, const double* k, int32_t V, uint32_t* notint) {
+// Integral weights (with degrees below 2^30: bucket_count_kernel) allow an
+// exact int32 accumulator.  Only for a CSR whose build did not tell.
+__global__ void int_weights_kernel(const float* cw, int64_t nnz, uint32_t* notint) {
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  bool frac = false;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nnz; e += stride) {
     float x = cw[e];
-    if (x != truncf(x)) atomicOr(notint, 1u);
+    frac |= x != truncf(x);
   }
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < V; i += stride)
-    if (!(k[i] < 1073741824.0)) atomicOr(notint, 1u);
+  if (__any_sync(0xffffffffu, frac) && (threadIdx.x & 31) == 0) atomicOr(notint, 1u);
 }
 
 // Hubs: rows longer than block_max.  A pass aggregates a hub's neighbour
@@ -1995,34 +1977,42 @@ MoveArgs move_args(const LevelGraph& g, CommState& st) {
 
 // ============================================================================ host
 
-bool validate_edges(const int32_t* src, const int32_t* dst, const float* w, int64_t E, int32_t V, Arena& a,
-                    cudaStream_t s) {
-  if (E == 0) return true;
-  HiScope hs(a);
-  uint32_t* bad = a.hi_n<uint32_t>(1);
-  LVG_CUDA(cudaMemsetAsync(bad, 0, sizeof(uint32_t), s));
-  validate_kernel<<<sm_grid(E, kThreads), kThreads, 0, s>>>(src, dst, w, E, V, bad);
+namespace {
+// One pass of list_facts_kernel over [b, e_end).
+void launch_facts(const int32_t* src, const int32_t* dst, const float* w, int64_t b, int64_t e_end, int32_t V,
+                  unsigned long long* chk, uint32_t* cnt, double* gpart, cudaStream_t s) {
+  const int64_t ng = (e_end - b + kGroup - 1) / kGroup;
+  const unsigned grid = (unsigned)std::min<int64_t>(ng, (int64_t)sm_count() * 8);
+  list_facts_kernel<<<grid, kThreads, 0, s>>>(src, dst, w, b, e_end, V, (uint32_t*)chk, chk + 1, cnt, gpart);
   LVG_LAUNCH();
-  uint32_t h = 0;
-  LVG_CUDA(cudaMemcpyAsync(&h, bad, sizeof h, cudaMemcpyDeviceToHost, s));
-  LVG_CUDA(cudaStreamSynchronize(s));
-  return h == 0;
 }
+}  // namespace
 
-bool check_edges(const int32_t* src, const int32_t* dst, const float* w, int64_t E, int32_t V, bool* sorted_symmetric,
-                 Arena& a, cudaStream_t s) {
-  *sorted_symmetric = false;
-  if (E == 0) return true;
+ListFacts list_facts(const int32_t* src, const int32_t* dst, const float* w, int64_t E, int32_t V, Arena& a,
+                     cudaStream_t s) {
+  ListFacts F;
+  if (E <= 0) return F;
+  const int64_t ng = (E + kGroup - 1) / kGroup;
+  F.pos = a.hi_n<uint32_t>(ng + 1);
   HiScope hs(a);
+  double* gpart = a.hi_n<double>(ng);
+  double* d_m = a.hi_n<double>(1);
   unsigned long long* chk = a.hi_n<unsigned long long>(3);   // flags, two fingerprint sums
   LVG_CUDA(cudaMemsetAsync(chk, 0, 3 * sizeof(unsigned long long), s));
-  list_check_kernel<<<sm_grid(E, kThreads), kThreads, 0, s>>>(src, dst, w, E, V, (uint32_t*)chk, chk + 1);
-  LVG_LAUNCH();
-  unsigned long long h[3] = {0, 0, 0};
-  LVG_CUDA(cudaMemcpyAsync(h, chk, sizeof h, cudaMemcpyDeviceToHost, s));
-  LVG_CUDA(cudaStreamSynchronize(s));
-  *sorted_symmetric = h[0] == 0 && h[1] == 0 && h[2] == 0;
-  return (h[0] & kBadEntry) == 0;
+  launch_facts(src, dst, w, 0, E, V, chk, F.pos, gpart, s);
+  scan_u32(F.pos, F.pos, ng, a, s);
+  tree_finish(gpart, ng, d_m, a, s);   // NeighbourCompute.cu:46
+  Fetch f(a, s);
+  const unsigned long long* h = f.add(chk, 3);
+  const uint32_t* n = f.add(F.pos + ng);
+  const double* m = f.add(d_m);
+  f.wait();
+  F.ok = (h[0] & kBadEntry) == 0;
+  F.sorted_symmetric = F.ok && (h[0] & kNotSorted) == 0 && h[1] == 0 && h[2] == 0;
+  F.integral = (h[0] & kNotIntegral) == 0;
+  F.nonloop = *n;
+  F.m = *m;
+  return F;
 }
 
 bool stream_load_level0(const int32_t* hsrc, const int32_t* hdst, const float* hw, int32_t* src, int32_t* dst,
@@ -2041,8 +2031,8 @@ bool stream_load_level0(const int32_t* hsrc, const int32_t* hdst, const float* h
   bool valid = false, bad = false;
   {
     HiScope hs(a);
-    uint32_t* pos = a.hi_n<uint32_t>(E + 1);
     const int64_t ngroups = (E + kGroup - 1) / kGroup;
+    uint32_t* pos = a.hi_n<uint32_t>(ngroups + nchunks + 1);   // per chunk: its groups' counts and their total
     double* gpart = a.hi_n<double>(ngroups);
     double* d_m = a.hi_n<double>(1);
     unsigned long long* chk = a.hi_n<unsigned long long>(3);   // flags, two fingerprint sums
@@ -2077,16 +2067,14 @@ bool stream_load_level0(const int32_t* hsrc, const int32_t* hdst, const float* h
       const int64_t b = i * chunk, n = std::min(chunk, E - b);
       if (i + 1 < nchunks) issue_copy(i + 1);
       LVG_CUDA(cudaStreamWaitEvent(s, evs[i], 0));
-      pre_chunk_kernel<<<grid_for(n, kThreads), kThreads, 0, s>>>(src, dst, w, b, b + n, V, (uint32_t*)chk, chk + 1,
-                                                                   (unsigned long long*)pre.off, pos);
+      const int64_t ng = (n + kGroup - 1) / kGroup;
+      uint32_t* cpos = pos + b / kGroup + i;
+      launch_facts(src, dst, w, b, b + n, V, chk, cpos, gpart + b / kGroup, s);
+      scan_u32(cpos, cpos, ng, a, s);
+      pre_carry_kernel<<<1, 1, 0, s>>>(carry, i, cpos + ng);
       LVG_LAUNCH();
-      scan_u32(pos + b, pos + b, n, a, s);
-      pre_carry_kernel<<<1, 1, 0, s>>>(carry, i, pos + b + n);
-      LVG_LAUNCH();
-      pre_emit_kernel<<<grid_for(n, kThreads), kThreads, 0, s>>>(src, dst, w, b, b + n, V, pos, carry + i, pre.col,
-                                                                  pre.cw, pre.k, pre.loopw, pre.has_loop);
-      LVG_LAUNCH();
-      pre_group_kernel<<<(unsigned)((n + kGroup - 1) / kGroup), kRedThreads, 0, s>>>(w + b, n, gpart + b / kGroup);
+      csr_emit_rows_kernel<<<(unsigned)ng, kThreads, 0, s>>>(src, dst, w, b, b + n, V, cpos, carry + i, pre.col,
+                                                             pre.cw, pre.k, pre.loopw, pre.has_loop, pre.off);
       LVG_LAUNCH();
     }
     tree_finish(gpart, ngroups, d_m, a, s);
@@ -2095,11 +2083,11 @@ bool stream_load_level0(const int32_t* hsrc, const int32_t* hdst, const float* h
     LVG_CUDA(cudaMemcpyAsync(&pre.m, d_m, sizeof(double), cudaMemcpyDeviceToHost, s));
     LVG_CUDA(cudaStreamSynchronize(s));
     bad = (h[0] & kBadEntry) != 0;
-    valid = !bad && h[0] == 0 && h[1] == 0 && h[2] == 0;
+    valid = !bad && (h[0] & kNotSorted) == 0 && h[1] == 0 && h[2] == 0;
+    pre.integral = (h[0] & kNotIntegral) == 0;
     if (valid) {
-      scan_i64(pre.off, pre.off, V, a, s);   // non-loop entries before each row
-      LVG_CUDA(cudaMemcpyAsync(&pre.nnz, pre.off + V, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-      LVG_CUDA(cudaStreamSynchronize(s));
+      scan_max_i64(pre.off, pre.off, V, a, s);   // row ends -> row starts
+      pre.nnz = fetch_one(pre.off + V, a, s);
     }
   }
   if (!valid) {
@@ -2110,56 +2098,131 @@ bool stream_load_level0(const int32_t* hsrc, const int32_t* hdst, const float* h
   return !bad;
 }
 
-// Sort-free CSR build; returns false (and builds nothing) unless the level
-// list is strictly sorted and symmetric.
 static void set_move_attributes();
 
-static bool build_csr_fast(LevelGraph& g, Arena& a, cudaStream_t s) {
-  const int32_t V = g.V;
+// CSR of a list known to be sorted and symmetric (g.off zeroed here).
+static void build_csr_fast(LevelGraph& g, const ListFacts& F, Arena& a, cudaStream_t s) {
   const int64_t E = g.E;
-  if (E >= ((int64_t)1 << 32) - 1) return false;
-  HiScope hs(a);
-  int64_t* rowstart = a.hi_n<int64_t>(V + 1);
-  unsigned long long* chk = a.hi_n<unsigned long long>(3);   // flags, two fingerprint sums
-  LVG_CUDA(cudaMemsetAsync(chk, 0, 3 * sizeof(unsigned long long), s));
-  list_check_kernel<<<sm_grid(E, kThreads), kThreads, 0, s>>>(g.src, g.dst, g.w, E, V, (uint32_t*)chk, chk + 1);
+  g.nnz = F.nonloop;
+  g.col = a.lo_n<int32_t>(g.nnz);
+  g.cw = a.lo_n<float>(g.nnz);
+  LVG_CUDA(cudaMemsetAsync(g.off, 0, sizeof(int64_t) * ((size_t)g.V + 1), s));
+  csr_emit_rows_kernel<<<grid_for(E, kGroup), kThreads, 0, s>>>(g.src, g.dst, g.w, 0, E, g.V, F.pos, nullptr, g.col,
+                                                                g.cw, g.k, g.loopw, g.has_loop, g.off);
   LVG_LAUNCH();
-  unsigned long long h[3] = {0, 0, 0};
-  LVG_CUDA(cudaMemcpyAsync(h, chk, sizeof h, cudaMemcpyDeviceToHost, s));
-  LVG_CUDA(cudaStreamSynchronize(s));
-  if (h[0] != 0 || h[1] != 0 || h[2] != 0) return false;
-  LVG_CUDA(cudaMemsetAsync(rowstart, 0, sizeof(int64_t) * (V + 1), s));
-  row_count_kernel<<<grid_for(E, kThreads), kThreads, 0, s>>>(g.src, E, rowstart);
-  LVG_LAUNCH();
-  scan_i64(rowstart, rowstart, V, a, s);
-  uint32_t* pos = a.hi_n<uint32_t>(E + 1);
-  nonloop_flag_kernel<<<sm_grid(E, kThreads), kThreads, 0, s>>>(g.src, g.dst, E, pos);
-  LVG_LAUNCH();
-  scan_u32(pos, pos, E, a, s);
-  uint32_t nnz = 0;
-  LVG_CUDA(cudaMemcpyAsync(&nnz, pos + E, sizeof nnz, cudaMemcpyDeviceToHost, s));
-  LVG_CUDA(cudaStreamSynchronize(s));
-  g.nnz = nnz;
-  g.col = a.lo_n<int32_t>(nnz);
-  g.cw = a.lo_n<float>(nnz);
-  csr_fast_emit_kernel<<<grid_for(E, kThreads), kThreads, 0, s>>>(g.src, g.dst, g.w, E, pos, g.col, g.cw, g.k,
-                                                                    g.loopw, g.has_loop);
-  LVG_LAUNCH();
-  row_off_kernel<<<sm_grid(V + 1, kThreads), kThreads, 0, s>>>(rowstart, pos, V, g.off);
-  LVG_LAUNCH();
-  return true;
+  scan_max_i64(g.off, g.off, g.V, a, s);   // row ends -> row starts
 }
 
-void build_level(LevelGraph& g, const Tuning& t, Arena& a, cudaStream_t s) {
+// Hubs: chunks of kHubChunk entries and ~kHubBucketTarget entries per bucket.
+// be: first and last CSR entry of every hub.
+static void build_hubs(LevelGraph& g, const std::vector<int64_t>& be, Arena& a, cudaStream_t s) {
+  const int64_t nhub = (int64_t)be.size() / 2;
+  std::vector<int32_t> plog(nhub), cb0(nhub + 1), bb0(nhub + 1), chub, bhub;
+  std::vector<int64_t> cbeg, cbo, cstg;
+  int64_t noff = 0, nstg = 0;
+  for (int64_t h = 0; h < nhub; ++h) {
+    const int64_t d = be[2 * h + 1] - be[2 * h];
+    int l = 0;
+    while (l < kHubMaxBucketsLog && ((int64_t)kHubBucketTarget << l) < d) ++l;
+    plog[h] = l;
+    cb0[h] = (int32_t)chub.size();
+    bb0[h] = (int32_t)bhub.size();
+    for (int64_t b = be[2 * h]; b < be[2 * h + 1]; b += kHubChunk) {
+      chub.push_back((int32_t)h);
+      cbeg.push_back(b);
+      cbo.push_back(noff);
+      cstg.push_back(nstg + (b - be[2 * h]));
+      noff += ((int64_t)1 << l) + 1;
+    }
+    nstg += d;
+    bhub.insert(bhub.end(), (size_t)1 << l, (int32_t)h);
+  }
+  cb0[nhub] = (int32_t)chub.size();
+  bb0[nhub] = (int32_t)bhub.size();
+  g.nchunk = (int64_t)chub.size();
+  g.nhub_bucket = (int64_t)bhub.size();
+  g.chunk_hub = a.lo_n<int32_t>(g.nchunk);
+  g.chunk_beg = a.lo_n<int64_t>(g.nchunk);
+  g.chunk_cbo = a.lo_n<int64_t>(g.nchunk);
+  g.chunk_stg = a.lo_n<int64_t>(g.nchunk);
+  g.hub_plog = a.lo_n<int32_t>(nhub);
+  g.hub_cb0 = a.lo_n<int32_t>(nhub + 1);
+  g.hub_bb0 = a.lo_n<int32_t>(nhub + 1);
+  g.bucket_hub = a.lo_n<int32_t>(g.nhub_bucket);
+  g.cb_off = a.lo_n<uint16_t>(noff);
+  g.stage = a.lo_n<unsigned long long>(nstg);
+  g.hub_sawown = a.lo_n<uint32_t>(nhub);
+  g.hub_part = a.lo_n<HubPartial>(g.nhub_bucket);
+  LVG_CUDA(cudaMemcpyAsync(g.chunk_hub, chub.data(), sizeof(int32_t) * g.nchunk, cudaMemcpyHostToDevice, s));
+  LVG_CUDA(cudaMemcpyAsync(g.chunk_beg, cbeg.data(), sizeof(int64_t) * g.nchunk, cudaMemcpyHostToDevice, s));
+  LVG_CUDA(cudaMemcpyAsync(g.chunk_cbo, cbo.data(), sizeof(int64_t) * g.nchunk, cudaMemcpyHostToDevice, s));
+  LVG_CUDA(cudaMemcpyAsync(g.chunk_stg, cstg.data(), sizeof(int64_t) * g.nchunk, cudaMemcpyHostToDevice, s));
+  LVG_CUDA(cudaMemcpyAsync(g.hub_plog, plog.data(), sizeof(int32_t) * nhub, cudaMemcpyHostToDevice, s));
+  LVG_CUDA(cudaMemcpyAsync(g.hub_cb0, cb0.data(), sizeof(int32_t) * (nhub + 1), cudaMemcpyHostToDevice, s));
+  LVG_CUDA(cudaMemcpyAsync(g.hub_bb0, bb0.data(), sizeof(int32_t) * (nhub + 1), cudaMemcpyHostToDevice, s));
+  LVG_CUDA(cudaMemcpyAsync(g.bucket_hub, bhub.data(), sizeof(int32_t) * g.nhub_bucket, cudaMemcpyHostToDevice,
+                           s));
+  LVG_CUDA(cudaMemsetAsync(g.hub_sawown, 0, sizeof(uint32_t) * nhub, s));
+  LVG_CUDA(cudaStreamSynchronize(s));  // host vectors go out of scope
+}
+
+// CSR of any list: the doubled list sorted by (src, dst), equal pairs merged.
+static void build_csr_sorted(LevelGraph& g, Arena& a, cudaStream_t s) {
+  const int32_t V = g.V;
+  const int64_t E = g.E, n = 2 * E;
+  HiScope hs(a);
+  const int B = std::max(1, bits_for(V));
+  uint64_t* k0 = a.hi_n<uint64_t>(n);
+  float* v0 = a.hi_n<float>(n);
+  uint64_t* k1 = a.hi_n<uint64_t>(n);
+  float* v1 = a.hi_n<float>(n);
+  uint32_t* head = a.hi_n<uint32_t>(n + 1);
+  uint32_t* pos = a.hi_n<uint32_t>(n + 1);
+  int64_t* rowcnt = a.hi_n<int64_t>(V + 1);
+  LVG_CUDA(cudaMemsetAsync(rowcnt, 0, sizeof(int64_t) * (V + 1), s));
+  if (E > 0) {
+    make_keys_kernel<<<sm_grid(E, kThreads), kThreads, 0, s>>>(g.src, g.dst, g.w, E, B, k0, v0);
+    LVG_LAUNCH();
+  }
+  int which = radix_sort_pairs(k0, v0, k1, v1, n, 2 * B, a, s);   // NeighbourCompute.cu:82
+  uint64_t* keys = which ? k1 : k0;
+  float* vals = which ? v1 : v0;
+  if (n > 0) {
+    csr_scan_kernel<<<grid_for(n, kThreads), kThreads, 0, s>>>(keys, vals, n, B, head, rowcnt, g.k, g.loopw,
+                                                                g.has_loop);
+    LVG_LAUNCH();
+  }
+  scan_u32(head, pos, n, a, s);
+  scan_i64(rowcnt, g.off, V, a, s);
+  const int64_t nnz = fetch_one(g.off + V, a, s);
+  g.nnz = nnz;
+  // exact CSR on the low end
+  g.col = a.lo_n<int32_t>(nnz);
+  g.cw = a.lo_n<float>(nnz);
+  double* wsum = (double*)(which ? k0 : k1);   // the sort's other key buffer: nnz <= n
+  LVG_CUDA(cudaMemsetAsync(wsum, 0, sizeof(double) * nnz, s));
+  if (n > 0) {
+    csr_emit_kernel<<<grid_for(n, kThreads), kThreads, 0, s>>>(keys, vals, n, B, pos, head, g.col, wsum);
+    LVG_LAUNCH();
+  }
+  if (nnz > 0) {
+    to_float_kernel<<<sm_grid(nnz, kThreads), kThreads, 0, s>>>(wsum, g.cw, nnz);
+    LVG_LAUNCH();
+  }
+}
+
+void build_level(LevelGraph& g, const Tuning& t, Arena& a, cudaStream_t s, const ListFacts* facts) {
   const int32_t V = g.V;
   const int64_t E = g.E;
-  const int64_t n = 2 * E;
-  if (n >= ((int64_t)1 << 32)) throw Error(LVG_ERR_CAPACITY, "doubled edge list exceeds 2^32-1 entries");
+  if (2 * E >= ((int64_t)1 << 32)) throw Error(LVG_ERR_CAPACITY, "doubled edge list exceeds 2^32-1 entries");
   // per-vertex arrays (low end, level lifetime)
-  const bool pre = g.pre && g.pre->valid;
   g.kfrac = a.lo_n<double>(V);
-  double* d_m = a.lo_n<double>(1);
-  if (pre) {   // level 0 built while it streamed in (stream_load_level0)
+  HiScope outer(a);
+  uint32_t* small = a.hi_n<uint32_t>(kNumBuckets + 3);   // class starts, entries, flags: read together
+  uint32_t* notint = small + kNumBuckets + 1;            // [0] a weight, [1] a degree
+  LVG_CUDA(cudaMemsetAsync(notint, 0, 2 * sizeof(uint32_t), s));
+  bool integral = true;   // as far as the build tells
+  if (g.pre && g.pre->valid) {   // written by the upload or the coarsening
     g.off = g.pre->off;
     g.col = g.pre->col;
     g.cw = g.pre->cw;
@@ -2167,9 +2230,15 @@ void build_level(LevelGraph& g, const Tuning& t, Arena& a, cudaStream_t s) {
     g.loopw = g.pre->loopw;
     g.has_loop = g.pre->has_loop;
     g.nnz = g.pre->nnz;
-    LVG_CUDA(cudaMemcpyAsync(d_m, &g.pre->m, sizeof(double), cudaMemcpyHostToDevice, s));
+    g.m = g.pre->m;
+    integral = g.pre->integral;
     g.sorted_symmetric = true;
   } else {
+    ListFacts own;
+    if (!facts) {
+      own = list_facts(g.src, g.dst, g.w, E, V, a, s);
+      facts = &own;
+    }
     g.off = a.lo_n<int64_t>(V + 1);
     g.k = a.lo_n<double>(V);
     g.loopw = a.lo_n<float>(V);
@@ -2177,79 +2246,47 @@ void build_level(LevelGraph& g, const Tuning& t, Arena& a, cudaStream_t s) {
     LVG_CUDA(cudaMemsetAsync(g.k, 0, sizeof(double) * std::max<int32_t>(V, 1), s));
     LVG_CUDA(cudaMemsetAsync(g.loopw, 0, sizeof(float) * std::max<int32_t>(V, 1), s));
     LVG_CUDA(cudaMemsetAsync(g.has_loop, 0, std::max<int32_t>(V, 1), s));
-    tree_sum_f32(g.w, E, d_m, a, s);                                  // NeighbourCompute.cu:46
-    g.sorted_symmetric = E > 0 && build_csr_fast(g, a, s);
-  }
-  if (!g.sorted_symmetric) {
-    HiScope hs(a);
-    const int B = std::max(1, bits_for(V));
-    uint64_t* k0 = a.hi_n<uint64_t>(n);
-    float* v0 = a.hi_n<float>(n);
-    uint64_t* k1 = a.hi_n<uint64_t>(n);
-    float* v1 = a.hi_n<float>(n);
-    uint32_t* head = a.hi_n<uint32_t>(n + 1);
-    uint32_t* pos = a.hi_n<uint32_t>(n + 1);
-    int64_t* rowcnt = a.hi_n<int64_t>(V + 1);
-    LVG_CUDA(cudaMemsetAsync(rowcnt, 0, sizeof(int64_t) * (V + 1), s));
-    if (E > 0) {
-      make_keys_kernel<<<sm_grid(E, kThreads), kThreads, 0, s>>>(g.src, g.dst, g.w, E, B, k0, v0);
-      LVG_LAUNCH();
-    }
-    int which = radix_sort_pairs(k0, v0, k1, v1, n, 2 * B, a, s);   // NeighbourCompute.cu:82
-    uint64_t* keys = which ? k1 : k0;
-    float* vals = which ? v1 : v0;
-    if (n > 0) {
-      csr_scan_kernel<<<grid_for(n, kThreads), kThreads, 0, s>>>(keys, vals, n, B, head, rowcnt, g.k, g.loopw,
-                                                                  g.has_loop);
-      LVG_LAUNCH();
-    }
-    scan_u32(head, pos, n, a, s);
-    scan_i64(rowcnt, g.off, V, a, s);
-    int64_t nnz = 0;
-    LVG_CUDA(cudaMemcpyAsync(&nnz, g.off + V, sizeof nnz, cudaMemcpyDeviceToHost, s));
-    LVG_CUDA(cudaStreamSynchronize(s));
-    g.nnz = nnz;
-    // exact CSR on the low end
-    g.col = a.lo_n<int32_t>(nnz);
-    g.cw = a.lo_n<float>(nnz);
-    double* wsum = a.hi_n<double>(nnz);
-    LVG_CUDA(cudaMemsetAsync(wsum, 0, sizeof(double) * std::max<int64_t>(nnz, 1), s));
-    if (n > 0) {
-      csr_emit_kernel<<<grid_for(n, kThreads), kThreads, 0, s>>>(keys, vals, n, B, pos, head, g.col, wsum);
-      LVG_LAUNCH();
-    }
-    if (nnz > 0) {
-      to_float_kernel<<<sm_grid(nnz, kThreads), kThreads, 0, s>>>(wsum, g.cw, nnz);
-      LVG_LAUNCH();
+    g.m = facts->m;
+    g.sorted_symmetric = facts->sorted_symmetric;
+    if (g.sorted_symmetric) {
+      build_csr_fast(g, *facts, a, s);
+      integral = facts->integral;
+    } else {
+      build_csr_sorted(g, a, s);
+      if (g.nnz > 0) {
+        int_weights_kernel<<<sm_grid(g.nnz, kThreads), kThreads, 0, s>>>(g.cw, g.nnz, notint);
+        LVG_LAUNCH();
+      }
     }
   }
-  LVG_CUDA(cudaMemcpyAsync(&g.m, d_m, sizeof(double), cudaMemcpyDeviceToHost, s));
-  LVG_CUDA(cudaStreamSynchronize(s));
   // degree buckets (stable by vertex index)
   g.blist = a.lo_n<int32_t>(V);
   {
     HiScope hs(a);
-    int64_t nblk = (V + 2047) / 2048;
-    if (nblk == 0) nblk = 1;
+    const int64_t nblk = std::max<int64_t>(1, ((int64_t)V + 2047) / 2048);
     uint32_t* cnt = a.hi_n<uint32_t>(kNumBuckets * nblk + 1);
-    bucket_count_kernel<<<(unsigned)nblk, kThreads, 0, s>>>(V, g.off, g.k, t.warp_max, t.block_max, cnt, nblk);
+    bucket_count_kernel<<<(unsigned)nblk, kThreads, 0, s>>>(V, g.off, g.k, t.warp_max, t.block_max, cnt, nblk,
+                                                            notint + 1);
     LVG_LAUNCH();
-    std::vector<uint32_t> host_cnt(kNumBuckets * nblk);
-    LVG_CUDA(cudaMemcpyAsync(host_cnt.data(), cnt, sizeof(uint32_t) * kNumBuckets * nblk, cudaMemcpyDeviceToHost,
-                             s));
     scan_u32(cnt, cnt, kNumBuckets * nblk, a, s);
+    bucket_starts_kernel<<<1, 32, 0, s>>>(cnt, nblk, small);
+    LVG_LAUNCH();
     bucket_scatter_kernel<<<(unsigned)nblk, kThreads, 0, s>>>(V, g.off, g.k, t.warp_max, t.block_max, cnt, nblk,
                                                               g.blist);
     LVG_LAUNCH();
-    LVG_CUDA(cudaStreamSynchronize(s));
-    int64_t acc = 0;
-    for (int b = 0; b < kNumBuckets; ++b) {
-      int64_t c = 0;
-      for (int64_t j = 0; j < nblk; ++j) c += host_cnt[b * nblk + j];
-      g.nbucket[b] = c;
-      g.bstart[b] = acc;
-      acc += c;
+    // k/2m while the class sizes come back
+    if (V > 0) {
+      kfrac_kernel<<<sm_grid(V, kThreads), kThreads, 0, s>>>(V, g.k, g.m, g.gm, g.vgid, g.kfrac);
+      LVG_LAUNCH();
     }
+    Fetch f(a, s);
+    const uint32_t* h = f.add(small, kNumBuckets + 3);
+    f.wait();
+    for (int b = 0; b < kNumBuckets; ++b) {
+      g.bstart[b] = h[b];
+      g.nbucket[b] = (int64_t)h[b + 1] - h[b];
+    }
+    g.int_acc = integral && h[kNumBuckets + 1] == 0 && h[kNumBuckets + 2] == 0;
   }
   // sliced-ELL copies of the degree classes up to 32
   {
@@ -2271,11 +2308,7 @@ void build_level(LevelGraph& g, const Tuning& t, Arena& a, cudaStream_t s) {
       LVG_LAUNCH();
     }
   }
-  // k/2m and the class-ordered vertex facts of the thread kernels
-  if (V > 0) {
-    kfrac_kernel<<<sm_grid(V, kThreads), kThreads, 0, s>>>(V, g.k, g.m, g.gm, g.vgid, g.kfrac);
-    LVG_LAUNCH();
-  }
+  // the class-ordered vertex facts of the thread kernels
   {
     int64_t nitems = g.bstart[kB32] + g.nbucket[kB32] - g.bstart[kB4];
     g.ell_info = a.lo_n<VInfo>(nitems);
@@ -2285,36 +2318,6 @@ void build_level(LevelGraph& g, const Tuning& t, Arena& a, cudaStream_t s) {
       LVG_LAUNCH();
     }
   }
-  // tiles of the small-degree bucket
-  g.ntiles = 0;
-  const int64_t n0 = g.nbucket[kBTile];
-  const int32_t* tlist = g.blist + g.bstart[kBTile];
-  g.tile_start = a.lo_n<int32_t>(n0 + 2);
-  if (n0 > 0) {
-    HiScope hs(a);
-    int64_t* cum = a.hi_n<int64_t>(n0 + 1);
-    tile_cost_kernel<<<sm_grid(n0, kThreads), kThreads, 0, s>>>(tlist, n0, g.off, cum);
-    LVG_LAUNCH();
-    scan_i64(cum, cum, n0, a, s);
-    tile_start_kernel<<<sm_grid(n0, kThreads), kThreads, 0, s>>>(cum, n0, g.tile_start);
-    LVG_LAUNCH();
-    int64_t last = 0;
-    LVG_CUDA(cudaMemcpyAsync(&last, cum + n0 - 1, sizeof last, cudaMemcpyDeviceToHost, s));
-    LVG_CUDA(cudaStreamSynchronize(s));
-    g.ntiles = last / kTileCost + 1;
-  }
-  {
-    HiScope hs(a);
-    uint32_t* notint = a.hi_n<uint32_t>(1);
-    LVG_CUDA(cudaMemsetAsync(notint, 0, sizeof(uint32_t), s));
-    int_weights_kernel<<<sm_grid(std::max<int64_t>(g.nnz, V), kThreads), kThreads, 0, s>>>(g.cw, g.nnz, g.k, V,
-                                                                                          notint);
-    LVG_LAUNCH();
-    uint32_t h = 0;
-    LVG_CUDA(cudaMemcpyAsync(&h, notint, sizeof h, cudaMemcpyDeviceToHost, s));
-    LVG_CUDA(cudaStreamSynchronize(s));
-    g.int_acc = h == 0;
-  }
   // the first pass gathers a neighbour's singleton total k as int32 when exact
   g.k32 = nullptr;
   if (g.int_acc && V > 0) {
@@ -2322,95 +2325,57 @@ void build_level(LevelGraph& g, const Tuning& t, Arena& a, cudaStream_t s) {
     k32_kernel<<<sm_grid(V, kThreads), kThreads, 0, s>>>(V, g.k, g.k32);
     LVG_LAUNCH();
   }
-  // hubs: chunks of kHubChunk entries and ~kHubBucketTarget entries per bucket
+  // Rows longer than 32: tiles of the small-degree bucket, warp chunks of the
+  // first pass, the hubs' extents; their sizes are read with one wait.
+  const int64_t n0 = g.nbucket[kBTile];
+  const int32_t* tlist = g.blist + g.bstart[kBTile];
+  const int64_t nl = g.nbucket[kBTile] + g.nbucket[kBBlock] + g.nbucket[kBHub];
+  const int64_t nhub = g.nbucket[kBHub];
+  g.ntiles = 0;
   g.nchunk = 0;
   g.nhub_bucket = 0;
-  const int64_t nhub = g.nbucket[kBHub];
-  if (nhub > 0) {
-    const int32_t* hubs = g.blist + g.bstart[kBHub];
+  g.sp_nchunk = 0;
+  g.sp_nmulti = 0;
+  g.tile_start = a.lo_n<int32_t>(n0 + 2);
+  if (nl > 0) {
+    HiScope hs(a);
+    Fetch f(a, s);
+    const int64_t* h_last = nullptr;
+    if (n0 > 0) {
+      int64_t* cum = a.hi_n<int64_t>(n0 + 1);
+      tile_cost_kernel<<<sm_grid(n0, kThreads), kThreads, 0, s>>>(tlist, n0, g.off, cum);
+      LVG_LAUNCH();
+      scan_i64(cum, cum, n0, a, s);
+      tile_start_kernel<<<sm_grid(n0, kThreads), kThreads, 0, s>>>(cum, n0, g.tile_start);
+      LVG_LAUNCH();
+      h_last = f.add(cum + n0 - 1);
+    }
+    uint32_t* cnt = a.hi_n<uint32_t>(nl + 1);
+    uint32_t* mul = a.hi_n<uint32_t>(nl + 1);
+    sp_count_kernel<<<sm_grid(nl, kThreads), kThreads, 0, s>>>(tlist, nl, g.off, cnt, mul);
+    LVG_LAUNCH();
+    scan_u32(cnt, cnt, nl, a, s);
+    scan_u32(mul, mul, nl, a, s);
+    const uint32_t* h_cnt = f.add(cnt + nl);
+    const uint32_t* h_mul = f.add(mul + nl);
     std::vector<int64_t> be(2 * nhub);
-    {
-      HiScope hs(a);
+    if (nhub > 0) {
+      const int32_t* hubs = g.blist + g.bstart[kBHub];
       int64_t* d_be = a.hi_n<int64_t>(2 * nhub);
       hub_info_kernel<<<grid_for(nhub, kThreads), kThreads, 0, s>>>(hubs, nhub, g.off, d_be);
       LVG_LAUNCH();
       LVG_CUDA(cudaMemcpyAsync(be.data(), d_be, sizeof(int64_t) * 2 * nhub, cudaMemcpyDeviceToHost, s));
-      LVG_CUDA(cudaStreamSynchronize(s));
     }
-    std::vector<int32_t> plog(nhub), cb0(nhub + 1), bb0(nhub + 1), chub, bhub;
-    std::vector<int64_t> cbeg, cbo, cstg;
-    int64_t noff = 0, nstg = 0;
-    for (int64_t h = 0; h < nhub; ++h) {
-      const int64_t d = be[2 * h + 1] - be[2 * h];
-      int l = 0;
-      while (l < kHubMaxBucketsLog && ((int64_t)kHubBucketTarget << l) < d) ++l;
-      plog[h] = l;
-      cb0[h] = (int32_t)chub.size();
-      bb0[h] = (int32_t)bhub.size();
-      for (int64_t b = be[2 * h]; b < be[2 * h + 1]; b += kHubChunk) {
-        chub.push_back((int32_t)h);
-        cbeg.push_back(b);
-        cbo.push_back(noff);
-        cstg.push_back(nstg + (b - be[2 * h]));
-        noff += ((int64_t)1 << l) + 1;
-      }
-      nstg += d;
-      bhub.insert(bhub.end(), (size_t)1 << l, (int32_t)h);
-    }
-    cb0[nhub] = (int32_t)chub.size();
-    bb0[nhub] = (int32_t)bhub.size();
-    g.nchunk = (int64_t)chub.size();
-    g.nhub_bucket = (int64_t)bhub.size();
-    g.chunk_hub = a.lo_n<int32_t>(g.nchunk);
-    g.chunk_beg = a.lo_n<int64_t>(g.nchunk);
-    g.chunk_cbo = a.lo_n<int64_t>(g.nchunk);
-    g.chunk_stg = a.lo_n<int64_t>(g.nchunk);
-    g.hub_plog = a.lo_n<int32_t>(nhub);
-    g.hub_cb0 = a.lo_n<int32_t>(nhub + 1);
-    g.hub_bb0 = a.lo_n<int32_t>(nhub + 1);
-    g.bucket_hub = a.lo_n<int32_t>(g.nhub_bucket);
-    g.cb_off = a.lo_n<uint16_t>(noff);
-    g.stage = a.lo_n<unsigned long long>(nstg);
-    g.hub_sawown = a.lo_n<uint32_t>(nhub);
-    g.hub_part = a.lo_n<HubPartial>(g.nhub_bucket);
-    LVG_CUDA(cudaMemcpyAsync(g.chunk_hub, chub.data(), sizeof(int32_t) * g.nchunk, cudaMemcpyHostToDevice, s));
-    LVG_CUDA(cudaMemcpyAsync(g.chunk_beg, cbeg.data(), sizeof(int64_t) * g.nchunk, cudaMemcpyHostToDevice, s));
-    LVG_CUDA(cudaMemcpyAsync(g.chunk_cbo, cbo.data(), sizeof(int64_t) * g.nchunk, cudaMemcpyHostToDevice, s));
-    LVG_CUDA(cudaMemcpyAsync(g.chunk_stg, cstg.data(), sizeof(int64_t) * g.nchunk, cudaMemcpyHostToDevice, s));
-    LVG_CUDA(cudaMemcpyAsync(g.hub_plog, plog.data(), sizeof(int32_t) * nhub, cudaMemcpyHostToDevice, s));
-    LVG_CUDA(cudaMemcpyAsync(g.hub_cb0, cb0.data(), sizeof(int32_t) * (nhub + 1), cudaMemcpyHostToDevice, s));
-    LVG_CUDA(cudaMemcpyAsync(g.hub_bb0, bb0.data(), sizeof(int32_t) * (nhub + 1), cudaMemcpyHostToDevice, s));
-    LVG_CUDA(cudaMemcpyAsync(g.bucket_hub, bhub.data(), sizeof(int32_t) * g.nhub_bucket, cudaMemcpyHostToDevice,
-                             s));
-    LVG_CUDA(cudaMemsetAsync(g.hub_sawown, 0, sizeof(uint32_t) * nhub, s));
-    LVG_CUDA(cudaStreamSynchronize(s));  // host vectors go out of scope
-  }
-  // singleton first pass: warp chunks of the rows longer than 32
-  g.sp_nchunk = 0;
-  g.sp_nmulti = 0;
-  {
-    const int64_t nl = g.nbucket[kBTile] + g.nbucket[kBBlock] + g.nbucket[kBHub];
-    const int32_t* llist = g.blist + g.bstart[kBTile];
-    if (nl > 0) {
-      HiScope hs(a);
-      uint32_t* cnt = a.hi_n<uint32_t>(nl + 1);
-      uint32_t* mul = a.hi_n<uint32_t>(nl + 1);
-      sp_count_kernel<<<sm_grid(nl, kThreads), kThreads, 0, s>>>(llist, nl, g.off, cnt, mul);
-      LVG_LAUNCH();
-      scan_u32(cnt, cnt, nl, a, s);
-      scan_u32(mul, mul, nl, a, s);
-      uint32_t tot[2] = {0, 0};
-      LVG_CUDA(cudaMemcpyAsync(&tot[0], cnt + nl, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-      LVG_CUDA(cudaMemcpyAsync(&tot[1], mul + nl, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-      LVG_CUDA(cudaStreamSynchronize(s));
-      g.sp_nchunk = tot[0];
-      g.sp_nmulti = tot[1];
-      g.sp_chunk = a.lo_n<int2>(g.sp_nchunk);
-      g.sp_multi = a.lo_n<int2>(g.sp_nmulti);
-      g.sp_part = a.lo_n<HubPartial>(g.sp_nmulti > 0 ? g.sp_nchunk : 0);
-      sp_fill_kernel<<<sm_grid(nl, kThreads), kThreads, 0, s>>>(llist, nl, g.off, cnt, mul, g.sp_chunk, g.sp_multi);
-      LVG_LAUNCH();
-    }
+    f.wait();
+    if (n0 > 0) g.ntiles = *h_last / kTileCost + 1;
+    g.sp_nchunk = *h_cnt;
+    g.sp_nmulti = *h_mul;
+    g.sp_chunk = a.lo_n<int2>(g.sp_nchunk);
+    g.sp_multi = a.lo_n<int2>(g.sp_nmulti);
+    g.sp_part = a.lo_n<HubPartial>(g.sp_nmulti > 0 ? g.sp_nchunk : 0);
+    sp_fill_kernel<<<sm_grid(nl, kThreads), kThreads, 0, s>>>(tlist, nl, g.off, cnt, mul, g.sp_chunk, g.sp_multi);
+    LVG_LAUNCH();
+    if (nhub > 0) build_hubs(g, be, a, s);
   }
   g.block_max = t.block_max;
   set_move_attributes();
@@ -2766,6 +2731,7 @@ static void move_down(const CoarseList& hi, const PreCsr& hi_csr, int32_t C, siz
   down(next.has_loop, hi_csr.has_loop, C);
   next.m = hi_csr.m;
   next.nnz = hi_csr.nnz;
+  next.integral = hi_csr.integral;
   next.valid = true;
 }
 

@@ -44,6 +44,7 @@ struct PreCsr {
   uint8_t* has_loop = nullptr;
   double m = 0.0;
   int64_t nnz = 0;
+  bool integral = false;   // every weight of cw integral
 };
 
 // One level of the graph on the device.
@@ -148,18 +149,22 @@ struct Tuning {
 // Coarsening methods of a level (lvg_config.coarsen_mode).
 enum : int32_t { kCoarsenAuto = 0, kCoarsenChunks = 1, kCoarsenTransposed = 2, kCoarsenSort = 3 };
 
-// Validate an input list on the device: ids in range, weights finite >= 0.
-bool validate_edges(const int32_t* src, const int32_t* dst, const float* w, int64_t E, int32_t V,
-                    Arena& a, cudaStream_t s);
-
-// The same check with the list's form: *sorted_symmetric when it is strictly
-// sorted by (src, dst) and symmetric with bitwise-equal weights.
-bool check_edges(const int32_t* src, const int32_t* dst, const float* w, int64_t E, int32_t V, bool* sorted_symmetric,
-                 Arena& a, cudaStream_t s);
+// What one pass over a list tells (list_facts).
+struct ListFacts {
+  bool ok = true;                 // ids in range, weights finite and >= 0
+  bool sorted_symmetric = false;  // strictly sorted by (src, dst), symmetric with bitwise-equal weights
+  bool integral = false;          // every merged weight 2w integral
+  int64_t nonloop = 0;            // entries that are not self loops
+  double m = 0.0;                 // sum of the weights (fixed tree)
+  uint32_t* pos = nullptr;        // non-loop entries before each 2048-entry block (caller's high scratch)
+};
+ListFacts list_facts(const int32_t* src, const int32_t* dst, const float* w, int64_t E, int32_t V, Arena& a,
+                     cudaStream_t s);
 
 // Build the level CSR, degrees, loops and buckets (NeighbourCompute.cu:42-117,
 // InitKernel.cu:245-339).  Level arrays go to the arena's low end.
-void build_level(LevelGraph& g, const Tuning& t, Arena& a, cudaStream_t s);
+// facts: of the list, when its caller has them (else they are taken here).
+void build_level(LevelGraph& g, const Tuning& t, Arena& a, cudaStream_t s, const ListFacts* facts = nullptr);
 // Copies a host list into (src, dst, w) in chunks of `chunk` entries on
 // `copy` while kernels on `s` check each arrived chunk (ids in range, finite
 // non-negative weights, strict order, symmetry fingerprints) and build the

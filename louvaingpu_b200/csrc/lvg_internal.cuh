@@ -39,7 +39,9 @@ void count_launch();
 struct Arena {
   char* base = nullptr;
   size_t cap = 0, lo = 0, hi = 0, peak = 0;
+  char* box = nullptr;   // pinned host memory for small reads (Fetch)
   static constexpr size_t kAlign = 256;
+  static constexpr size_t kBox = (size_t)64 << 10;
   void reserve(size_t bytes) {
     bytes = (bytes + ((size_t)2 << 20) - 1) & ~(((size_t)2 << 20) - 1);  // both ends stay 256-aligned
     if (bytes <= cap) { lo = 0; hi = cap; return; }
@@ -50,6 +52,11 @@ struct Arena {
   void release() {
     if (base) cudaFree(base);
     base = nullptr; cap = lo = hi = 0;
+  }
+  void destroy() {
+    release();
+    if (box) cudaFreeHost(box);
+    box = nullptr;
   }
   static size_t up(size_t x) { return (x + kAlign - 1) & ~(kAlign - 1); }
   void* alloc_lo(size_t bytes) {
@@ -84,6 +91,31 @@ struct HiScope {  // releases high-end scratch on scope exit
   explicit HiScope(Arena& ar) : a(ar), mark(ar.hi) {}
   ~HiScope() { a.hi = mark; }
 };
+
+// A few small device values read with one wait: every add() queues a copy
+// into the arena's pinned box, wait() waits for the stream.  (A copy into
+// pageable memory waits for the stream by itself, once per value.)
+struct Fetch {
+  Arena& a;
+  cudaStream_t s;
+  size_t used = 0;
+  Fetch(Arena& ar, cudaStream_t st) : a(ar), s(st) {}
+  template <typename T> const T* add(const T* dev, size_t n = 1) {
+    const size_t bytes = sizeof(T) * n, at = (used + 15) & ~(size_t)15;
+    if (!a.box) LVG_CUDA(cudaMallocHost(&a.box, Arena::kBox));
+    if (at + bytes > Arena::kBox) throw Error(LVG_ERR_CAPACITY, "read-back box too small");
+    LVG_CUDA(cudaMemcpyAsync(a.box + at, dev, bytes, cudaMemcpyDeviceToHost, s));
+    used = at + bytes;
+    return reinterpret_cast<const T*>(a.box + at);
+  }
+  void wait() { LVG_CUDA(cudaStreamSynchronize(s)); }
+};
+template <typename T> T fetch_one(const T* dev, Arena& a, cudaStream_t s) {
+  Fetch f(a, s);
+  const T* h = f.add(dev);
+  f.wait();
+  return *h;
+}
 
 inline int bits_for(int64_t n) {  // bits needed to hold values 0..n-1
   int b = 0;

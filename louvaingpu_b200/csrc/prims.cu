@@ -26,19 +26,53 @@ __device__ __forceinline__ T block_exclusive_scan(T v, T* total) {
   return block_exclusive_scan256<T>(v, total);
 }
 
-template <typename T>
+struct AddOp {
+  template <typename T> static __device__ __forceinline__ T of(T a, T b) { return a + b; }
+};
+struct MaxOp {   // of values >= 0
+  template <typename T> static __device__ __forceinline__ T of(T a, T b) { return a > b ? a : b; }
+};
+
+// Exclusive scan of one value per thread over the block, and its total.
+template <typename Op, typename T>
+__device__ __forceinline__ T block_exclusive_op(T v, T* total) {
+  __shared__ T wsum[8];
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  T inc = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const T u = __shfl_up_sync(full, inc, o);
+    if (lane >= o) inc = Op::of(u, inc);
+  }
+  if (lane == 31) wsum[w] = inc;
+  __syncthreads();
+  T base = T(0), tot = T(0);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    if (k < w) base = Op::of(base, wsum[k]);
+    tot = Op::of(tot, wsum[k]);
+  }
+  *total = tot;
+  __syncthreads();
+  T ex = __shfl_up_sync(full, inc, 1);
+  if (lane == 0) ex = T(0);
+  return Op::of(base, ex);
+}
+
+template <typename Op, typename T>
 __global__ void __launch_bounds__(kScanThreads) scan_reduce_kernel(const T* in, int64_t n, T* bsum) {
-  int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
+  int64_t base = (int64_t)blockIdx.x * kScanTile + threadIdx.x;
   T s = 0;
 #pragma unroll
-  for (int j = 0; j < kScanItems; ++j)
-    if (base + j < n) s += in[base + j];
+  for (int j = 0; j < kScanItems; ++j)   // any order: the block's total alone
+    if (base + j * kScanThreads < n) s = Op::of(s, in[base + j * kScanThreads]);
   T tot;
-  block_exclusive_scan(s, &tot);
+  block_exclusive_op<Op, T>(s, &tot);
   if (threadIdx.x == 0) bsum[blockIdx.x] = tot;
 }
 
-template <typename T>
+template <typename Op, typename T>
 __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const T* in, T* out, int64_t n,
                                                                   const T* bscan) {
   int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
@@ -47,21 +81,21 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const T* in, T
 #pragma unroll
   for (int j = 0; j < kScanItems; ++j) {
     v[j] = base + j < n ? in[base + j] : T(0);
-    s += v[j];
+    s = Op::of(s, v[j]);
   }
   T tot;
-  T pre = block_exclusive_scan(s, &tot);
-  T off = (bscan ? bscan[blockIdx.x] : T(0)) + pre;
+  T pre = block_exclusive_op<Op, T>(s, &tot);
+  const T before = bscan ? bscan[blockIdx.x] : T(0);
+  T off = Op::of(before, pre);
 #pragma unroll
   for (int j = 0; j < kScanItems; ++j) {
     if (base + j < n) out[base + j] = off;
-    off += v[j];
+    off = Op::of(off, v[j]);
   }
-  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0)
-    out[n] = (bscan ? bscan[blockIdx.x] : T(0)) + tot;
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = Op::of(before, tot);
 }
 
-template <typename T>
+template <typename Op, typename T>
 void scan_impl(const T* in, T* out, int64_t n, Arena& a, cudaStream_t s) {
   if (n <= 0) {
     LVG_CUDA(cudaMemsetAsync(out, 0, sizeof(T), s));
@@ -72,12 +106,12 @@ void scan_impl(const T* in, T* out, int64_t n, Arena& a, cudaStream_t s) {
   T* bscan = nullptr;
   if (nb > 1) {
     T* bsum = a.hi_n<T>(nb + 1);
-    scan_reduce_kernel<T><<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, bsum);
+    scan_reduce_kernel<Op, T><<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, bsum);
     LVG_LAUNCH();
-    scan_impl<T>(bsum, bsum, nb, a, s);
+    scan_impl<Op, T>(bsum, bsum, nb, a, s);
     bscan = bsum;
   }
-  scan_apply_kernel<T><<<(unsigned)nb, kScanThreads, 0, s>>>(in, out, n, bscan);
+  scan_apply_kernel<Op, T><<<(unsigned)nb, kScanThreads, 0, s>>>(in, out, n, bscan);
   LVG_LAUNCH();
 }
 
@@ -265,10 +299,13 @@ __global__ void __launch_bounds__(kRsThreads) rs_onesweep_kernel(const uint64_t*
 }  // namespace
 
 void scan_u32(const uint32_t* in, uint32_t* out, int64_t n, Arena& a, cudaStream_t s) {
-  scan_impl<uint32_t>(in, out, n, a, s);
+  scan_impl<AddOp, uint32_t>(in, out, n, a, s);
 }
 void scan_i64(const int64_t* in, int64_t* out, int64_t n, Arena& a, cudaStream_t s) {
-  scan_impl<int64_t>(in, out, n, a, s);
+  scan_impl<AddOp, int64_t>(in, out, n, a, s);
+}
+void scan_max_i64(const int64_t* in, int64_t* out, int64_t n, Arena& a, cudaStream_t s) {
+  scan_impl<MaxOp, int64_t>(in, out, n, a, s);
 }
 
 void tree_sum_f64(const double* x, int64_t n, double* d_out, Arena& a, cudaStream_t s) {

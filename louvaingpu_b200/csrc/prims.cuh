@@ -11,6 +11,9 @@ namespace lvg {
 void scan_u32(const uint32_t* in, uint32_t* out, int64_t n, Arena& a, cudaStream_t s);
 void scan_i64(const int64_t* in, int64_t* out, int64_t n, Arena& a, cudaStream_t s);
 
+// out[0..n] = exclusive running maximum of in[0..n) (values >= 0; 0 first).
+void scan_max_i64(const int64_t* in, int64_t* out, int64_t n, Arena& a, cudaStream_t s);
+
 // Fixed-tree sum (see lvg_internal.cuh) of n doubles or floats into *d_out.
 void tree_sum_f64(const double* x, int64_t n, double* d_out, Arena& a, cudaStream_t s);
 void tree_sum_f32(const float* x, int64_t n, double* d_out, Arena& a, cudaStream_t s);

@@ -48,6 +48,29 @@ __device__ __forceinline__ bool seg_warp_last(K seg, bool valid) {
   return valid && (lane == 31 || !nvalid || nx != seg);
 }
 
+// Runs of equal `seg` in a warp (lanes hold consecutive list entries): the
+// lane's distance from its run's first lane, and whether it is the run's last.
+// Two votes and a shuffle, where a scan that shuffles `seg` along needs one a
+// step: the shuffles are what bounds the scans below.
+__device__ __forceinline__ int run_depth(int32_t seg, bool& last) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int32_t before = __shfl_up_sync(full, seg, 1);
+  const unsigned heads = __ballot_sync(full, lane == 0 || before != seg);
+  last = lane == 31 || ((heads >> (lane + 1)) & 1u);
+  return lane - (31 - __clz(heads & (0xffffffffu >> (31 - lane))));
+}
+
+// Inclusive sum over the lanes of v's run up to this one, from run_depth.
+__device__ __forceinline__ double run_sum(double v, int depth) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double u = __shfl_up_sync(0xffffffffu, v, o);
+    if (o <= depth) v = __dadd_rn(v, u);
+  }
+  return v;
+}
+
 __device__ __forceinline__ uint64_t edge_hash(uint32_t u, uint32_t v, uint32_t wb, uint64_t key) {
   return mix64(mix64((((uint64_t)u << 32) | v) ^ key) + (uint64_t)wb * 0x9E3779B97F4A7C15ull + key);
 }

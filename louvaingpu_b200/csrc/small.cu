@@ -429,19 +429,6 @@ struct List {
 
 __device__ __forceinline__ double merged_w(float w) { return (double)__double2float_rn(__dadd_rn((double)w, (double)w)); }
 
-// Runs of equal `seg` in a warp (lanes hold consecutive list entries): the
-// lane's distance from its run's first lane, and whether it is the run's last.
-// Two votes and a shuffle, where a scan that shuffles `seg` along needs one a
-// step: the shuffles are what bounds the scans below.
-__device__ __forceinline__ int run_depth(int32_t seg, bool& last) {
-  const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  const int32_t before = __shfl_up_sync(full, seg, 1);
-  const unsigned heads = __ballot_sync(full, lane == 0 || before != seg);
-  last = lane == 31 || ((heads >> (lane + 1)) & 1u);
-  return lane - (31 - __clz(heads & (0xffffffffu >> (31 - lane))));
-}
-
 // First pass of a level: every neighbour is its own candidate.
 template <typename X>
 __device__ __forceinline__ void moves_first_body(const List L, int32_t v, int32_t vend, bool last_pass) {
@@ -449,7 +436,7 @@ __device__ __forceinline__ void moves_first_body(const List L, int32_t v, int32_
   auto& S = X::S();
   auto& W = X::W();
   const unsigned full = 0xffffffffu;
-  const int tid = threadIdx.x, lane = tid & 31;
+  const int tid = threadIdx.x;
 #pragma unroll 1
   while (v < vend) {
     const int nv = tile_rows<X>(W.roff, v, vend, Tile<NT>::kInt);
