@@ -12,6 +12,7 @@
 // round-to-nearest intrinsics so it rounds exactly as the CPU oracle does.
 #include <algorithm>
 #include <climits>
+#include <cstring>
 #include <mutex>
 #include <vector>
 
@@ -104,7 +105,7 @@ __global__ void csr_emit_kernel(const uint64_t* keys, const float* vals, int64_t
 // (Seven passes before -- checks, m, order and symmetry, row counts, loop
 // flags and their scan, the CSR, integral weights: 20.1 ms of an R-MAT scale
 // 24 load, 520 M entries; BUILDFIG now.)
-enum : uint32_t { kNotSorted = 1u, kBadEntry = 4u, kNotIntegral = 8u };
+enum : uint32_t { kNotSorted = 1u, kBadEntry = 4u, kNotIntegral = 8u, kNotWhole = 16u };
 constexpr int kListItems = kGroup / kThreads;   // entries per thread
 
 // Order (exact), symmetry, ids and weights, m's group sums, and the non-loop
@@ -117,14 +118,14 @@ constexpr int kListItems = kGroup / kThreads;   // entries per thread
 __global__ void __launch_bounds__(kThreads) list_facts_kernel(const int32_t* src, const int32_t* dst, const float* w,
                                                               int64_t b, int64_t e_end, int32_t V, uint32_t* flags,
                                                               unsigned long long* sums, uint32_t* cnt,
-                                                              double* gpart) {
+                                                              double* gpart) {   // flags[1]: largest weight
   const uint64_t K1 = 0x243F6A8885A308D3ull, K2 = 0x13198A2E03707344ull;
   __shared__ double ws[8];
   __shared__ uint32_t wc[kThreads / 32];
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   uint64_t d1 = 0, d2 = 0;
-  uint32_t f = 0;
+  uint32_t f = 0, top = 0;
   const int64_t ngroups = (e_end - b + kGroup - 1) / kGroup;
   for (int64_t g = blockIdx.x; g < ngroups; g += gridDim.x) {
     const int64_t e0 = b + g * kGroup + threadIdx.x;
@@ -154,6 +155,8 @@ __global__ void __launch_bounds__(kThreads) list_facts_kernel(const int32_t* src
       if (in && e > 0 && !(u[j] > up || (u[j] == up && v[j] > vp))) f |= kNotSorted;
       const float x2 = __fadd_rn(x[j], x[j]);
       if (in && x2 != truncf(x2)) f |= kNotIntegral;
+      if (in && x[j] != truncf(x[j])) f |= kNotWhole;
+      if (ok) top = max(top, __float_as_uint(x[j]));   // (bits of weights >= 0 order as they do)
       if (ok && u[j] != v[j]) {
         const uint64_t key = ((uint64_t)(uint32_t)min(u[j], v[j]) << 32) | (uint32_t)max(u[j], v[j]);
         const uint64_t h1 = mix64((key ^ K1) + (uint64_t)__float_as_uint(x[j]) * 0x9E3779B97F4A7C15ull);
@@ -180,10 +183,12 @@ __global__ void __launch_bounds__(kThreads) list_facts_kernel(const int32_t* src
     d2 += __shfl_down_sync(full, d2, o);
   }
   f = __reduce_or_sync(full, f);
+  top = __reduce_max_sync(full, top);
   if (lane == 0) {
     if (d1) atomicAdd(&sums[0], (unsigned long long)d1);
     if (d2) atomicAdd(&sums[1], (unsigned long long)d2);
     if (f) atomicOr(flags, f);
+    atomicMax(flags + 1, top);
   }
 }
 
@@ -1988,6 +1993,14 @@ void launch_facts(const int32_t* src, const int32_t* dst, const float* w, int64_
 }
 }  // namespace
 
+// The largest weight, in the upper half of the flags word.
+static float weight_of(unsigned long long h) {
+  const uint32_t bits = (uint32_t)(h >> 32);
+  float x;
+  std::memcpy(&x, &bits, sizeof x);
+  return x;
+}
+
 ListFacts list_facts(const int32_t* src, const int32_t* dst, const float* w, int64_t E, int32_t V, Arena& a,
                      cudaStream_t s) {
   ListFacts F;
@@ -1997,7 +2010,7 @@ ListFacts list_facts(const int32_t* src, const int32_t* dst, const float* w, int
   HiScope hs(a);
   double* gpart = a.hi_n<double>(ng);
   double* d_m = a.hi_n<double>(1);
-  unsigned long long* chk = a.hi_n<unsigned long long>(3);   // flags, two fingerprint sums
+  unsigned long long* chk = a.hi_n<unsigned long long>(3);   // flags and largest weight, two fingerprint sums
   LVG_CUDA(cudaMemsetAsync(chk, 0, 3 * sizeof(unsigned long long), s));
   launch_facts(src, dst, w, 0, E, V, chk, F.pos, gpart, s);
   scan_u32(F.pos, F.pos, ng, a, s);
@@ -2010,6 +2023,8 @@ ListFacts list_facts(const int32_t* src, const int32_t* dst, const float* w, int
   F.ok = (h[0] & kBadEntry) == 0;
   F.sorted_symmetric = F.ok && (h[0] & kNotSorted) == 0 && h[1] == 0 && h[2] == 0;
   F.integral = (h[0] & kNotIntegral) == 0;
+  F.whole = (h[0] & kNotWhole) == 0;
+  F.max_w = weight_of(h[0]);
   F.nonloop = *n;
   F.m = *m;
   return F;
@@ -2085,6 +2100,8 @@ bool stream_load_level0(const int32_t* hsrc, const int32_t* hdst, const float* h
     bad = (h[0] & kBadEntry) != 0;
     valid = !bad && (h[0] & kNotSorted) == 0 && h[1] == 0 && h[2] == 0;
     pre.integral = (h[0] & kNotIntegral) == 0;
+    pre.whole = (h[0] & kNotWhole) == 0;
+    pre.max_w = weight_of(h[0]);
     if (valid) {
       scan_max_i64(pre.off, pre.off, V, a, s);   // row ends -> row starts
       pre.nnz = fetch_one(pre.off + V, a, s);
@@ -2232,6 +2249,8 @@ void build_level(LevelGraph& g, const Tuning& t, Arena& a, cudaStream_t s, const
     g.nnz = g.pre->nnz;
     g.m = g.pre->m;
     integral = g.pre->integral;
+    g.whole = g.pre->whole;
+    g.max_w = g.pre->max_w;
     g.sorted_symmetric = true;
   } else {
     ListFacts own;
@@ -2247,6 +2266,8 @@ void build_level(LevelGraph& g, const Tuning& t, Arena& a, cudaStream_t s, const
     LVG_CUDA(cudaMemsetAsync(g.loopw, 0, sizeof(float) * std::max<int32_t>(V, 1), s));
     LVG_CUDA(cudaMemsetAsync(g.has_loop, 0, std::max<int32_t>(V, 1), s));
     g.m = facts->m;
+    g.whole = facts->whole;
+    g.max_w = facts->max_w;
     g.sorted_symmetric = facts->sorted_symmetric;
     if (g.sorted_symmetric) {
       build_csr_fast(g, *facts, a, s);
@@ -2732,6 +2753,8 @@ static void move_down(const CoarseList& hi, const PreCsr& hi_csr, int32_t C, siz
   next.m = hi_csr.m;
   next.nnz = hi_csr.nnz;
   next.integral = hi_csr.integral;
+  next.whole = hi_csr.whole;
+  next.max_w = hi_csr.max_w;
   next.valid = true;
 }
 

@@ -45,6 +45,8 @@ struct PreCsr {
   double m = 0.0;
   int64_t nnz = 0;
   bool integral = false;   // every weight of cw integral
+  bool whole = false;      // every weight of the list integral
+  float max_w = 0.0f;      // largest weight of the list
 };
 
 // One level of the graph on the device.
@@ -64,6 +66,8 @@ struct LevelGraph {
   uint8_t* has_loop = nullptr;
   double m = 0.0;                 // sum of input weights (NeighbourCompute.cu:46)
   bool sorted_symmetric = false;  // CSR built without sorting (list sorted and symmetric)
+  bool whole = false;             // every weight of the list integral
+  float max_w = 0.0f;             // largest weight of the list
   const PreCsr* pre = nullptr;    // level 0 only: CSR built during the upload
   const double* gm = nullptr;     // batched runs: m of each graph (device)
   const int32_t* vgid = nullptr;  // batched runs: graph of each vertex (device)
@@ -154,6 +158,8 @@ struct ListFacts {
   bool ok = true;                 // ids in range, weights finite and >= 0
   bool sorted_symmetric = false;  // strictly sorted by (src, dst), symmetric with bitwise-equal weights
   bool integral = false;          // every merged weight 2w integral
+  bool whole = false;             // every weight integral
+  float max_w = 0.0f;             // largest weight
   int64_t nonloop = 0;            // entries that are not self loops
   double m = 0.0;                 // sum of the weights (fixed tree)
   uint32_t* pos = nullptr;        // non-loop entries before each 2048-entry block (caller's high scratch)
