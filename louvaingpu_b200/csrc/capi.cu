@@ -1310,6 +1310,7 @@ void batch_union(lvg_ctx* c, const BatchInput& in, int32_t* part_out, double* q_
   const size_t base_lo = a.lo;
   std::vector<double> mod(G0, 0.0);
   std::vector<int32_t> levels(G0, 0), comms(G0, 0), status(G0, 0);
+  bool symmetric0 = false;   // of the union list
   BatchLevel L;
   L.act.resize(G0);
   std::iota(L.act.begin(), L.act.end(), 0);
@@ -1340,6 +1341,7 @@ void batch_union(lvg_ctx* c, const BatchInput& in, int32_t* part_out, double* q_
     g.gm = gm;
     g.vgid = vgid;
     build_level(g, c->tune, a, s);
+    if (level == 0) symmetric0 = g.sorted_symmetric;
     CommState& st = c->st;
     alloc_state(g, st, a);
     // commit plan: groups of 2048 communities per graph
@@ -1534,7 +1536,7 @@ void batch_union(lvg_ctx* c, const BatchInput& in, int32_t* part_out, double* q_
     cp.blk_g = bg_d;
     cp.blk_c0 = bc_d;
     cp.gblk0 = gb_d;
-    batch_modularity(src0, dst0, w0, E0, gid0, local0, cp, cg_d, Ctot, G0, q_d, a, s);
+    batch_modularity(src0, dst0, w0, E0, gid0, local0, V0, symmetric0, cp, cg_d, Ctot, G0, q_d, a, s);
     if (q_out) LVG_CUDA(cudaMemcpyAsync(q_out, q_d, sizeof(double) * G0, cudaMemcpyDeviceToHost, s));
     if (scatter) {
       int32_t* from_d = a.hi_n<int32_t>(G0 + 1);

@@ -1847,81 +1847,189 @@ __global__ void run_sum_kernel(const uint64_t* keys, const float* vals, int64_t 
 
 // ------------------------------------------------------------------ modularity
 // Community strength Kc (both endpoints of every entry) and internal weight
-// Ain (2w for entries inside one community).  Few communities: block-private
-// shared-memory sums flushed once per block; many: global atomics.
-constexpr int kNmSmemMax = 4096;
-// Lanes of a warp holding the same key add their values before one atomic:
-// large communities (the last levels have few) would otherwise serialise on a
-// handful of addresses.  Every lane gets its group's sum; the lowest lane of
-// the group adds it.  Lanes with key < 0 take no part.
-__device__ __forceinline__ void warp_group_add(double* arr, int32_t key, double x) {
-  const unsigned full = 0xffffffffu;
-  const unsigned peers = __match_any_sync(full, key);
-  double sum = 0.0;
+// Ain (2w for entries inside one community).
+//
+// The last levels leave a few very large communities, and one global atomic
+// an entry into those few addresses would serialise at the L2.  Each block
+// takes one contiguous range of the list and keeps
+//  - the kNmTop communities most frequent in a sample of its range, in
+//    registers: every lane adds to sums of its own, no atomics;
+//  - the others in a small open-addressing table in shared memory (a community
+//    that finds no slot within a few probes updates the global sums);
+// and flushes both once.  SYM: the list holds (v, u, w) for every (u, v, w)
+// and is sorted by source, so the destination side of Kc equals the source
+// side: an entry adds 2w to its source's community, and the lanes of one row
+// add first by a segmented warp sum.  (Lanes of equal communities used to be
+// gathered by match instructions and 32-lane shuffle loops: 2.84 -> 0.18 ms on
+// 3.9 M entries in any order, 0.42 -> 0.15 ms on the LFR graph of 2^20
+// vertices, 4.5 -> 3.7 ms on R-MAT scale 24, 2.8 -> 0.7 ms on 128 graphs.)
+constexpr int kNmHotLog = 9;        // 512 slots
+constexpr int kNmHot = 1 << kNmHotLog;
+constexpr int kNmHotProbes = 8;
+constexpr int kNmTop = 4;
+constexpr int kNmItems = 4;         // entries per thread in flight
+constexpr int kNmStep = kNmItems * kThreads;
+constexpr int kNmBlocksPerSm = 8;
+
+struct NmSmem {
+  int32_t key[kNmHot];
+  double K[kNmHot], A[kNmHot];
+  uint32_t cnt[kNmHot];
+  double topK[kNmTop], topA[kNmTop];
+  int32_t top[kNmTop];
+  uint32_t best;
+};
+
+__device__ __forceinline__ void nm_count(NmSmem& S, int32_t c) {   // a sampled community
+  uint32_t h = hash_c(c, kNmHotLog);
+  for (int p = 0; p < kNmHotProbes; ++p) {
+    const int32_t prev = atomicCAS(&S.key[h], -1, c);
+    if (prev == -1 || prev == c) { atomicAdd(&S.cnt[h], 1u); return; }
+    h = (h + 1) & (kNmHot - 1);
+  }
+}
+
+struct NmSums {
+  int32_t top[kNmTop];
+  double k[kNmTop], a[kNmTop];
+  __device__ __forceinline__ void add(NmSmem& S, double* Kc, double* Ain, int32_t c, double kin, double ain) {
+    bool done = c < 0;
 #pragma unroll
-  for (int l = 0; l < 32; ++l) {
-    const double v = __shfl_sync(full, x, l);
-    if ((peers >> l) & 1u) sum += v;
+    for (int t = 0; t < kNmTop; ++t) {   // (no early return: the sums stay in registers)
+      const bool hit = c == top[t];
+      k[t] = __dadd_rn(k[t], hit ? kin : 0.0);
+      a[t] = __dadd_rn(a[t], hit ? ain : 0.0);
+      done |= hit;
+    }
+    if (done) return;
+    uint32_t h = hash_c(c, kNmHotLog);
+    for (int p = 0; p < kNmHotProbes; ++p) {
+      int32_t cur = *reinterpret_cast<volatile int32_t*>(&S.key[h]);
+      if (cur == -1) {
+        cur = atomicCAS(&S.key[h], -1, c);
+        if (cur == -1) cur = c;
+      }
+      if (cur == c) {
+        atomicAdd(&S.K[h], kin);
+        if (ain != 0.0) atomicAdd(&S.A[h], ain);
+        return;
+      }
+      h = (h + 1) & (kNmHot - 1);
+    }
+    atomicAdd(&Kc[c], kin);
+    if (ain != 0.0) atomicAdd(&Ain[c], ain);
   }
-  if (key >= 0 && (threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&arr[key], sum);
+};
+
+// Community of a vertex as an accumulation key: -1 (no part in the sums) for
+// an id outside [0, C), which also sets *bad when the caller passes a flag
+// (callers that validated the ids on the host pass none).
+__device__ __forceinline__ int32_t nm_key(int32_t c, int32_t C, uint32_t* bad) {
+  if ((uint32_t)c < (uint32_t)C) return c;
+  if (bad) atomicOr(bad, 1u);
+  return -1;
 }
 
-// Community ids of an entry's endpoints as accumulation keys: -1 (no part in
-// the sums) for a lane past the end, and for an id outside [0, C), which also
-// sets *bad when the caller passes a flag (callers that validated the ids on
-// the host pass none).
-__device__ __forceinline__ void nm_keys(const int32_t* part, const int32_t* src, const int32_t* dst, int64_t e,
-                                        bool ok, int32_t C, uint32_t* bad, int32_t& a, int32_t& b) {
-  a = ok ? part[src[e]] : -1;
-  b = ok ? part[dst[e]] : -1;
-  const bool oob = ok && ((uint32_t)a >= (uint32_t)C || (uint32_t)b >= (uint32_t)C);
-  if (oob) {
-    if (bad) atomicOr(bad, 1u);
-    a = (uint32_t)a < (uint32_t)C ? a : -1;
-    b = (uint32_t)b < (uint32_t)C ? b : -1;
-  }
-}
-
-__global__ void __launch_bounds__(kThreads) nm_accum_smem_kernel(const int32_t* src, const int32_t* dst,
-                                                                 const float* w, int64_t E, const int32_t* part,
-                                                                 int32_t C, double* Kc, double* Ain, uint32_t* bad) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  double* sK = reinterpret_cast<double*>(smem);
-  double* sA = sK + C;
-  for (int c = threadIdx.x; c < 2 * C; c += kThreads) sK[c] = 0.0;
+template <bool SYM>
+__global__ void __launch_bounds__(kThreads) nm_accum_kernel(const int32_t* src, const int32_t* dst, const float* w,
+                                                            int64_t E, const int32_t* part, int32_t C, double* Kc,
+                                                            double* Ain, uint32_t* bad) {
+  __shared__ NmSmem S;
+  const int tid = threadIdx.x, lane = tid & 31;
+  for (int x = tid; x < kNmHot; x += kThreads) { S.key[x] = -1; S.K[x] = 0.0; S.A[x] = 0.0; S.cnt[x] = 0u; }
+  if (tid < kNmTop) { S.topK[tid] = 0.0; S.topA[tid] = 0.0; }
+  if (tid == 0) S.best = 0u;
   __syncthreads();
-  // few communities: lanes with the same community add first (warp-uniform loop)
-  for (int64_t e0 = blockIdx.x * (int64_t)blockDim.x; e0 < E; e0 += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t e = e0 + threadIdx.x;
-    const bool ok = e < E;
-    const double x = ok ? (double)w[e] : 0.0;
-    int32_t a, b;
-    nm_keys(part, src, dst, e, ok, C, bad, a, b);
-    warp_group_add(sK, a, x);
-    warp_group_add(sK, b, x);
-    warp_group_add(sA, (a >= 0 && a == b) ? a : -1, 2.0 * x);
+  const int64_t steps = (E + kNmStep - 1) / kNmStep;
+  const int64_t per = (steps + gridDim.x - 1) / gridDim.x;
+  const int64_t e0 = (int64_t)blockIdx.x * per * kNmStep, e1 = min(E, e0 + per * kNmStep);
+  if (e0 >= E) return;   // whole blocks
+  {   // the range's most frequent communities
+    const int64_t stride = max((int64_t)1, (e1 - e0) / kThreads), e = e0 + tid * stride;
+    if (e < e1) {
+      const int32_t a = part[src[e]], b = SYM ? -1 : part[dst[e]];
+      if ((uint32_t)a < (uint32_t)C) nm_count(S, a);
+      if (!SYM && (uint32_t)b < (uint32_t)C) nm_count(S, b);
+    }
+    __syncthreads();
+    for (int t = 0; t < kNmTop; ++t) {
+      uint32_t m = 0u;
+      for (int x = tid; x < kNmHot; x += kThreads) m = max(m, (S.cnt[x] << kNmHotLog) | (uint32_t)x);
+      m = __reduce_max_sync(0xffffffffu, m);
+      if (lane == 0) atomicMax(&S.best, m);
+      __syncthreads();
+      const uint32_t best = S.best;
+      __syncthreads();
+      if (tid == 0) {
+        const bool hot = (best >> kNmHotLog) >= 4u;   // above 1 in 64 or so
+        S.top[t] = hot ? S.key[best & (kNmHot - 1)] : -2;
+        S.cnt[best & (kNmHot - 1)] = 0u;
+        S.best = 0u;
+      }
+      __syncthreads();
+    }
+    for (int x = tid; x < kNmHot; x += kThreads) S.key[x] = -1;
+    __syncthreads();
+  }
+  NmSums R;
+#pragma unroll
+  for (int t = 0; t < kNmTop; ++t) {
+    R.top[t] = S.top[t];
+    R.k[t] = 0.0;
+    R.a[t] = 0.0;
+  }
+  for (int64_t b0 = e0; b0 < e1; b0 += kNmStep) {
+    int32_t u[kNmItems], a[kNmItems], b[kNmItems];
+    double x[kNmItems];
+#pragma unroll
+    for (int j = 0; j < kNmItems; ++j) {
+      const int64_t e = b0 + j * kThreads + tid;
+      const bool in = e < e1;
+      u[j] = in ? src[e] : -1;
+      b[j] = in ? dst[e] : -1;
+      x[j] = in ? (double)w[e] : 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < kNmItems; ++j) {
+      a[j] = u[j] >= 0 ? nm_key(part[u[j]], C, bad) : -1;
+      b[j] = u[j] >= 0 ? nm_key(part[b[j]], C, bad) : -1;
+    }
+#pragma unroll
+    for (int j = 0; j < kNmItems; ++j) {
+      if (SYM) {
+        bool last;
+        const int depth = run_depth(u[j], last);
+        const double kin = run_sum(2.0 * x[j], depth);
+        const double ain = run_sum(a[j] == b[j] ? 2.0 * x[j] : 0.0, depth);
+        if (last) R.add(S, Kc, Ain, a[j], kin, ain);
+      } else {
+        R.add(S, Kc, Ain, a[j], x[j], a[j] == b[j] ? 2.0 * x[j] : 0.0);
+        R.add(S, Kc, Ain, b[j], x[j], 0.0);
+      }
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < kNmTop; ++t) {
+    double k = R.k[t], a = R.a[t];
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+      k += __shfl_xor_sync(0xffffffffu, k, o);
+      a += __shfl_xor_sync(0xffffffffu, a, o);
+    }
+    if (lane == 0 && k != 0.0) atomicAdd(&S.topK[t], k);
+    if (lane == 0 && a != 0.0) atomicAdd(&S.topA[t], a);
   }
   __syncthreads();
-  for (int c = threadIdx.x; c < C; c += kThreads) {
-    if (sK[c] != 0.0) atomicAdd(&Kc[c], sK[c]);
-    if (sA[c] != 0.0) atomicAdd(&Ain[c], sA[c]);
+  if (tid < kNmTop && S.top[tid] >= 0) {
+    atomicAdd(&Kc[S.top[tid]], S.topK[tid]);
+    if (S.topA[tid] != 0.0) atomicAdd(&Ain[S.top[tid]], S.topA[tid]);
   }
-}
-
-// Kc, Ain of modularity_fp64 for many communities: grid-stride over whole
-// warps, warp-aggregated atomics.
-__global__ void nm_accum_agg_kernel(const int32_t* src, const int32_t* dst, const float* w, int64_t E,
-                                    const int32_t* part, int32_t C, double* Kc, double* Ain, uint32_t* bad) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t e0 = blockIdx.x * (int64_t)blockDim.x; e0 < E; e0 += stride) {
-    const int64_t e = e0 + threadIdx.x;
-    const bool ok = e < E;
-    const double x = ok ? (double)w[e] : 0.0;
-    int32_t a, b;
-    nm_keys(part, src, dst, e, ok, C, bad, a, b);
-    warp_group_add(Kc, a, x);
-    warp_group_add(Kc, b, x);
-    warp_group_add(Ain, (a >= 0 && a == b) ? a : -1, 2.0 * x);
+  for (int x = tid; x < kNmHot; x += kThreads) {
+    const int32_t c = S.key[x];
+    if (c >= 0) {
+      atomicAdd(&Kc[c], S.K[x]);
+      if (S.A[x] != 0.0) atomicAdd(&Ain[c], S.A[x]);
+    }
   }
 }
 
@@ -2835,104 +2943,13 @@ void induce(const LevelGraph& g, const int32_t* part, int32_t C, size_t base_lo,
   LVG_CUDA(cudaStreamSynchronize(s));
 }
 
-// Kc and Ain of a list known to be symmetric (every (u, v, w) has its
-// (v, u, w)) and sorted by source: the destination side of Kc equals the
-// source side, so each entry adds 2w to its source's community only, and 2w
-// to Ain when both ends share a community.  Lanes holding entries of one
-// source row add them by a segmented warp scan; the last lane of each row
-// piece makes one atomic update of each sum -- a few updates per row instead
-// of one per entry, and no shuffle loop over all 32 lanes.
-//
-// The row pieces then add into a small block-private table of communities in
-// shared memory (open addressing, a few probes; a community that finds no
-// slot adds to the global sums directly), flushed once per block.  The last
-// levels leave a few very large communities, and one global atomic per row
-// piece into those few addresses would serialise at the L2: with the table
-// each block makes one global update per large community.  Each block takes
-// one contiguous range of the list (whole 256-entry steps, so every warp
-// stays converged), whose rows meet the same large communities again and
-// again.
-constexpr int kNmHotLog = 9;        // 512 slots: 10 KB, eight blocks per SM
-constexpr int kNmHot = 1 << kNmHotLog;
-constexpr int kNmHotProbes = 8;
-constexpr int kNmSymBlocksPerSm = 8;
-
-__device__ __forceinline__ void nm_hot_add(int32_t* hk, double* hK, double* hA, double* Kc, double* Ain, int32_t a,
-                                           double kin, double ain) {
-  uint32_t h = hash_c(a, kNmHotLog);
-  for (int p = 0; p < kNmHotProbes; ++p) {
-    const int32_t prev = atomicCAS(&hk[h], -1, a);
-    if (prev == -1 || prev == a) {
-      atomicAdd(&hK[h], kin);
-      if (ain != 0.0) atomicAdd(&hA[h], ain);
-      return;
-    }
-    h = (h + 1) & (kNmHot - 1);
-  }
-  atomicAdd(&Kc[a], kin);
-  if (ain != 0.0) atomicAdd(&Ain[a], ain);
-}
-
-__global__ void __launch_bounds__(kThreads) nm_accum_sym_kernel(const int32_t* src, const int32_t* dst,
-                                                                const float* w, int64_t E, const int32_t* part,
-                                                                double* Kc, double* Ain) {
-  __shared__ int32_t hk[kNmHot];
-  __shared__ double hK[kNmHot], hA[kNmHot];
-  for (int x = threadIdx.x; x < kNmHot; x += kThreads) { hk[x] = -1; hK[x] = 0.0; hA[x] = 0.0; }
-  __syncthreads();
-  const int64_t steps = (E + kThreads - 1) / kThreads;
-  const int64_t per = (steps + gridDim.x - 1) / gridDim.x;
-  const int64_t s0 = (int64_t)blockIdx.x * per;
-  const int64_t s1 = min(steps, s0 + per);
-  for (int64_t st = s0; st < s1; ++st) {
-    const int64_t e = st * kThreads + threadIdx.x;
-    const bool ok = e < E;
-    const int32_t u = ok ? src[e] : -1;
-    const double x = ok ? 2.0 * (double)w[e] : 0.0;
-    const int32_t a = ok ? part[u] : -1, b = ok ? part[dst[e]] : -1;
-    const double kin = seg_warp_sum<int32_t>(x, u);
-    const double ain = seg_warp_sum<int32_t>(a == b ? x : 0.0, u);
-    if (seg_warp_last<int32_t>(u, ok)) nm_hot_add(hk, hK, hA, Kc, Ain, a, kin, ain);
-  }
-  __syncthreads();
-  for (int x = threadIdx.x; x < kNmHot; x += kThreads) {
-    const int32_t a = hk[x];
-    if (a >= 0) {
-      atomicAdd(&Kc[a], hK[x]);
-      if (hA[x] != 0.0) atomicAdd(&Ain[a], hA[x]);
-    }
-  }
-}
-
-// Raises the dynamic shared memory limit of nm_accum_smem_kernel on the
-// current device to at least `smem` bytes.  The limit only ever grows, under
-// one lock shared by every caller, so a launch never finds it lowered by a
-// smaller request made in between.
-static void nm_smem_attr(size_t smem) {
-  if (smem <= 48 * 1024) return;
-  constexpr int kDevs = 64;
-  static std::mutex mu;
-  static size_t attr[kDevs] = {};
-  int dev = 0;
-  LVG_CUDA(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> lock(mu);
-  if (dev >= 0 && dev < kDevs && smem <= attr[dev]) return;
-  LVG_CUDA(cudaFuncSetAttribute(nm_accum_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  if (dev >= 0 && dev < kDevs) attr[dev] = smem;
-}
-
-// Kc and Ain of every community: shared-memory sums when they fit, else
-// warp-aggregated global atomics.
+// Kc and Ain of every community (zeroed by the caller).
 static void nm_accum(const int32_t* src, const int32_t* dst, const float* w, int64_t E, int32_t C,
-                     const int32_t* part, double* Kc, double* Ain, uint32_t* bad, cudaStream_t s) {
+                     const int32_t* part, double* Kc, double* Ain, bool symmetric, uint32_t* bad, cudaStream_t s) {
   if (E <= 0) return;
-  if (C <= kNmSmemMax) {
-    const size_t smem = sizeof(double) * 2 * (size_t)C;
-    nm_smem_attr(smem);
-    nm_accum_smem_kernel<<<sm_grid(E, kThreads), kThreads, smem, s>>>(src, dst, w, E, part, C, Kc, Ain, bad);
-  } else {
-    nm_accum_agg_kernel<<<sm_grid(E, kThreads), kThreads, 0, s>>>(src, dst, w, E, part, C, Kc, Ain, bad);
-  }
+  const unsigned grid = std::min<unsigned>(grid_for(E, kNmStep), (unsigned)(sm_count() * kNmBlocksPerSm));
+  if (symmetric) nm_accum_kernel<true><<<grid, kThreads, 0, s>>>(src, dst, w, E, part, C, Kc, Ain, bad);
+  else nm_accum_kernel<false><<<grid, kThreads, 0, s>>>(src, dst, w, E, part, C, Kc, Ain, bad);
   LVG_LAUNCH();
 }
 
@@ -2945,21 +2962,12 @@ double modularity_fp64(const int32_t* src, const int32_t* dst, const float* w, i
   double* twoW = a.hi_n<double>(2);
   LVG_CUDA(cudaMemsetAsync(Kc, 0, sizeof(double) * std::max(C, 1), s));
   LVG_CUDA(cudaMemsetAsync(Ain, 0, sizeof(double) * std::max(C, 1), s));
-  if (symmetric && E > 0 && C > kNmSmemMax) {
-    const unsigned grid = std::min<unsigned>(grid_for(E, kThreads), (unsigned)(sm_count() * kNmSymBlocksPerSm));
-    nm_accum_sym_kernel<<<grid, kThreads, 0, s>>>(src, dst, w, E, part, Kc, Ain);
-    LVG_LAUNCH();
-  } else {
-    nm_accum(src, dst, w, E, C, part, Kc, Ain, nullptr, s);   // ids checked on the host
-  }
+  nm_accum(src, dst, w, E, C, part, Kc, Ain, symmetric, nullptr, s);   // ids checked on the host
   tree_sum_f64(Kc, C, twoW, a, s);
   nm_term_kernel<<<sm_grid(C, kThreads), kThreads, 0, s>>>(Kc, Ain, C, twoW, t);
   LVG_LAUNCH();
   tree_sum_f64(t, C, twoW + 1, a, s);
-  double q = 0.0;
-  LVG_CUDA(cudaMemcpyAsync(&q, twoW + 1, sizeof q, cudaMemcpyDeviceToHost, s));
-  LVG_CUDA(cudaStreamSynchronize(s));
-  return q;
+  return fetch_one(twoW + 1, a, s);
 }
 
 // The modularity kernels of modularity_fp64 with every scratch array given by
@@ -2970,7 +2978,7 @@ void modularity_fp64_scratch(const int32_t* src, const int32_t* dst, const float
                              double* twoW_q, uint32_t* bad, cudaStream_t s) {
   LVG_CUDA(cudaMemsetAsync(Kc, 0, sizeof(double) * C, s));
   LVG_CUDA(cudaMemsetAsync(Ain, 0, sizeof(double) * C, s));
-  nm_accum(src, dst, w, E, C, part, Kc, Ain, bad, s);
+  nm_accum(src, dst, w, E, C, part, Kc, Ain, false, bad, s);
   // the fixed tree of tree_sum_f64, partials from the caller
   auto tree = [&](const double* x, double* out) {
     int64_t nb = ((int64_t)C + kGroup - 1) / kGroup;
@@ -3246,27 +3254,11 @@ __global__ void batch_scatter_kernel(const int32_t* local, const int32_t* gid, c
   }
 }
 
-// Newman modularity per graph over its level-0 entries (global community
-// ids coff[g] + local id).
-__global__ void batch_nm_accum_kernel(const int32_t* src, const int32_t* dst, const float* w, int64_t E,
-                                      const int32_t* gid0, const int32_t* local0, const int32_t* coff, double* Kc,
-                                      double* Ain) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t e0 = blockIdx.x * (int64_t)blockDim.x; e0 < E; e0 += stride) {
-    const int64_t e = e0 + threadIdx.x;
-    const bool ok = e < E;
-    double x = 0.0;
-    int32_t a = -1, b = -1;
-    if (ok) {
-      const int32_t g = gid0[src[e]];
-      x = (double)w[e];
-      a = coff[g] + local0[src[e]];
-      b = coff[g] + local0[dst[e]];
-    }
-    warp_group_add(Kc, a, x);
-    warp_group_add(Kc, b, x);
-    warp_group_add(Ain, (ok && a == b) ? a : -1, 2.0 * x);
-  }
+// Communities numbered over all graphs: graph g's start at coff[g].
+__global__ void batch_comm_kernel(const int32_t* gid0, const int32_t* local0, const int32_t* coff, int32_t V,
+                                  int32_t* comm) {
+  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V; v += (int64_t)gridDim.x * blockDim.x)
+    comm[v] = coff[gid0[v]] + local0[v];
 }
 
 // Per-graph fixed-tree sums: block b sums x over communities blk_c0[b] ..
@@ -3486,9 +3478,10 @@ void batch_scatter(const int32_t* local, const int32_t* gid, const int32_t* from
 }
 
 void batch_modularity(const int32_t* src, const int32_t* dst, const float* w, int64_t E, const int32_t* gid0,
-                      const int32_t* local0, const BatchPlan& cp, const int32_t* cg, int32_t Ctot, int32_t G,
-                      double* q, Arena& a, cudaStream_t s) {
+                      const int32_t* local0, int32_t V, bool symmetric, const BatchPlan& cp, const int32_t* cg,
+                      int32_t Ctot, int32_t G, double* q, Arena& a, cudaStream_t s) {
   HiScope hs(a);
+  int32_t* comm = a.hi_n<int32_t>(V);
   double* Kc = a.hi_n<double>(Ctot);
   double* Ain = a.hi_n<double>(Ctot);
   double* t = a.hi_n<double>(Ctot);
@@ -3497,8 +3490,9 @@ void batch_modularity(const int32_t* src, const int32_t* dst, const float* w, in
   LVG_CUDA(cudaMemsetAsync(Kc, 0, sizeof(double) * std::max(Ctot, 1), s));
   LVG_CUDA(cudaMemsetAsync(Ain, 0, sizeof(double) * std::max(Ctot, 1), s));
   if (E > 0) {
-    batch_nm_accum_kernel<<<sm_grid(E, kThreads), kThreads, 0, s>>>(src, dst, w, E, gid0, local0, cp.vbase, Kc, Ain);
+    batch_comm_kernel<<<sm_grid(V, kThreads), kThreads, 0, s>>>(gid0, local0, cp.vbase, V, comm);
     LVG_LAUNCH();
+    nm_accum(src, dst, w, E, Ctot, comm, Kc, Ain, symmetric, nullptr, s);
   }
   if (cp.nblk > 0) {
     batch_group_kernel<<<(unsigned)cp.nblk, kRedThreads, 0, s>>>(Kc, cp.blk_g, cp.blk_c0, cp.vbase, partials);

@@ -326,9 +326,10 @@ void batch_compose(int32_t* local0, const int32_t* gid0, int64_t n, const int32_
 // FP64 Newman modularity of every graph: community ids coff[g] + local0[v]
 // with coff = cp.vbase, cp the 2048-groups of each graph's communities,
 // cg[c] = graph of community c; q[g] on the device, summed on the fixed tree.
+// symmetric: as modularity_fp64's.
 void batch_modularity(const int32_t* src, const int32_t* dst, const float* w, int64_t E, const int32_t* gid0,
-                      const int32_t* local0, const BatchPlan& cp, const int32_t* cg, int32_t Ctot, int32_t G,
-                      double* q, Arena& a, cudaStream_t s);
+                      const int32_t* local0, int32_t V, bool symmetric, const BatchPlan& cp, const int32_t* cg,
+                      int32_t Ctot, int32_t G, double* q, Arena& a, cudaStream_t s);
 
 // out[to_off[g] + i] = local[from_off[g] + i] for the vertices i of graph gid = g.
 void batch_scatter(const int32_t* local, const int32_t* gid, const int32_t* from_off, const int32_t* to_off, int32_t V,
