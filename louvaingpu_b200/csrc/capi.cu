@@ -89,6 +89,8 @@ struct lvg_ctx {
   PreCsr pre0;                    // level-0 CSR built during a chunked host upload
   PreCsr pre_next;                // CSR of the level just coarsened into, written by the coarsening
   cudaStream_t copy_stream = nullptr;   // host-list upload chunks (lvg_load_edges)
+  cudaStream_t small_streams[4] = {};   // small graphs of a batch, beside the others
+  cudaEvent_t small_ev = nullptr;
   std::vector<cudaEvent_t> load_ev;     // one per upload chunk
 };
 
@@ -677,6 +679,9 @@ lvg_status lvg_destroy(lvg_ctx* c) {
   }
   for (cudaEvent_t e : c->load_ev) cudaEventDestroy(e);
   if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
+  for (cudaStream_t st : c->small_streams)
+    if (st) cudaStreamDestroy(st);
+  if (c->small_ev) cudaEventDestroy(c->small_ev);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
   delete c;
   return LVG_OK;
@@ -1562,34 +1567,45 @@ int small_blocks(int64_t E) {
   return E <= 16 * 1024 ? 1 : E <= 48 * 1024 ? 2 : E <= 128 * 1024 ? 4 : 8;
 }
 
-// Runs the small graphs of a batch, each by its own cluster; marks the graphs
-// that are finished, their partitions at part_d + voff[g].  Leaves the arena
-// as it was.  A graph whose list is not in the form small_run takes stays
-// unmarked.
-void batch_small(lvg_ctx* c, const BatchInput& in, int32_t* part_d, std::vector<char>& done, double* q_out,
-                 int32_t* levels_out, int32_t* comms_out, int32_t* status_out) {
+// The small graphs of a batch while they run, each by its own cluster, on
+// streams of their own beside the batch's other work.
+struct SmallBatch {
+  std::vector<int32_t> which;
+  SmallResult* res = nullptr;
+};
+
+// Starts the small graphs; their partitions go to part_d + voff[g].  Their
+// memory stays taken from the arena's high end (the caller's scope).
+SmallBatch batch_small_start(lvg_ctx* c, const BatchInput& in, int32_t* part_d) {
   Arena& a = c->arena;
   cudaStream_t s = c->stream;
-  std::vector<int32_t> which;
+  SmallBatch B;
+  std::vector<int32_t>& which = B.which;
   for (int32_t g = 0; g < in.G; ++g)
     if (small_fits(in.voff[g + 1] - in.voff[g], in.eoff[g + 1] - in.eoff[g], kSmallBatchEntries)) which.push_back(g);
-  if (which.empty()) return;
+  if (which.empty()) return B;
   auto entries = [&](int32_t g) { return in.eoff[g + 1] - in.eoff[g]; };
   std::sort(which.begin(), which.end(), [&](int32_t x, int32_t y) {   // longest first
     return entries(x) != entries(y) ? entries(x) > entries(y) : x < y;
   });
   const int64_t n = (int64_t)which.size();
   size_t lists = 0, work = 0;
+  int64_t others = in.eoff[in.G], other_v = in.voff[in.G];
   for (int32_t g : which) {
     lists += Arena::up(small_list_bytes(entries(g)));
     work += Arena::up(small_work_bytes(in.voff[g + 1] - in.voff[g], entries(g)));
+    others -= entries(g);
+    other_v -= in.voff[g + 1] - in.voff[g];
   }
   const size_t need = lists + work + n * (sizeof(SmallJob) + sizeof(SmallResult)) + 8 * Arena::kAlign;
-  if (a.hi < a.lo || a.hi - a.lo < need) return;   // the union path takes them all
-  HiScope hs(a);
+  const size_t rest = others > 0 ? arena_estimate(other_v, others, true) : 0;
+  if (a.hi < a.lo || a.hi - a.lo < need + rest) {   // the union path takes them all
+    which.clear();
+    return B;
+  }
   char* lp = (char*)a.alloc_hi(lists);
   char* wp = (char*)a.alloc_hi(work);
-  SmallResult* res = a.hi_n<SmallResult>(n);
+  B.res = a.hi_n<SmallResult>(n);
   SmallJob* jobs_d = a.hi_n<SmallJob>(n);
   std::vector<SmallJob> jobs((size_t)n);
   for (int64_t k = 0; k < n; ++k) {
@@ -1606,34 +1622,46 @@ void batch_small(lvg_ctx* c, const BatchInput& in, int32_t* part_d, std::vector<
     lp += Arena::up(small_list_bytes(J.E));
     wp += Arena::up(small_work_bytes(J.V, J.E));
     J.comp = part_d + in.voff[g];
-    J.res = res + k;
+    J.res = B.res + k;
     J.check = 1;
     J.want_q = 1;
   }
+  if (!c->small_ev) {
+    for (cudaStream_t& st : c->small_streams) LVG_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    LVG_CUDA(cudaEventCreateWithFlags(&c->small_ev, cudaEventDisableTiming));
+  }
   LVG_CUDA(cudaMemcpyAsync(jobs_d, jobs.data(), sizeof(SmallJob) * n, cudaMemcpyHostToDevice, s));
-  LVG_CUDA(cudaMemsetAsync(res, 0, sizeof(SmallResult) * n, s));
+  LVG_CUDA(cudaMemsetAsync(B.res, 0, sizeof(SmallResult) * n, s));
+  LVG_CUDA(cudaEventRecord(c->small_ev, s));
   const SmallCfg cfg{c->cfg.pass_min_gain, c->cfg.level_min_gain, c->cfg.max_passes, c->cfg.max_levels};
-  // one launch per cluster size, side by side
-  LVG_CUDA(cudaEventRecord(c->side.fork, s));
-  for (int k = 0; k < 3; ++k) LVG_CUDA(cudaStreamWaitEvent(c->side.side[k], c->side.fork, 0));
-  const cudaStream_t streams[4] = {s, c->side.side[0], c->side.side[1], c->side.side[2]};
   int slot = 0;
-  for (int64_t k0 = 0; k0 < n;) {
+  for (int64_t k0 = 0; k0 < n;) {   // one launch per cluster size, side by side
     const int K = small_blocks(jobs[k0].E);
     int64_t k1 = k0;
     while (k1 < n && small_blocks(jobs[k1].E) == K) ++k1;
-    small_run(jobs_d + k0, (int)(k1 - k0), K, cfg, streams[slot++ & 3]);
+    cudaStream_t st = c->small_streams[slot++ & 3];
+    LVG_CUDA(cudaStreamWaitEvent(st, c->small_ev, 0));
+    small_run(jobs_d + k0, (int)(k1 - k0), K, cfg, st);
     k0 = k1;
   }
-  for (int k = 0; k < 3; ++k) {
-    LVG_CUDA(cudaEventRecord(c->side.join[k], c->side.side[k]));
-    LVG_CUDA(cudaStreamWaitEvent(s, c->side.join[k], 0));
+  return B;
+}
+
+// Waits for the small graphs and marks those that are finished; one whose list
+// is not in the form small_run takes stays unmarked.
+void batch_small_finish(lvg_ctx* c, const SmallBatch& B, std::vector<char>& done, double* q_out,
+                        int32_t* levels_out, int32_t* comms_out, int32_t* status_out) {
+  cudaStream_t s = c->stream;
+  for (cudaStream_t st : c->small_streams) {
+    LVG_CUDA(cudaEventRecord(c->small_ev, st));
+    LVG_CUDA(cudaStreamWaitEvent(s, c->small_ev, 0));
   }
-  std::vector<SmallResult> o((size_t)n);
-  LVG_CUDA(cudaMemcpyAsync(o.data(), res, sizeof(SmallResult) * n, cudaMemcpyDeviceToHost, s));
+  const size_t n = B.which.size();
+  std::vector<SmallResult> o(n);
+  LVG_CUDA(cudaMemcpyAsync(o.data(), B.res, sizeof(SmallResult) * n, cudaMemcpyDeviceToHost, s));
   sync(c);
-  for (int64_t k = 0; k < n; ++k) {
-    const int32_t g = which[k];
+  for (size_t k = 0; k < n; ++k) {
+    const int32_t g = B.which[k];
     require(!o[k].bad, LVG_ERR_INVALID_ARG,
             "edge list has a vertex id out of its graph or a negative / non-finite weight");
     if (o[k].open || !o[k].finished) continue;
@@ -1642,6 +1670,41 @@ void batch_small(lvg_ctx* c, const BatchInput& in, int32_t* part_d, std::vector<
     if (levels_out) levels_out[g] = o[k].n_levels;
     if (comms_out) comms_out[g] = o[k].n_comms;
     if (status_out) status_out[g] = o[k].status;
+  }
+}
+
+// The graphs of `in` not marked done, as a batch of their own.
+void batch_rest(lvg_ctx* c, const BatchInput& in, std::vector<char>& done, const std::vector<char>& skip,
+                int32_t* part_d, double* q_out, int32_t* levels_out, int32_t* comms_out, int32_t* status_out) {
+  std::vector<int32_t> rest, rvoff(1, 0), to;
+  std::vector<int64_t> reoff(1, 0);
+  BatchInput sub;
+  for (int32_t g = 0; g < in.G; ++g) {
+    if (done[g] || skip[g]) continue;
+    rest.push_back(g);
+    to.push_back(in.voff[g]);
+    rvoff.push_back(rvoff.back() + in.voff[g + 1] - in.voff[g]);
+    reoff.push_back(reoff.back() + in.eoff[g + 1] - in.eoff[g]);
+    sub.src.push_back(in.src[g]);
+    sub.dst.push_back(in.dst[g]);
+    sub.w.push_back(in.w[g]);
+  }
+  if (rest.empty()) return;
+  sub.G = (int32_t)rest.size();
+  sub.eoff = reoff.data();
+  sub.voff = rvoff.data();
+  std::vector<double> q(rest.size());
+  std::vector<int32_t> lev(rest.size()), com(rest.size()), stat(rest.size());
+  const size_t lo0 = c->arena.lo;
+  batch_union(c, sub, nullptr, q.data(), lev.data(), com.data(), stat.data(), part_d, to.data());
+  c->arena.lo = lo0;
+  for (size_t k = 0; k < rest.size(); ++k) {
+    const int32_t g = rest[k];
+    done[g] = 1;
+    if (q_out) q_out[g] = q[k];
+    if (levels_out) levels_out[g] = lev[k];
+    if (comms_out) comms_out[g] = com[k];
+    if (status_out) status_out[g] = stat[k];
   }
 }
 
@@ -1699,41 +1762,24 @@ void batch_run(lvg_ctx* c, const BatchInput& given, int32_t* part_out, double* q
   }
   const size_t lo0 = a.lo;
   int32_t* part_d = a.lo_n<int32_t>(V0);
-  std::vector<char> done((size_t)G0, 0);
-  batch_small(c, in, part_d, done, q_out, levels_out, comms_out, status_out);
-  const int64_t ndone = std::count(done.begin(), done.end(), (char)1);
-  if (ndone == 0) {
-    a.lo = lo0;
-    batch_union(c, in, part_out, q_out, levels_out, comms_out, status_out, nullptr, nullptr);
-    return;
-  }
-  if (ndone < G0) {   // the other graphs, as a batch of their own
-    std::vector<int32_t> rest, rvoff(1, 0), to;
-    std::vector<int64_t> reoff(1, 0);
-    BatchInput sub;
-    for (int32_t g = 0; g < G0; ++g) {
-      if (done[g]) continue;
-      rest.push_back(g);
-      to.push_back(voff[g]);
-      rvoff.push_back(rvoff.back() + voff[g + 1] - voff[g]);
-      reoff.push_back(reoff.back() + eoff[g + 1] - eoff[g]);
-      sub.src.push_back(in.src[g]);
-      sub.dst.push_back(in.dst[g]);
-      sub.w.push_back(in.w[g]);
+  SmallBatch small;
+  try {
+    small = batch_small_start(c, in, part_d);
+    if (small.which.empty()) {
+      a.lo = lo0;
+      batch_union(c, in, part_out, q_out, levels_out, comms_out, status_out, nullptr, nullptr);
+      return;
     }
-    sub.G = (int32_t)rest.size();
-    sub.eoff = reoff.data();
-    sub.voff = rvoff.data();
-    std::vector<double> q(rest.size());
-    std::vector<int32_t> lev(rest.size()), com(rest.size()), stat(rest.size());
-    batch_union(c, sub, nullptr, q.data(), lev.data(), com.data(), stat.data(), part_d, to.data());
-    for (size_t k = 0; k < rest.size(); ++k) {
-      const int32_t g = rest[k];
-      if (q_out) q_out[g] = q[k];
-      if (levels_out) levels_out[g] = lev[k];
-      if (comms_out) comms_out[g] = com[k];
-      if (status_out) status_out[g] = stat[k];
-    }
+    std::vector<char> done((size_t)G0, 0), started((size_t)G0, 0);
+    const std::vector<char> none((size_t)G0, 0);
+    for (int32_t g : small.which) started[g] = 1;
+    batch_rest(c, in, done, started, part_d, q_out, levels_out, comms_out, status_out);
+    batch_small_finish(c, small, done, q_out, levels_out, comms_out, status_out);
+    batch_rest(c, in, done, none, part_d, q_out, levels_out, comms_out, status_out);
+  } catch (...) {   // nothing of the batch may still run when its memory is given up
+    for (cudaStream_t st : c->small_streams)
+      if (st) cudaStreamSynchronize(st);
+    throw;
   }
   if (part_out && V0 > 0)
     LVG_CUDA(cudaMemcpyAsync(part_out, part_d, sizeof(int32_t) * V0, cudaMemcpyDeviceToHost, s));
