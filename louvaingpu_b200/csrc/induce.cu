@@ -36,6 +36,7 @@
 
 #include "louvain.cuh"
 #include "prims.cuh"
+#include "rules.cuh"
 
 namespace lvg {
 namespace {
@@ -760,24 +761,29 @@ constexpr int kTxItems = kIcChunk / kTxThreads;   // 16 consecutive positions (e
 
 // Per member of a chunk: start relative to the chunk (0 for the member
 // holding the chunk's first position), list index of its first position
-// minus its start, community.
+// minus its start (mod 2^32: lists are shorter), community.
 struct TxSmem {
   int32_t rs[kIcChunk + 2];
-  int64_t eb[kIcChunk + 1];
+  uint32_t eb[kIcChunk + 1];
   int32_t yc[kIcChunk + 1];
 };
+constexpr int kTxLayThreads = 512;
+constexpr int kTxLayItems = kIcChunk / kTxLayThreads;   // 8 positions per thread
 
 // Keys (dense community of d << Bb | community of u: the caller passes the
 // dense ids of the vertices as `part`) and weights (0 counted as 1) of the
-// entries
-// in segment order, a block per 4096 positions.  The chunk's members are
-// staged in shared memory; a thread takes 16 positions 256 apart, finds the
-// member of each by a binary search, then issues all 16 list loads and all
-// 16 community gathers before it uses any of them.
+// entries in segment order, a block per 4096 positions.  The chunk's members
+// are staged in shared memory; a thread takes 8 positions 512 apart, finds the
+// member of each by a binary search, then issues all its list loads and all
+// its community gathers before it uses any of them.  Bound by the latency of
+// those gathers, so by the warps in flight: 512 threads of 8 positions and a
+// 48 KB table fit two blocks an SM (32 warps), 256 of 16 with 64-bit
+// list indices also fitted two (16 warps): R-MAT scale 24, 850 M entries, 14.0 ->
+// 10.2 ms.
 // PACKED (whole weights that fit): the weight rides in the key's bits from
 // `wshift` up, and no values are written.
 template <bool PACKED>
-__global__ void __launch_bounds__(kTxThreads) tx_layout_kernel(
+__global__ void __launch_bounds__(kTxLayThreads, 2) tx_layout_kernel(
     int64_t E, int32_t nz, int Bb, int wshift, const int32_t* mem, const int32_t* mcomm, const int64_t* mscan,
     const int32_t* cfirst, const int64_t* off, const uint32_t* lscan, const int32_t* ldst, const float* lw,
     const int32_t* part, uint64_t* keys, float* vals) {
@@ -791,67 +797,67 @@ __global__ void __launch_bounds__(kTxThreads) tx_layout_kernel(
   const int32_t j0 = cfirst[c];
   const int32_t jend = min(cfirst[c + 1] + 1, nz);
   const int nm = jend - j0;
-  {   // stage the members: every thread's loads issued before any is used
-    constexpr int kStage = (kIcChunk + 2 + kTxThreads - 1) / kTxThreads;
-    int64_t st[kStage];
-    int32_t uu[kStage], yy[kStage];
+  // stage the members, four of a thread's at a time
+#pragma unroll 1
+  for (int t0 = threadIdx.x; t0 <= nm; t0 += 4 * kTxLayThreads) {
+    int64_t st[4];
+    int32_t uu[4], yy[4];
 #pragma unroll
-    for (int x = 0; x < kStage; ++x) {
-      const int t = threadIdx.x + x * kTxThreads;
+    for (int x = 0; x < 4; ++x) {
+      const int t = t0 + x * kTxLayThreads;
       st[x] = t <= nm ? mscan[j0 + t] : 0;
       uu[x] = t < nm ? mem[j0 + t] : 0;
       yy[x] = t < nm ? mcomm[j0 + t] : 0;
     }
-    int64_t ob[kStage];
+    uint32_t ob[4];
 #pragma unroll
-    for (int x = 0; x < kStage; ++x) {
-      const int t = threadIdx.x + x * kTxThreads;
-      ob[x] = t < nm ? off[uu[x]] + (int64_t)lscan[uu[x]] : 0;
-    }
+    for (int x = 0; x < 4; ++x) ob[x] = t0 + x * kTxLayThreads < nm ? (uint32_t)off[uu[x]] + lscan[uu[x]] : 0u;
 #pragma unroll
-    for (int x = 0; x < kStage; ++x) {
-      const int t = threadIdx.x + x * kTxThreads;
+    for (int x = 0; x < 4; ++x) {
+      const int t = t0 + x * kTxLayThreads;
       if (t <= nm) {
         const int64_t r = st[x] - p0;
         S.rs[t] = (int32_t)(r < 0 ? 0 : (r > kIcChunk ? kIcChunk : r));
       }
       if (t < nm) {
-        S.eb[t] = ob[x] - st[x];
+        S.eb[t] = ob[x] - (uint32_t)st[x];
         S.yc[t] = yy[x];
       }
     }
   }
   __syncthreads();
-  // position q = i * 256 + thread: a warp's loads and stores are contiguous
+  // position q = i * 512 + thread: a warp's loads and stores are contiguous
   // along the rows; the member of each position by a branch-free binary
-  // search over the staged starts (all 16 searches independent)
-  int64_t e[kTxItems];
-  int32_t y[kTxItems];
+  // search over the staged starts (all searches independent)
+  int top = 0;
+  while ((1 << (top + 1)) <= nm) ++top;   // uniform: chunks of long rows search few members
+  uint32_t e[kTxLayItems];
+  int32_t y[kTxLayItems];
 #pragma unroll
-  for (int i = 0; i < kTxItems; ++i) {
-    const int q = i * kTxThreads + threadIdx.x;
+  for (int i = 0; i < kTxLayItems; ++i) {
+    const int q = i * kTxLayThreads + threadIdx.x;
     int lo = 0;
-#pragma unroll
-    for (int b = 12; b >= 0; --b) {   // nm <= kIcChunk + 1 < 2^13
+#pragma unroll 1
+    for (int b = top; b >= 0; --b) {
       const int cand = lo + (1 << b);
       if (cand < nm && S.rs[cand] <= q) lo = cand;
     }
-    e[i] = q < n ? S.eb[lo] + p0 + q : 0;
+    e[i] = S.eb[lo] + (uint32_t)(p0 + q);
     y[i] = S.yc[lo];
   }
-  int32_t d[kTxItems];
-  float wv[kTxItems];
+  int32_t d[kTxLayItems];
+  float wv[kTxLayItems];
 #pragma unroll
-  for (int i = 0; i < kTxItems; ++i) {
-    const bool ok = i * kTxThreads + (int)threadIdx.x < n;
+  for (int i = 0; i < kTxLayItems; ++i) {
+    const bool ok = i * kTxLayThreads + (int)threadIdx.x < n;
     d[i] = ok ? __ldg(ldst + e[i]) : 0;
     wv[i] = ok ? __ldg(lw + e[i]) : 1.0f;
   }
 #pragma unroll
-  for (int i = 0; i < kTxItems; ++i) d[i] = __ldg(part + d[i]);
+  for (int i = 0; i < kTxLayItems; ++i) d[i] = __ldg(part + d[i]);
 #pragma unroll
-  for (int i = 0; i < kTxItems; ++i) {
-    const int q = i * kTxThreads + threadIdx.x;
+  for (int i = 0; i < kTxLayItems; ++i) {
+    const int q = i * kTxLayThreads + threadIdx.x;
     if (q < n) {
       const float x = wv[i] == 0.0f ? 1.0f : wv[i];   // InducedGraphKernel.cu:38-39
       uint64_t key = ((uint64_t)(uint32_t)d[i] << Bb) | (uint32_t)y[i];
@@ -862,36 +868,36 @@ __global__ void __launch_bounds__(kTxThreads) tx_layout_kernel(
   }
 }
 
-// The 16 sorted keys and weights of a thread (16-byte loads when whole).
+// The N consecutive sorted keys and weights of a thread (16-byte loads when whole).
 // Without values: weights from the keys' bits from wshift up, when WEIGHTS.
-template <bool WEIGHTS>
-__device__ __forceinline__ int tx_load16(const uint64_t* k, const float* v, int64_t i0, int64_t n, int wshift,
-                                         uint64_t (&kk)[kTxItems], float (&vv)[kTxItems]) {
-  const int m = (int)max((int64_t)0, min((int64_t)kTxItems, n - i0));
-  if (m == kTxItems) {
+template <int N, bool WEIGHTS>
+__device__ __forceinline__ int tx_load_keys(const uint64_t* k, const float* v, int64_t i0, int64_t n, int wshift,
+                                         uint64_t (&kk)[N], float (&vv)[N]) {
+  const int m = (int)max((int64_t)0, min((int64_t)N, n - i0));
+  if (m == N) {
 #pragma unroll
-    for (int i = 0; i < kTxItems; i += 2) {
+    for (int i = 0; i < N; i += 2) {
       const ulonglong2 x = reinterpret_cast<const ulonglong2*>(k + i0)[i / 2];
       kk[i] = x.x;
       kk[i + 1] = x.y;
     }
     if (v) {
 #pragma unroll
-      for (int i = 0; i < kTxItems; i += 4) {
+      for (int i = 0; i < N; i += 4) {
         const float4 x = reinterpret_cast<const float4*>(v + i0)[i / 4];
         vv[i] = x.x; vv[i + 1] = x.y; vv[i + 2] = x.z; vv[i + 3] = x.w;
       }
     }
   } else {
 #pragma unroll
-    for (int i = 0; i < kTxItems; ++i) {
+    for (int i = 0; i < N; ++i) {
       kk[i] = i < m ? k[i0 + i] : ~0ull;
       if (v) vv[i] = i < m ? v[i0 + i] : 0.0f;
     }
   }
   const uint64_t kmask = ~0ull >> (64 - wshift);
 #pragma unroll
-  for (int i = 0; i < kTxItems; ++i) {
+  for (int i = 0; i < N; ++i) {
     if (WEIGHTS && !v) vv[i] = (float)(kk[i] >> wshift);
     kk[i] &= kmask;
   }
@@ -909,7 +915,7 @@ __global__ void __launch_bounds__(kTxThreads) tx_count_kernel(const uint64_t* k,
   const int64_t i0 = blockIdx.x * (int64_t)kIcChunk + (int64_t)threadIdx.x * kTxItems;
   uint64_t kk[kTxItems];
   float unused[kTxItems];
-  const int m = tx_load16<false>(k, nullptr, i0, n, wshift, kk, unused);
+  const int m = tx_load_keys<kTxItems, false>(k, nullptr, i0, n, wshift, kk, unused);
   uint64_t prev = (i0 > 0 && m > 0) ? k[i0 - 1] & (~0ull >> (64 - wshift)) : ~0ull;
   unsigned long long cnt = 0;
 #pragma unroll
@@ -923,31 +929,18 @@ __global__ void __launch_bounds__(kTxThreads) tx_count_kernel(const uint64_t* k,
   if (threadIdx.x == 0) tcount[blockIdx.x] = (int64_t)tot;
 }
 
-__device__ __forceinline__ double tx_seg_sum(double v, int64_t seg) {
-  const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const double u = __shfl_up_sync(full, v, o);
-    const int64_t t = __shfl_up_sync(full, seg, o);
-    if (lane >= o && t == seg) v = __dadd_rn(v, u);
-  }
-  return v;
-}
-
-__device__ __forceinline__ bool tx_seg_last(int64_t seg, bool valid) {
-  const unsigned full = 0xffffffffu;
-  const int64_t nx = __shfl_down_sync(full, seg, 1);
-  const bool nvalid = __shfl_down_sync(full, valid, 1);
-  return valid && ((threadIdx.x & 31) == 31 || !nvalid || nx != seg);
-}
+// (512 threads of 8 entries at 64 registers: 32 warps an SM where 256 of 16
+// entries at 80 gave 24; row sums from run_depth: R-MAT scale 24, four levels,
+// 10.1 -> 9.6 ms.  Bound by issue and the serial pieces of long runs.)
+constexpr int kTxEmitThreads = 512;
+constexpr int kTxEmitItems = kIcChunk / kTxEmitThreads;   // 8 consecutive entries per thread
 
 struct TxEmitSmem {
   uint64_t key[kIcChunk];     // key of the tile's i-th distinct entry
   double sum[kIcChunk];       // its summed weight; -1: the run is still open at the tile's end
   uint16_t lp[kIcChunk];      // coarse self loops among the tile's distinct entries before it
-  double lead[kTxThreads];    // sum of a thread's entries before its first head
-  uint8_t anyhead[kTxThreads];
+  double lead[kTxEmitThreads];    // sum of a thread's entries before its first head
+  uint8_t anyhead[kTxEmitThreads];
 };
 
 __device__ __forceinline__ uint32_t tx_lo(int64_t x) { return (uint32_t)((uint64_t)x & 0xffffffffull); }
@@ -974,7 +967,7 @@ __device__ __forceinline__ double tx_csr_entry(const IcCsrOut& O, int32_t a, int
 }
 
 // Each run of equal keys (dense first community, mapped back by und; the
-// second community as it is) once, a block per 4096-entry tile, 16 consecutive
+// second community as it is) once, a block per 4096-entry tile, 8 consecutive
 // entries per thread.  A thread sums the runs that start in its entries in
 // entry order (FP64); a run that goes on past the thread is finished by the
 // thread holding its head, which adds the leading pieces of the threads after
@@ -984,7 +977,7 @@ __device__ __forceinline__ double tx_csr_entry(const IcCsrOut& O, int32_t a, int
 // entry and the row degrees.  The tile's last run, when it goes on into the
 // next tiles, is summed with atomics into opensum[tile] (its continuations
 // find the tile by a binary search) and finished by tx_open_kernel.
-__global__ void __launch_bounds__(kTxThreads) tx_emit_kernel(const uint64_t* k, const float* v, int64_t n, int Bb,
+__global__ void __launch_bounds__(kTxEmitThreads, 2) tx_emit_kernel(const uint64_t* k, const float* v, int64_t n, int Bb,
                                                              int wshift, const int64_t* tscan, const int32_t* und,
                                                              int32_t* osrc, int32_t* odst, float* ow, double* opensum,
                                                              uint32_t* openflag, uint32_t* hl, uint32_t* dcount,
@@ -994,14 +987,14 @@ __global__ void __launch_bounds__(kTxThreads) tx_emit_kernel(const uint64_t* k, 
   const uint64_t mask = (1ull << Bb) - 1ull;
   const int t = threadIdx.x;
   const int64_t tile = blockIdx.x;
-  const int64_t i0 = tile * kIcChunk + (int64_t)t * kTxItems;
-  uint64_t kk[kTxItems];
-  float vv[kTxItems];
-  const int m = tx_load16<true>(k, v, i0, n, wshift, kk, vv);
+  const int64_t i0 = tile * kIcChunk + (int64_t)t * kTxEmitItems;
+  uint64_t kk[kTxEmitItems];
+  float vv[kTxEmitItems];
+  const int m = tx_load_keys<kTxEmitItems, true>(k, v, i0, n, wshift, kk, vv);
   uint64_t prev = (i0 > 0 && m > 0) ? k[i0 - 1] & (~0ull >> (64 - wshift)) : ~0ull;
   uint32_t hmask = 0, nloop = 0;
 #pragma unroll
-  for (int i = 0; i < kTxItems; ++i) {
+  for (int i = 0; i < kTxEmitItems; ++i) {
     if (i < m && (i0 + i == 0 || kk[i] != prev)) {
       hmask |= 1u << i;
       nloop += (uint64_t)und[(int32_t)(kk[i] >> Bb)] == (kk[i] & mask) ? 1u : 0u;
@@ -1010,14 +1003,14 @@ __global__ void __launch_bounds__(kTxThreads) tx_emit_kernel(const uint64_t* k, 
   }
   unsigned long long both;
   const unsigned long long ex =
-      block_exclusive_scan256<unsigned long long>(((unsigned long long)nloop << 32) | (uint32_t)__popc(hmask), &both);
+      block_exclusive_scan512<unsigned long long>(((unsigned long long)nloop << 32) | (uint32_t)__popc(hmask), &both);
   const uint32_t tot = (uint32_t)both;
   int loc = (int)(uint32_t)ex - 1;
   uint32_t lc = (uint32_t)(ex >> 32);   // self loops among the tile's distinct entries before the next head
   double s = 0.0;
   bool started = false;
 #pragma unroll
-  for (int i = 0; i < kTxItems; ++i) {
+  for (int i = 0; i < kTxEmitItems; ++i) {
     if (i < m) {
       if ((hmask >> i) & 1u) {
         if (started) S.sum[loc] = s;   // a run that began and ended in this thread
@@ -1041,7 +1034,7 @@ __global__ void __launch_bounds__(kTxThreads) tx_emit_kernel(const uint64_t* k, 
     // entries before the tile's first head continue the last run of an
     // earlier tile h: the run with distinct index tb - 1
     double x = 0.0;
-    for (int u = 0; u < kTxThreads; ++u) {
+    for (int u = 0; u < kTxEmitThreads; ++u) {
       x = __dadd_rn(x, S.lead[u]);
       if (S.anyhead[u]) break;
     }
@@ -1056,11 +1049,11 @@ __global__ void __launch_bounds__(kTxThreads) tx_emit_kernel(const uint64_t* k, 
   if (started) {   // the thread's last run takes the leading pieces after it
     double x = s;
     bool open = true;
-    for (int u = t + 1; u < kTxThreads; ++u) {
+    for (int u = t + 1; u < kTxEmitThreads; ++u) {
       x = __dadd_rn(x, S.lead[u]);
       if (S.anyhead[u]) { open = false; break; }
     }
-    if (open && i0 + kIcChunk - (int64_t)t * kTxItems < n) {   // goes on into the next tile
+    if (open && i0 + kIcChunk - (int64_t)t * kTxEmitItems < n) {   // goes on into the next tile
       atomicAdd(&opensum[tile], x);
       openflag[tile] = 1u;
       S.sum[loc] = -1.0;
@@ -1073,7 +1066,7 @@ __global__ void __launch_bounds__(kTxThreads) tx_emit_kernel(const uint64_t* k, 
   const int64_t lt = tx_hi(tscan[tile]);
   const int lane = t & 31;
   uint32_t top = 0;   // bits of the largest weight written
-  for (uint32_t l0 = 0; l0 < tot; l0 += kTxThreads) {
+  for (uint32_t l0 = 0; l0 < tot; l0 += kTxEmitThreads) {
     const uint32_t l = l0 + t;
     const bool valid = l < tot;
     const int64_t r = tb + l;
@@ -1093,16 +1086,13 @@ __global__ void __launch_bounds__(kTxThreads) tx_emit_kernel(const uint64_t* k, 
     if (closed) ow[r] = wf;
     top = max(top, __float_as_uint(wf));
     // distinct entries per row: lanes of one row are consecutive
-    const int32_t ap = __shfl_up_sync(0xffffffffu, a, 1);
-    const unsigned starts = __ballot_sync(0xffffffffu, valid && (lane == 0 || ap != a));
-    const bool last = tx_seg_last(a, valid);
-    if (last) {
-      const int first = 31 - __clz(starts & (0xffffffffu >> (31 - lane)));
-      atomicAdd(&dcount[a], (uint32_t)(lane - first + 1));
-    }
+    bool last;
+    const int depth = run_depth(a, last);
+    last = last && valid;
+    if (last) atomicAdd(&dcount[a], (uint32_t)depth + 1u);
     if (O.col) {
       const double kd = closed ? tx_csr_entry(O, a, b, wf, r, lt + (valid ? S.lp[l] : 0)) : 0.0;
-      const double ks = tx_seg_sum(kd, a);
+      const double ks = run_sum(kd, depth);
       if (last && ks != 0.0) atomicAdd(&O.k[a], ks);
     }
   }
@@ -1253,10 +1243,10 @@ bool induce_transposed(const LevelGraph& g, const int32_t* part, int32_t C, int6
   float* v1 = packed ? nullptr : a.hi_n<float>(E);
   tx_attributes();
   if (packed)
-    tx_layout_kernel<true><<<(unsigned)nchunks, kTxThreads, sizeof(TxSmem), s>>>(
+    tx_layout_kernel<true><<<(unsigned)nchunks, kTxLayThreads, sizeof(TxSmem), s>>>(
         E, h_nz, Bb, wshift, mem, mcomm, mscan, cfirst, g.off, lscan, g.dst, g.w, pd, k0, v0);
   else
-    tx_layout_kernel<false><<<(unsigned)nchunks, kTxThreads, sizeof(TxSmem), s>>>(
+    tx_layout_kernel<false><<<(unsigned)nchunks, kTxLayThreads, sizeof(TxSmem), s>>>(
         E, h_nz, Bb, wshift, mem, mcomm, mscan, cfirst, g.off, lscan, g.dst, g.w, pd, k0, v0);
   LVG_LAUNCH();
   const int w2 = radix_sort_range(k0, v0, k1, v1, E, Bb, Bd, a, s);
@@ -1320,7 +1310,7 @@ bool induce_transposed(const LevelGraph& g, const int32_t* part, int32_t C, int6
     LVG_CUDA(cudaMemsetAsync(next.has_loop, 0, (size_t)C, s));
     O = IcCsrOut{next.col, next.cw, next.k, next.loopw, next.has_loop, hl, nullptr};
   }
-  tx_emit_kernel<<<(unsigned)nchunks, kTxThreads, sizeof(TxEmitSmem), s>>>(keys, vals, E, Bb, wshift, tscan, und, osrc,
+  tx_emit_kernel<<<(unsigned)nchunks, kTxEmitThreads, sizeof(TxEmitSmem), s>>>(keys, vals, E, Bb, wshift, tscan, und, osrc,
                                                                            odst, ow, opensum, openflag, hl, dcount,
                                                                            max_w, O);
   LVG_LAUNCH();
