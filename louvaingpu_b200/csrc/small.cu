@@ -60,7 +60,9 @@ constexpr unsigned long long kEmpty = ~0ull;
 static_assert(kSmallMaxV <= (1 << kCommBits), "packed keys hold 18-bit communities");
 
 enum : uint32_t { fNotInt = 1u, fUnfit = 2u, fBad = 4u, fUnsorted = 8u };
-enum : int32_t { kPhaseNone = 0, kPhaseTail = 1, kPhaseEnd = 2 };
+// kPhaseMid: the grid left the level to a cluster; kPhaseTail: a level fits
+// one block's shared memory; kPhaseEnd: the levels are done.
+enum : int32_t { kPhaseNone = 0, kPhaseMid = 1, kPhaseTail = 2, kPhaseEnd = 3 };
 enum : int32_t { kCompDone = 0, kCompTail = 1, kCompTailAll = 2 };
 
 // Control words of a level's blocks.
@@ -1033,7 +1035,7 @@ struct At {
   int64_t E;
   int32_t ncomms = 0;
   int buf = -1, nlev = 0, status = LVG_OK;
-  bool open = false, symmetric = true, bad = false, tail = false;
+  bool open = false, symmetric = true, bad = false, tail = false, mid = false;
   double mod = 0.0, lower = 0.0;
   int64_t part_off = 0;
 };
@@ -1071,6 +1073,10 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
     if (at.nlev >= kSmallLevels || (J.parts && at.part_off + 2 * (int64_t)V > J.parts_cap)) { at.open = true; return true; }
     if (!X::kResident) {
       if (V <= kResV && E <= kResE) { at.tail = true; return true; }
+      // below this a cluster's barriers save more than the chip's width does
+      // (a level of 117 Ki entries takes 154 us on the grid, 199 on a cluster;
+      // one of 12 Ki 96 and 68)
+      if (T.mode == kModeGrid && E <= kSmallClusterEntries) { at.mid = true; return true; }
       // few entries for so many blocks: the last ones leave
       if (T.mode == kModeGrid && T.K_ > 1) {
         T.K_ = (int)min((int64_t)T.K_, (E + kGridEntries - 1) / kGridEntries);
@@ -1357,9 +1363,23 @@ __device__ __forceinline__ void store_between(Between& B, const At& at) {
   B.lower = at.lower;
 }
 
-// First launch: the levels until one fits a block's shared memory.
+__device__ __forceinline__ void load_between(const Between& B, At& at) {
+  at.V = B.V;
+  at.E = B.E;
+  at.ncomms = B.ncomms;
+  at.buf = B.buf;
+  at.nlev = B.nlev;
+  at.symmetric = B.symmetric != 0;
+  at.mod = B.mod;
+  at.lower = B.lower;
+  at.part_off = B.part_off;
+}
+
+// First launch (and the second, a cluster's, behind a grid's): the levels
+// until one fits a block's shared memory.
 template <int NT>
-__global__ void __launch_bounds__(NT, 1024 / NT) small_kernel(const SmallJob* jobs, int K, int mode, SmallCfg cfg) {
+__global__ void __launch_bounds__(NT, 1024 / NT) small_kernel(const SmallJob* jobs, int K, int mode, int resume,
+                                                               SmallCfg cfg) {
   using X = Multi<NT>;
   load_job<X>(jobs + blockIdx.x / K);
   const SmallJob& J = X::S().J;
@@ -1376,14 +1396,19 @@ __global__ void __launch_bounds__(NT, 1024 / NT) small_kernel(const SmallJob* jo
   at.E = J.E;
   at.symmetric = J.check == 0;
   at.mod = J.mod;
+  Between& B = *X::W().bt;
+  if (resume) {   // from where the grid stopped
+    if (B.phase != kPhaseMid) return;
+    load_between(B, at);
+    if (!T.sync()) return;   // before the first block writes it again
+  }
   if (!run_levels<X>(T, cfg, at)) return;
   if (T.lead()) {
-    Between& B = *X::W().bt;
     store_between(B, at);
     const long long ticks = clock64() - c0;
     B.ms_per_tick = ticks > 0 ? 1e-6 * (double)(now_ns() - ns0) / (double)ticks : 0.0;
     B.comp = kCompDone;
-    B.phase = at.tail ? kPhaseTail : kPhaseEnd;
+    B.phase = at.mid ? kPhaseMid : at.tail ? kPhaseTail : kPhaseEnd;
   }
 }
 
@@ -1409,15 +1434,7 @@ __global__ void __launch_bounds__(kResThreads, 1) small_tail_kernel(const SmallJ
       W.ghist = g.ghist;
     }
     At at;
-    at.V = B.V;
-    at.E = B.E;
-    at.ncomms = ncomms;
-    at.buf = B.buf;
-    at.nlev = B.nlev;
-    at.symmetric = B.symmetric != 0;
-    at.mod = B.mod;
-    at.lower = B.lower;
-    at.part_off = B.part_off;
+    load_between(B, at);
     const bool first = at.nlev == 0;
     const int32_t nlev0 = at.nlev, v0 = at.V;
     __syncthreads();
@@ -1561,8 +1578,7 @@ void set_attributes() {
 }
 
 template <int NT>
-void launch(const SmallJob* jobs, int n, int K, int mode, const SmallCfg& cfg, cudaStream_t s) {
-  set_attributes();
+void launch_levels(const SmallJob* jobs, int n, int K, int mode, int resume, const SmallCfg& cfg, cudaStream_t s) {
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3((unsigned)(n * K));
   lc.blockDim = dim3(NT);
@@ -1580,8 +1596,12 @@ void launch(const SmallJob* jobs, int n, int K, int mode, const SmallCfg& cfg, c
   }
   lc.attrs = at;
   lc.numAttrs = mode == kModeGrid || K > 1 ? 1 : 0;
-  LVG_CUDA(cudaLaunchKernelEx(&lc, small_kernel<NT>, jobs, K, mode, cfg));
+  LVG_CUDA(cudaLaunchKernelEx(&lc, small_kernel<NT>, jobs, K, mode, resume, cfg));
   count_launch();
+}
+
+// The launches behind the levels: the tail, and the results by K blocks a job.
+void launch_rest(const SmallJob* jobs, int n, int K, const SmallCfg& cfg, cudaStream_t s) {
   small_tail_kernel<<<(unsigned)n, kResThreads, sizeof(Tail::Smem), s>>>(jobs, cfg);
   LVG_LAUNCH();
   small_sum_kernel<<<(unsigned)(n * K), kQThreads, 0, s>>>(jobs, K);
@@ -1609,8 +1629,10 @@ bool small_fits(int64_t V, int64_t E, int64_t max_entries) {
 
 void small_run(const SmallJob* d_jobs, int n, int K, const SmallCfg& cfg, cudaStream_t s) {
   if (n <= 0) return;
-  if (K >= 8) launch<1024>(d_jobs, n, K, kModeCluster, cfg, s);
-  else launch<512>(d_jobs, n, K, kModeCluster, cfg, s);
+  set_attributes();
+  if (K >= 8) launch_levels<1024>(d_jobs, n, K, kModeCluster, 0, cfg, s);
+  else launch_levels<512>(d_jobs, n, K, kModeCluster, 0, cfg, s);
+  launch_rest(d_jobs, n, K, cfg, s);
 }
 
 int small_grid_blocks() {
@@ -1633,7 +1655,10 @@ int small_grid_blocks() {
 void small_run_grid(const SmallJob* d_job, void* work, int K, const SmallCfg& cfg, cudaStream_t s) {
   // the barrier's words, and the phase, should a wait run out
   LVG_CUDA(cudaMemsetAsync(work, 0, up256(sizeof(Ctl)) + up256(sizeof(Between)), s));
-  launch<1024>(d_job, 1, K, kModeGrid, cfg, s);
+  set_attributes();
+  launch_levels<1024>(d_job, 1, K, kModeGrid, 0, cfg, s);
+  launch_levels<1024>(d_job, 1, kSmallClusterBlocks, kModeCluster, 1, cfg, s);
+  launch_rest(d_job, 1, K, cfg, s);
 }
 
 }  // namespace lvg
