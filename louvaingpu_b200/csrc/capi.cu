@@ -183,8 +183,9 @@ void prepare_level(lvg_ctx* c, const ListFacts* facts = nullptr) {
   c->renumbered = false;
 }
 
-// Largest list small_run takes (1.9 M entries: a level takes 0.57 ms on the
-// cooperative grid, 0.95 by the level kernels; 13 M: 2.7 and 2.0).
+// Largest list small_run takes: at 1.9 M entries a level takes 0.57 ms on the
+// cooperative grid, 0.95 by the level kernels.  (Above 4 Mi the tree of m
+// would have more partials than finish_sum adds.)
 constexpr int64_t kSmallRunEntries = 2 * 1024 * 1024;
 
 // `copied`: the list lies in the arena.  facts: of the list, unless it was

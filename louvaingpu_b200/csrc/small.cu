@@ -17,11 +17,12 @@
 //   pass 1   singletons: the best candidate of a row is an argmax over its
 //            entries (segmented warp argmax, then shared-memory max / min)
 //   pass 2+  tiles of consecutive rows hashed as (row, community) pairs in
-//            shared memory: packed 64-bit slots when the weights are integral,
-//            key + FP64 sum otherwise
+//            shared memory: 32-bit keys and sums when the weights are integral,
+//            key + FP64 sum otherwise; a row longer than a tile is a block's
+//            work alone, its communities split over several tables in turn
 //   renumber by smallest member; coarse keys (cu << b | cv) sorted by a stable
 //            LSD radix sort across the cluster, runs summed in FP64
-// A list that is not sorted and symmetric, a row longer than a tile, or more
+// A list that is not sorted and symmetric, a row beyond kLongRow, or more
 // levels or passes than the tables hold end the launch with the level left
 // open; the caller goes on with the level kernels from the same list.
 #include <algorithm>
@@ -53,13 +54,14 @@ struct Tile {
 constexpr int kCommBits = 18;              // community bits of a packed key
 constexpr int kDigits = 256;
 constexpr int64_t kGridEntries = 4096;     // grid mode: entries a block, at least
+constexpr int kLongRow = 1 << 16;          // longest row (32 parts: the row is read 32 times a pass by one block)
 constexpr int kResThreads = 512;
 constexpr int kResV = 512, kResE = 6144;   // a level this small lives in one block's shared memory
 constexpr unsigned long long kWaitNs = 4000000000ull;   // limit of a grid barrier's wait
 constexpr unsigned long long kEmpty = ~0ull;
 static_assert(kSmallMaxV <= (1 << kCommBits), "packed keys hold 18-bit communities");
 
-enum : uint32_t { fNotInt = 1u, fUnfit = 2u, fBad = 4u, fUnsorted = 8u };
+enum : uint32_t { fNotInt = 1u, fUnfit = 2u, fBad = 4u, fUnsorted = 8u, fFull = 16u, fLong = 32u };
 // kPhaseMid: the grid left the level to a cluster; kPhaseTail: a level fits
 // one block's shared memory; kPhaseEnd: the levels are done.
 enum : int32_t { kPhaseNone = 0, kPhaseMid = 1, kPhaseTail = 2, kPhaseEnd = 3 };
@@ -185,6 +187,9 @@ struct Space {
   double ws[8];
   double bcast;
   uint32_t wtot[NT / 32];
+  double rg[NT / 32], rw[NT / 32];   // long rows: each warp's best candidate
+  int32_t rc[NT / 32];
+  int32_t saw;
   int32_t nclaimed, row0, row1;
   unsigned long long goal;   // grid barrier: arrivals awaited
   int32_t alive;
@@ -431,9 +436,49 @@ struct List {
 
 __device__ __forceinline__ double merged_w(float w) { return (double)__double2float_rn(__dadd_rn((double)w, (double)w)); }
 
-// First pass of a level: every neighbour is its own candidate.
+// The block's best candidate from each thread's, in thread 0.
 template <typename X>
-__device__ __forceinline__ void moves_first_body(const List L, int32_t v, int32_t vend, bool last_pass) {
+__device__ __forceinline__ void block_best(double& g, int32_t& c, double& w) {
+  auto& S = X::S();
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) {
+    const double g2 = __shfl_xor_sync(full, g, o), w2 = __shfl_xor_sync(full, w, o);
+    const int32_t c2 = __shfl_xor_sync(full, c, o);
+    if (better(g2, c2, g, c)) { g = g2; c = c2; w = w2; }
+  }
+  if (lane == 0) { S.rg[wid] = g; S.rc[wid] = c; S.rw[wid] = w; }
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int k = 1; k < X::NT / 32; ++k)
+      if (better(S.rg[k], S.rc[k], g, c)) { g = S.rg[k]; c = S.rc[k]; w = S.rw[k]; }
+  __syncthreads();
+}
+
+// A row longer than a tile, in the first pass: the block strides over it.
+template <typename X>
+__device__ __noinline__ void long_first(const List L, int32_t v, bool last_pass) {
+  auto& W = X::W();
+  const int32_t beg = W.roff[v], end = W.roff[v + 1];
+  const double kf = W.kfrac[v];
+  double bg = 0.0, bw = 0.0;
+  int32_t bc = kNone;
+#pragma unroll 4
+  for (int32_t e = beg + (int)threadIdx.x; e < end; e += X::NT) {
+    const int32_t c = L.dst[e];
+    const double w = merged_w(L.w[e]);
+    const double g = __dsub_rn(w, __dmul_rn(W.k[c], kf));
+    if (c != v && w != 0.0 && g > 0.0 && better(g, c, bg, bc)) { bg = g; bc = c; bw = w; }
+  }
+  block_best<X>(bg, bc, bw);
+  if (threadIdx.x == 0) decide<X, true>(v, v, bc, bw, end - beg, last_pass);
+}
+
+// First pass of a level: every neighbour is its own candidate.  Returns the
+// first row longer than a tile, else vend.
+template <typename X>
+__device__ __forceinline__ int32_t moves_first_body(const List L, int32_t v, int32_t vend, bool last_pass) {
   constexpr int NT = X::NT;
   auto& S = X::S();
   auto& W = X::W();
@@ -442,7 +487,7 @@ __device__ __forceinline__ void moves_first_body(const List L, int32_t v, int32_
 #pragma unroll 1
   while (v < vend) {
     const int nv = tile_rows<X>(W.roff, v, vend, Tile<NT>::kInt);
-    if (nv == 0) return;   // cannot happen: rows longer than a tile leave the level open
+    if (nv == 0) return v;
     const int32_t base = W.roff[v];
     const int n = W.roff[v + nv] - base;
     if (n > 0) {
@@ -525,6 +570,7 @@ __device__ __forceinline__ void moves_first_body(const List L, int32_t v, int32_
     }
     v += nv;
   }
+  return vend;
 }
 
 // (row, community) tables.  Integral weights: a 32-bit key (row << 18 |
@@ -541,23 +587,28 @@ struct Table {
     return reinterpret_cast<uint32_t*>(slot);
   }
   static __device__ __forceinline__ uint32_t* sum_of(unsigned long long* slot) { return key_of(slot) + kSlots; }
-  static __device__ __forceinline__ void insert(unsigned long long* slot, int32_t* ncl, uint16_t* claimed, int j,
+  // GUARD: the keys may be more than the list of claimed slots holds; false if so
+  template <bool GUARD>
+  static __device__ __forceinline__ bool insert(unsigned long long* slot, int32_t* ncl, uint16_t* claimed, int j,
                                                 int32_t c, double w) {
     uint32_t *keys = key_of(slot), *sums = sum_of(slot);
     const uint32_t key = ((uint32_t)j << kCommBits) | (uint32_t)c;
     uint32_t h = (uint32_t)(((unsigned long long)key * 0x9E3779B97F4A7C15ull) >> (64 - Tile<NT>::kLog));
-    for (int p = 0; p < kSlots; ++p) {   // at most half the slots are ever taken
+    for (int p = 0; p < kSlots; ++p) {   // a tile takes at most half the slots
       uint32_t cur = *reinterpret_cast<volatile uint32_t*>(&keys[h]);
       if (cur == kNoKey) {
         cur = atomicCAS(&keys[h], kNoKey, key);
         if (cur == kNoKey) {
-          claimed[atomicAdd(ncl, 1)] = (uint16_t)h;
+          const int n = atomicAdd(ncl, 1);
+          if (GUARD && n >= kTile) return false;
+          claimed[n] = (uint16_t)h;
           cur = key;
         }
       }
-      if (cur == key) { atomicAdd(&sums[h], (uint32_t)w); return; }
+      if (cur == key) { atomicAdd(&sums[h], (uint32_t)w); return true; }
       h = (h + 1) & (kSlots - 1);
     }
+    return false;
   }
   static __device__ __forceinline__ void get(unsigned long long* slot, int s, int& j, int32_t& c, double& w) {
     const uint32_t key = key_of(slot)[s];
@@ -577,17 +628,23 @@ struct Table<NT, false> {
   static constexpr int kTile = Tile<NT>::kF64;
   static constexpr int kHalf = Tile<NT>::kSlots / 2;   // keys below, FP64 sums above
   static constexpr int kUsed = kHalf;
-  static __device__ __forceinline__ void insert(unsigned long long* slot, int32_t* ncl, uint16_t* claimed, int j,
+  template <bool GUARD>
+  static __device__ __forceinline__ bool insert(unsigned long long* slot, int32_t* ncl, uint16_t* claimed, int j,
                                                 int32_t c, double w) {
     const unsigned long long key = ((unsigned long long)j << 32) | (uint32_t)c;
     double* sum = reinterpret_cast<double*>(slot + kHalf);
     uint32_t h = (uint32_t)((key * 0x9E3779B97F4A7C15ull) >> (64 - Tile<NT>::kLog + 1));
     for (int p = 0; p < kHalf; ++p) {
       const unsigned long long prev = atomicCAS(&slot[h], kEmpty, key);
-      if (prev == kEmpty) claimed[atomicAdd(ncl, 1)] = (uint16_t)h;
-      if (prev == kEmpty || prev == key) { atomicAdd(&sum[h], w); return; }
+      if (prev == kEmpty) {
+        const int n = atomicAdd(ncl, 1);
+        if (GUARD && n >= kTile) return false;
+        claimed[n] = (uint16_t)h;
+      }
+      if (prev == kEmpty || prev == key) { atomicAdd(&sum[h], w); return true; }
       h = (h + 1) & (kHalf - 1);
     }
+    return false;
   }
   static __device__ __forceinline__ void get(unsigned long long* slot, int s, int& j, int32_t& c, double& w) {
     const unsigned long long key = slot[s];
@@ -601,9 +658,67 @@ struct Table<NT, false> {
   }
 };
 
-// A later pass: rows hashed tile by tile.
+// A row longer than a tile, in a later pass: its communities are split by a
+// second hash into as many parts as leave a part half a tile on average, and
+// the row is read once for each.  A part that overflows all the same leaves
+// the level open.
 template <typename X, bool INT>
-__device__ __forceinline__ void moves_hash_body(const List L, int32_t v, int32_t vend, bool last_pass) {
+__device__ __noinline__ void long_hash(const List L, int32_t v, bool last_pass) {
+  using Tab = Table<X::NT, INT>;
+  auto& S = X::S();
+  auto& W = X::W();
+  unsigned long long* slot = S.u.slot;
+  const int tid = threadIdx.x;
+  const int32_t beg = W.roff[v], end = W.roff[v + 1], own = W.comm[v];
+  const double kf = W.kfrac[v];
+  int parts = 0;
+  while (((Tab::kTile / 2) << parts) < end - beg) ++parts;
+  if (tid == 0) S.saw = 0;
+  __syncthreads();
+  double bg = 0.0, bw = 0.0;
+  int32_t bc = kNone, nseg = 0;
+  bool full = false, saw = false;
+#pragma unroll 1
+  for (uint32_t part = 0; part < (1u << parts); ++part) {
+#pragma unroll 2
+    for (int32_t e = beg + tid; e < end; e += X::NT) {
+      const int32_t d = L.dst[e];
+      if (d == v) continue;
+      const int32_t c = W.comm[d];
+      saw |= c == own;
+      if (parts == 0 || (uint32_t)(((uint64_t)(uint32_t)c * 0xD6E8FEB86659FD93ull) >> (64 - parts)) == part)
+        if (!Tab::template insert<true>(slot, &S.nclaimed, S.claimed, 0, c, merged_w(L.w[e]))) full = true;
+    }
+    __syncthreads();
+    const int nc = min(S.nclaimed, Tab::kTile);
+    nseg += nc;
+#pragma unroll 1
+    for (int x = tid; x < nc; x += X::NT) {
+      const int sl = S.claimed[x];
+      int j;
+      int32_t c;
+      double w;
+      Tab::get(slot, sl, j, c, w);
+      Tab::clear(slot, sl);
+      if (w != 0.0) {
+        const double g = __dsub_rn(w, __dmul_rn(W.tot[c], kf));
+        if (g > 0.0 && better(g, c, bg, bc)) { bg = g; bc = c; bw = w; }
+      }
+    }
+    __syncthreads();
+    if (tid == 0) S.nclaimed = 0;
+    __syncthreads();
+  }
+  if (saw) S.saw = 1;
+  if (full) atomicOr(&W.ctl->flags2, fFull);
+  block_best<X>(bg, bc, bw);   // (its barriers order saw too)
+  if (tid == 0) decide<X, false>(v, own, bc, bw, nseg + ((W.hasl[v] && !S.saw) ? 1 : 0), last_pass);
+  __syncthreads();
+}
+
+// A later pass: rows hashed tile by tile.  Returns as moves_first_body.
+template <typename X, bool INT>
+__device__ __forceinline__ int32_t moves_hash_body(const List L, int32_t v, int32_t vend, bool last_pass) {
   constexpr int NT = X::NT;
   using Tab = Table<NT, INT>;
   constexpr int kItems = Tab::kTile / NT;
@@ -618,7 +733,7 @@ __device__ __forceinline__ void moves_hash_body(const List L, int32_t v, int32_t
 #pragma unroll 1
   while (v < vend) {
     const int nv = tile_rows<X>(W.roff, v, vend, Tab::kTile);
-    if (nv == 0) return;   // cannot happen, as above
+    if (nv == 0) return v;
     const int32_t base = W.roff[v];
     const int n = W.roff[v + nv] - base;
     if (n > 0) {
@@ -653,7 +768,7 @@ __device__ __forceinline__ void moves_hash_body(const List L, int32_t v, int32_t
       for (int q = 0; q < kItems; ++q) {
         if (jj[q] >= 0) {
           if (cc[q] == S.own[jj[q]]) atomicOr(&S.nseg[jj[q]], 1 << 30);
-          Tab::insert(slot, &S.nclaimed, S.claimed, jj[q], cc[q], wd[q]);
+          Tab::template insert<false>(slot, &S.nclaimed, S.claimed, jj[q], cc[q], wd[q]);
         }
       }
       __syncthreads();
@@ -710,16 +825,37 @@ __device__ __forceinline__ void moves_hash_body(const List L, int32_t v, int32_t
     }
     v += nv;
   }
+  return vend;
 }
 
-// Out of line over device memory, where registers are short.
+// Over device memory: out of line, where registers are short, with the long
+// rows between (inside the tiles' loops they cost every graph 2-3 %).  A level
+// in shared memory has no row longer than a tile.
 template <typename X>
-__device__ __noinline__ void moves_first_call(const List L, int32_t v, int32_t vend, bool last) {
-  moves_first_body<X>(L, v, vend, last);
+__device__ __noinline__ int32_t moves_first_call(const List L, int32_t v, int32_t vend, bool last) {
+  return moves_first_body<X>(L, v, vend, last);
 }
 template <typename X, bool INT>
-__device__ __noinline__ void moves_hash_call(const List L, int32_t v, int32_t vend, bool last) {
-  moves_hash_body<X, INT>(L, v, vend, last);
+__device__ __noinline__ int32_t moves_hash_call(const List L, int32_t v, int32_t vend, bool last) {
+  return moves_hash_body<X, INT>(L, v, vend, last);
+}
+template <typename X>
+__device__ __forceinline__ void moves_first(const List L, int32_t v, int32_t vend, bool last) {
+  if constexpr (X::kResident) {
+    moves_first_body<X>(L, v, vend, last);
+  } else {
+#pragma unroll 1
+    while ((v = moves_first_call<X>(L, v, vend, last)) < vend) long_first<X>(L, v++, last);
+  }
+}
+template <typename X, bool INT>
+__device__ __forceinline__ void moves_hash(const List L, int32_t v, int32_t vend, bool last) {
+  if constexpr (X::kResident && INT) {
+    moves_hash_body<X, INT>(L, v, vend, last);
+  } else {
+#pragma unroll 1
+    while ((v = moves_hash_call<X, INT>(L, v, vend, last)) < vend) long_hash<X, INT>(L, v++, last);
+  }
 }
 
 struct Committed {
@@ -1168,7 +1304,6 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
     const double m = finish_sum<X>(W.mpart, E);
     const double twom = __dmul_rn(2.0, m);
     {
-      const int32_t longest = integral ? Tile<NT>::kInt : Tile<NT>::kF64;
       uint32_t f = 0;
       group_partials<X>(
           T, V, W.qpart, [&](int64_t i) { return Row{W.k[i], W.loopw[i], W.roff[i + 1] - W.roff[i]}; },
@@ -1183,7 +1318,7 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
             W.cand[i] = -1;
             W.kfrac[i] = m > 0.0 ? __ddiv_rn(r.k, twom) : 0.0;   // OneLevelKernel.cu:307
             W.minidx[i] = kNone;
-            if (r.len > longest) f |= fUnfit;
+            if (r.len > Tile<NT>::kF64) f |= r.len > kLongRow ? fUnfit : fLong;
             if (!(r.k < 1073741824.0)) f |= fNotInt;
             return q_term(x, r.k, m, twom);
           });
@@ -1192,8 +1327,7 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
     if (!T.sync()) return false;
     const uint32_t f2 = W.ctl->flags2;
     const bool packed = integral && !(f2 & fNotInt);
-    // sums beyond 32 bits take the FP64 tiles, whose rows are shorter
-    if ((f2 & fUnfit) || (integral && !packed)) { at.open = true; return true; }
+    if (f2 & fUnfit) { at.open = true; return true; }
     const double q0 = finish_sum<X>(W.qpart, V);
     at.lower = level == 0 ? q0 : at.mod;        // LouvainCPP.cpp:356,446
     find_rows<X>(T, V, E);
@@ -1212,15 +1346,14 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
       const bool stop = __dsub_rn(q_prev, floor_q) < cfg.pass_min;
       const bool capped = cfg.max_passes >= 0 && pass >= cfg.max_passes;
       if (pass == 1) {
-        if constexpr (X::kResident) moves_first_body<X>(L, v0, v1, stop || capped);
-        else moves_first_call<X>(L, v0, v1, stop || capped);
+        moves_first<X>(L, v0, v1, stop || capped);
       } else if (packed) {
-        if constexpr (X::kResident) moves_hash_body<X, true>(L, v0, v1, stop || capped);
-        else moves_hash_call<X, true>(L, v0, v1, stop || capped);
+        moves_hash<X, true>(L, v0, v1, stop || capped);
       } else {
-        moves_hash_call<X, false>(L, v0, v1, stop || capped);
+        moves_hash<X, false>(L, v0, v1, stop || capped);
       }
       if (!T.sync()) return false;
+      if ((f2 & fLong) && (W.ctl->flags2 & fFull)) { at.open = true; return true; }
       if (pass <= 2) pass_ticks[pass - 1] = (float)(clock64() - p0);
       if (stop || capped) {
         st = stop ? LVG_OK : LVG_ERR_NOT_CONVERGED;

@@ -59,7 +59,7 @@ def graph(gen, oracle, name):
     return gen.sbm(n, max(2, n // 60), 0.25, 3.0 / n, 1, 4, seed=n)
 
 
-NAMES = ["one:", "loop:", "star:4095", "star:4096", "star:4097", "star:9000", "stars8:2048", "stars8:2049",
+NAMES = ["one:", "loop:", "star:4095", "star:4096", "star:4097", "star:9000", "star:66000", "stars8:2048", "stars8:2049",
          "isolated:65536", "isolated:65537", "case:loops_zeros_isolated", "case:odd_sizes", "case:weighted",
          "eighths:900", "eighths:4001", "heavy:", "dense:64", "dense:511", "dense:513", "sbm:70", "sbm:1025",
          "sbm:2049", "sbm:8193", "sbm:14001"]
@@ -76,7 +76,7 @@ def test_run_equals_the_oracle(Louvain, oracle, gen, name):
             run_equal(lv, lv.run(), orun, n, s, d, w, oracle)
 
 
-@pytest.mark.parametrize("name", ["sbm:1025", "eighths:900", "star:4097", "case:loops_zeros_isolated"])
+@pytest.mark.parametrize("name", ["sbm:1025", "eighths:900", "star:4097", "star:9000", "case:loops_zeros_isolated"])
 def test_calls_after_a_run_see_its_last_level(Louvain, oracle, gen, name):
     """The last level's CSR, Q and list, its coarsening, and a step-by-step
     run on the same load, after a run that built none of its levels."""
