@@ -459,7 +459,9 @@ bool run_small(lvg_ctx* c, RunState& R) {
   a.hi = c->run_hi;
   constexpr int kRoomLevels = 12;
   const int64_t parts_cap = 2 * (int64_t)kRoomLevels * V;
-  const size_t need = small_list_bytes(E) + small_work_bytes(V, E) + sizeof(int32_t) * ((size_t)parts_cap + V) +
+  // level 0: checked at load; later lists are symmetric when their CSR was written
+  const bool any_order = c->level > 0 && !c->pre_next.valid;
+  const size_t need = small_list_bytes(E) + small_work_bytes(V, E, any_order) + sizeof(int32_t) * ((size_t)parts_cap + V) +
                       sizeof(SmallOut) + sizeof(SmallJob) + 16 * Arena::kAlign;
   if (a.hi < a.lo || a.hi - a.lo < need) return false;
   c->pristine = false;
@@ -476,13 +478,12 @@ bool run_small(lvg_ctx* c, RunState& R) {
   J.parts = a.hi_n<int32_t>(parts_cap);
   J.parts_cap = parts_cap;
   const size_t run_hi = a.hi;
-  // level 0: checked at load; later lists are symmetric when their CSR was written
-  J.check = c->level == 0 || c->pre_next.valid ? 0 : 1;
+  J.check = J.dbl = any_order ? 1 : 0;
   J.want_q = c->level == 0 ? 1 : 0;
   SmallOut o;
   {
     HiScope hs(a);
-    J.work = (char*)a.alloc_hi(small_work_bytes(V, E));
+    J.work = (char*)a.alloc_hi(small_work_bytes(V, E, any_order));
     J.comp = c->level == 0 ? c->composed : a.hi_n<int32_t>(V);
     SmallOut* d_out = a.hi_n<SmallOut>(1);
     J.res = &d_out->res;
@@ -491,7 +492,7 @@ bool run_small(lvg_ctx* c, RunState& R) {
     LVG_CUDA(cudaMemcpyAsync(d_job, &J, sizeof J, cudaMemcpyHostToDevice, s));
     const SmallCfg cfg{c->cfg.pass_min_gain, c->cfg.level_min_gain, c->cfg.max_passes, c->cfg.max_levels};
     LVG_CUDA(cudaMemsetAsync(J.res, 0, sizeof(SmallResult), s));
-    if (E <= kSmallClusterEntries) small_run(d_job, 1, kSmallClusterBlocks, cfg, s);
+    if (E + V <= kSmallClusterEntries) small_run(d_job, 1, kSmallClusterBlocks, cfg, s);
     else small_run_grid(d_job, J.work, small_grid_blocks(), cfg, s);
     LVG_CUDA(cudaMemcpyAsync(&o, d_out, sizeof o, cudaMemcpyDeviceToHost, s));
     if (c->level > 0) {   // a launch that finishes no level leaves no composition
@@ -1592,7 +1593,7 @@ SmallBatch batch_small_start(lvg_ctx* c, const BatchInput& in, int32_t* part_d) 
   int64_t others = in.eoff[in.G], other_v = in.voff[in.G];
   for (int32_t g : which) {
     lists += Arena::up(small_list_bytes(entries(g)));
-    work += Arena::up(small_work_bytes(in.voff[g + 1] - in.voff[g], entries(g)));
+    work += Arena::up(small_work_bytes(in.voff[g + 1] - in.voff[g], entries(g), false));
     others -= entries(g);
     other_v -= in.voff[g + 1] - in.voff[g];
   }
@@ -1619,7 +1620,7 @@ SmallBatch batch_small_start(lvg_ctx* c, const BatchInput& in, int32_t* part_d) 
     J.lists = lp;
     J.work = wp;
     lp += Arena::up(small_list_bytes(J.E));
-    wp += Arena::up(small_work_bytes(J.V, J.E));
+    wp += Arena::up(small_work_bytes(J.V, J.E, false));
     J.comp = part_d + in.voff[g];
     J.res = B.res + k;
     J.check = 1;

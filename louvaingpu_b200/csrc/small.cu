@@ -9,22 +9,24 @@
 // a batch each graph has its own cluster, so the graphs' levels need not wait
 // for one another.
 //
-// A level's list is strictly sorted by (src, dst) and symmetric, so a row is a
-// contiguous range of the list and the merged CSR entry of (u, v, w) is
-// (u, v, 2w); no CSR is written.  The rules are the level kernels' (rules.cuh):
+// Where a level's list is strictly sorted by (src, dst) and symmetric, a row is
+// a contiguous range of the list and the merged CSR entry of (u, v, w) is
+// (u, v, 2w); no CSR is written.  Other lists (coarse ones of a graph whose
+// edges are listed once) have the doubled list sorted and merged into a CSR
+// first.  The rules are the level kernels' (rules.cuh):
 //   build    row starts, degrees and self loops from one pass over the list,
 //            m and every Q on the fixed tree
 //   pass 1   singletons: the best candidate of a row is an argmax over its
 //            entries (segmented warp argmax, then shared-memory max / min)
 //   pass 2+  tiles of consecutive rows hashed as (row, community) pairs in
 //            shared memory: 32-bit keys and sums when the weights are integral,
-//            key + FP64 sum otherwise; a row longer than a tile is a block's
-//            work alone, its communities split over several tables in turn
+//            key + FP64 sum otherwise; rows longer than a tile in tables in
+//            device memory, by all blocks
 //   renumber by smallest member; coarse keys (cu << b | cv) sorted by a stable
 //            LSD radix sort across the cluster, runs summed in FP64
-// A list that is not sorted and symmetric, a row beyond kLongRow, or more
-// levels or passes than the tables hold end the launch with the level left
-// open; the caller goes on with the level kernels from the same list.
+// A list in any order without room for its CSR, or more levels or passes than
+// the tables hold, end the launch with the level left open; the caller goes on
+// with the level kernels from the same list.
 #include <algorithm>
 #include <cooperative_groups.h>
 #include <mutex>
@@ -54,14 +56,16 @@ struct Tile {
 constexpr int kCommBits = 18;              // community bits of a packed key
 constexpr int kDigits = 256;
 constexpr int64_t kGridEntries = 4096;     // grid mode: entries a block, at least
-constexpr int kLongRow = 1 << 16;          // longest row (32 parts: the row is read 32 times a pass by one block)
+constexpr int kShortRow = kItems * 512 / 2;   // the smaller blocks' FP64 tile: no row up to this is long
+constexpr int kGaps = 64;                  // runs of empty rows a block fills together
+constexpr int kHubs = 32;                  // long rows a block looks up at a time
 constexpr int kResThreads = 512;
 constexpr int kResV = 512, kResE = 6144;   // a level this small lives in one block's shared memory
 constexpr unsigned long long kWaitNs = 4000000000ull;   // limit of a grid barrier's wait
 constexpr unsigned long long kEmpty = ~0ull;
 static_assert(kSmallMaxV <= (1 << kCommBits), "packed keys hold 18-bit communities");
 
-enum : uint32_t { fNotInt = 1u, fUnfit = 2u, fBad = 4u, fUnsorted = 8u, fFull = 16u, fLong = 32u };
+enum : uint32_t { fNotInt = 1u, fBad = 4u, fUnsorted = 8u, fLong = 16u };
 // kPhaseMid: the grid left the level to a cluster; kPhaseTail: a level fits
 // one block's shared memory; kPhaseEnd: the levels are done.
 enum : int32_t { kPhaseNone = 0, kPhaseMid = 1, kPhaseTail = 2, kPhaseEnd = 3 };
@@ -70,6 +74,7 @@ enum : int32_t { kCompDone = 0, kCompTail = 1, kCompTailAll = 2 };
 // Control words of a level's blocks.
 struct Ctl {
   uint32_t flags, flags2, check, loops;
+  uint32_t nlong;               // rows in Work::longs
   unsigned long long sums[2];
   uint32_t count[2][kSmallMaxBlocks];
   unsigned long long arrived;   // grid barrier: arrivals so far
@@ -100,12 +105,17 @@ struct Work {
   int32_t* rc;               // composition of the resident levels
   float* val[2];
   double* wsum;
+  int32_t* longs;            // rows longer than a tile of FP64 sums
+  int32_t *csrc, *cdst;      // CSR of a list that is not symmetric, row by row
+  float* cw;
 };
 
 __host__ __device__ inline size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-__host__ __device__ inline size_t carve(char* base, int64_t V, int64_t E, Work& W) {
+// dbl: room for the doubled list of a level and the CSR made from it.
+__host__ __device__ inline size_t carve(char* base, int64_t V, int64_t E, bool dbl, Work& W) {
   size_t o = 0;
+  const int64_t n = dbl ? 2 * E : E;
   auto take = [&](size_t bytes) {
     char* p = base + o;
     o += up256(bytes);
@@ -129,11 +139,15 @@ __host__ __device__ inline size_t carve(char* base, int64_t V, int64_t E, Work& 
   W.newid = (int32_t*)take(4 * V);
   W.loopw = (float*)take(4 * V);
   W.hasl = (int32_t*)take(4 * V);
-  W.key[0] = (uint64_t*)take(8 * E);
-  W.key[1] = (uint64_t*)take(8 * E);
-  W.val[0] = (float*)take(4 * E);
-  W.val[1] = (float*)take(4 * E);
-  W.wsum = (double*)take(8 * E);
+  W.key[0] = (uint64_t*)take(8 * n);
+  W.key[1] = (uint64_t*)take(16 * n);   // wsum behind it: together the sums of the long rows' tables
+  W.wsum = (double*)W.key[1] + n;
+  W.val[0] = (float*)take(4 * n);
+  W.val[1] = (float*)take(4 * n);
+  W.csrc = dbl ? (int32_t*)take(4 * n) : nullptr;
+  W.cdst = dbl ? (int32_t*)take(4 * n) : nullptr;
+  W.cw = dbl ? (float*)take(4 * n) : nullptr;
+  W.longs = (int32_t*)take(4 * (n / kShortRow + 1));
   W.ghist = (uint32_t*)take(4 * kDigits * kSmallMaxBlocks);
   W.rc = (int32_t*)take(4 * kResV);
   return o;
@@ -189,7 +203,9 @@ struct Space {
   uint32_t wtot[NT / 32];
   double rg[NT / 32], rw[NT / 32];   // long rows: each warp's best candidate
   int32_t rc[NT / 32];
-  int32_t saw;
+  int32_t nhub, hub[kHubs];
+  int32_t ngap;
+  int4 gap[kGaps];
   int32_t nclaimed, row0, row1;
   unsigned long long goal;   // grid barrier: arrivals awaited
   int32_t alive;
@@ -389,18 +405,52 @@ __device__ __forceinline__ void find_rows(const Team<X> T, int32_t V, int64_t E)
   const int64_t x0 = E * T.rank() / T.K(), x1 = E * (T.rank() + 1) / T.K();
   if (threadIdx.x == 0) {   // a share that starts or ends at entry 0 does so at row 0
     S.row0 = 0;
-    S.row1 = T.rank() == T.K() - 1 ? V : 0;
+    S.row1 = T.K() == 1 ? V : 0;
   }
   __syncthreads();
-  if (T.K() > 1) {
+  if (T.K() > 1) {   // (the rows behind the last entry are nobody's: they have nothing to decide)
     const int32_t* roff = X::W().roff;
 #pragma unroll 2
     for (int32_t v = 1 + (int)threadIdx.x; v <= V; v += X::NT) {
       const int32_t a = roff[v - 1], b = roff[v];
       if (T.rank() > 0 && a < x0 && b >= x0) S.row0 = v;
-      if (T.rank() < T.K() - 1 && a < x1 && b >= x1) S.row1 = v;
+      if (a < x1 && b >= x1) S.row1 = v;
     }
     __syncthreads();
+  }
+}
+
+// Rows r0..r1 start at entry e: few of them by the thread that met them, many
+// by its block (long_gaps).  A coarse list ends in a gap of all vertices
+// without edges: 189,000 written by one thread took 5.2 ms a level.
+template <typename X>
+__device__ __forceinline__ void row_starts(int32_t r0, int32_t r1, int32_t e) {
+  auto& S = X::S();
+  if constexpr (!X::kResident) {
+    if (r1 - r0 >= 64) {
+      const int p = atomicAdd(&S.ngap, 1);
+      if (p < kGaps) {
+        S.gap[p] = make_int4(r0, r1, e, 0);
+        return;
+      }
+    }
+  }
+  int32_t* roff = X::W().roff;
+#pragma unroll 1
+  for (int32_t r = r0; r <= r1; ++r) roff[r] = e;
+}
+
+template <typename X>
+__device__ __forceinline__ void long_gaps() {
+  auto& S = X::S();
+  int32_t* roff = X::W().roff;
+  __syncthreads();
+  const int n = min(S.ngap, kGaps);
+#pragma unroll 1
+  for (int g = 0; g < n; ++g) {
+    const int4 x = S.gap[g];
+#pragma unroll 2
+    for (int32_t r = x.x + (int)threadIdx.x; r <= x.y; r += X::NT) roff[r] = x.z;
   }
 }
 
@@ -428,13 +478,18 @@ __device__ __forceinline__ int tile_rows(const int32_t* roff, int32_t v0, int32_
   return __syncthreads_count(v <= vend && roff[v] - base <= cap);
 }
 
+// A list's rows: those of a symmetric list as it is (self loops among them,
+// each entry standing for itself and its mirror), or of a merged CSR.
 struct List {
   const int32_t* src;
   const int32_t* dst;
   const float* w;
+  float copies;              // of an entry in the merged doubled list: 2, or 1 once merged
+  __device__ __forceinline__ int32_t loop_apart(int32_t hasl) const { return copies == 1.0f ? hasl : 0; }
 };
 
-__device__ __forceinline__ double merged_w(float w) { return (double)__double2float_rn(__dadd_rn((double)w, (double)w)); }
+// Weight of a row's entry in the merged doubled list.
+__device__ __forceinline__ double merged_w(const List& L, float w) { return (double)__fmul_rn(w, L.copies); }
 
 // The block's best candidate from each thread's, in thread 0.
 template <typename X>
@@ -467,12 +522,12 @@ __device__ __noinline__ void long_first(const List L, int32_t v, bool last_pass)
 #pragma unroll 4
   for (int32_t e = beg + (int)threadIdx.x; e < end; e += X::NT) {
     const int32_t c = L.dst[e];
-    const double w = merged_w(L.w[e]);
+    const double w = merged_w(L, L.w[e]);
     const double g = __dsub_rn(w, __dmul_rn(W.k[c], kf));
     if (c != v && w != 0.0 && g > 0.0 && better(g, c, bg, bc)) { bg = g; bc = c; bw = w; }
   }
   block_best<X>(bg, bc, bw);
-  if (threadIdx.x == 0) decide<X, true>(v, v, bc, bw, end - beg, last_pass);
+  if (threadIdx.x == 0) decide<X, true>(v, v, bc, bw, end - beg + L.loop_apart(W.hasl[v]), last_pass);
 }
 
 // First pass of a level: every neighbour is its own candidate.  Returns the
@@ -507,7 +562,7 @@ __device__ __forceinline__ int32_t moves_first_body(const List L, int32_t v, int
         if (x < n) {
           jj[q] = L.src[base + x] - v;
           cc[q] = L.dst[base + x];
-          wd[q] = merged_w(L.w[base + x]);
+          wd[q] = merged_w(L, L.w[base + x]);
         }
       }
 #pragma unroll
@@ -564,7 +619,8 @@ __device__ __forceinline__ int32_t moves_first_body(const List L, int32_t v, int
         const int32_t i = v + tid, len = W.roff[i + 1] - W.roff[i];
         const int32_t c = S.bestc[tid];
         // distinct candidates: one per neighbour, and the own community with a self loop
-        if (len > 0) decide<X, true>(i, i, c, c == kNone ? 0.0 : S.bestw[tid], len, last_pass);
+        if (len > 0)
+          decide<X, true>(i, i, c, c == kNone ? 0.0 : S.bestw[tid], len + L.loop_apart(W.hasl[i]), last_pass);
       }
       __syncthreads();
     }
@@ -587,9 +643,7 @@ struct Table {
     return reinterpret_cast<uint32_t*>(slot);
   }
   static __device__ __forceinline__ uint32_t* sum_of(unsigned long long* slot) { return key_of(slot) + kSlots; }
-  // GUARD: the keys may be more than the list of claimed slots holds; false if so
-  template <bool GUARD>
-  static __device__ __forceinline__ bool insert(unsigned long long* slot, int32_t* ncl, uint16_t* claimed, int j,
+  static __device__ __forceinline__ void insert(unsigned long long* slot, int32_t* ncl, uint16_t* claimed, int j,
                                                 int32_t c, double w) {
     uint32_t *keys = key_of(slot), *sums = sum_of(slot);
     const uint32_t key = ((uint32_t)j << kCommBits) | (uint32_t)c;
@@ -599,16 +653,13 @@ struct Table {
       if (cur == kNoKey) {
         cur = atomicCAS(&keys[h], kNoKey, key);
         if (cur == kNoKey) {
-          const int n = atomicAdd(ncl, 1);
-          if (GUARD && n >= kTile) return false;
-          claimed[n] = (uint16_t)h;
+          claimed[atomicAdd(ncl, 1)] = (uint16_t)h;
           cur = key;
         }
       }
-      if (cur == key) { atomicAdd(&sums[h], (uint32_t)w); return true; }
+      if (cur == key) { atomicAdd(&sums[h], (uint32_t)w); return; }
       h = (h + 1) & (kSlots - 1);
     }
-    return false;
   }
   static __device__ __forceinline__ void get(unsigned long long* slot, int s, int& j, int32_t& c, double& w) {
     const uint32_t key = key_of(slot)[s];
@@ -628,23 +679,17 @@ struct Table<NT, false> {
   static constexpr int kTile = Tile<NT>::kF64;
   static constexpr int kHalf = Tile<NT>::kSlots / 2;   // keys below, FP64 sums above
   static constexpr int kUsed = kHalf;
-  template <bool GUARD>
-  static __device__ __forceinline__ bool insert(unsigned long long* slot, int32_t* ncl, uint16_t* claimed, int j,
+  static __device__ __forceinline__ void insert(unsigned long long* slot, int32_t* ncl, uint16_t* claimed, int j,
                                                 int32_t c, double w) {
     const unsigned long long key = ((unsigned long long)j << 32) | (uint32_t)c;
     double* sum = reinterpret_cast<double*>(slot + kHalf);
     uint32_t h = (uint32_t)((key * 0x9E3779B97F4A7C15ull) >> (64 - Tile<NT>::kLog + 1));
     for (int p = 0; p < kHalf; ++p) {
       const unsigned long long prev = atomicCAS(&slot[h], kEmpty, key);
-      if (prev == kEmpty) {
-        const int n = atomicAdd(ncl, 1);
-        if (GUARD && n >= kTile) return false;
-        claimed[n] = (uint16_t)h;
-      }
-      if (prev == kEmpty || prev == key) { atomicAdd(&sum[h], w); return true; }
+      if (prev == kEmpty) claimed[atomicAdd(ncl, 1)] = (uint16_t)h;
+      if (prev == kEmpty || prev == key) { atomicAdd(&sum[h], w); return; }
       h = (h + 1) & (kHalf - 1);
     }
-    return false;
   }
   static __device__ __forceinline__ void get(unsigned long long* slot, int s, int& j, int32_t& c, double& w) {
     const unsigned long long key = slot[s];
@@ -658,62 +703,162 @@ struct Table<NT, false> {
   }
 };
 
-// A row longer than a tile, in a later pass: its communities are split by a
-// second hash into as many parts as leave a part half a tile on average, and
-// the row is read once for each.  A part that overflows all the same leaves
-// the level open.
+// Rows longer than a tile, in a later pass.  Each has a table of its own in
+// device memory, twice as many slots as entries (keys over key[0], FP64 sums
+// over key[1] and wsum, which the sort does not need meanwhile), so that the
+// whole team works on it: a block reads the entries of long rows within its
+// share of the list, adds them up in shared memory a tile at a time, and adds
+// each tile's communities to the row's table (hub_insert); then a block per
+// row takes the best and leaves the table empty (hub_pick).  One block alone,
+// hashing a row of 60,000 entries part by part in shared memory, took 1 ms a
+// pass with integral weights and 7 with others.
+template <typename X>
+struct HubTable {
+  int32_t* key;
+  double* sum;
+  uint32_t slots;
+  __device__ __forceinline__ explicit HubTable(int32_t v) {
+    auto& W = X::W();
+    const int64_t beg = W.roff[v];
+    key = (int32_t*)W.key[0] + 2 * beg;
+    sum = (double*)W.key[1] + 2 * beg;
+    slots = 2u * (uint32_t)(W.roff[v + 1] - beg);
+  }
+};
+
+template <typename X>
+__device__ __noinline__ void hub_clear(const Team<X> T) {
+  auto& W = X::W();
+  const int n = (int)W.ctl->nlong;
+#pragma unroll 1
+  for (int i = T.rank(); i < n; i += T.K()) {
+    const HubTable<X> H(W.longs[i]);
+#pragma unroll 4
+    for (uint32_t x = threadIdx.x; x < H.slots; x += X::NT) {
+      H.key[x] = kNone;
+      H.sum[x] = 0.0;
+    }
+  }
+}
+
+// (Behind moves_hash, which leaves its table empty.)
 template <typename X, bool INT>
-__device__ __noinline__ void long_hash(const List L, int32_t v, bool last_pass) {
+__device__ __noinline__ void hub_insert(const Team<X> T, const List L, int64_t E) {
   using Tab = Table<X::NT, INT>;
   auto& S = X::S();
   auto& W = X::W();
   unsigned long long* slot = S.u.slot;
   const int tid = threadIdx.x;
-  const int32_t beg = W.roff[v], end = W.roff[v + 1], own = W.comm[v];
-  const double kf = W.kfrac[v];
-  int parts = 0;
-  while (((Tab::kTile / 2) << parts) < end - beg) ++parts;
-  if (tid == 0) S.saw = 0;
-  __syncthreads();
-  double bg = 0.0, bw = 0.0;
-  int32_t bc = kNone, nseg = 0;
-  bool full = false, saw = false;
+  const int n = (int)W.ctl->nlong;
+  const int32_t x0 = (int32_t)(E * T.rank() / T.K()), x1 = (int32_t)(E * (T.rank() + 1) / T.K());
 #pragma unroll 1
-  for (uint32_t part = 0; part < (1u << parts); ++part) {
-#pragma unroll 2
-    for (int32_t e = beg + tid; e < end; e += X::NT) {
-      const int32_t d = L.dst[e];
-      if (d == v) continue;
-      const int32_t c = W.comm[d];
-      saw |= c == own;
-      if (parts == 0 || (uint32_t)(((uint64_t)(uint32_t)c * 0xD6E8FEB86659FD93ull) >> (64 - parts)) == part)
-        if (!Tab::template insert<true>(slot, &S.nclaimed, S.claimed, 0, c, merged_w(L.w[e]))) full = true;
+  for (int i0 = 0; i0 < n; i0 += X::NT) {
+    const int32_t v = i0 + tid < n ? W.longs[i0 + tid] : -1;
+    bool mine = false;
+    if (v >= 0) {
+      const int32_t beg = W.roff[v], end = W.roff[v + 1];
+      mine = end - beg > Tab::kTile && beg < x1 && end > x0;
     }
-    __syncthreads();
-    const int nc = min(S.nclaimed, Tab::kTile);
-    nseg += nc;
+    for (;;) {   // a few of the rows at a time
+      if (tid == 0) S.nhub = 0;
+      __syncthreads();
+      if (mine) {
+        const int p = atomicAdd(&S.nhub, 1);
+        if (p < kHubs) {
+          S.hub[p] = v;
+          mine = false;
+        }
+      }
+      __syncthreads();
+      const int found = min(S.nhub, kHubs);
 #pragma unroll 1
-    for (int x = tid; x < nc; x += X::NT) {
-      const int sl = S.claimed[x];
-      int j;
-      int32_t c;
-      double w;
-      Tab::get(slot, sl, j, c, w);
-      Tab::clear(slot, sl);
+      for (int h = 0; h < found; ++h) {
+        const int32_t row = S.hub[h];
+        const HubTable<X> H(row);
+        const int32_t lo = max(W.roff[row], x0), hi = min(W.roff[row + 1], x1);
+#pragma unroll 1
+        for (int32_t e0 = lo; e0 < hi; e0 += Tab::kTile) {
+#pragma unroll 4
+          for (int q = 0; q < Tab::kTile / X::NT; ++q) {
+            const int32_t e = e0 + q * X::NT + tid;
+            if (e < hi) {
+              const int32_t d = L.dst[e];
+              if (d != row) Tab::insert(slot, &S.nclaimed, S.claimed, 0, W.comm[d], merged_w(L, L.w[e]));
+            }
+          }
+          __syncthreads();
+          const int nc = S.nclaimed;
+#pragma unroll 1
+          for (int x = tid; x < nc; x += X::NT) {
+            int j;
+            int32_t c;
+            double w;
+            Tab::get(slot, S.claimed[x], j, c, w);
+            Tab::clear(slot, S.claimed[x]);
+            uint32_t at = (uint32_t)(((uint64_t)((uint32_t)c * 0x9E3779B1u) * H.slots) >> 32);
+            for (uint32_t p = 0; p < H.slots; ++p) {   // at most half are ever taken
+              const int32_t cur = atomicCAS(&H.key[at], kNone, c);
+              if (cur == kNone || cur == c) {
+                atomicAdd(&H.sum[at], w);
+                break;
+              }
+              if (++at == H.slots) at = 0;
+            }
+          }
+          __syncthreads();
+          if (tid == 0) S.nclaimed = 0;
+          __syncthreads();
+        }
+      }
+      if (!__syncthreads_or(mine)) break;
+    }
+  }
+}
+
+template <typename X, bool INT>
+__device__ __noinline__ void hub_pick(const Team<X> T, bool last_pass) {
+  auto& S = X::S();
+  auto& W = X::W();
+  const int n = (int)W.ctl->nlong;
+#pragma unroll 1
+  for (int i = T.rank(); i < n; i += T.K()) {
+    const int32_t v = W.longs[i];
+    const HubTable<X> H(v);
+    if (H.slots <= 2u * Table<X::NT, INT>::kTile) continue;
+    if (threadIdx.x == 0) S.nhub = 0;
+    __syncthreads();
+    const double kf = W.kfrac[v];
+    const int32_t own = W.comm[v];
+    double bg = 0.0, bw = 0.0;
+    int32_t bc = kNone;
+    uint32_t met = 0;   // communities, and bit 31: the row's own
+#pragma unroll 4
+    for (uint32_t x = threadIdx.x; x < H.slots; x += X::NT) {
+      const int32_t c = H.key[x];
+      if (c == kNone) continue;
+      const double w = H.sum[x];
+      H.key[x] = kNone;
+      H.sum[x] = 0.0;
+      met = (met + 1) | (c == own ? 1u << 31 : 0u);
       if (w != 0.0) {
         const double g = __dsub_rn(w, __dmul_rn(W.tot[c], kf));
         if (g > 0.0 && better(g, c, bg, bc)) { bg = g; bc = c; bw = w; }
       }
     }
-    __syncthreads();
-    if (tid == 0) S.nclaimed = 0;
+    const uint32_t many = __reduce_add_sync(0xffffffffu, met & 0x7fffffffu);
+    const uint32_t own_met = __reduce_or_sync(0xffffffffu, met & (1u << 31));
+    if ((threadIdx.x & 31) == 0) {
+      atomicAdd(&S.nhub, (int)many);
+      if (own_met) atomicOr(&S.nhub, 1 << 30);   // (sums stay far below)
+    }
+    block_best<X>(bg, bc, bw);   // (its barriers order nhub too)
+    if (threadIdx.x == 0) {
+      const int32_t s = S.nhub;
+      const int32_t nseg = (s & ((1 << 30) - 1)) + ((W.hasl[v] && !(s >> 30)) ? 1 : 0);
+      decide<X, false>(v, own, bc, bw, nseg, last_pass);
+    }
     __syncthreads();
   }
-  if (saw) S.saw = 1;
-  if (full) atomicOr(&W.ctl->flags2, fFull);
-  block_best<X>(bg, bc, bw);   // (its barriers order saw too)
-  if (tid == 0) decide<X, false>(v, own, bc, bw, nseg + ((W.hasl[v] && !S.saw) ? 1 : 0), last_pass);
-  __syncthreads();
 }
 
 // A later pass: rows hashed tile by tile.  Returns as moves_first_body.
@@ -757,7 +902,7 @@ __device__ __forceinline__ int32_t moves_hash_body(const List L, int32_t v, int3
           const int32_t u = L.src[base + x], d = L.dst[base + x];
           if (u != d) jj[q] = u - v;
           cc[q] = d;
-          wd[q] = merged_w(L.w[base + x]);
+          wd[q] = merged_w(L, L.w[base + x]);
         }
       }
 #pragma unroll
@@ -768,7 +913,7 @@ __device__ __forceinline__ int32_t moves_hash_body(const List L, int32_t v, int3
       for (int q = 0; q < kItems; ++q) {
         if (jj[q] >= 0) {
           if (cc[q] == S.own[jj[q]]) atomicOr(&S.nseg[jj[q]], 1 << 30);
-          Tab::template insert<false>(slot, &S.nclaimed, S.claimed, jj[q], cc[q], wd[q]);
+          Tab::insert(slot, &S.nclaimed, S.claimed, jj[q], cc[q], wd[q]);
         }
       }
       __syncthreads();
@@ -854,7 +999,7 @@ __device__ __forceinline__ void moves_hash(const List L, int32_t v, int32_t vend
     moves_hash_body<X, INT>(L, v, vend, last);
   } else {
 #pragma unroll 1
-    while ((v = moves_hash_call<X, INT>(L, v, vend, last)) < vend) long_hash<X, INT>(L, v++, last);
+    while ((v = moves_hash_call<X, INT>(L, v, vend, last)) < vend) ++v;   // hub_insert's
   }
 }
 
@@ -934,87 +1079,38 @@ __device__ __forceinline__ bool cells_fit(int32_t C) {
   return X::kResident && C <= 1024 && C * C <= X::kCells;
 }
 
-// The coarse list of a level of C communities (new ids W.newid of the labels
-// W.comm) into (osrc, odst, ow); returns its length (-1: a barrier's wait ran
-// out).  Stable LSD sort of the entries' keys over the team: block r owns the
-// r-th share of the positions, counts its digits, and places its keys after
-// those of all blocks before it.
-template <typename X, typename Key>
-__device__ __noinline__ int64_t coarsen(const Team<X> T, const List L, int64_t E, int32_t C, bool integral,
-                                        int32_t* osrc, int32_t* odst, float* ow) {
+// Stable LSD sort over the team of n keys by their low `bits` bits, made with
+// their values by gen(i, key, val): block r owns the r-th share of the
+// positions, counts its digits, and places its keys after those of all blocks
+// before it.  Clears wsum.  Returns which of W.key / W.val holds the result
+// (-1: a barrier's wait ran out).
+template <typename X, typename Key, typename G>
+__device__ __forceinline__ int sort_keys(const Team<X> T, int64_t n, int bits, G gen) {
   constexpr int NT = X::NT, kIt = 4, kQ = NT / kDigits;
   auto& S = X::S();
   auto& W = X::W();
   const unsigned full = 0xffffffffu;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const unsigned lt = (1u << lane) - 1u;
-  if (cells_fit<X>(C)) {
-    // few communities, one block: a sum for every pair of them, the pairs met
-    // (sums are positive: weight 0 counts 1) written in order, to the resident
-    // list as well
-    const int cells = C * C;
-#pragma unroll 1
-    for (int x = tid; x < cells; x += NT) S.u.cell[x] = 0.0;
-    __syncthreads();
-#pragma unroll 4
-    for (int64_t e = tid; e < E; e += NT) {
-      const float x = L.w[e];
-      const int cell = W.newid[W.comm[L.src[e]]] * C + W.newid[W.comm[L.dst[e]]];
-      // integral weights add as integers (shared memory adds those in place)
-      if (integral) atomicAdd(reinterpret_cast<unsigned long long*>(&S.u.cell[cell]),
-                              x == 0.0f ? 1ull : (unsigned long long)x);       // InducedGraphKernel.cu:38-39
-      else atomicAdd(&S.u.cell[cell], x == 0.0f ? 1.0 : (double)x);
-    }
-    __syncthreads();
-    // a run of consecutive cells a thread
-    const int per = (cells + NT - 1) / NT, x0 = min(tid * per, cells), x1 = min(x0 + per, cells);
-    uint32_t met = 0;
-#pragma unroll 4
-    for (int x = x0; x < x1; ++x) met += S.u.cell[x] != 0.0 ? 1u : 0u;   // (an integer's bits are 0 for 0 alone)
-    uint32_t all;
-    uint32_t r = block_excl<X>(met, &all);
-    int row = x0 / C, column = x0 % C;
-    if constexpr (X::kResident) {
-#pragma unroll 1
-      for (int x = x0; x < x1; ++x) {
-        const double sum = S.u.cell[x];
-        if (sum != 0.0) {
-          const float w = __double2float_rn(integral ? (double)__double_as_longlong(sum) : sum);
-          W.src[r] = osrc[r] = row;
-          W.dst[r] = odst[r] = column;
-          W.w[r] = ow[r] = w;
-          ++r;
-        }
-        if (++column == C) {
-          column = 0;
-          ++row;
-        }
-      }
-    }
-    __syncthreads();
-    return (int64_t)all;
-  }
-  int b = 1;
-  while ((1 << b) < C) ++b;
   Key* const keys[2] = {(Key*)W.key[0], (Key*)W.key[1]};
-  const int bits = 2 * b, np = (bits + 7) / 8, width = (bits + np - 1) / np;
+  const int np = (bits + 7) / 8, width = (bits + np - 1) / np;
   const uint32_t dmask = (1u << width) - 1u;
-  const int64_t s0 = E * T.rank() / T.K(), s1 = E * (T.rank() + 1) / T.K();
+  const int64_t s0 = n * T.rank() / T.K(), s1 = n * (T.rank() + 1) / T.K();
   int cur = 0;
 #pragma unroll 1
   for (int p = 0; p < np; ++p) {
     if (tid < kDigits) S.hist[tid] = 0;
     __syncthreads();
     if (p == 0) {
-      const int32_t *comm = W.comm, *newid = W.newid;
       double* wsum = W.wsum;
       float* val = W.val[0];
 #pragma unroll 2
       for (int64_t e = s0 + tid; e < s1; e += NT) {
-        const Key key = ((Key)newid[comm[L.src[e]]] << b) | (Key)newid[comm[L.dst[e]]];
-        const float x = L.w[e];
+        Key key;
+        float x;
+        gen(e, key, x);
         keys[0][e] = key;
-        val[e] = x == 0.0f ? 1.0f : x;       // InducedGraphKernel.cu:38-39
+        val[e] = x;
         wsum[e] = 0.0;
         atomicAdd(&S.hist[(uint32_t)key & dmask], 1u);
       }
@@ -1103,20 +1199,26 @@ __device__ __noinline__ int64_t coarsen(const Team<X> T, const List L, int64_t E
     if (!T.sync()) return -1;
     cur ^= 1;
   }
-  // runs of equal keys: heads counted per block, then each run's pieces added
-  const Key* key = keys[cur];
-  const float* val = W.val[cur];
-  double* wsum = W.wsum;
+  return cur;
+}
+
+// Runs of equal keys that `counts` at their first entry: those started before
+// the block's share, and all of them.  False: a barrier's wait ran out.
+template <typename X, typename Key, typename P>
+__device__ __forceinline__ bool count_runs(const Team<X> T, const Key* key, int64_t s0, int64_t s1, uint32_t& run,
+                                           uint32_t& cnt, P counts) {
+  auto& W = X::W();
   uint32_t heads = 0;
 #pragma unroll 1
-  for (int64_t i0 = s0; i0 < s1; i0 += NT) {
-    const int64_t i = i0 + tid;
-    heads += __syncthreads_count(i < s1 && (i == 0 || key[i] != key[i - 1]));
+  for (int64_t i0 = s0; i0 < s1; i0 += X::NT) {
+    const int64_t i = i0 + threadIdx.x;
+    heads += __syncthreads_count(i < s1 && (i == 0 || key[i] != key[i - 1]) && counts(key[i]));
   }
-  uint32_t run = 0, cnt = heads;
+  run = 0;
+  cnt = heads;
   if (T.K() > 1) {
-    if (tid == 0) W.ctl->count[1][T.rank()] = heads;
-    if (!T.sync()) return -1;
+    if (threadIdx.x == 0) W.ctl->count[1][T.rank()] = heads;
+    if (!T.sync()) return false;
     cnt = 0;
 #pragma unroll 4
     for (int r = 0; r < T.K(); ++r) {
@@ -1125,6 +1227,81 @@ __device__ __noinline__ int64_t coarsen(const Team<X> T, const List L, int64_t E
       cnt += c;
     }
   }
+  return true;
+}
+
+// The coarse list of a level of C communities (new ids W.newid of the labels
+// W.comm) into (osrc, odst, ow); returns its length (-1: a barrier's wait ran
+// out).
+template <typename X, typename Key>
+__device__ __noinline__ int64_t coarsen(const Team<X> T, const List L, int64_t E, int32_t C, bool integral,
+                                        int32_t* osrc, int32_t* odst, float* ow) {
+  constexpr int NT = X::NT, kIt = 4;
+  auto& S = X::S();
+  auto& W = X::W();
+  const int tid = threadIdx.x;
+  if (cells_fit<X>(C)) {
+    // few communities, one block: a sum for every pair of them, the pairs met
+    // (sums are positive: weight 0 counts 1) written in order, to the resident
+    // list as well
+    const int cells = C * C;
+#pragma unroll 1
+    for (int x = tid; x < cells; x += NT) S.u.cell[x] = 0.0;
+    __syncthreads();
+#pragma unroll 4
+    for (int64_t e = tid; e < E; e += NT) {
+      const float x = L.w[e];
+      const int cell = W.newid[W.comm[L.src[e]]] * C + W.newid[W.comm[L.dst[e]]];
+      // integral weights add as integers (shared memory adds those in place)
+      if (integral) atomicAdd(reinterpret_cast<unsigned long long*>(&S.u.cell[cell]),
+                              x == 0.0f ? 1ull : (unsigned long long)x);       // InducedGraphKernel.cu:38-39
+      else atomicAdd(&S.u.cell[cell], x == 0.0f ? 1.0 : (double)x);
+    }
+    __syncthreads();
+    // a run of consecutive cells a thread
+    const int per = (cells + NT - 1) / NT, x0 = min(tid * per, cells), x1 = min(x0 + per, cells);
+    uint32_t met = 0;
+#pragma unroll 4
+    for (int x = x0; x < x1; ++x) met += S.u.cell[x] != 0.0 ? 1u : 0u;   // (an integer's bits are 0 for 0 alone)
+    uint32_t all;
+    uint32_t r = block_excl<X>(met, &all);
+    int row = x0 / C, column = x0 % C;
+    if constexpr (X::kResident) {
+#pragma unroll 1
+      for (int x = x0; x < x1; ++x) {
+        const double sum = S.u.cell[x];
+        if (sum != 0.0) {
+          const float w = __double2float_rn(integral ? (double)__double_as_longlong(sum) : sum);
+          W.src[r] = osrc[r] = row;
+          W.dst[r] = odst[r] = column;
+          W.w[r] = ow[r] = w;
+          ++r;
+        }
+        if (++column == C) {
+          column = 0;
+          ++row;
+        }
+      }
+    }
+    __syncthreads();
+    return (int64_t)all;
+  }
+  int b = 1;
+  while ((1 << b) < C) ++b;
+  const int32_t *comm = W.comm, *newid = W.newid;
+  const int cur = sort_keys<X, Key>(T, E, 2 * b, [&](int64_t e, Key& k, float& x) {
+    k = ((Key)newid[comm[L.src[e]]] << b) | (Key)newid[comm[L.dst[e]]];
+    x = L.w[e];
+    x = x == 0.0f ? 1.0f : x;       // InducedGraphKernel.cu:38-39
+  });
+  if (cur < 0) return -1;
+  // runs of equal keys: heads counted per block, then each run's pieces added
+  const Key* key = (const Key*)W.key[cur];
+  const float* val = W.val[cur];
+  double* wsum = W.wsum;
+  const int64_t s0 = E * T.rank() / T.K(), s1 = E * (T.rank() + 1) / T.K();
+  uint32_t run, cnt;
+  if (!count_runs<X>(T, key, s0, s1, run, cnt, [](Key) { return true; })) return -1;
   const Key cmask = (Key(1) << b) - 1;
 #pragma unroll 1
   for (int64_t t0 = s0; t0 < s1; t0 += NT * kIt) {
@@ -1165,6 +1342,86 @@ __device__ __noinline__ int64_t coarsen(const Team<X> T, const List L, int64_t E
   return (int64_t)cnt;
 }
 
+// CSR of a list that is not sorted and symmetric: the doubled list sorted by
+// (src, dst), equal pairs merged, row by row in W.csrc / cdst / cw; degrees
+// and self loops on the way (as csr_scan_kernel).  Returns the entries (-1: a
+// barrier's wait ran out).
+template <typename X, typename Key>
+__device__ __noinline__ int64_t build_csr(const Team<X> T, const List L, int64_t E, int32_t V) {
+  constexpr int NT = X::NT, kIt = 4;
+  auto& W = X::W();
+  int b = 1;
+  while ((1 << b) < V) ++b;
+  const int64_t n = 2 * E;
+  const int cur = sort_keys<X, Key>(T, n, 2 * b, [&](int64_t e, Key& k, float& x) {
+    const int64_t q = e < E ? e : e - E;
+    const Key u = (Key)L.src[q], d = (Key)L.dst[q];
+    k = e < E ? (u << b) | d : (d << b) | u;
+    x = L.w[q];
+  });
+  if (cur < 0) return -1;
+  const Key* key = (const Key*)W.key[cur];
+  const float* val = W.val[cur];
+  double* wsum = W.wsum;
+  const Key cmask = (Key(1) << b) - 1;
+  const int64_t s0 = n * T.rank() / T.K(), s1 = n * (T.rank() + 1) / T.K();
+  uint32_t run, cnt;
+  if (!count_runs<X>(T, key, s0, s1, run, cnt, [&](Key k) { return (k >> b) != (k & cmask); })) return -1;
+#pragma unroll 1
+  for (int64_t t0 = s0; t0 < s1; t0 += NT * kIt) {
+    const int64_t i0 = t0 + (int64_t)threadIdx.x * kIt;
+    Key k[kIt + 2];
+    uint32_t hm = 0;
+    k[0] = i0 > 0 && i0 < s1 ? key[i0 - 1] : Key(0);
+#pragma unroll
+    for (int j = 0; j <= kIt; ++j) k[j + 1] = i0 + j < n && i0 < s1 ? key[i0 + j] : Key(0);
+#pragma unroll
+    for (int j = 0; j < kIt; ++j)
+      if (i0 + j < s1 && (i0 + j == 0 || k[j + 1] != k[j]) && (k[j + 1] >> b) != (k[j + 1] & cmask)) hm |= 1u << j;
+    uint32_t all;
+    uint32_t r = run + block_excl<X>((uint32_t)__popc(hm), &all);
+    run += all;
+    double s = 0.0, deg = 0.0;
+    bool any = false;
+#pragma unroll
+    for (int j = 0; j < kIt; ++j) {
+      const int64_t i = i0 + j;
+      if (i < s1) {
+        const int32_t u = (int32_t)(k[j + 1] >> b), d = (int32_t)(k[j + 1] & cmask);
+        const float x = val[i];
+        if ((hm >> j) & 1u) {
+          if (any) atomicAdd(&wsum[r - 1], s);
+          s = 0.0;
+          any = false;
+          W.csrc[r] = u;
+          W.cdst[r] = d;
+          ++r;
+        }
+        if (u != d) {
+          s = __dadd_rn(s, (double)x);
+          any = true;
+        } else if (i == n - 1 || k[j + 2] != k[j + 1]) {   // the last self-loop entry (InitKernel.cu:181-194)
+          W.loopw[u] = x;
+          W.hasl[u] = 1;
+        }
+        float f = x == 0.0f ? 1.0f : x;                    // InitKernel.cu:165-170
+        if (u == d) f *= 2.0f;
+        deg = __dadd_rn(deg, (double)f);
+        if (j == kIt - 1 || i == s1 - 1 || (int32_t)(k[j + 2] >> b) != u) {
+          atomicAdd(&W.k[u], deg);
+          deg = 0.0;
+        }
+      }
+    }
+    if (any) atomicAdd(&wsum[r - 1], s);
+  }
+  if (!T.sync()) return -1;
+#pragma unroll 2
+  for (int64_t i = T.gt(); i < cnt; i += T.stride()) W.cw[i] = __double2float_rn(wsum[i]);
+  if (!T.sync()) return -1;
+  return (int64_t)cnt;
+}
+
 // Where a job's levels stand, the same in every thread of its team.
 struct At {
   int32_t V;
@@ -1172,6 +1429,7 @@ struct At {
   int32_t ncomms = 0;
   int buf = -1, nlev = 0, status = LVG_OK;
   bool open = false, symmetric = true, bad = false, tail = false, mid = false;
+  bool any_order = false;   // the list may be other than sorted and symmetric, and there is room for that
   double mod = 0.0, lower = 0.0;
   int64_t part_off = 0;
 };
@@ -1192,12 +1450,12 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
   auto& W = X::W();
   const SmallJob& J = S.J;
   const bool lead = T.lead();
-  List L{J.src, J.dst, J.w};
+  List L{J.src, J.dst, J.w, 2.0f};
   if (at.buf >= 0) {
     int32_t *ls, *ld;
     float* lw;
     list_of(J.lists, J.E, at.buf, &ls, &ld, &lw);
-    L = List{ls, ld, lw};
+    L = List{ls, ld, lw, 2.0f};
   }
   int64_t res_v = 0;
   bool list_here = false;   // the resident list is already this level's
@@ -1208,14 +1466,14 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
     const int64_t E = at.E;
     if (at.nlev >= kSmallLevels || (J.parts && at.part_off + 2 * (int64_t)V > J.parts_cap)) { at.open = true; return true; }
     if (!X::kResident) {
-      if (V <= kResV && E <= kResE) { at.tail = true; return true; }
+      if (V <= kResV && E <= kResE && !at.any_order) { at.tail = true; return true; }
       // below this a cluster's barriers save more than the chip's width does
       // (a level of 117 Ki entries takes 154 us on the grid, 199 on a cluster;
       // one of 12 Ki 96 and 68)
-      if (T.mode == kModeGrid && E <= kSmallClusterEntries) { at.mid = true; return true; }
+      if (T.mode == kModeGrid && E + V <= kSmallClusterEntries) { at.mid = true; return true; }
       // few entries for so many blocks: the last ones leave
       if (T.mode == kModeGrid && T.K_ > 1) {
-        T.K_ = (int)min((int64_t)T.K_, (E + kGridEntries - 1) / kGridEntries);
+        T.K_ = (int)min((int64_t)T.K_, (E + V + kGridEntries - 1) / kGridEntries);
         if (T.rank_ >= T.K_) return true;
       }
     }
@@ -1236,7 +1494,7 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
           W.w[e] = x;
         }
       }
-      L = List{W.src, W.dst, W.w};
+      L = List{W.src, W.dst, W.w, 2.0f};
     }
 #pragma unroll 1
     for (int32_t i = T.gt(); i < V; i += T.stride()) {
@@ -1245,18 +1503,47 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
       W.hasl[i] = 0;
     }
     if (lead) {
-      W.ctl->flags = W.ctl->flags2 = W.ctl->check = W.ctl->loops = 0u;
+      W.ctl->flags = W.ctl->flags2 = W.ctl->check = W.ctl->loops = W.ctl->nlong = 0u;
       W.ctl->sums[0] = W.ctl->sums[1] = 0ull;
     }
     if (!T.sync()) return false;
+    bool any_order = false;
     if (!at.symmetric) {
       check_list<X>(T, L, E, V);
       if (!T.sync()) return false;
       const uint32_t f = W.ctl->check;
       if (f & fBad) { at.bad = true; return true; }
-      if (f != 0u || W.ctl->sums[0] != 0ull || W.ctl->sums[1] != 0ull) { at.open = true; return true; }
+      any_order = f != 0u || W.ctl->sums[0] != 0ull || W.ctl->sums[1] != 0ull;
+      if (any_order && (X::kResident || !J.dbl)) { at.open = true; return true; }
+      at.any_order = any_order;
     }
-    {
+    if constexpr (!X::kResident) {
+      if (threadIdx.x == 0) S.ngap = 0;
+      __syncthreads();
+    }
+    // The list of rows M, of EM entries: the list itself, or its CSR.
+    List M = L;
+    int64_t EM = E;
+    if constexpr (!X::kResident) {
+      if (any_order) {
+        EM = V <= (1 << 16) ? build_csr<X, uint32_t>(T, L, E, V) : build_csr<X, uint64_t>(T, L, E, V);
+        if (EM < 0) return false;
+        M = List{W.csrc, W.cdst, W.cw, 1.0f};
+        if (EM == 0)
+          for (int32_t r = T.gt(); r <= V; r += T.stride()) W.roff[r] = 0;
+        uint32_t f = 0;
+#pragma unroll 1
+        for (int64_t e = T.gt(); e < EM; e += T.stride()) {
+          const int32_t u = M.src[e], up = e > 0 ? M.src[e - 1] : -1;
+          row_starts<X>(up + 1, u, (int32_t)e);
+          if (e == EM - 1) row_starts<X>(u + 1, V, (int32_t)EM);
+          const float x = M.w[e];
+          if (x != truncf(x)) f |= fNotInt;
+        }
+        if (f) atomicOr(&W.ctl->flags, f);
+      }
+    }
+    if (!any_order) {
       uint32_t f = 0, nl = 0;
 #pragma unroll 1
       for (int64_t e0 = (int64_t)T.rank() * NT; e0 < E; e0 += T.stride()) {
@@ -1267,12 +1554,8 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
         const int32_t up = in && e > 0 ? L.src[e - 1] : -1;
         const float x = in ? L.w[e] : 0.0f;
         if (in) {
-#pragma unroll 1
-          for (int32_t r = up + 1; r <= u; ++r) W.roff[r] = (int32_t)e;
-          if (e == E - 1) {
-#pragma unroll 1
-            for (int32_t r = u + 1; r <= V; ++r) W.roff[r] = (int32_t)E;
-          }
+          row_starts<X>(up + 1, u, (int32_t)e);
+          if (e == E - 1) row_starts<X>(u + 1, V, (int32_t)E);
           if (x != truncf(x)) f |= fNotInt;
           if (u == d) { W.loopw[u] = x; W.hasl[u] = 1; ++nl; }
         }
@@ -1294,13 +1577,15 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
         if (f) atomicOr(&W.ctl->flags, f);
         if (nl) atomicAdd(&W.ctl->loops, nl);
       }
-      group_partials<X>(   // NeighbourCompute.cu:46
-          T, E, W.mpart, [&](int64_t e) { return L.w[e]; }, [&](int64_t, float x) { return (double)x; });
     }
+    if constexpr (!X::kResident) long_gaps<X>();
+    group_partials<X>(   // NeighbourCompute.cu:46
+        T, E, W.mpart, [&](int64_t e) { return L.w[e]; }, [&](int64_t, float x) { return (double)x; });
     if (!T.sync()) return false;
     const bool integral = !(W.ctl->flags & fNotInt);
-    at.symmetric = integral;   // of the next list: exact sums round alike in both directions
-    const int64_t nnz = E - (int64_t)W.ctl->loops;
+    // of the next list: exact sums round alike in both directions
+    at.symmetric = integral && !any_order;
+    const int64_t nnz = EM - (int64_t)W.ctl->loops;
     const double m = finish_sum<X>(W.mpart, E);
     const double twom = __dmul_rn(2.0, m);
     {
@@ -1318,7 +1603,12 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
             W.cand[i] = -1;
             W.kfrac[i] = m > 0.0 ? __ddiv_rn(r.k, twom) : 0.0;   // OneLevelKernel.cu:307
             W.minidx[i] = kNone;
-            if (r.len > Tile<NT>::kF64) f |= r.len > kLongRow ? fUnfit : fLong;
+            if constexpr (!X::kResident) {
+              if (r.len > Tile<NT>::kF64) {
+                f |= fLong;
+                W.longs[atomicAdd(&W.ctl->nlong, 1u)] = (int32_t)i;
+              }
+            }
             if (!(r.k < 1073741824.0)) f |= fNotInt;
             return q_term(x, r.k, m, twom);
           });
@@ -1327,10 +1617,10 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
     if (!T.sync()) return false;
     const uint32_t f2 = W.ctl->flags2;
     const bool packed = integral && !(f2 & fNotInt);
-    if (f2 & fUnfit) { at.open = true; return true; }
+    const bool longs = !X::kResident && (f2 & fLong);
     const double q0 = finish_sum<X>(W.qpart, V);
     at.lower = level == 0 ? q0 : at.mod;        // LouvainCPP.cpp:356,446
-    find_rows<X>(T, V, E);
+    find_rows<X>(T, V, EM);
     const int32_t v0 = S.row0, v1 = S.row1;
     const long long t1 = clock64();
     // ---- passes
@@ -1346,14 +1636,29 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
       const bool stop = __dsub_rn(q_prev, floor_q) < cfg.pass_min;
       const bool capped = cfg.max_passes >= 0 && pass >= cfg.max_passes;
       if (pass == 1) {
-        moves_first<X>(L, v0, v1, stop || capped);
+        if constexpr (!X::kResident) {
+          if (longs) hub_clear<X>(T);
+        }
+        moves_first<X>(M, v0, v1, stop || capped);
       } else if (packed) {
-        moves_hash<X, true>(L, v0, v1, stop || capped);
+        moves_hash<X, true>(M, v0, v1, stop || capped);
       } else {
-        moves_hash<X, false>(L, v0, v1, stop || capped);
+        moves_hash<X, false>(M, v0, v1, stop || capped);
+      }
+      if constexpr (!X::kResident) {
+        if (longs && pass > 1) {
+          if (packed) hub_insert<X, true>(T, M, EM);
+          else hub_insert<X, false>(T, M, EM);
+        }
       }
       if (!T.sync()) return false;
-      if ((f2 & fLong) && (W.ctl->flags2 & fFull)) { at.open = true; return true; }
+      if constexpr (!X::kResident) {
+        if (longs && pass > 1) {
+          if (packed) hub_pick<X, true>(T, stop || capped);
+          else hub_pick<X, false>(T, stop || capped);
+          if (!T.sync()) return false;
+        }
+      }
       if (pass <= 2) pass_ticks[pass - 1] = (float)(clock64() - p0);
       if (stop || capped) {
         st = stop ? LVG_OK : LVG_ERR_NOT_CONVERGED;
@@ -1466,7 +1771,7 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
     ++at.nlev;
     if (last) return true;
     at.buf = (at.nlev - 1) & 1;
-    L = List{ns, nd, nw};
+    L = List{ns, nd, nw, 2.0f};
     list_here = cells_fit<X>((int32_t)C);
     at.V = (int32_t)C;
     at.E = E1;
@@ -1484,7 +1789,7 @@ __device__ __forceinline__ void load_job(const SmallJob* job) {
 __device__ __forceinline__ void store_between(Between& B, const At& at) {
   B.nlev = at.nlev;
   B.buf = at.buf;
-  B.symmetric = at.symmetric ? 1 : 0;
+  B.symmetric = (at.symmetric ? 1 : 0) | (at.any_order ? 2 : 0);
   B.V = at.V;
   B.ncomms = at.ncomms;
   B.open = at.open ? 1 : 0;
@@ -1502,7 +1807,8 @@ __device__ __forceinline__ void load_between(const Between& B, At& at) {
   at.ncomms = B.ncomms;
   at.buf = B.buf;
   at.nlev = B.nlev;
-  at.symmetric = B.symmetric != 0;
+  at.symmetric = (B.symmetric & 1) != 0;
+  at.any_order = (B.symmetric & 2) != 0;
   at.mod = B.mod;
   at.lower = B.lower;
   at.part_off = B.part_off;
@@ -1517,7 +1823,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) small_kernel(const SmallJob* jo
   load_job<X>(jobs + blockIdx.x / K);
   const SmallJob& J = X::S().J;
   if (threadIdx.x == 0) {
-    carve(J.work, J.V, J.E, X::W());
+    carve(J.work, J.V, J.E, J.dbl != 0, X::W());
     X::S().goal = 0ull;
   }
   __syncthreads();
@@ -1528,6 +1834,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) small_kernel(const SmallJob* jo
   at.V = J.V;
   at.E = J.E;
   at.symmetric = J.check == 0;
+  at.any_order = J.dbl != 0;
   at.mod = J.mod;
   Between& B = *X::W().bt;
   if (resume) {   // from where the grid stopped
@@ -1552,7 +1859,7 @@ __global__ void __launch_bounds__(kResThreads, 1) small_tail_kernel(const SmallJ
   load_job<X>(jobs + blockIdx.x);
   const SmallJob& J = X::S().J;
   Work g;
-  carve(J.work, J.V, J.E, g);
+  carve(J.work, J.V, J.E, J.dbl != 0, g);
   Between& B = *g.bt;
   const int32_t phase = B.phase;
   int32_t ncomms = B.ncomms;
@@ -1603,7 +1910,7 @@ constexpr int kQThreads = 512;
 __global__ void __launch_bounds__(kQThreads) small_sum_kernel(const SmallJob* jobs, int K) {
   const SmallJob& J = jobs[blockIdx.x / K];
   Work g;
-  carve(J.work, J.V, J.E, g);
+  carve(J.work, J.V, J.E, J.dbl != 0, g);
   const Between& B = *g.bt;
   if (!wants_q(J, B)) return;
   const int32_t how = B.comp;
@@ -1651,7 +1958,7 @@ struct QSpace {
 __global__ void __launch_bounds__(kQThreads) small_end_kernel(const SmallJob* jobs, int K) {
   const SmallJob& J = jobs[blockIdx.x / K];
   Work g;
-  carve(J.work, J.V, J.E, g);
+  carve(J.work, J.V, J.E, J.dbl != 0, g);
   const Between& B = *g.bt;
   if (B.phase != kPhaseEnd) return;   // a barrier's wait ran out: no result
   const int32_t how = B.comp;
@@ -1747,9 +2054,9 @@ void launch_rest(const SmallJob* jobs, int n, int K, const SmallCfg& cfg, cudaSt
 
 size_t small_list_bytes(int64_t E) { return 6 * up256(4 * (size_t)E); }
 
-size_t small_work_bytes(int32_t V, int64_t E) {
+size_t small_work_bytes(int32_t V, int64_t E, bool dbl) {
   Work W;
-  return carve(nullptr, V, E, W);
+  return carve(nullptr, V, E, dbl, W);
 }
 
 void small_list(char* lists, int64_t E, int buf, int32_t** src, int32_t** dst, float** w) {

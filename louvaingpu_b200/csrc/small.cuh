@@ -60,6 +60,8 @@ struct SmallJob {
   SmallLevel* lv;           // [kSmallLevels], or nullptr
   int32_t check;            // 1: ids, weights, order and symmetry not checked yet
   int32_t want_q;
+  int32_t dbl;              // 1: work has room for lists in any order (small_work_bytes with dbl)
+  int32_t pad;
 };
 
 struct SmallCfg {
@@ -68,7 +70,7 @@ struct SmallCfg {
 };
 
 size_t small_list_bytes(int64_t E);           // both coarse list buffers
-size_t small_work_bytes(int32_t V, int64_t E);
+size_t small_work_bytes(int32_t V, int64_t E, bool dbl);
 // Coarse list buffer `buf` of a job's lists.
 void small_list(char* lists, int64_t E, int buf, int32_t** src, int32_t** dst, float** w);
 // True when the sizes are ones this path takes.

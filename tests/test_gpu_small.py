@@ -131,6 +131,36 @@ def test_larger_graphs(Louvain, oracle, gen, n, comms, p_in):
         run_equal(lv, lv.run(), oracle.Run(n, s, d, w), n, s, d, w, oracle)
 
 
+@pytest.mark.parametrize("kind", ["sbm:9001", "sbm:30011", "linked:70001", "hub:60001"])
+@pytest.mark.parametrize("scale", [1.0, 0.125])
+def test_coarse_lists_in_one_direction(Louvain, oracle, gen, kind, scale):
+    """Edges listed once, in any order: coarse lists are sorted but not
+    symmetric (of more vertices than 16 bits hold, or with a row longer than a
+    tile, for the linked triangles)."""
+    rng = np.random.default_rng(8)
+    n = int(kind.split(":")[1])
+    if kind.startswith("sbm"):
+        _, s, d, w = gen.sbm(n, n // 60, 0.25, 3.0 / n, 1, 4, seed=n)
+        up = s <= d
+        s, d, w = s[up], d[up], w[up]
+    else:                       # triangles, linked at random, or all to the first
+        t = np.arange(n, dtype=np.int32) * 3
+        other = t[rng.integers(0, n, n)] if kind.startswith("linked") else np.zeros(n, np.int32)
+        s = np.concatenate([t, t, t + 1, t[1:], t[::5]])
+        d = np.concatenate([t + 1, t + 2, t + 2, other[1:], t[::5]])
+        w = np.concatenate([np.full(3 * n, 8), np.ones(n - 1), np.full(len(t[::5]), 2)]).astype(np.float32)
+        n = 3 * n
+    o = rng.permutation(len(s))
+    s, d, w = s[o], d[o], (w[o] * np.float32(scale)).astype(np.float32)
+    flip = rng.random(len(s)) < 0.5
+    s, d = np.where(flip, d, s), np.where(flip, s, d)
+    orun = oracle.Run(n, s, d, w)
+    with Louvain() as lv:
+        lv.load_edges(s, d, w, n)
+        run_equal(lv, lv.run(), orun, n, s, d, w, oracle)
+        run_equal(lv, lv.run(), orun, n, s, d, w, oracle)
+
+
 def test_batch_mixes_the_paths(Louvain, oracle, gen):
     """Graphs for clusters of 1, 2, 4 and 8 blocks, ones the launch leaves
     open (unsorted, a row too long), larger ones, and one without entries:
