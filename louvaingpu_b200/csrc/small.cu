@@ -184,7 +184,10 @@ struct Space {
   static constexpr int kSlots = Tile<NT>::kSlots, kTileRows = Tile<NT>::kRows, kTileInt = Tile<NT>::kInt;
   union {
     unsigned long long slot[kSlots];
-    uint32_t wc[NT / 32][kDigits + 1];
+    struct {
+      uint32_t wc[NT / 32][kDigits];     // a warp's keys of each digit
+      uint32_t meet[NT / 32][kDigits];   // its lanes that hold one
+    } sort;
     uint32_t part[2][NT / kDigits][kDigits];
     double stage[kGroup];
     double cell[CELLS];        // sums of a coarse graph of few communities
@@ -1089,7 +1092,6 @@ __device__ __forceinline__ int sort_keys(const Team<X> T, int64_t n, int bits, G
   constexpr int NT = X::NT, kIt = 4, kQ = NT / kDigits;
   auto& S = X::S();
   auto& W = X::W();
-  const unsigned full = 0xffffffffu;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const unsigned lt = (1u << lane) - 1u;
   Key* const keys[2] = {(Key*)W.key[0], (Key*)W.key[1]};
@@ -1104,6 +1106,8 @@ __device__ __forceinline__ int sort_keys(const Team<X> T, int64_t n, int bits, G
     if (p == 0) {
       double* wsum = W.wsum;
       float* val = W.val[0];
+#pragma unroll 4
+      for (int x = tid; x < (NT / 32) * kDigits; x += NT) (&S.u.sort.meet[0][0])[x] = 0;
 #pragma unroll 2
       for (int64_t e = s0 + tid; e < s1; e += NT) {
         Key key;
@@ -1153,7 +1157,7 @@ __device__ __forceinline__ int sort_keys(const Team<X> T, int64_t n, int bits, G
 #pragma unroll 1
     for (int64_t t0 = s0; t0 < s1; t0 += NT * kIt) {
 #pragma unroll 2
-      for (int x = tid; x < (NT / 32) * (kDigits + 1); x += NT) (&S.u.wc[0][0])[x] = 0;
+      for (int x = tid; x < (NT / 32) * kDigits; x += NT) (&S.u.sort.wc[0][0])[x] = 0;
       Key key[kIt];
       uint32_t rank[kIt], dg[kIt];
       float val[kIt];
@@ -1168,11 +1172,19 @@ __device__ __forceinline__ int sort_keys(const Team<X> T, int64_t n, int bits, G
       __syncthreads();
 #pragma unroll
       for (int j = 0; j < kIt; ++j) {
-        const unsigned peers = __match_any_sync(full, dg[j]);
-        const uint32_t before = S.u.wc[wid][dg[j]];
+        // lanes of a digit meet in a shared word (a match instruction takes
+        // 62 cycles of an SM a warp, this some 15)
+        const bool in = dg[j] < (uint32_t)kDigits;
+        if (in) atomicOr(&S.u.sort.meet[wid][dg[j]], 1u << lane);
+        __syncwarp();
+        const unsigned peers = in ? S.u.sort.meet[wid][dg[j]] : 0u;
+        const uint32_t before = in ? S.u.sort.wc[wid][dg[j]] : 0u;
         rank[j] = before + __popc(peers & lt);
         __syncwarp();
-        if ((peers & lt) == 0) S.u.wc[wid][dg[j]] = before + __popc(peers);
+        if (in && (peers & lt) == 0) {
+          S.u.sort.wc[wid][dg[j]] = before + __popc(peers);
+          S.u.sort.meet[wid][dg[j]] = 0u;
+        }
         __syncwarp();
       }
       __syncthreads();
@@ -1180,8 +1192,8 @@ __device__ __forceinline__ int sort_keys(const Team<X> T, int64_t n, int bits, G
         uint32_t run = S.dbase[tid];
 #pragma unroll 8
         for (int w = 0; w < NT / 32; ++w) {
-          const uint32_t c = S.u.wc[w][tid];
-          S.u.wc[w][tid] = run;
+          const uint32_t c = S.u.sort.wc[w][tid];
+          S.u.sort.wc[w][tid] = run;
           run += c;
         }
         S.dbase[tid] = run;
@@ -1190,7 +1202,7 @@ __device__ __forceinline__ int sort_keys(const Team<X> T, int64_t n, int bits, G
 #pragma unroll
       for (int j = 0; j < kIt; ++j)
         if (dg[j] < (uint32_t)kDigits) {
-          const uint32_t o = S.u.wc[wid][dg[j]] + rank[j];
+          const uint32_t o = S.u.sort.wc[wid][dg[j]] + rank[j];
           keys[cur ^ 1][o] = key[j];
           W.val[cur ^ 1][o] = val[j];
         }
