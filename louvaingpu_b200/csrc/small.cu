@@ -1082,6 +1082,38 @@ __device__ __forceinline__ bool cells_fit(int32_t C) {
   return X::kResident && C <= 1024 && C * C <= X::kCells;
 }
 
+// Keys with their values: 32-bit keys side by side with them, one scattered
+// store of 8 bytes each a pass instead of two of 4 (coarsening 1.9 M entries:
+// 275 us before, 237 now).
+template <typename Key>
+struct Keyed {
+  uint64_t* key;
+  float* val;
+  static constexpr bool kPair = sizeof(Key) == 4;
+  __device__ __forceinline__ Key at(int64_t i) const {
+    if constexpr (kPair) return reinterpret_cast<const uint2*>(key)[i].x;
+    else return key[i];
+  }
+  __device__ __forceinline__ void get(int64_t i, Key& k, float& x) const {
+    if constexpr (kPair) {
+      const uint2 p = reinterpret_cast<const uint2*>(key)[i];
+      k = p.x;
+      x = __uint_as_float(p.y);
+    } else {
+      k = key[i];
+      x = val[i];
+    }
+  }
+  __device__ __forceinline__ void put(int64_t i, Key k, float x) const {
+    if constexpr (kPair) {
+      reinterpret_cast<uint2*>(key)[i] = make_uint2(k, __float_as_uint(x));
+    } else {
+      key[i] = k;
+      val[i] = x;
+    }
+  }
+};
+
 // Stable LSD sort over the team of n keys by their low `bits` bits, made with
 // their values by gen(i, key, val): block r owns the r-th share of the
 // positions, counts its digits, and places its keys after those of all blocks
@@ -1094,18 +1126,17 @@ __device__ __forceinline__ int sort_keys(const Team<X> T, int64_t n, int bits, G
   auto& W = X::W();
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const unsigned lt = (1u << lane) - 1u;
-  Key* const keys[2] = {(Key*)W.key[0], (Key*)W.key[1]};
   const int np = (bits + 7) / 8, width = (bits + np - 1) / np;
   const uint32_t dmask = (1u << width) - 1u;
   const int64_t s0 = n * T.rank() / T.K(), s1 = n * (T.rank() + 1) / T.K();
   int cur = 0;
 #pragma unroll 1
   for (int p = 0; p < np; ++p) {
+    const Keyed<Key> from{W.key[cur], W.val[cur]}, to{W.key[cur ^ 1], W.val[cur ^ 1]};
     if (tid < kDigits) S.hist[tid] = 0;
     __syncthreads();
     if (p == 0) {
       double* wsum = W.wsum;
-      float* val = W.val[0];
 #pragma unroll 4
       for (int x = tid; x < (NT / 32) * kDigits; x += NT) (&S.u.sort.meet[0][0])[x] = 0;
 #pragma unroll 2
@@ -1113,15 +1144,14 @@ __device__ __forceinline__ int sort_keys(const Team<X> T, int64_t n, int bits, G
         Key key;
         float x;
         gen(e, key, x);
-        keys[0][e] = key;
-        val[e] = x;
+        from.put(e, key, x);
         wsum[e] = 0.0;
         atomicAdd(&S.hist[(uint32_t)key & dmask], 1u);
       }
     } else {
 #pragma unroll 4
       for (int64_t e = s0 + tid; e < s1; e += NT)
-        atomicAdd(&S.hist[(uint32_t)(keys[cur][e] >> (p * width)) & dmask], 1u);
+        atomicAdd(&S.hist[(uint32_t)(from.at(e) >> (p * width)) & dmask], 1u);
     }
     __syncthreads();
     uint32_t tot = 0, pre = 0;
@@ -1165,8 +1195,9 @@ __device__ __forceinline__ int sort_keys(const Team<X> T, int64_t n, int bits, G
 #pragma unroll
       for (int j = 0; j < kIt; ++j) {
         const int64_t i = base + j * 32 + lane;
-        key[j] = i < s1 ? keys[cur][i] : Key(0);
-        val[j] = i < s1 ? W.val[cur][i] : 0.0f;
+        key[j] = Key(0);
+        val[j] = 0.0f;
+        if (i < s1) from.get(i, key[j], val[j]);
         dg[j] = i < s1 ? (uint32_t)(key[j] >> (p * width)) & dmask : (uint32_t)kDigits;
       }
       __syncthreads();
@@ -1203,8 +1234,7 @@ __device__ __forceinline__ int sort_keys(const Team<X> T, int64_t n, int bits, G
       for (int j = 0; j < kIt; ++j)
         if (dg[j] < (uint32_t)kDigits) {
           const uint32_t o = S.u.sort.wc[wid][dg[j]] + rank[j];
-          keys[cur ^ 1][o] = key[j];
-          W.val[cur ^ 1][o] = val[j];
+          to.put(o, key[j], val[j]);
         }
       __syncthreads();
     }
@@ -1217,14 +1247,15 @@ __device__ __forceinline__ int sort_keys(const Team<X> T, int64_t n, int bits, G
 // Runs of equal keys that `counts` at their first entry: those started before
 // the block's share, and all of them.  False: a barrier's wait ran out.
 template <typename X, typename Key, typename P>
-__device__ __forceinline__ bool count_runs(const Team<X> T, const Key* key, int64_t s0, int64_t s1, uint32_t& run,
+__device__ __forceinline__ bool count_runs(const Team<X> T, const Keyed<Key> key, int64_t s0, int64_t s1, uint32_t& run,
                                            uint32_t& cnt, P counts) {
   auto& W = X::W();
   uint32_t heads = 0;
 #pragma unroll 1
   for (int64_t i0 = s0; i0 < s1; i0 += X::NT) {
     const int64_t i = i0 + threadIdx.x;
-    heads += __syncthreads_count(i < s1 && (i == 0 || key[i] != key[i - 1]) && counts(key[i]));
+    const Key k = i < s1 ? key.at(i) : Key(0);
+    heads += __syncthreads_count(i < s1 && (i == 0 || k != key.at(i - 1)) && counts(k));
   }
   run = 0;
   cnt = heads;
@@ -1308,8 +1339,7 @@ __device__ __noinline__ int64_t coarsen(const Team<X> T, const List L, int64_t E
   });
   if (cur < 0) return -1;
   // runs of equal keys: heads counted per block, then each run's pieces added
-  const Key* key = (const Key*)W.key[cur];
-  const float* val = W.val[cur];
+  const Keyed<Key> key{W.key[cur], W.val[cur]};
   double* wsum = W.wsum;
   const int64_t s0 = E * T.rank() / T.K(), s1 = E * (T.rank() + 1) / T.K();
   uint32_t run, cnt;
@@ -1319,11 +1349,13 @@ __device__ __noinline__ int64_t coarsen(const Team<X> T, const List L, int64_t E
   for (int64_t t0 = s0; t0 < s1; t0 += NT * kIt) {
     const int64_t i0 = t0 + (int64_t)tid * kIt;
     Key k[kIt + 1];
+    float xs[kIt];
     uint32_t hm = 0;
-    k[0] = i0 > 0 && i0 < s1 ? key[i0 - 1] : Key(0);
+    k[0] = i0 > 0 && i0 < s1 ? key.at(i0 - 1) : Key(0);
 #pragma unroll
     for (int j = 0; j < kIt; ++j) {
-      k[j + 1] = i0 + j < s1 ? key[i0 + j] : Key(0);
+      k[j + 1] = Key(0);
+      if (i0 + j < s1) key.get(i0 + j, k[j + 1], xs[j]);
       if (i0 + j < s1 && (i0 + j == 0 || k[j + 1] != k[j])) hm |= 1u << j;
     }
     uint32_t all;
@@ -1341,7 +1373,7 @@ __device__ __noinline__ int64_t coarsen(const Team<X> T, const List L, int64_t E
           odst[r] = (int32_t)(k[j + 1] & cmask);
           ++r;
         }
-        s = __dadd_rn(s, (double)val[i0 + j]);
+        s = __dadd_rn(s, (double)xs[j]);
         any = true;
       }
     }
@@ -1372,8 +1404,7 @@ __device__ __noinline__ int64_t build_csr(const Team<X> T, const List L, int64_t
     x = L.w[q];
   });
   if (cur < 0) return -1;
-  const Key* key = (const Key*)W.key[cur];
-  const float* val = W.val[cur];
+  const Keyed<Key> key{W.key[cur], W.val[cur]};
   double* wsum = W.wsum;
   const Key cmask = (Key(1) << b) - 1;
   const int64_t s0 = n * T.rank() / T.K(), s1 = n * (T.rank() + 1) / T.K();
@@ -1383,10 +1414,14 @@ __device__ __noinline__ int64_t build_csr(const Team<X> T, const List L, int64_t
   for (int64_t t0 = s0; t0 < s1; t0 += NT * kIt) {
     const int64_t i0 = t0 + (int64_t)threadIdx.x * kIt;
     Key k[kIt + 2];
+    float xs[kIt + 1];
     uint32_t hm = 0;
-    k[0] = i0 > 0 && i0 < s1 ? key[i0 - 1] : Key(0);
+    k[0] = i0 > 0 && i0 < s1 ? key.at(i0 - 1) : Key(0);
 #pragma unroll
-    for (int j = 0; j <= kIt; ++j) k[j + 1] = i0 + j < n && i0 < s1 ? key[i0 + j] : Key(0);
+    for (int j = 0; j <= kIt; ++j) {
+      k[j + 1] = Key(0);
+      if (i0 + j < n && i0 < s1) key.get(i0 + j, k[j + 1], xs[j]);
+    }
 #pragma unroll
     for (int j = 0; j < kIt; ++j)
       if (i0 + j < s1 && (i0 + j == 0 || k[j + 1] != k[j]) && (k[j + 1] >> b) != (k[j + 1] & cmask)) hm |= 1u << j;
@@ -1400,7 +1435,7 @@ __device__ __noinline__ int64_t build_csr(const Team<X> T, const List L, int64_t
       const int64_t i = i0 + j;
       if (i < s1) {
         const int32_t u = (int32_t)(k[j + 1] >> b), d = (int32_t)(k[j + 1] & cmask);
-        const float x = val[i];
+        const float x = xs[j];
         if ((hm >> j) & 1u) {
           if (any) atomicAdd(&wsum[r - 1], s);
           s = 0.0;
