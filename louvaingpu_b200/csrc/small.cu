@@ -400,26 +400,45 @@ __device__ __forceinline__ double finish_sum(const double* partials, int64_t n) 
   return x;
 }
 
-// The block's share of the rows: those starting in its share of the list.
-// row0 and row1 become the first rows starting at or after the share's ends.
+// The block's share of the rows: those starting in its share of the entries
+// and rows together (by entries alone, one block of 30 could own 100,000 empty
+// rows: .3 ms a pass).  row0 and row1 become the first rows starting at or
+// after the share's ends.
 template <typename X>
 __device__ __forceinline__ void find_rows(const Team<X> T, int32_t V, int64_t E) {
   auto& S = X::S();
-  const int64_t x0 = E * T.rank() / T.K(), x1 = E * (T.rank() + 1) / T.K();
-  if (threadIdx.x == 0) {   // a share that starts or ends at entry 0 does so at row 0
+  const int64_t x0 = (E + V) * T.rank() / T.K(), x1 = (E + V) * (T.rank() + 1) / T.K();
+  if (threadIdx.x == 0) {   // a share that starts or ends at 0 does so at row 0
     S.row0 = 0;
     S.row1 = T.K() == 1 ? V : 0;
   }
   __syncthreads();
-  if (T.K() > 1) {   // (the rows behind the last entry are nobody's: they have nothing to decide)
+  if (T.K() > 1) {
     const int32_t* roff = X::W().roff;
 #pragma unroll 2
     for (int32_t v = 1 + (int)threadIdx.x; v <= V; v += X::NT) {
-      const int32_t a = roff[v - 1], b = roff[v];
+      const int64_t a = (int64_t)roff[v - 1] + v - 1, b = (int64_t)roff[v] + v;
       if (T.rank() > 0 && a < x0 && b >= x0) S.row0 = v;
       if (a < x1 && b >= x1) S.row1 = v;
     }
     __syncthreads();
+  }
+}
+
+// Row starts of a list of fewer than two entries a row, each row looking for
+// its own: its gaps may be many and long.
+template <typename X>
+__device__ __forceinline__ void search_starts(const Team<X> T, const int32_t* src, int64_t E, int32_t V) {
+  int32_t* roff = X::W().roff;
+#pragma unroll 1
+  for (int32_t r = T.gt(); r <= V; r += T.stride()) {
+    int32_t lo = 0, hi = (int32_t)E;
+    while (lo < hi) {
+      const int32_t mid = (lo + hi) >> 1;
+      if (src[mid] < r) lo = mid + 1;
+      else hi = mid;
+    }
+    roff[r] = lo;
   }
 }
 
@@ -1571,19 +1590,22 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
     // The list of rows M, of EM entries: the list itself, or its CSR.
     List M = L;
     int64_t EM = E;
+    bool sparse = E < 2 * (int64_t)V;
     if constexpr (!X::kResident) {
       if (any_order) {
         EM = V <= (1 << 16) ? build_csr<X, uint32_t>(T, L, E, V) : build_csr<X, uint64_t>(T, L, E, V);
         if (EM < 0) return false;
         M = List{W.csrc, W.cdst, W.cw, 1.0f};
-        if (EM == 0)
-          for (int32_t r = T.gt(); r <= V; r += T.stride()) W.roff[r] = 0;
+        sparse = EM < 2 * (int64_t)V;
+        if (sparse) search_starts<X>(T, M.src, EM, V);
         uint32_t f = 0;
 #pragma unroll 1
         for (int64_t e = T.gt(); e < EM; e += T.stride()) {
           const int32_t u = M.src[e], up = e > 0 ? M.src[e - 1] : -1;
-          row_starts<X>(up + 1, u, (int32_t)e);
-          if (e == EM - 1) row_starts<X>(u + 1, V, (int32_t)EM);
+          if (!sparse) {
+            row_starts<X>(up + 1, u, (int32_t)e);
+            if (e == EM - 1) row_starts<X>(u + 1, V, (int32_t)EM);
+          }
           const float x = M.w[e];
           if (x != truncf(x)) f |= fNotInt;
         }
@@ -1591,6 +1613,9 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
       }
     }
     if (!any_order) {
+      if constexpr (!X::kResident) {
+        if (sparse) search_starts<X>(T, L.src, E, V);
+      }
       uint32_t f = 0, nl = 0;
 #pragma unroll 1
       for (int64_t e0 = (int64_t)T.rank() * NT; e0 < E; e0 += T.stride()) {
@@ -1601,8 +1626,10 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
         const int32_t up = in && e > 0 ? L.src[e - 1] : -1;
         const float x = in ? L.w[e] : 0.0f;
         if (in) {
-          row_starts<X>(up + 1, u, (int32_t)e);
-          if (e == E - 1) row_starts<X>(u + 1, V, (int32_t)E);
+          if (X::kResident || !sparse) {
+            row_starts<X>(up + 1, u, (int32_t)e);
+            if (e == E - 1) row_starts<X>(u + 1, V, (int32_t)E);
+          }
           if (x != truncf(x)) f |= fNotInt;
           if (u == d) { W.loopw[u] = x; W.hasl[u] = 1; ++nl; }
         }
