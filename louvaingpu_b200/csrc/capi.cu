@@ -183,10 +183,11 @@ void prepare_level(lvg_ctx* c, const ListFacts* facts = nullptr) {
   c->renumbered = false;
 }
 
-// Largest list small_run takes: at 1.9 M entries a level takes 0.57 ms on the
-// cooperative grid, 0.95 by the level kernels.  (Above 4 Mi the tree of m
-// would have more partials than finish_sum adds.)
-constexpr int64_t kSmallRunEntries = 2 * 1024 * 1024;
+// Largest list small_run takes, the last whose sums' tree has no more partials
+// than finish_sum adds: at 3.3 M entries a level takes 0.77 ms on the
+// cooperative grid, 0.99 by the level kernels; an SBM of 3.0 M entries runs in
+// 2.86 ms instead of 4.38.
+constexpr int64_t kSmallRunEntries = 4 * 1024 * 1024;
 
 // `copied`: the list lies in the arena.  facts: of the list, unless it was
 // built while it streamed in.

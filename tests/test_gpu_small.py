@@ -119,12 +119,12 @@ def test_caps_and_thresholds(Louvain, oracle, gen, kw):
     assert out[0] == out[1]
 
 
-@pytest.mark.parametrize("n,comms,p_in", [(30011, 150, 0.06), (90001, 450, 0.06), (200003, 900, 0.05)])
+@pytest.mark.parametrize("n,comms,p_in", [(30011, 150, 0.06), (90001, 450, 0.06), (200003, 900, 0.05), (240003, 600, 0.05)])
 def test_larger_graphs(Louvain, oracle, gen, n, comms, p_in):
     """A cooperative grid for the whole run (coarse keys of 32 and of 64 bits),
     and for the last levels of a run whose first are too large for it."""
     n, s, d, w = gen.sbm(n, comms, p_in, 2.0 / n, 1, 3, seed=9)
-    assert (len(s) > 64 * 1024) and ((len(s) > 2 * 1024 * 1024) == (n > 200000))
+    assert (len(s) > 64 * 1024) and ((len(s) > 4 * 1024 * 1024) == (n > 240000))
     with Louvain() as lv:
         lv.load_edges(s, d, w, n)
         run_equal(lv, lv.run(), oracle.Run(n, s, d, w), n, s, d, w, oracle)
