@@ -645,6 +645,7 @@ lvg_status lvg_create(const lvg_config* cfg, lvg_ctx** out) {
     }
     LVG_CUDA(cudaEventCreateWithFlags(&c->side.fork, cudaEventDisableTiming));
     c->have_side = true;
+    c->arena.open_box();   // with the streams: pinning it takes 1 to 3 ms
     cudaDeviceProp prop;
     LVG_CUDA(cudaGetDeviceProperties(&prop, c->device));
     c->persist_max = (size_t)prop.persistingL2CacheMaxSize;

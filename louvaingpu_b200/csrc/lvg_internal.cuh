@@ -53,6 +53,9 @@ struct Arena {
     if (base) cudaFree(base);
     base = nullptr; cap = lo = hi = 0;
   }
+  void open_box() {
+    if (!box) LVG_CUDA(cudaMallocHost(&box, kBox));
+  }
   void destroy() {
     release();
     if (box) cudaFreeHost(box);
@@ -102,7 +105,7 @@ struct Fetch {
   Fetch(Arena& ar, cudaStream_t st) : a(ar), s(st) {}
   template <typename T> const T* add(const T* dev, size_t n = 1) {
     const size_t bytes = sizeof(T) * n, at = (used + 15) & ~(size_t)15;
-    if (!a.box) LVG_CUDA(cudaMallocHost(&a.box, Arena::kBox));
+    a.open_box();
     if (at + bytes > Arena::kBox) throw Error(LVG_ERR_CAPACITY, "read-back box too small");
     LVG_CUDA(cudaMemcpyAsync(a.box + at, dev, bytes, cudaMemcpyDeviceToHost, s));
     used = at + bytes;

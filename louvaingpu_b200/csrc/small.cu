@@ -1535,7 +1535,8 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
       if (V <= kResV && E <= kResE && !at.any_order) { at.tail = true; return true; }
       // below this a cluster's barriers save more than the chip's width does
       // (a level of 117 Ki entries takes 154 us on the grid, 199 on a cluster;
-      // one of 12 Ki 96 and 68)
+      // one of 12 Ki 96 and 68; one of 2 Ki entries and 189,000 vertices 504
+      // and 561: vertices count as entries do)
       if (T.mode == kModeGrid && E + V <= kSmallClusterEntries) { at.mid = true; return true; }
       // few entries for so many blocks: the last ones leave
       if (T.mode == kModeGrid && T.K_ > 1) {

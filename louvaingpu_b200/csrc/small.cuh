@@ -6,7 +6,7 @@ namespace lvg {
 
 constexpr int32_t kSmallMaxV = 1 << 18;     // communities of a packed table slot
 constexpr int kSmallMaxBlocks = 160;
-constexpr int kSmallClusterBlocks = 16;     // a single run's cluster, up to this many entries;
+constexpr int kSmallClusterBlocks = 16;     // a single run's cluster, up to this many entries and vertices;
 constexpr int64_t kSmallClusterEntries = 64 * 1024;   // above, a cooperative grid of the whole chip
 constexpr int32_t kSmallLevels = 48;        // levels one launch may record
 constexpr int32_t kSmallPassCap = 4096;     // passes of a level before it is left to the caller

@@ -55,6 +55,12 @@ def graph(gen, oracle, name):
         n = int(arg)
         s, d = np.divmod(np.arange(n * n, dtype=np.int32), np.int32(n))
         return n, s[s != d], d[s != d], np.ones(n * n - n, np.float32)
+    if kind == "gaps":          # cliques with runs of vertices without edges between them, more than a block records
+        size, gap, count = map(int, arg.split(":"))
+        i, j = np.divmod(np.arange(size * size), size)
+        at = (np.arange(count) * (size + gap))[:, None]
+        s, d = ((at + x[i != j]).ravel().astype(np.int32) for x in (i, j))
+        return count * (size + gap), s, d, np.ones(len(s), np.float32)
     n = int(arg)                # sbm:<n>
     return gen.sbm(n, max(2, n // 60), 0.25, 3.0 / n, 1, 4, seed=n)
 
@@ -62,7 +68,7 @@ def graph(gen, oracle, name):
 NAMES = ["one:", "loop:", "star:4095", "star:4096", "star:4097", "star:9000", "star:66000", "stars8:2048", "stars8:2049",
          "isolated:65536", "isolated:65537", "case:loops_zeros_isolated", "case:odd_sizes", "case:weighted",
          "eighths:900", "eighths:4001", "heavy:", "dense:64", "dense:511", "dense:513", "sbm:70", "sbm:1025",
-         "sbm:2049", "sbm:8193", "sbm:14001"]
+         "sbm:2049", "sbm:8193", "sbm:14001", "gaps:15:66:70", "gaps:100:200:60"]
 
 
 @pytest.mark.parametrize("name", NAMES)
