@@ -2624,6 +2624,16 @@ static void launch_thread(const LevelGraph& g, MoveArgs P, int bucket, cudaStrea
   LVG_LAUNCH();
 }
 
+// Blocks an SM of the persistent hub and tile kernels: as many as fit would
+// keep the other classes, which wait on gathers, off the chip until they are
+// done.  Level-0 passes (both, ms) of R-MAT 25 / 24 / 22 at the default
+// thresholds, with 8 and 5 blocks (all that fit) 48.4 / 20.5 / 4.3, 5 and 4
+// 46.9 / 20.3 / 4.3, 4 and 3 45.0 / 20.0 / 4.2, 4 and 2 49.7 / 21.1 / 4.9.
+// With fewer block-class rows than a wave of their kernel, or in a batch, whose
+// rows are mostly the tiles', there is little to make room for (128 mixed
+// graphs: 39.4 ms without the limit, 40.5 with it).
+constexpr int kHubBlocks = 4, kTileBlocks = 3;
+
 // The degree classes are independent within a pass (each writes only its own
 // vertices' decisions and atomically adds into the deltas), so the small-grid
 // classes run on side streams, forked from and joined back into `s`.
@@ -2639,6 +2649,7 @@ void launch_moves(const LevelGraph& g, CommState& st, cudaStream_t s, const Side
     for (int k = 0; k < 3; ++k) LVG_CUDA(cudaStreamWaitEvent(ss->side[k], ss->fork, 0));
     sh = ss->side[0]; sb = ss->side[1]; st2 = ss->side[2];
   }
+  const bool room = !q && g.nbucket[kBBlock] >= 8 * (int64_t)sm_count();
   const int64_t nhub = g.nbucket[kBHub];
   if (nhub > 0) {
     HubArgs H;
@@ -2650,7 +2661,7 @@ void launch_moves(const LevelGraph& g, CommState& st, cudaStream_t s, const Side
     hub_part_kernel<<<(unsigned)g.nchunk, kHubPartThreads, 0, sh>>>(P, H);
     LVG_LAUNCH();
     const size_t smem = g.int_acc ? agg_smem_bytes<true>() : agg_smem_bytes<false>();
-    const int per_sm = std::max(1, std::min(8, (int)((227u * 1024u) / (smem + 1024))));
+    const int per_sm = std::max(1, std::min(room ? kHubBlocks : 8, (int)((227u * 1024u) / (smem + 1024))));
     const int64_t grid = std::min<int64_t>(g.nhub_bucket, (int64_t)sm_count() * per_sm);
     MoveArgs PA = P;
     PA.queue = q ? q + 0 : nullptr;
@@ -2691,7 +2702,7 @@ void launch_moves(const LevelGraph& g, CommState& st, cudaStream_t s, const Side
     if (g.int_acc && g.V <= kTilePackedMaxComm) {
       Q.queue = q ? q + 1 : nullptr;
       const size_t smem = sizeof(TilePackedSmem);
-      const int per_sm = std::max(1, std::min(8, (int)((227u * 1024u) / (smem + 1024))));
+      const int per_sm = std::max(1, std::min(room ? kTileBlocks : 8, (int)((227u * 1024u) / (smem + 1024))));
       const int64_t grid = std::min<int64_t>(g.ntiles, (int64_t)sm_count() * per_sm);
       move_tile_packed_kernel<<<(unsigned)std::max<int64_t>(grid, 1), kThreads, smem, st2>>>(Q, g.tile_start,
                                                                                             g.ntiles);
