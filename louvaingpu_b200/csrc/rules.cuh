@@ -112,7 +112,7 @@ __device__ __forceinline__ double q_term(double in, double tot, double m, double
 }
 
 __device__ __forceinline__ bool entry_ok(int32_t u, int32_t v, float x, int32_t V) {
-  return u >= 0 && u < V && v >= 0 && v < V && x >= 0.0f && !isinf(x);   // as validate_kernel
+  return u >= 0 && u < V && v >= 0 && v < V && x >= 0.0f && !isinf(x);   // as list_facts_kernel
 }
 
 }  // namespace lvg

@@ -1059,7 +1059,7 @@ __device__ __forceinline__ void commit(const Team<X> T, int32_t V, double m) {
 }
 
 // Entries of the list checked: ids and weights, strict order, and symmetry by
-// the fingerprints of list_check_kernel.
+// the fingerprints of list_facts_kernel.
 template <typename X>
 __device__ __noinline__ void check_list(const Team<X> T, const List L, int64_t E, int32_t V) {
   const uint64_t K1 = 0x243F6A8885A308D3ull, K2 = 0x13198A2E03707344ull;
@@ -1980,7 +1980,7 @@ __device__ __forceinline__ bool wants_q(const SmallJob& J, const Between& B) {
 constexpr int kQThreads = 512;
 
 // Third launch (K blocks a job): community strengths and internal weights of
-// the final communities over the job's list, as nm_accum_sym_kernel: the list
+// the final communities over the job's list, as nm_accum_kernel<true>: the list
 // is symmetric, so each entry adds 2w to its source's community.
 __global__ void __launch_bounds__(kQThreads) small_sum_kernel(const SmallJob* jobs, int K) {
   const SmallJob& J = jobs[blockIdx.x / K];
