@@ -1294,9 +1294,11 @@ __device__ __forceinline__ bool count_runs(const Team<X> T, const Keyed<Key> key
 
 // The coarse list of a level of C communities (new ids W.newid of the labels
 // W.comm) into (osrc, odst, ow); returns its length (-1: a barrier's wait ran
-// out).
+// out).  packed: whole weights and degrees below 2^30, so that a sum over the
+// level stays far below 2^63 (a whole weight alone may be any float from 2^23
+// up, and 2^64 fits no integer).
 template <typename X, typename Key>
-__device__ __noinline__ int64_t coarsen(const Team<X> T, const List L, int64_t E, int32_t C, bool integral,
+__device__ __noinline__ int64_t coarsen(const Team<X> T, const List L, int64_t E, int32_t C, bool packed,
                                         int32_t* osrc, int32_t* odst, float* ow) {
   constexpr int NT = X::NT, kIt = 4;
   auto& S = X::S();
@@ -1314,8 +1316,8 @@ __device__ __noinline__ int64_t coarsen(const Team<X> T, const List L, int64_t E
     for (int64_t e = tid; e < E; e += NT) {
       const float x = L.w[e];
       const int cell = W.newid[W.comm[L.src[e]]] * C + W.newid[W.comm[L.dst[e]]];
-      // integral weights add as integers (shared memory adds those in place)
-      if (integral) atomicAdd(reinterpret_cast<unsigned long long*>(&S.u.cell[cell]),
+      // those add as integers (shared memory adds them in place)
+      if (packed) atomicAdd(reinterpret_cast<unsigned long long*>(&S.u.cell[cell]),
                               x == 0.0f ? 1ull : (unsigned long long)x);       // InducedGraphKernel.cu:38-39
       else atomicAdd(&S.u.cell[cell], x == 0.0f ? 1.0 : (double)x);
     }
@@ -1333,7 +1335,7 @@ __device__ __noinline__ int64_t coarsen(const Team<X> T, const List L, int64_t E
       for (int x = x0; x < x1; ++x) {
         const double sum = S.u.cell[x];
         if (sum != 0.0) {
-          const float w = __double2float_rn(integral ? (double)__double_as_longlong(sum) : sum);
+          const float w = __double2float_rn(packed ? (double)__double_as_longlong(sum) : sum);
           W.src[r] = osrc[r] = row;
           W.dst[r] = odst[r] = column;
           W.w[r] = ow[r] = w;
@@ -1820,8 +1822,8 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
     float* nw = nullptr;
     if (!last) {
       list_of(J.lists, J.E, at.nlev & 1, &ns, &nd, &nw);
-      if (X::kResident || C <= (1u << 16)) E1 = coarsen<X, uint32_t>(T, L, E, (int32_t)C, integral, ns, nd, nw);
-      else E1 = coarsen<X, uint64_t>(T, L, E, (int32_t)C, integral, ns, nd, nw);
+      if (X::kResident || C <= (1u << 16)) E1 = coarsen<X, uint32_t>(T, L, E, (int32_t)C, packed, ns, nd, nw);
+      else E1 = coarsen<X, uint64_t>(T, L, E, (int32_t)C, packed, ns, nd, nw);
       if (E1 < 0) return false;
     }
     if (lead && J.lv) {
