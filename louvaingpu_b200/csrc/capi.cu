@@ -1254,6 +1254,11 @@ extern "C" lvg_status lvg_autotune(lvg_ctx* c, const lvg_tune_space* sp, lvg_tun
 // launches over the disjoint union of the graphs still running.
 namespace {
 
+// Device bytes for a batch of G graphs with V vertices and E entries in all.
+size_t batch_estimate(int64_t V, int64_t E, int64_t G) {
+  return arena_estimate(V, E, true) + 256 * (size_t)G + 8 * (size_t)V;
+}
+
 struct BatchLevel {
   std::vector<int32_t> act;     // original graph of each level graph
   std::vector<int32_t> vbase;   // [G+1] vertex ranges of the level graphs
@@ -1269,6 +1274,8 @@ struct BatchInput {
   std::vector<const int32_t*> src, dst;
   std::vector<const float*> w;
   bool host = false;
+  size_t free_hi = 0;   // the lists are staged below this mark of the arena's high end and may be
+                        // given up once they are packed (0: they may not)
 };
 
 // Every level of the graphs of `in` (device lists) in shared launches over
@@ -1314,6 +1321,7 @@ void batch_union(lvg_ctx* c, const BatchInput& in, int32_t* part_out, double* q_
     sync(c);
     require(h == 0, LVG_ERR_INVALID_ARG, "edge list has a vertex id out of its graph or a negative / non-finite weight");
   }
+  if (in.free_hi) a.hi = in.free_hi;
   const size_t base_lo = a.lo;
   std::vector<double> mod(G0, 0.0);
   std::vector<int32_t> levels(G0, 0), comms(G0, 0), status(G0, 0);
@@ -1600,7 +1608,7 @@ SmallBatch batch_small_start(lvg_ctx* c, const BatchInput& in, int32_t* part_d) 
     other_v -= in.voff[g + 1] - in.voff[g];
   }
   const size_t need = lists + work + n * (sizeof(SmallJob) + sizeof(SmallResult)) + 8 * Arena::kAlign;
-  const size_t rest = others > 0 ? arena_estimate(other_v, others, true) : 0;
+  const size_t rest = others > 0 ? batch_estimate(other_v, others, in.G - n) : 0;
   if (a.hi < a.lo || a.hi - a.lo < need + rest) {   // the union path takes them all
     which.clear();
     return B;
@@ -1675,9 +1683,11 @@ void batch_small_finish(lvg_ctx* c, const SmallBatch& B, std::vector<char>& done
   }
 }
 
-// The graphs of `in` not marked done, as a batch of their own.
+// The graphs of `in` not marked done, as a batch of their own.  free_hi: as
+// BatchInput's.
 void batch_rest(lvg_ctx* c, const BatchInput& in, std::vector<char>& done, const std::vector<char>& skip,
-                int32_t* part_d, double* q_out, int32_t* levels_out, int32_t* comms_out, int32_t* status_out) {
+                int32_t* part_d, double* q_out, int32_t* levels_out, int32_t* comms_out, int32_t* status_out,
+                size_t free_hi) {
   std::vector<int32_t> rest, rvoff(1, 0), to;
   std::vector<int64_t> reoff(1, 0);
   BatchInput sub;
@@ -1695,6 +1705,7 @@ void batch_rest(lvg_ctx* c, const BatchInput& in, std::vector<char>& done, const
   sub.G = (int32_t)rest.size();
   sub.eoff = reoff.data();
   sub.voff = rvoff.data();
+  sub.free_hi = free_hi;
   std::vector<double> q(rest.size());
   std::vector<int32_t> lev(rest.size()), com(rest.size()), stat(rest.size());
   const size_t lo0 = c->arena.lo;
@@ -1730,8 +1741,7 @@ void batch_run(lvg_ctx* c, const BatchInput& given, int32_t* part_out, double* q
   c->pre0 = PreCsr();   // the batch reuses the arena
   c->loaded = false;
   c->have_state = false;
-  size_t need = c->cfg.arena_bytes > 0 ? (size_t)c->cfg.arena_bytes
-                                       : arena_estimate(V0, E0, true) + 256 * (size_t)G0 + 8 * (size_t)V0;
+  size_t need = c->cfg.arena_bytes > 0 ? (size_t)c->cfg.arena_bytes : batch_estimate(V0, E0, G0);
   c->arena.reserve(need);
   Arena& a = c->arena;
   BatchInput in = given;
@@ -1762,22 +1772,33 @@ void batch_run(lvg_ctx* c, const BatchInput& given, int32_t* part_out, double* q
     }
     in.host = false;
   }
+  // What a union needs beside its own arrays is given up before it: the staged
+  // lists once it has packed them, the small graphs' memory once they are done
+  // (graphs they leave open go to a second union, in the room of the batch's
+  // estimate).
+  const size_t free_hi = given.host ? hs.mark : 0;
   const size_t lo0 = a.lo;
   int32_t* part_d = a.lo_n<int32_t>(V0);
-  SmallBatch small;
   try {
-    small = batch_small_start(c, in, part_d);
-    if (small.which.empty()) {
+    std::vector<char> done((size_t)G0, 0);
+    {
+      HiScope held(a);
+      const SmallBatch small = batch_small_start(c, in, part_d);
+      if (!small.which.empty()) {
+        std::vector<char> started((size_t)G0, 0);
+        for (int32_t g : small.which) started[g] = 1;
+        batch_rest(c, in, done, started, part_d, q_out, levels_out, comms_out, status_out, 0);
+        batch_small_finish(c, small, done, q_out, levels_out, comms_out, status_out);
+      }
+    }
+    if (std::find(done.begin(), done.end(), 1) == done.end()) {   // no graph has run yet
       a.lo = lo0;
+      in.free_hi = free_hi;
       batch_union(c, in, part_out, q_out, levels_out, comms_out, status_out, nullptr, nullptr);
       return;
     }
-    std::vector<char> done((size_t)G0, 0), started((size_t)G0, 0);
     const std::vector<char> none((size_t)G0, 0);
-    for (int32_t g : small.which) started[g] = 1;
-    batch_rest(c, in, done, started, part_d, q_out, levels_out, comms_out, status_out);
-    batch_small_finish(c, small, done, q_out, levels_out, comms_out, status_out);
-    batch_rest(c, in, done, none, part_d, q_out, levels_out, comms_out, status_out);
+    batch_rest(c, in, done, none, part_d, q_out, levels_out, comms_out, status_out, free_hi);
   } catch (...) {   // nothing of the batch may still run when its memory is given up
     for (cudaStream_t st : c->small_streams)
       if (st) cudaStreamSynchronize(st);
@@ -1868,8 +1889,7 @@ extern "C" lvg_status lvg_reserve(lvg_ctx* c, int64_t bytes) {
 
 extern "C" lvg_status lvg_batch_footprint(int64_t n_vertices, int64_t n_entries, int32_t n_graphs, int64_t* bytes) {
   if (!bytes || n_vertices < 0 || n_entries < 0 || n_graphs < 0) return LVG_ERR_INVALID_ARG;
-  *bytes = (int64_t)(arena_estimate(n_vertices, n_entries, true) + 256 * (size_t)n_graphs +
-                     8 * (size_t)n_vertices);
+  *bytes = (int64_t)batch_estimate(n_vertices, n_entries, n_graphs);
   return LVG_OK;
 }
 

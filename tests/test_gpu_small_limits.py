@@ -41,3 +41,74 @@ def test_whole_weights_beyond_integers(Louvain, oracle, gen, unit):
             run_equal(lv, lv.run(), orun, n, s, d, w, oracle)
             np.testing.assert_array_equal(b.part(g), orun.final)
             assert b.n_levels[g] == len(orun.levels)
+
+
+def listed_once(n, degree, seed):
+    """A graph of 50-vertex blocks, every edge listed once, in any order."""
+    rng = np.random.default_rng(seed)
+    s = rng.integers(0, n, n * degree)
+    d = np.where(rng.random(len(s)) < 0.8, s // 50 * 50 + rng.integers(0, 50, len(s)), rng.integers(0, n, len(s)))
+    d = np.minimum(d, n - 1)
+    keep = s != d
+    return n, s[keep].astype(np.int32), d[keep].astype(np.int32), rng.integers(1, 5, keep.sum()).astype(np.float32)
+
+
+@pytest.fixture(scope="module")
+def unsorted_graphs():
+    """6.3 M entries in graphs a cluster starts and leaves open."""
+    return [listed_once(5000, 10, k) for k in range(128)]
+
+
+def check_sample(oracle, graphs, part, n_levels, sample=(0, 31, 64, 127)):
+    for g in sample:
+        orun = oracle.Run(*graphs[g])
+        np.testing.assert_array_equal(part(g), orun.final, err_msg=str(g))
+        assert n_levels[g] == len(orun.levels)
+
+
+@pytest.mark.parametrize("others", [0, 1])
+@pytest.mark.parametrize("where", ["host", "device"])
+def test_batches_of_unsorted_small_graphs_fit_the_default_arena(Louvain, oracle, gen, unsorted_graphs, where, others):
+    """The union that takes the graphs left open needs the memory they were
+    started in, and the staged copies of host lists.  others: beside a graph
+    that is no small run, and ones that are and finish."""
+    graphs = list(unsorted_graphs)
+    if others:
+        graphs += [gen.sbm(40000, 200, 0.06, 2.0 / 40000, 1, 4, seed=1), gen.sbm(900, 20, 0.3, 0.01, 1, 4, seed=2)]
+    with Louvain() as lv:
+        if where == "host":
+            b = lv.run_batch(graphs)
+        else:
+            import torch
+            from louvaingpu_b200.louvain import pack_graphs
+            s, d, w, eoff, voff = pack_graphs(graphs)
+            t = [torch.from_numpy(x).cuda() for x in (s, d, w)]
+            torch.cuda.synchronize()
+            b = lv.run_batch_device(*(x.data_ptr() for x in t), eoff, voff)
+    assert not b.status.any()
+    check_sample(oracle, graphs, b.part, b.n_levels, (0, 31, 64, 127) + tuple(range(128, len(graphs))))
+
+
+def test_server_groups_of_unsorted_small_graphs_stay_whole(oracle, unsorted_graphs):
+    """A slot of just the footprint of all requests runs them as one group (a
+    group that exhausts the arena would be split in two)."""
+    import ctypes
+    import torch
+    from louvaingpu_b200 import _lib
+    from louvaingpu_b200.serving import Server
+    graphs = unsorted_graphs
+    t = [[torch.from_numpy(x).cuda() for x in g[1:]] for g in graphs]
+    torch.cuda.synchronize()
+    E, V, size = sum(len(g[1]) for g in graphs), sum(g[0] for g in graphs), ctypes.c_int64()
+    assert _lib.load().lvg_batch_footprint(V, E, len(graphs), ctypes.byref(size)) == 0
+    parts = [np.zeros(g[0], np.int32) for g in graphs]
+    with Server(n_slots=1, hbm_budget=size.value, max_batch_entries=E, max_batch_graphs=len(graphs)) as srv:
+        ids = [srv.submit(*(x.data_ptr() for x in a), len(g[1]), g[0], part_out=p)
+               for a, g, p in zip(t, graphs, parts)]
+        srv.drain(timeout_ms=60000)
+        got = {r.id: r for r in srv.poll(len(graphs))}
+        taken = srv.stats()["batches"]
+    assert all(got[i].status == 0 for i in ids)
+    sizes = [got[i].batch_graphs for i in ids]
+    assert sum(sizes.count(k) // k for k in set(sizes)) == taken   # groups as the slot took them
+    check_sample(oracle, graphs, lambda g: parts[g], [got[i].n_levels for i in ids])
