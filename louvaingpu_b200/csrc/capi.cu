@@ -65,8 +65,8 @@ struct lvg_ctx {
   bool renumbered = false;
   bool built = false;            // the level's CSR and state exist (c->g, c->st); else only its list
   bool small0 = false;           // level 0 is a list small_run takes
-  bool replay = false;           // not built because small_run finished the run on this level:
-  double replay_lower = 0.0;     //   its state is that of a one-level phase with this floor
+  const double* kept = nullptr;  // not built because small_run finished the run on this level: the state
+                                 //   it ended in (SmallJob::state), with the last level's labels
   bool timed = false;            // the last level's renumbering is between pev[2] and pev[3]
   bool pristine = false;         // level 0 as loaded: no pass, state change or renumbering since
   bool symmetric0 = false;       // the level-0 list was found sorted and symmetric at load
@@ -218,7 +218,7 @@ void load_common(lvg_ctx* c, const int32_t* d_src, const int32_t* d_dst, const f
   c->g.w = d_w;
   c->g.pre = &c->pre0;
   c->small0 = ready;
-  c->replay = false;
+  c->kept = nullptr;
   c->built = false;
   if (ready) {
     c->have_state = true;
@@ -246,7 +246,7 @@ void reset_to_level0(lvg_ctx* c, bool build = true) {
   c->g.dst = c->dst0;
   c->g.w = c->w0;
   c->g.pre = &c->pre0;
-  c->replay = false;
+  c->kept = nullptr;
   c->built = false;
   c->renumbered = false;
   if (build) prepare_level(c);
@@ -415,7 +415,7 @@ void induce_level(lvg_ctx* c) {
   c->g.pre = &c->pre_next;
   c->level += 1;
   c->built = false;
-  c->replay = false;
+  c->kept = nullptr;
   c->renumbered = false;
 }
 
@@ -424,16 +424,10 @@ void ensure_built(lvg_ctx* c) {
   if (c->built) return;
   const bool renumbered = c->renumbered, pristine = c->pristine;
   prepare_level(c);
-  if (c->replay) {
-    const std::vector<float> ms = c->pass_ms, move_ms = c->move_pass_ms;
-    const double total = c->move_ms;
-    const int64_t passes = c->move_passes;
-    one_level(c, c->replay_lower, nullptr, nullptr, nullptr, nullptr);
-    c->pass_ms = ms;
-    c->move_pass_ms = move_ms;
-    c->move_ms = total;
-    c->move_passes = passes;
-    c->replay = false;
+  if (c->kept) {
+    set_state(c->g, c->st, c->levels.back().d_labels, c->kept, c->kept + c->g.V,
+              reinterpret_cast<const int32_t*>(c->kept + 2 * (size_t)c->g.V), c->stream);
+    c->kept = nullptr;
   }
   c->renumbered = renumbered;
   c->pristine = pristine;
@@ -463,7 +457,7 @@ bool run_small(lvg_ctx* c, RunState& R) {
   // level 0: checked at load; later lists are symmetric when their CSR was written
   const bool any_order = c->level > 0 && !c->pre_next.valid;
   const size_t need = small_list_bytes(E) + small_work_bytes(V, E, any_order) + sizeof(int32_t) * ((size_t)parts_cap + V) +
-                      sizeof(SmallOut) + sizeof(SmallJob) + 16 * Arena::kAlign;
+                      small_state_bytes(V) + sizeof(SmallOut) + sizeof(SmallJob) + 16 * Arena::kAlign;
   if (a.hi < a.lo || a.hi - a.lo < need) return false;
   c->pristine = false;
   const size_t lo0 = a.lo, hi0 = a.hi;
@@ -478,6 +472,7 @@ bool run_small(lvg_ctx* c, RunState& R) {
   J.lists = (char*)a.alloc_lo(small_list_bytes(E));
   J.parts = a.hi_n<int32_t>(parts_cap);
   J.parts_cap = parts_cap;
+  J.state = (double*)a.alloc_hi(small_state_bytes(V));
   const size_t run_hi = a.hi;
   J.check = J.dbl = any_order ? 1 : 0;
   J.want_q = c->level == 0 ? 1 : 0;
@@ -562,8 +557,7 @@ bool run_small(lvg_ctx* c, RunState& R) {
   c->pre_next = PreCsr();
   c->g.pre = nullptr;
   c->renumbered = !o.res.open;
-  c->replay = !o.res.open;
-  c->replay_lower = o.res.lower;
+  c->kept = o.res.open ? nullptr : J.state;
   if (o.res.open) {
     R.no_small = true;
     return false;

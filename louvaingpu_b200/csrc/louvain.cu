@@ -2805,6 +2805,21 @@ void set_state_from(const LevelGraph& g, CommState& st, const int32_t* d_comm, c
   clear_deltas(g, st, s);
 }
 
+void set_state(const LevelGraph& g, CommState& st, const int32_t* comm, const double* tot, const double* in,
+               const int32_t* size, cudaStream_t s) {
+  const size_t V = (size_t)g.V;
+  if (V == 0) return;
+  auto put = [&](void* to, const void* from, size_t bytes) {
+    LVG_CUDA(cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToDevice, s));
+  };
+  put(st.comm, comm, sizeof(int32_t) * V);
+  put(st.next, comm, sizeof(int32_t) * V);
+  put(st.tot, tot, sizeof(double) * V);
+  put(st.in, in, sizeof(double) * V);
+  put(st.size, size, sizeof(int32_t) * V);
+  clear_deltas(g, st, s);
+}
+
 void reset_ctl(CommState& st, double lower, double pass_min, int32_t max_passes, cudaStream_t s) {
   ctl_init_kernel<<<1, 1, 0, s>>>(st.ctl, lower, pass_min, max_passes);
   LVG_LAUNCH();

@@ -209,6 +209,9 @@ void launch_merge(const LevelGraph& g, CommState& st, cudaStream_t s);
 void launch_q(const LevelGraph& g, CommState& st, double* dst, cudaStream_t s);
 // Overwrite the committed state from comm (device) and recompute totals.
 void set_state_from(const LevelGraph& g, CommState& st, const int32_t* d_comm, cudaStream_t s);
+// Committed state as given (device arrays), deltas clear.
+void set_state(const LevelGraph& g, CommState& st, const int32_t* comm, const double* tot, const double* in,
+               const int32_t* size, cudaStream_t s);
 void clear_deltas(const LevelGraph& g, CommState& st, cudaStream_t s);
 void reset_ctl(CommState& st, double lower, double pass_min, int32_t max_passes, cudaStream_t s);
 

@@ -88,7 +88,7 @@ struct Between {
   int32_t V, ncomms, open, bad, status;
   int32_t comp;              // kComp*: what the composition still needs
   int64_t E, part_off;
-  double mod, lower;
+  double mod;
   double ms_per_tick;
 };
 
@@ -1058,6 +1058,23 @@ __device__ __forceinline__ void commit(const Team<X> T, int32_t V, double m) {
       });
 }
 
+// The state behind the level's last commit, which left its totals where they
+// were: for the calls that follow a run (its labels go with the partitions).
+template <typename X>
+__device__ __noinline__ void keep_state(const Team<X> T, int32_t V, double* state) {
+  auto& W = X::W();
+  double *tot = state, *in = state + V;
+  int32_t* size = reinterpret_cast<int32_t*>(in + V);
+#pragma unroll 1
+  for (int32_t c = T.gt(); c < V; c += T.stride()) {
+    Committed x{W.delta[c], W.tot[c], W.in[c], W.k[c], W.size[c], 0};
+    delta_commit(x.d, x.k, x.tot, x.in, x.size);
+    tot[c] = x.tot;
+    in[c] = x.in;
+    size[c] = x.size;
+  }
+}
+
 // Entries of the list checked: ids and weights, strict order, and symmetry by
 // the fingerprints of list_facts_kernel.
 template <typename X>
@@ -1498,7 +1515,7 @@ struct At {
   int buf = -1, nlev = 0, status = LVG_OK;
   bool open = false, symmetric = true, bad = false, tail = false, mid = false;
   bool any_order = false;   // the list may be other than sorted and symmetric, and there is room for that
-  double mod = 0.0, lower = 0.0;
+  double mod = 0.0;
   int64_t part_off = 0;
 };
 
@@ -1696,7 +1713,7 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
     const bool packed = integral && !(f2 & fNotInt);
     const bool longs = !X::kResident && (f2 & fLong);
     const double q0 = finish_sum<X>(W.qpart, V);
-    at.lower = level == 0 ? q0 : at.mod;        // LouvainCPP.cpp:356,446
+    const double lower = level == 0 ? q0 : at.mod;   // LouvainCPP.cpp:356,446
     find_rows<X>(T, V, EM);
     const int32_t v0 = S.row0, v1 = S.row1;
     const long long t1 = clock64();
@@ -1744,7 +1761,7 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
       commit<X, false>(T, V, m);
       if (!T.sync()) return false;
       const double q = finish_sum<X>(W.qpart, V);
-      floor_q = q_prev < at.lower ? at.lower : q_prev;
+      floor_q = q_prev < lower ? lower : q_prev;
       q_prev = q;
       if (pass >= kSmallPassCap) { at.open = true; return true; }
     }
@@ -1816,6 +1833,7 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
     if (st != LVG_OK) { at.status = st; last = true; }
     else if (level > 0 && (ql - at.mod) < cfg.level_min) last = true;
     else if (cfg.max_levels >= 0 && level + 1 >= cfg.max_levels) { at.status = LVG_ERR_NOT_CONVERGED; last = true; }
+    if (last && J.state) keep_state<X>(T, V, J.state);
     at.mod = ql;
     int64_t E1 = 0;
     int32_t *ns = nullptr, *nd = nullptr;
@@ -1875,7 +1893,6 @@ __device__ __forceinline__ void store_between(Between& B, const At& at) {
   B.E = at.E;
   B.part_off = at.part_off;
   B.mod = at.mod;
-  B.lower = at.lower;
 }
 
 __device__ __forceinline__ void load_between(const Between& B, At& at) {
@@ -1887,7 +1904,6 @@ __device__ __forceinline__ void load_between(const Between& B, At& at) {
   at.symmetric = (B.symmetric & 1) != 0;
   at.any_order = (B.symmetric & 2) != 0;
   at.mod = B.mod;
-  at.lower = B.lower;
   at.part_off = B.part_off;
 }
 
@@ -2072,7 +2088,6 @@ __global__ void __launch_bounds__(kQThreads) small_end_kernel(const SmallJob* jo
     O.E = B.E;
     O.ms_per_tick = B.ms_per_tick;
     O.mod = B.mod;
-    O.lower = B.lower;
     O.q_final = q;
     O.finished = 1;
   }

@@ -33,7 +33,6 @@ struct SmallResult {
   int64_t E;
   double ms_per_tick;
   double mod;               // Q of the last finished level
-  double lower;             // floor of the last finished level's pass loop
   double q_final;           // FP64 modularity of comp over the job's list (want_q)
 };
 
@@ -56,6 +55,8 @@ struct SmallJob {
   int32_t* parts;           // per-level partitions and labels, or nullptr
   int64_t parts_cap;        // ints
   int32_t* comp;            // [V] composition of the levels' partitions
+  double* state;            // small_state_bytes(V), or nullptr: the state the run ends in, over the last
+                            // level's communities: tot, in, then (int32) sizes, one array behind the other
   SmallResult* res;
   SmallLevel* lv;           // [kSmallLevels], or nullptr
   int32_t check;            // 1: ids, weights, order and symmetry not checked yet
@@ -71,6 +72,7 @@ struct SmallCfg {
 
 size_t small_list_bytes(int64_t E);           // both coarse list buffers
 size_t small_work_bytes(int32_t V, int64_t E, bool dbl);
+inline size_t small_state_bytes(int32_t V) { return (2 * sizeof(double) + sizeof(int32_t)) * (size_t)V; }
 // Coarse list buffer `buf` of a job's lists.
 void small_list(char* lists, int64_t E, int buf, int32_t** src, int32_t** dst, float** w);
 // True when the sizes are ones this path takes.

@@ -112,3 +112,29 @@ def test_server_groups_of_unsorted_small_graphs_stay_whole(oracle, unsorted_grap
     sizes = [got[i].batch_graphs for i in ids]
     assert sum(sizes.count(k) // k for k in set(sizes)) == taken   # groups as the slot took them
     check_sample(oracle, graphs, lambda g: parts[g], [got[i].n_levels for i in ids])
+
+
+@pytest.mark.parametrize("max_levels", [1, 2, -1])
+@pytest.mark.parametrize("n,blocks", [(60, 4), (400, 12), (3001, 60), (30011, 300), (90001, 450)])
+def test_state_after_a_run_is_the_runs_own(Louvain, gen, n, blocks, max_levels):
+    """Weights over 60 binary orders, so that sums depend on their order: Q
+    and labels that a call after the run sees are those the run ended in, not
+    those of its passes run again."""
+    from louvaingpu_b200 import LvgError
+    n, s, d, _ = gen.sbm(n, blocks, min(0.5, 15.0 * blocks / n), 2.0 / n, 1, 1, seed=n)
+    for seed in range(4):
+        x = np.random.default_rng(seed).random(n) * 30.0
+        w = np.exp2(x[s] + x[d] - 30.0).astype(np.float32)
+        with Louvain(max_levels=max_levels) as lv:
+            lv.load_edges(s, d, w, n)
+            try:
+                lv.run()
+            except LvgError as e:
+                assert e.status == 4 and max_levels > 0   # the level cap
+            last = lv.n_levels - 1
+            labels, part, info = lv.level_labels(last), lv.level_partition(last), lv.level_info(last)
+            assert lv.modularity() == info.q_level
+            again, comms = lv.renumber()
+            np.testing.assert_array_equal(again, part)
+            assert comms == info.n_comms
+            np.testing.assert_array_equal(lv.level_labels(last + 1), labels)
