@@ -1670,10 +1670,10 @@ void batch_small_finish(lvg_ctx* c, const SmallBatch& B, std::vector<char>& done
             "edge list has a vertex id out of its graph or a negative / non-finite weight");
     if (o[k].open || !o[k].finished) continue;
     done[g] = 1;
-    if (q_out) q_out[g] = o[k].q_final;
-    if (levels_out) levels_out[g] = o[k].n_levels;
-    if (comms_out) comms_out[g] = o[k].n_comms;
-    if (status_out) status_out[g] = o[k].status;
+    q_out[g] = o[k].q_final;
+    levels_out[g] = o[k].n_levels;
+    comms_out[g] = o[k].n_comms;
+    status_out[g] = o[k].status;
   }
 }
 
@@ -1708,10 +1708,10 @@ void batch_rest(lvg_ctx* c, const BatchInput& in, std::vector<char>& done, const
   for (size_t k = 0; k < rest.size(); ++k) {
     const int32_t g = rest[k];
     done[g] = 1;
-    if (q_out) q_out[g] = q[k];
-    if (levels_out) levels_out[g] = lev[k];
-    if (comms_out) comms_out[g] = com[k];
-    if (status_out) status_out[g] = stat[k];
+    q_out[g] = q[k];
+    levels_out[g] = lev[k];
+    comms_out[g] = com[k];
+    status_out[g] = stat[k];
   }
 }
 
@@ -1773,6 +1773,10 @@ void batch_run(lvg_ctx* c, const BatchInput& given, int32_t* part_out, double* q
   const size_t free_hi = given.host ? hs.mark : 0;
   const size_t lo0 = a.lo;
   int32_t* part_d = a.lo_n<int32_t>(V0);
+  // A list of a small graph may be refused when others have run: nothing is
+  // written to the caller's arrays before all are done.
+  std::vector<double> q((size_t)G0);
+  std::vector<int32_t> lev((size_t)G0), com((size_t)G0), stat((size_t)G0);
   try {
     std::vector<char> done((size_t)G0, 0);
     {
@@ -1781,8 +1785,8 @@ void batch_run(lvg_ctx* c, const BatchInput& given, int32_t* part_out, double* q
       if (!small.which.empty()) {
         std::vector<char> started((size_t)G0, 0);
         for (int32_t g : small.which) started[g] = 1;
-        batch_rest(c, in, done, started, part_d, q_out, levels_out, comms_out, status_out, 0);
-        batch_small_finish(c, small, done, q_out, levels_out, comms_out, status_out);
+        batch_rest(c, in, done, started, part_d, q.data(), lev.data(), com.data(), stat.data(), 0);
+        batch_small_finish(c, small, done, q.data(), lev.data(), com.data(), stat.data());
       }
     }
     if (std::find(done.begin(), done.end(), 1) == done.end()) {   // no graph has run yet
@@ -1792,7 +1796,7 @@ void batch_run(lvg_ctx* c, const BatchInput& given, int32_t* part_out, double* q
       return;
     }
     const std::vector<char> none((size_t)G0, 0);
-    batch_rest(c, in, done, none, part_d, q_out, levels_out, comms_out, status_out, free_hi);
+    batch_rest(c, in, done, none, part_d, q.data(), lev.data(), com.data(), stat.data(), free_hi);
   } catch (...) {   // nothing of the batch may still run when its memory is given up
     for (cudaStream_t st : c->small_streams)
       if (st) cudaStreamSynchronize(st);
@@ -1801,6 +1805,10 @@ void batch_run(lvg_ctx* c, const BatchInput& given, int32_t* part_out, double* q
   if (part_out && V0 > 0)
     LVG_CUDA(cudaMemcpyAsync(part_out, part_d, sizeof(int32_t) * V0, cudaMemcpyDeviceToHost, s));
   sync(c);
+  if (q_out) std::copy(q.begin(), q.end(), q_out);
+  if (levels_out) std::copy(lev.begin(), lev.end(), levels_out);
+  if (comms_out) std::copy(com.begin(), com.end(), comms_out);
+  if (status_out) std::copy(stat.begin(), stat.end(), status_out);
   c->levels.clear();
   c->g = LevelGraph();
   c->st = CommState();

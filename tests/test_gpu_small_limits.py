@@ -138,3 +138,26 @@ def test_state_after_a_run_is_the_runs_own(Louvain, gen, n, blocks, max_levels):
             np.testing.assert_array_equal(again, part)
             assert comms == info.n_comms
             np.testing.assert_array_equal(lv.level_labels(last + 1), labels)
+
+
+@pytest.mark.parametrize("fault", ["id", "weight"])
+def test_a_refused_batch_writes_nothing(gen, fault):
+    """A bad entry of a small graph is found beside the union of the others:
+    the call is refused with every output as it was."""
+    from louvaingpu_b200 import _lib, Louvain
+    from louvaingpu_b200.louvain import pack_graphs
+    bad = gen.sbm(500, 10, 0.3, 0.01, 1, 4, seed=3)
+    if fault == "id":
+        bad[2][-1] = 500
+    else:
+        bad[3][7] = -1.0
+    graphs = [gen.sbm(60001, 300, 0.06, 0.00005, 1, 3, seed=9), gen.sbm(900, 20, 0.3, 0.01, 1, 4, seed=2), bad]
+    s, d, w, eoff, voff = pack_graphs(graphs)
+    p = lambda x: x.ctypes.data
+    outs = [np.full(voff[-1], -7, np.int32), np.full(3, -7.0), *(np.full(3, -7, np.int32) for _ in range(3))]
+    L = _lib.load()
+    with Louvain(arena_bytes=1 << 30) as lv:   # room for both at once
+        assert L.lvg_batch_run(lv._h, p(s), p(d), p(w), p(eoff), p(voff), 3, *map(p, outs)) == 1
+        assert all((x == -7).all() for x in outs)
+        b = lv.run_batch(graphs[:2])
+        assert not b.status.any()
