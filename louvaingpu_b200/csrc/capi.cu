@@ -64,7 +64,8 @@ struct lvg_ctx {
   bool have_state = false;
   bool renumbered = false;
   bool built = false;            // the level's CSR and state exist (c->g, c->st); else only its list
-  bool small0 = false;           // level 0 is a list small_run takes
+  bool small0 = false;           // level 0 is a list small_run takes; what the load learnt of it,
+  ListFacts facts0;              //   for a call that needs its build after all
   const double* kept = nullptr;  // not built because small_run finished the run on this level: the state
                                  //   it ended in (SmallJob::state), with the last level's labels
   bool timed = false;            // the last level's renumbering is between pev[2] and pev[3]
@@ -189,6 +190,11 @@ void prepare_level(lvg_ctx* c, const ListFacts* facts = nullptr) {
 // 2.86 ms instead of 4.38.
 constexpr int64_t kSmallRunEntries = 4 * 1024 * 1024;
 
+// Where the facts of a list that may wait with its build are kept.
+uint32_t* facts_room(lvg_ctx* c, int32_t V, int64_t E) {
+  return small_fits(V, E, kSmallRunEntries) ? c->arena.lo_n<uint32_t>(facts_words(E)) : nullptr;
+}
+
 // `copied`: the list lies in the arena.  facts: of the list, unless it was
 // built while it streamed in.
 void load_common(lvg_ctx* c, const int32_t* d_src, const int32_t* d_dst, const float* d_w, int64_t E,
@@ -218,6 +224,7 @@ void load_common(lvg_ctx* c, const int32_t* d_src, const int32_t* d_dst, const f
   c->g.w = d_w;
   c->g.pre = &c->pre0;
   c->small0 = ready;
+  if (ready) c->facts0 = *facts;
   c->kept = nullptr;
   c->built = false;
   if (ready) {
@@ -249,7 +256,7 @@ void reset_to_level0(lvg_ctx* c, bool build = true) {
   c->kept = nullptr;
   c->built = false;
   c->renumbered = false;
-  if (build) prepare_level(c);
+  if (build) prepare_level(c, c->small0 ? &c->facts0 : nullptr);
   c->pristine = true;
 }
 
@@ -423,7 +430,7 @@ void induce_level(lvg_ctx* c) {
 void ensure_built(lvg_ctx* c) {
   if (c->built) return;
   const bool renumbered = c->renumbered, pristine = c->pristine;
-  prepare_level(c);
+  prepare_level(c, c->small0 && c->level == 0 ? &c->facts0 : nullptr);
   if (c->kept) {
     set_state(c->g, c->st, c->levels.back().d_labels, c->kept, c->kept + c->g.V,
               reinterpret_cast<const int32_t*>(c->kept + 2 * (size_t)c->g.V), c->stream);
@@ -721,7 +728,7 @@ lvg_status lvg_load_edges(lvg_ctx* c, const int32_t* src, const int32_t* dst, co
         LVG_CUDA(cudaMemcpyAsync(d, dst, sizeof(int32_t) * E, cudaMemcpyHostToDevice, c->stream));
         LVG_CUDA(cudaMemcpyAsync(ww, w, sizeof(float) * E, cudaMemcpyHostToDevice, c->stream));
       }
-      facts = list_facts(s, d, ww, E, V, c->arena, c->stream);
+      facts = list_facts(s, d, ww, E, V, c->arena, c->stream, facts_room(c, V, E));
       ok = facts.ok;
     }
     require(ok, LVG_ERR_INVALID_ARG, "edge list has a vertex id out of range or a negative / non-finite weight");
@@ -740,7 +747,7 @@ lvg_status lvg_load_edges_device(lvg_ctx* c, const int32_t* src, const int32_t* 
     size_t need = c->cfg.arena_bytes > 0 ? (size_t)c->cfg.arena_bytes : arena_estimate(V, E, false);
     c->arena.reserve(need);
     HiScope hs(c->arena);
-    const ListFacts facts = list_facts(src, dst, w, E, V, c->arena, c->stream);
+    const ListFacts facts = list_facts(src, dst, w, E, V, c->arena, c->stream, facts_room(c, V, E));
     require(facts.ok, LVG_ERR_INVALID_ARG,
             "edge list has a vertex id out of range or a negative / non-finite weight");
     load_common(c, src, dst, w, E, V, false, &facts);

@@ -2110,11 +2110,11 @@ static float weight_of(unsigned long long h) {
 }
 
 ListFacts list_facts(const int32_t* src, const int32_t* dst, const float* w, int64_t E, int32_t V, Arena& a,
-                     cudaStream_t s) {
+                     cudaStream_t s, uint32_t* pos) {
   ListFacts F;
   if (E <= 0) return F;
   const int64_t ng = (E + kGroup - 1) / kGroup;
-  F.pos = a.hi_n<uint32_t>(ng + 1);
+  F.pos = pos ? pos : a.hi_n<uint32_t>(facts_words(E));
   HiScope hs(a);
   double* gpart = a.hi_n<double>(ng);
   double* d_m = a.hi_n<double>(1);

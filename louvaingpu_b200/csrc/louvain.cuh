@@ -162,10 +162,12 @@ struct ListFacts {
   float max_w = 0.0f;             // largest weight
   int64_t nonloop = 0;            // entries that are not self loops
   double m = 0.0;                 // sum of the weights (fixed tree)
-  uint32_t* pos = nullptr;        // non-loop entries before each 2048-entry block (caller's high scratch)
+  uint32_t* pos = nullptr;        // non-loop entries before each 2048-entry block
 };
+inline int64_t facts_words(int64_t E) { return (E + kGroup - 1) / kGroup + 1; }   // of ListFacts::pos
+// pos: facts_words(E) words that outlive the facts (nullptr: the caller's high scratch).
 ListFacts list_facts(const int32_t* src, const int32_t* dst, const float* w, int64_t E, int32_t V, Arena& a,
-                     cudaStream_t s);
+                     cudaStream_t s, uint32_t* pos = nullptr);
 
 // Build the level CSR, degrees, loops and buckets (NeighbourCompute.cu:42-117,
 // InitKernel.cu:245-339).  Level arrays go to the arena's low end.

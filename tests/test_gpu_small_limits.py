@@ -161,3 +161,25 @@ def test_a_refused_batch_writes_nothing(gen, fault):
         assert all((x == -7).all() for x in outs)
         b = lv.run_batch(graphs[:2])
         assert not b.status.any()
+
+
+def test_a_build_after_the_load_reads_no_facts_again(Louvain, oracle, gen):
+    """A list that waits with its build keeps what the load learnt of it: the
+    launches up to Q are those of a load that builds at once (as it does in an
+    arena without room for any list's build)."""
+    import ctypes
+    from louvaingpu_b200 import _lib
+    from test_gpu_parity import csr_equal
+    n, s, d, w = gen.sbm(3001, 60, 0.2, 0.001, 1, 4, seed=1)
+    L, counts = _lib.load(), []
+    for arena in (0, 24 << 20):
+        with Louvain(arena_bytes=arena) as lv:
+            lv.load_edges(s, d, w, n)          # (the first sizes the arena)
+            at = [ctypes.c_int64(), ctypes.c_int64()]
+            L.lvg_kernel_launches(ctypes.byref(at[0]))
+            lv.load_edges(s, d, w, n)
+            lv.modularity()
+            L.lvg_kernel_launches(ctypes.byref(at[1]))
+            counts.append(at[1].value - at[0].value)
+            csr_equal(lv, oracle.Csr(n, s, d, w))
+    assert counts[0] == counts[1]
