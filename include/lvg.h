@@ -320,6 +320,14 @@ lvg_status lvg_modularity_fp64_noalloc(const int32_t* d_src, const int32_t* d_ds
  * restore normal operation.  Process-wide; for tests only. */
 lvg_status lvg_debug_radix_hold(int32_t spin_limit, int64_t hold_tile);
 
+/* Test hook of the path back from small runs (lists of at most 4 Mi entries,
+ * whose levels run inside a few launches).  Process-wide; for tests only.
+ *
+ * error != 0: launching their levels fails with that cudaError_t, without a
+ * launch.  Where it says that such a launch is not possible here, lvg_run and
+ * batches go on with the level kernels, else they return LVG_ERR_CUDA. */
+lvg_status lvg_debug_small_launch(int32_t error);
+
 /* Bytes of device memory the context holds (arena capacity) and its peak use. */
 lvg_status lvg_memory(const lvg_ctx* ctx, int64_t* capacity, int64_t* peak);
 

@@ -484,6 +484,7 @@ bool run_small(lvg_ctx* c, RunState& R) {
   J.check = J.dbl = any_order ? 1 : 0;
   J.want_q = c->level == 0 ? 1 : 0;
   SmallOut o;
+  std::memset(&o.res, 0, sizeof o.res);
   {
     HiScope hs(a);
     J.work = (char*)a.alloc_hi(small_work_bytes(V, E, any_order));
@@ -495,9 +496,10 @@ bool run_small(lvg_ctx* c, RunState& R) {
     LVG_CUDA(cudaMemcpyAsync(d_job, &J, sizeof J, cudaMemcpyHostToDevice, s));
     const SmallCfg cfg{c->cfg.pass_min_gain, c->cfg.level_min_gain, c->cfg.max_passes, c->cfg.max_levels};
     LVG_CUDA(cudaMemsetAsync(J.res, 0, sizeof(SmallResult), s));
-    if (E + V <= kSmallClusterEntries) small_run(d_job, 1, kSmallClusterBlocks, cfg, s);
-    else small_run_grid(d_job, J.work, small_grid_blocks(), cfg, s);
-    LVG_CUDA(cudaMemcpyAsync(&o, d_out, sizeof o, cudaMemcpyDeviceToHost, s));
+    const bool taken = E + V <= kSmallClusterEntries
+                           ? small_run(d_job, 1, kSmallClusterBlocks, cfg, s)
+                           : small_run_grid(d_job, J.work, small_grid_blocks(), cfg, s);
+    if (taken) LVG_CUDA(cudaMemcpyAsync(&o, d_out, sizeof o, cudaMemcpyDeviceToHost, s));
     if (c->level > 0) {   // a launch that finishes no level leaves no composition
       sync(c);
       if (o.res.finished && o.res.n_levels > 0) compose(c->composed, J.comp, c->V0, s);
@@ -1652,7 +1654,7 @@ SmallBatch batch_small_start(lvg_ctx* c, const BatchInput& in, int32_t* part_d) 
     while (k1 < n && small_blocks(jobs[k1].E) == K) ++k1;
     cudaStream_t st = c->small_streams[slot++ & 3];
     LVG_CUDA(cudaStreamWaitEvent(st, c->small_ev, 0));
-    small_run(jobs_d + k0, (int)(k1 - k0), K, cfg, st);
+    small_run(jobs_d + k0, (int)(k1 - k0), K, cfg, st);   // refused: not finished, the union takes them
     k0 = k1;
   }
   return B;

@@ -28,6 +28,7 @@
 // the tables hold, end the launch with the level left open; the caller goes on
 // with the level kernels from the same list.
 #include <algorithm>
+#include <atomic>
 #include <cooperative_groups.h>
 #include <mutex>
 #include <type_traits>
@@ -2109,8 +2110,13 @@ void set_attributes() {
   if (dev >= 0 && dev < kDevs) done[dev] = true;
 }
 
+// Test hook (lvg_debug_small_launch): the error every launch of the levels meets.
+std::atomic<int32_t> g_launch_error{0};
+
+// False: such a launch is refused here (a cluster or a grid that must be on
+// the chip together, on a stream that may use a part of the chip).
 template <int NT>
-void launch_levels(const SmallJob* jobs, int n, int K, int mode, int resume, const SmallCfg& cfg, cudaStream_t s) {
+bool launch_levels(const SmallJob* jobs, int n, int K, int mode, int resume, const SmallCfg& cfg, cudaStream_t s) {
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3((unsigned)(n * K));
   lc.blockDim = dim3(NT);
@@ -2128,8 +2134,21 @@ void launch_levels(const SmallJob* jobs, int n, int K, int mode, int resume, con
   }
   lc.attrs = at;
   lc.numAttrs = mode == kModeGrid || K > 1 ? 1 : 0;
-  LVG_CUDA(cudaLaunchKernelEx(&lc, small_kernel<NT>, jobs, K, mode, resume, cfg));
+  cudaError_t e = (cudaError_t)g_launch_error.load();
+  if (e == cudaSuccess) e = cudaLaunchKernelEx(&lc, small_kernel<NT>, jobs, K, mode, resume, cfg);
+  switch (e) {
+    case cudaErrorCooperativeLaunchTooLarge:
+    case cudaErrorInvalidClusterSize:
+    case cudaErrorLaunchOutOfResources:
+    case cudaErrorInvalidConfiguration:
+    case cudaErrorNotSupported:
+      cudaGetLastError();
+      return false;
+    default:
+      LVG_CUDA(e);
+  }
   count_launch();
+  return true;
 }
 
 // The launches behind the levels: the tail, and the results by K blocks a job.
@@ -2159,12 +2178,14 @@ bool small_fits(int64_t V, int64_t E, int64_t max_entries) {
   return V > 0 && V <= kSmallMaxV && E > 0 && E <= max_entries;
 }
 
-void small_run(const SmallJob* d_jobs, int n, int K, const SmallCfg& cfg, cudaStream_t s) {
-  if (n <= 0) return;
+bool small_run(const SmallJob* d_jobs, int n, int K, const SmallCfg& cfg, cudaStream_t s) {
+  if (n <= 0) return true;
   set_attributes();
-  if (K >= 8) launch_levels<1024>(d_jobs, n, K, kModeCluster, 0, cfg, s);
-  else launch_levels<512>(d_jobs, n, K, kModeCluster, 0, cfg, s);
+  if (!(K >= 8 ? launch_levels<1024>(d_jobs, n, K, kModeCluster, 0, cfg, s)
+               : launch_levels<512>(d_jobs, n, K, kModeCluster, 0, cfg, s)))
+    return false;
   launch_rest(d_jobs, n, K, cfg, s);
+  return true;
 }
 
 int small_grid_blocks() {
@@ -2184,13 +2205,20 @@ int small_grid_blocks() {
   return n;
 }
 
-void small_run_grid(const SmallJob* d_job, void* work, int K, const SmallCfg& cfg, cudaStream_t s) {
+bool small_run_grid(const SmallJob* d_job, void* work, int K, const SmallCfg& cfg, cudaStream_t s) {
   // the barrier's words, and the phase, should a wait run out
   LVG_CUDA(cudaMemsetAsync(work, 0, up256(sizeof(Ctl)) + up256(sizeof(Between)), s));
   set_attributes();
-  launch_levels<1024>(d_job, 1, K, kModeGrid, 0, cfg, s);
+  if (!launch_levels<1024>(d_job, 1, K, kModeGrid, 0, cfg, s)) return false;
+  // (refused, it leaves levels that the grid did not finish undone: no result)
   launch_levels<1024>(d_job, 1, kSmallClusterBlocks, kModeCluster, 1, cfg, s);
   launch_rest(d_job, 1, K, cfg, s);
+  return true;
 }
 
 }  // namespace lvg
+
+extern "C" lvg_status lvg_debug_small_launch(int32_t error) {
+  lvg::g_launch_error.store(error);
+  return LVG_OK;
+}

@@ -78,11 +78,12 @@ void small_list(char* lists, int64_t E, int buf, int32_t** src, int32_t** dst, f
 // True when the sizes are ones this path takes.
 bool small_fits(int64_t V, int64_t E, int64_t max_entries);
 // Runs n jobs (device array), each by a cluster of K blocks.  The caller has
-// cleared the results (finished == 0).
-void small_run(const SmallJob* d_jobs, int n, int K, const SmallCfg& cfg, cudaStream_t s);
+// cleared the results (finished == 0).  False: the device, or the part of it
+// the stream may use, does not take such a launch; nothing has run.
+bool small_run(const SmallJob* d_jobs, int n, int K, const SmallCfg& cfg, cudaStream_t s);
 // Runs one job (work: its work area) by a cooperative grid of
-// K <= small_grid_blocks() blocks.
-void small_run_grid(const SmallJob* d_job, void* work, int K, const SmallCfg& cfg, cudaStream_t s);
+// K <= small_grid_blocks() blocks.  False: as small_run's.
+bool small_run_grid(const SmallJob* d_job, void* work, int K, const SmallCfg& cfg, cudaStream_t s);
 int small_grid_blocks();
 
 }  // namespace lvg

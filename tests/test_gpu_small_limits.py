@@ -183,3 +183,68 @@ def test_a_build_after_the_load_reads_no_facts_again(Louvain, oracle, gen):
             counts.append(at[1].value - at[0].value)
             csr_equal(lv, oracle.Csr(n, s, d, w))
     assert counts[0] == counts[1]
+
+
+@pytest.fixture
+def hooks():
+    from louvaingpu_b200 import _lib
+    L = _lib.load()
+    yield L
+    assert L.lvg_debug_small_launch(0) == 0
+
+
+def launches():
+    import ctypes
+    from louvaingpu_b200 import _lib
+    n = ctypes.c_int64()
+    _lib.load().lvg_kernel_launches(ctypes.byref(n))
+    return n.value
+
+
+def run_counted(lv):
+    n = launches()
+    res = lv.run()
+    return res, launches() - n
+
+
+# n, blocks: a cluster's list; a grid's; a grid's behind levels of the level
+# kernels, as the list is in no order
+@pytest.mark.parametrize("n,blocks,unsorted", [(2000, 40, False), (30011, 300, False), (30011, 300, True)])
+@pytest.mark.parametrize("error", [720, 912, 701, 9, 801])
+def test_a_refused_launch_leaves_the_run_to_the_level_kernels(Louvain, oracle, gen, hooks, n, blocks, unsorted, error):
+    n, s, d, w = gen.sbm(n, blocks, 15.0 * blocks / n, 2.0 / n, 1, 4, seed=5)
+    if unsorted:
+        o = np.random.default_rng(2).permutation(len(s))
+        s, d, w = s[o], d[o], w[o]
+    orun = oracle.Run(n, s, d, w)
+    with Louvain() as lv:
+        lv.load_edges(s, d, w, n)
+        ref, n_ref = run_counted(lv)
+        run_equal(lv, ref, orun, n, s, d, w, oracle)
+        lv.load_edges(s, d, w, n)          # (a second run would build level 0 again)
+        assert hooks.lvg_debug_small_launch(error) == 0
+        res, n_res = run_counted(lv)
+        assert n_res > n_ref + 20
+        run_equal(lv, res, orun, n, s, d, w, oracle)
+        lv.modularity()
+        b = lv.run_batch([(n, s, d, w), triangles()])
+        np.testing.assert_array_equal(b.part(0), orun.final)
+        assert hooks.lvg_debug_small_launch(0) == 0
+        lv.load_edges(s, d, w, n)
+        assert run_counted(lv) == (ref, n_ref)
+
+
+def test_other_launch_errors_are_reported(Louvain, gen, hooks):
+    from louvaingpu_b200 import LvgError
+    n, s, d, w = gen.sbm(2000, 40, 0.3, 0.001, 1, 4, seed=5)
+    with Louvain() as lv:
+        lv.load_edges(s, d, w, n)
+        ref = lv.run()
+        assert hooks.lvg_debug_small_launch(999) == 0
+        for call in (lv.run, lambda: lv.run_batch([(n, s, d, w)])):
+            with pytest.raises(LvgError) as e:
+                call()
+            assert e.value.status == 5
+        assert hooks.lvg_debug_small_launch(0) == 0
+        lv.load_edges(s, d, w, n)
+        assert lv.run() == ref
