@@ -320,13 +320,18 @@ lvg_status lvg_modularity_fp64_noalloc(const int32_t* d_src, const int32_t* d_ds
  * restore normal operation.  Process-wide; for tests only. */
 lvg_status lvg_debug_radix_hold(int32_t spin_limit, int64_t hold_tile);
 
-/* Test hook of the path back from small runs (lists of at most 4 Mi entries,
+/* Test hooks of the paths back from small runs (lists of at most 4 Mi entries,
  * whose levels run inside a few launches).  Process-wide; for tests only.
  *
  * error != 0: launching their levels fails with that cudaError_t, without a
  * launch.  Where it says that such a launch is not possible here, lvg_run and
  * batches go on with the level kernels, else they return LVG_ERR_CUDA. */
 lvg_status lvg_debug_small_launch(int32_t error);
+/* block >= 0: that block of a cooperative grid leaves before its first
+ * barrier, so that the others wait for it until wait_ns have passed (0: the
+ * default, 4 s) and the launch ends without a result; lvg_run goes on with the
+ * level kernels.  (-1, 0) restores normal operation. */
+lvg_status lvg_debug_small_hold(int32_t block, int64_t wait_ns);
 
 /* Bytes of device memory the context holds (arena capacity) and its peak use. */
 lvg_status lvg_memory(const lvg_ctx* ctx, int64_t* capacity, int64_t* peak);

@@ -130,6 +130,7 @@ SIGNATURES = {
     "lvg_get_level_edges": (i32, [P, ctypes.POINTER(i64), P, P, P]),
     "lvg_debug_radix_hold": (i32, [i32, i64]),
     "lvg_debug_small_launch": (i32, [i32]),
+    "lvg_debug_small_hold": (i32, [i32, i64]),
     "lvg_set_communities": (i32, [P, P]),
     "lvg_move_decide": (i32, [P, P, P]),
     "lvg_last_pass_times": (i32, [P, P, i32, ctypes.POINTER(i32)]),

@@ -62,7 +62,6 @@ constexpr int kGaps = 64;                  // runs of empty rows a block fills t
 constexpr int kHubs = 32;                  // long rows a block looks up at a time
 constexpr int kResThreads = 512;
 constexpr int kResV = 512, kResE = 6144;   // a level this small lives in one block's shared memory
-constexpr unsigned long long kWaitNs = 4000000000ull;   // limit of a grid barrier's wait
 constexpr unsigned long long kEmpty = ~0ull;
 static_assert(kSmallMaxV <= (1 << kCommBits), "packed keys hold 18-bit communities");
 
@@ -212,6 +211,7 @@ struct Space {
   int4 gap[kGaps];
   int32_t nclaimed, row0, row1;
   unsigned long long goal;   // grid barrier: arrivals awaited
+  unsigned long long wait_ns;   // and the limit of the wait
   int32_t alive;
   SmallJob J;
 };
@@ -256,13 +256,14 @@ __device__ __forceinline__ unsigned long long now_ns() {
 }
 
 // Waits until *p reaches `goal`; false when the wait's limit has passed.
-__device__ __forceinline__ bool wait_for(unsigned long long* p, unsigned long long goal, uint32_t* dead) {
+__device__ __forceinline__ bool wait_for(unsigned long long* p, unsigned long long goal, uint32_t* dead,
+                                         unsigned long long limit_ns) {
   unsigned long long t0 = 0ull;
   for (unsigned spin = 0;; ++spin) {
     if (*reinterpret_cast<volatile unsigned long long*>(p) >= goal) return true;
     if ((spin & 1023u) != 1023u) continue;
     if (t0 == 0ull) t0 = now_ns();
-    if (*reinterpret_cast<volatile uint32_t*>(dead) || now_ns() - t0 > kWaitNs) {
+    if (*reinterpret_cast<volatile uint32_t*>(dead) || now_ns() - t0 > limit_ns) {
       atomicOr(dead, 1u);
       return false;
     }
@@ -301,7 +302,7 @@ struct Team {
         X::S().goal += (unsigned long long)K;
         __threadfence();
         atomicAdd(&c->arrived, 1ull);
-        X::S().alive = wait_for(&c->arrived, X::S().goal, &c->dead) ? 1 : 0;
+        X::S().alive = wait_for(&c->arrived, X::S().goal, &c->dead, X::S().wait_ns) ? 1 : 0;
         __threadfence();
       }
     }
@@ -1914,11 +1915,13 @@ template <int NT>
 __global__ void __launch_bounds__(NT, 1024 / NT) small_kernel(const SmallJob* jobs, int K, int mode, int resume,
                                                                SmallCfg cfg) {
   using X = Multi<NT>;
+  if (mode == kModeGrid && (int)blockIdx.x == cfg.hold) return;
   load_job<X>(jobs + blockIdx.x / K);
   const SmallJob& J = X::S().J;
   if (threadIdx.x == 0) {
     carve(J.work, J.V, J.E, J.dbl != 0, X::W());
     X::S().goal = 0ull;
+    X::S().wait_ns = (unsigned long long)cfg.wait_ns;
   }
   __syncthreads();
   Team<X> T{K, (int)(blockIdx.x % K), mode};
@@ -2112,6 +2115,10 @@ void set_attributes() {
 
 // Test hook (lvg_debug_small_launch): the error every launch of the levels meets.
 std::atomic<int32_t> g_launch_error{0};
+// Test hook (lvg_debug_small_hold): a block that stays away from the grid's
+// barriers, and their limit.
+std::atomic<int32_t> g_hold{-1};
+std::atomic<int64_t> g_wait_ns{SmallCfg().wait_ns};
 
 // False: such a launch is refused here (a cluster or a grid that must be on
 // the chip together, on a stream that may use a part of the chip).
@@ -2205,7 +2212,10 @@ int small_grid_blocks() {
   return n;
 }
 
-bool small_run_grid(const SmallJob* d_job, void* work, int K, const SmallCfg& cfg, cudaStream_t s) {
+bool small_run_grid(const SmallJob* d_job, void* work, int K, const SmallCfg& given, cudaStream_t s) {
+  SmallCfg cfg = given;
+  cfg.hold = g_hold.load();
+  cfg.wait_ns = g_wait_ns.load();
   // the barrier's words, and the phase, should a wait run out
   LVG_CUDA(cudaMemsetAsync(work, 0, up256(sizeof(Ctl)) + up256(sizeof(Between)), s));
   set_attributes();
@@ -2220,5 +2230,12 @@ bool small_run_grid(const SmallJob* d_job, void* work, int K, const SmallCfg& cf
 
 extern "C" lvg_status lvg_debug_small_launch(int32_t error) {
   lvg::g_launch_error.store(error);
+  return LVG_OK;
+}
+
+extern "C" lvg_status lvg_debug_small_hold(int32_t block, int64_t wait_ns) {
+  if (wait_ns < 0) return LVG_ERR_INVALID_ARG;
+  lvg::g_hold.store(block);
+  lvg::g_wait_ns.store(wait_ns > 0 ? wait_ns : lvg::SmallCfg().wait_ns);
   return LVG_OK;
 }

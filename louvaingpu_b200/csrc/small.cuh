@@ -68,6 +68,8 @@ struct SmallJob {
 struct SmallCfg {
   double pass_min, level_min;
   int32_t max_passes, max_levels;
+  int32_t hold = -1;                // grid: a block that stays away (test hook)
+  int64_t wait_ns = 4000000000ll;   // limit of a grid barrier's wait
 };
 
 size_t small_list_bytes(int64_t E);           // both coarse list buffers

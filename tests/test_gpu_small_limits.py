@@ -190,7 +190,7 @@ def hooks():
     from louvaingpu_b200 import _lib
     L = _lib.load()
     yield L
-    assert L.lvg_debug_small_launch(0) == 0
+    assert L.lvg_debug_small_launch(0) == 0 and L.lvg_debug_small_hold(-1, 0) == 0
 
 
 def launches():
@@ -248,3 +248,26 @@ def test_other_launch_errors_are_reported(Louvain, gen, hooks):
         assert hooks.lvg_debug_small_launch(0) == 0
         lv.load_edges(s, d, w, n)
         assert lv.run() == ref
+
+
+@pytest.mark.parametrize("unsorted", [False, True])
+def test_a_grid_wait_runs_out(Louvain, oracle, gen, hooks, unsorted):
+    """A block that never comes to the grid's barriers: the others give up
+    after 20 ms and the level kernels run instead."""
+    n, s, d, w = gen.sbm(30011, 300, 0.15, 2.0 / 30011, 1, 4, seed=5)
+    if unsorted:
+        o = np.random.default_rng(2).permutation(len(s))
+        s, d, w = s[o], d[o], w[o]
+    orun = oracle.Run(n, s, d, w)
+    with Louvain() as lv:
+        lv.load_edges(s, d, w, n)
+        ref, n_ref = run_counted(lv)
+        for block in (0, 1):
+            lv.load_edges(s, d, w, n)      # (a second run would build level 0 again)
+            assert hooks.lvg_debug_small_hold(block, 20_000_000) == 0
+            res, n_res = run_counted(lv)
+            assert n_res > n_ref + 20
+            run_equal(lv, res, orun, n, s, d, w, oracle)
+        assert hooks.lvg_debug_small_hold(-1, 0) == 0
+        lv.load_edges(s, d, w, n)
+        assert run_counted(lv) == (ref, n_ref)
