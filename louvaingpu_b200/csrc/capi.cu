@@ -463,7 +463,9 @@ bool run_small(lvg_ctx* c, RunState& R) {
   const int64_t parts_cap = 2 * (int64_t)kRoomLevels * V;
   // level 0: checked at load; later lists are symmetric when their CSR was written
   const bool any_order = c->level > 0 && !c->pre_next.valid;
-  const size_t need = small_list_bytes(E) + small_work_bytes(V, E, any_order) + sizeof(int32_t) * ((size_t)parts_cap + V) +
+  const bool cluster = E + V <= kSmallClusterEntries;
+  const int blocks = cluster ? kSmallClusterBlocks : std::max(small_grid_blocks(), kSmallClusterBlocks);
+  const size_t need = small_list_bytes(E) + small_work_bytes(V, E, any_order, blocks) + sizeof(int32_t) * ((size_t)parts_cap + V) +
                       small_state_bytes(V) + sizeof(SmallOut) + sizeof(SmallJob) + 16 * Arena::kAlign;
   if (a.hi < a.lo || a.hi - a.lo < need) return false;
   c->pristine = false;
@@ -482,12 +484,13 @@ bool run_small(lvg_ctx* c, RunState& R) {
   J.state = (double*)a.alloc_hi(small_state_bytes(V));
   const size_t run_hi = a.hi;
   J.check = J.dbl = any_order ? 1 : 0;
+  J.blocks = blocks;
   J.want_q = c->level == 0 ? 1 : 0;
   SmallOut o;
   std::memset(&o.res, 0, sizeof o.res);
   {
     HiScope hs(a);
-    J.work = (char*)a.alloc_hi(small_work_bytes(V, E, any_order));
+    J.work = (char*)a.alloc_hi(small_work_bytes(V, E, any_order, blocks));
     J.comp = c->level == 0 ? c->composed : a.hi_n<int32_t>(V);
     SmallOut* d_out = a.hi_n<SmallOut>(1);
     J.res = &d_out->res;
@@ -496,7 +499,7 @@ bool run_small(lvg_ctx* c, RunState& R) {
     LVG_CUDA(cudaMemcpyAsync(d_job, &J, sizeof J, cudaMemcpyHostToDevice, s));
     const SmallCfg cfg{c->cfg.pass_min_gain, c->cfg.level_min_gain, c->cfg.max_passes, c->cfg.max_levels};
     LVG_CUDA(cudaMemsetAsync(J.res, 0, sizeof(SmallResult), s));
-    const bool taken = E + V <= kSmallClusterEntries
+    const bool taken = cluster
                            ? small_run(d_job, 1, kSmallClusterBlocks, cfg, s)
                            : small_run_grid(d_job, J.work, small_grid_blocks(), cfg, s);
     if (taken) LVG_CUDA(cudaMemcpyAsync(&o, d_out, sizeof o, cudaMemcpyDeviceToHost, s));
@@ -1606,7 +1609,7 @@ SmallBatch batch_small_start(lvg_ctx* c, const BatchInput& in, int32_t* part_d) 
   int64_t others = in.eoff[in.G], other_v = in.voff[in.G];
   for (int32_t g : which) {
     lists += Arena::up(small_list_bytes(entries(g)));
-    work += Arena::up(small_work_bytes(in.voff[g + 1] - in.voff[g], entries(g), false));
+    work += Arena::up(small_work_bytes(in.voff[g + 1] - in.voff[g], entries(g), false, small_blocks(entries(g))));
     others -= entries(g);
     other_v -= in.voff[g + 1] - in.voff[g];
   }
@@ -1633,7 +1636,8 @@ SmallBatch batch_small_start(lvg_ctx* c, const BatchInput& in, int32_t* part_d) 
     J.lists = lp;
     J.work = wp;
     lp += Arena::up(small_list_bytes(J.E));
-    wp += Arena::up(small_work_bytes(J.V, J.E, false));
+    J.blocks = small_blocks(J.E);
+    wp += Arena::up(small_work_bytes(J.V, J.E, false, J.blocks));
     J.comp = part_d + in.voff[g];
     J.res = B.res + k;
     J.check = 1;

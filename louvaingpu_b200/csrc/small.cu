@@ -113,7 +113,8 @@ struct Work {
 __host__ __device__ inline size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // dbl: room for the doubled list of a level and the CSR made from it.
-__host__ __device__ inline size_t carve(char* base, int64_t V, int64_t E, bool dbl, Work& W) {
+// blocks: of the job's team, at most (one has no counts to share).
+__host__ __device__ inline size_t carve(char* base, int64_t V, int64_t E, bool dbl, int blocks, Work& W) {
   size_t o = 0;
   const int64_t n = dbl ? 2 * E : E;
   auto take = [&](size_t bytes) {
@@ -148,7 +149,7 @@ __host__ __device__ inline size_t carve(char* base, int64_t V, int64_t E, bool d
   W.cdst = dbl ? (int32_t*)take(4 * n) : nullptr;
   W.cw = dbl ? (float*)take(4 * n) : nullptr;
   W.longs = (int32_t*)take(4 * (n / kShortRow + 1));
-  W.ghist = (uint32_t*)take(4 * kDigits * kSmallMaxBlocks);
+  W.ghist = (uint32_t*)take(blocks > 1 ? 4 * kDigits * blocks : 0);
   W.rc = (int32_t*)take(4 * kResV);
   return o;
 }
@@ -1919,7 +1920,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) small_kernel(const SmallJob* jo
   load_job<X>(jobs + blockIdx.x / K);
   const SmallJob& J = X::S().J;
   if (threadIdx.x == 0) {
-    carve(J.work, J.V, J.E, J.dbl != 0, X::W());
+    carve(J.work, J.V, J.E, J.dbl != 0, J.blocks, X::W());
     X::S().goal = 0ull;
     X::S().wait_ns = (unsigned long long)cfg.wait_ns;
   }
@@ -1956,7 +1957,7 @@ __global__ void __launch_bounds__(kResThreads, 1) small_tail_kernel(const SmallJ
   load_job<X>(jobs + blockIdx.x);
   const SmallJob& J = X::S().J;
   Work g;
-  carve(J.work, J.V, J.E, J.dbl != 0, g);
+  carve(J.work, J.V, J.E, J.dbl != 0, J.blocks, g);
   Between& B = *g.bt;
   const int32_t phase = B.phase;
   int32_t ncomms = B.ncomms;
@@ -2007,7 +2008,7 @@ constexpr int kQThreads = 512;
 __global__ void __launch_bounds__(kQThreads) small_sum_kernel(const SmallJob* jobs, int K) {
   const SmallJob& J = jobs[blockIdx.x / K];
   Work g;
-  carve(J.work, J.V, J.E, J.dbl != 0, g);
+  carve(J.work, J.V, J.E, J.dbl != 0, J.blocks, g);
   const Between& B = *g.bt;
   if (!wants_q(J, B)) return;
   const int32_t how = B.comp;
@@ -2055,7 +2056,7 @@ struct QSpace {
 __global__ void __launch_bounds__(kQThreads) small_end_kernel(const SmallJob* jobs, int K) {
   const SmallJob& J = jobs[blockIdx.x / K];
   Work g;
-  carve(J.work, J.V, J.E, J.dbl != 0, g);
+  carve(J.work, J.V, J.E, J.dbl != 0, J.blocks, g);
   const Between& B = *g.bt;
   if (B.phase != kPhaseEnd) return;   // a barrier's wait ran out: no result
   const int32_t how = B.comp;
@@ -2172,9 +2173,9 @@ void launch_rest(const SmallJob* jobs, int n, int K, const SmallCfg& cfg, cudaSt
 
 size_t small_list_bytes(int64_t E) { return 6 * up256(4 * (size_t)E); }
 
-size_t small_work_bytes(int32_t V, int64_t E, bool dbl) {
+size_t small_work_bytes(int32_t V, int64_t E, bool dbl, int blocks) {
   Work W;
-  return carve(nullptr, V, E, dbl, W);
+  return carve(nullptr, V, E, dbl, blocks, W);
 }
 
 void small_list(char* lists, int64_t E, int buf, int32_t** src, int32_t** dst, float** w) {

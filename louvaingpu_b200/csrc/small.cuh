@@ -51,7 +51,7 @@ struct SmallJob {
   int32_t level0;           // level of the given list in its run
   double mod;               // Q of the level before (level0 > 0)
   char* lists;              // two coarse list buffers of E entries each
-  char* work;               // small_work_bytes(V, E)
+  char* work;               // small_work_bytes(V, E, dbl, blocks)
   int32_t* parts;           // per-level partitions and labels, or nullptr
   int64_t parts_cap;        // ints
   int32_t* comp;            // [V] composition of the levels' partitions
@@ -62,7 +62,7 @@ struct SmallJob {
   int32_t check;            // 1: ids, weights, order and symmetry not checked yet
   int32_t want_q;
   int32_t dbl;              // 1: work has room for lists in any order (small_work_bytes with dbl)
-  int32_t pad;
+  int32_t blocks;           // most blocks that work on it at a time
 };
 
 struct SmallCfg {
@@ -73,7 +73,7 @@ struct SmallCfg {
 };
 
 size_t small_list_bytes(int64_t E);           // both coarse list buffers
-size_t small_work_bytes(int32_t V, int64_t E, bool dbl);
+size_t small_work_bytes(int32_t V, int64_t E, bool dbl, int blocks);
 inline size_t small_state_bytes(int32_t V) { return (2 * sizeof(double) + sizeof(int32_t)) * (size_t)V; }
 // Coarse list buffer `buf` of a job's lists.
 void small_list(char* lists, int64_t E, int buf, int32_t** src, int32_t** dst, float** w);

@@ -271,3 +271,16 @@ def test_a_grid_wait_runs_out(Louvain, oracle, gen, hooks, unsorted):
         assert hooks.lvg_debug_small_hold(-1, 0) == 0
         lv.load_edges(s, d, w, n)
         assert run_counted(lv) == (ref, n_ref)
+
+
+def test_thousands_of_tiny_graphs_run_by_clusters(Louvain, oracle):
+    """Their memory is a few KB each, so a default arena holds them all: one
+    launch of the levels and three behind it, not a union's."""
+    from test_gpu_batch_edges import cycle
+    graphs = [cycle(3 + k % 60, 1.0 + k % 5) for k in range(3000)]
+    with Louvain() as lv:
+        lv.run_batch(graphs)
+        n = launches()
+        b = lv.run_batch(graphs)
+        assert launches() - n <= 8
+    check_sample(oracle, graphs, b.part, b.n_levels, range(0, 3000, 97))
