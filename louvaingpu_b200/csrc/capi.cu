@@ -465,8 +465,9 @@ bool run_small(lvg_ctx* c, RunState& R) {
   const bool any_order = c->level > 0 && !c->pre_next.valid;
   const bool cluster = E + V <= kSmallClusterEntries;
   const int blocks = cluster ? kSmallClusterBlocks : std::max(small_grid_blocks(), kSmallClusterBlocks);
-  const size_t need = small_list_bytes(E) + small_work_bytes(V, E, any_order, blocks) + sizeof(int32_t) * ((size_t)parts_cap + V) +
-                      small_state_bytes(V) + sizeof(SmallOut) + sizeof(SmallJob) + 16 * Arena::kAlign;
+  const size_t need = small_list_bytes(E) + small_work_bytes(V, E, any_order, blocks) +
+                      sizeof(int32_t) * ((size_t)parts_cap + V) + small_state_bytes(V) +
+                      sizeof(float) * kSmallPassCap + sizeof(SmallOut) + sizeof(SmallJob) + 16 * Arena::kAlign;
   if (a.hi < a.lo || a.hi - a.lo < need) return false;
   c->pristine = false;
   const size_t lo0 = a.lo, hi0 = a.hi;
@@ -488,6 +489,7 @@ bool run_small(lvg_ctx* c, RunState& R) {
   J.want_q = c->level == 0 ? 1 : 0;
   SmallOut o;
   std::memset(&o.res, 0, sizeof o.res);
+  std::vector<float> ticks;   // moves of the last level's passes
   {
     HiScope hs(a);
     J.work = (char*)a.alloc_hi(small_work_bytes(V, E, any_order, blocks));
@@ -495,6 +497,7 @@ bool run_small(lvg_ctx* c, RunState& R) {
     SmallOut* d_out = a.hi_n<SmallOut>(1);
     J.res = &d_out->res;
     J.lv = d_out->lv;
+    J.pass_ticks = a.hi_n<float>(kSmallPassCap);
     SmallJob* d_job = a.hi_n<SmallJob>(1);
     LVG_CUDA(cudaMemcpyAsync(d_job, &J, sizeof J, cudaMemcpyHostToDevice, s));
     const SmallCfg cfg{c->cfg.pass_min_gain, c->cfg.level_min_gain, c->cfg.max_passes, c->cfg.max_levels};
@@ -503,11 +506,18 @@ bool run_small(lvg_ctx* c, RunState& R) {
                            ? small_run(d_job, 1, kSmallClusterBlocks, cfg, s)
                            : small_run_grid(d_job, J.work, small_grid_blocks(), cfg, s);
     if (taken) LVG_CUDA(cudaMemcpyAsync(&o, d_out, sizeof o, cudaMemcpyDeviceToHost, s));
-    if (c->level > 0) {   // a launch that finishes no level leaves no composition
-      sync(c);
-      if (o.res.finished && o.res.n_levels > 0) compose(c->composed, J.comp, c->V0, s);
-    }
     sync(c);
+    if (o.res.finished && o.res.n_levels > 0) {   // (a launch that finishes no level leaves no composition)
+      if (c->level > 0) compose(c->composed, J.comp, c->V0, s);
+      const SmallLevel& z = o.lv[o.res.n_levels - 1];
+      ticks.assign(z.pass_ticks, z.pass_ticks + std::min(z.passes, 2));
+      if (z.passes > 2 && !o.res.open) {
+        ticks.resize(z.passes);
+        LVG_CUDA(cudaMemcpyAsync(ticks.data() + 2, J.pass_ticks + 2, sizeof(float) * (z.passes - 2),
+                                 cudaMemcpyDeviceToHost, s));
+      }
+      if (c->level > 0 || z.passes > 2) sync(c);
+    }
   }
   if (!o.res.finished || o.res.n_levels == 0) {
     a.lo = lo0;
@@ -544,7 +554,7 @@ bool run_small(lvg_ctx* c, RunState& R) {
   c->C_cur = z.C;
   c->pass_ms.assign(1, (float)(z.ticks[1] * o.res.ms_per_tick));
   c->move_pass_ms.clear();
-  for (int p = 0; p < std::min(z.passes, 2); ++p) c->move_pass_ms.push_back((float)(z.pass_ticks[p] * o.res.ms_per_tick));
+  for (float t : ticks) c->move_pass_ms.push_back((float)(t * o.res.ms_per_tick));
   c->move_passes = z.passes;
   c->move_ms = 0.0;
   for (float ms : c->move_pass_ms) c->move_ms += ms;

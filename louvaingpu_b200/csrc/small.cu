@@ -1757,6 +1757,7 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
         }
       }
       if (pass <= 2) pass_ticks[pass - 1] = (float)(clock64() - p0);
+      else if (lead && J.pass_ticks) J.pass_ticks[pass - 1] = (float)(clock64() - p0);
       if (stop || capped) {
         st = stop ? LVG_OK : LVG_ERR_NOT_CONVERGED;
         break;

@@ -17,7 +17,7 @@ struct SmallLevel {
   int64_t E, nnz;
   double q_start, q_level;
   float ticks[kSmallPhases];
-  float pass_ticks[2];      // the moves of the first two passes
+  float pass_ticks[2];      // the moves of the first two passes; SmallJob::pass_ticks has any others
   int64_t part_off;         // partition at parts + part_off, labels V later
 };
 
@@ -59,6 +59,7 @@ struct SmallJob {
                             // level's communities: tot, in, then (int32) sizes, one array behind the other
   SmallResult* res;
   SmallLevel* lv;           // [kSmallLevels], or nullptr
+  float* pass_ticks;        // [kSmallPassCap] moves of the last level's passes from the third on, or nullptr
   int32_t check;            // 1: ids, weights, order and symmetry not checked yet
   int32_t want_q;
   int32_t dbl;              // 1: work has room for lists in any order (small_work_bytes with dbl)

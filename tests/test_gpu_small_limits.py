@@ -284,3 +284,21 @@ def test_thousands_of_tiny_graphs_run_by_clusters(Louvain, oracle):
         b = lv.run_batch(graphs)
         assert launches() - n <= 8
     check_sample(oracle, graphs, b.part, b.n_levels, range(0, 3000, 97))
+
+
+@pytest.mark.parametrize("n,blocks", [(300, 6), (2000, 40), (30011, 300)])
+@pytest.mark.parametrize("max_passes", [1, 2, 5, 40])
+def test_every_pass_of_the_last_level_has_its_time(Louvain, gen, n, blocks, max_passes):
+    """A gain below the threshold never ends this level: it takes all passes
+    it may (by one block, a cluster, a grid)."""
+    from louvaingpu_b200 import LvgError
+    n, s, d, w = gen.sbm(n, blocks, 15.0 * blocks / n, 2.0 / n, 1, 4, seed=5)
+    with Louvain(pass_min_gain=-2.0, max_passes=max_passes) as lv:
+        lv.load_edges(s, d, w, n)
+        with pytest.raises(LvgError) as e:
+            lv.run()
+        assert e.value.status == 4 and lv.n_levels == 1 and lv.level_info(0).passes == max_passes
+        times = lv.move_pass_times()
+        total, passes = lv.move_stats()
+    assert len(times) == passes == max_passes
+    assert all(t > 0 for t in times) and total == pytest.approx(sum(times), rel=1e-5)
