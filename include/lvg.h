@@ -60,9 +60,15 @@ typedef struct {
                               * while the level-0 CSR is built from the chunks already on the device
                               * (0: 2^25; rounded up to a multiple of 2048; lists of fewer than two
                               * chunks are copied whole, then built) */
+                           /* The settings from tile_max_degree to l2_persist, and coarsen_mode, are those
+                            * of the level kernels.  A sorted and symmetric list of at most 4 Mi entries
+                            * and 2^18 vertices that lvg_run starts from or reaches as a level (in a
+                            * batch: a graph of at most 256 Ki entries) has its levels run inside a few
+                            * launches instead, with the same results and without these settings. */
   int32_t coarsen_mode;    /* coarsening of a sorted symmetric level list (InducedGraphKernel.cu:50-113):
                             * 0 automatic, 1 segment chunks, 2 by transposition, 3 sort of all keys;
                             * every mode writes the same coarse list */
+  int32_t level_kernels;   /* 1: the level kernels for every list; 0: where they are the faster ones */
 } lvg_config;
 
 /* Per-level record of a run (the reference keeps one Partition per level,
@@ -97,8 +103,9 @@ const char* lvg_status_string(lvg_status s);
  * context's own stream. */
 lvg_status lvg_set_stream(lvg_ctx* ctx, void* stream);
 
-/* Load the level-0 edge list from HOST memory and build the level CSR, degrees
- * and self-loop weights.  Replaces the driver's H2D copies
+/* Load the level-0 edge list from HOST memory, check it, and build the level
+ * CSR, degrees and self-loop weights (of a list that lvg_run takes without them,
+ * with the first call that needs them).  Replaces the driver's H2D copies
  * (LouvainCPP.cpp:283-287) followed by CalculateNeighbour (NeighbourCompute.cu:42)
  * and initCUDA (InitKernel.cu:245). */
 lvg_status lvg_load_edges(lvg_ctx* ctx, const int32_t* src, const int32_t* dst, const float* w,
@@ -375,7 +382,8 @@ typedef struct {
  * the hashing passes.  Pairs within 2 % of the fastest defer to the context's
  * configured pair when it is among them (lvg_tune_pick).  The chosen pair is
  * then used by every level built afterwards (this graph's later levels,
- * lvg_run, batched runs of this context) and the context is left at level 0,
+ * lvg_run, batched runs of this context; not by lists that take no level
+ * kernels, see lvg_config) and the context is left at level 0,
  * rebuilt, as after a load.  Shape class = (device, floor(log2 V),
  * floor(log2 nnz), floor(log2 max degree), integral weights); the process-wide
  * cache keeps the pair of each class.  points (nullable, cap entries) receives

@@ -38,6 +38,7 @@ class LvgConfig(ctypes.Structure):
         ("l2_persist", ctypes.c_int32),
         ("load_chunk_entries", ctypes.c_int64),
         ("coarsen_mode", ctypes.c_int32),
+        ("level_kernels", ctypes.c_int32),
     ]
 
 

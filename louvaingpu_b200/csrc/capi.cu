@@ -203,7 +203,7 @@ void load_common(lvg_ctx* c, const int32_t* d_src, const int32_t* d_dst, const f
   // build until a call needs it -- if the arena has room for any list's build,
   // so that what a load refuses for lack of memory does not depend on the
   // list's order.
-  const bool ready = facts && facts->sorted_symmetric && small_fits(V, E, kSmallRunEntries) &&
+  const bool ready = !c->cfg.level_kernels && facts && facts->sorted_symmetric && small_fits(V, E, kSmallRunEntries) &&
                      c->arena.cap >= arena_estimate(V, E, copied);
   c->V0 = V;
   c->E0 = E;
@@ -455,7 +455,7 @@ struct RunState {
 bool run_small(lvg_ctx* c, RunState& R) {
   const int32_t V = c->g.V;
   const int64_t E = c->g.E;
-  if (R.no_small || !small_fits(V, E, kSmallRunEntries)) return false;
+  if (c->cfg.level_kernels || R.no_small || !small_fits(V, E, kSmallRunEntries)) return false;
   Arena& a = c->arena;
   cudaStream_t s = c->stream;
   a.hi = c->run_hi;
@@ -1607,6 +1607,7 @@ SmallBatch batch_small_start(lvg_ctx* c, const BatchInput& in, int32_t* part_d) 
   cudaStream_t s = c->stream;
   SmallBatch B;
   std::vector<int32_t>& which = B.which;
+  if (c->cfg.level_kernels) return B;
   for (int32_t g = 0; g < in.G; ++g)
     if (small_fits(in.voff[g + 1] - in.voff[g], in.eoff[g + 1] - in.eoff[g], kSmallBatchEntries)) which.push_back(g);
   if (which.empty()) return B;

@@ -81,7 +81,7 @@ def pack_graphs(graphs):
 class Louvain:
     def __init__(self, device=0, pass_min_gain=1e-7, level_min_gain=1e-7, max_passes=-1, max_levels=-1,
                  arena_bytes=0, tile_max_degree=0, block_max_degree=0, passes_per_sync=0, use_graphs=True, l2_persist=True,
-                 load_chunk_entries=0, coarsen_mode=0):
+                 load_chunk_entries=0, coarsen_mode=0, level_kernels=False):
         L = _lib.load()
         cfg = _lib.LvgConfig()
         L.lvg_config_default(ctypes.byref(cfg))
@@ -101,6 +101,7 @@ class Louvain:
         cfg.l2_persist = 1 if l2_persist else 0
         cfg.load_chunk_entries = int(load_chunk_entries)
         cfg.coarsen_mode = int(coarsen_mode)
+        cfg.level_kernels = 1 if level_kernels else 0
         self._L = L
         h = ctypes.c_void_p()
         _lib.check(None, L.lvg_create(ctypes.byref(cfg), ctypes.byref(h)))
