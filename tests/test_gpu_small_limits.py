@@ -302,3 +302,69 @@ def test_every_pass_of_the_last_level_has_its_time(Louvain, gen, n, blocks, max_
         total, passes = lv.move_stats()
     assert len(times) == passes == max_passes
     assert all(t > 0 for t in times) and total == pytest.approx(sum(times), rel=1e-5)
+
+
+def sized(n, entries, seed=0):
+    """A sorted symmetric list of exactly `entries` entries on n vertices in
+    blocks of 64 (an odd number has a self loop)."""
+    rng, pairs = np.random.default_rng(seed), entries // 2
+    at = np.zeros(0, np.int64)
+    while len(at) < pairs:
+        a = rng.integers(0, n, 2 * pairs)
+        b = np.where(rng.random(len(a)) < 0.7, a // 64 * 64 + rng.integers(0, 64, len(a)), rng.integers(0, n, len(a)))
+        b = np.minimum(b, n - 1)
+        at = np.union1d(at, (np.minimum(a, b) * n + np.maximum(a, b))[a != b])
+    a, b = np.divmod(rng.permutation(at)[:pairs], n)
+    w = rng.integers(1, 5, pairs)
+    loop = [n // 2] if entries % 2 else []
+    s, d, w = np.concatenate([a, b, loop]), np.concatenate([b, a, loop]), np.concatenate([w, w, [3] * len(loop)])
+    return in_order(n, s.astype(np.int32), d.astype(np.int32), w.astype(np.float32))
+
+
+MAX_V, MAX_E, CLUSTER, RESIDENT = 1 << 18, 1 << 22, 1 << 16, (512, 6144)
+
+
+@pytest.mark.parametrize("make,small", [
+    (lambda: sized(MAX_V, 1500000), True), (lambda: sized(MAX_V + 1, 1500000), False),
+    (lambda: sized(MAX_V, 20000), True), (lambda: sized(MAX_V + 1, 20000), False),
+    (lambda: sized(90000, MAX_E), True), (lambda: sized(90000, MAX_E + 1), False),
+    (lambda: sized(15536, CLUSTER - 15536), True), (lambda: sized(15536, CLUSTER - 15535), True),
+    (lambda: sized(*RESIDENT), True), (lambda: sized(RESIDENT[0] + 1, RESIDENT[1]), True),
+    (lambda: sized(RESIDENT[0], RESIDENT[1] + 1), True)],
+    ids=["V", "V+1", "sparse_V", "sparse_V+1", "E", "E+1", "cluster", "grid", "block", "block_V+1", "block_E+1"])
+def test_limits_of_a_run(Louvain, oracle, make, small):
+    n, s, d, w = make()
+    orun = oracle.Run(n, s, d, w)
+    with Louvain() as lv:
+        lv.load_edges(s, d, w, n)
+        res, count = run_counted(lv)
+        assert (count < 10) == small
+        run_equal(lv, res, orun, n, s, d, w, oracle)
+        assert lv.modularity() == lv.level_info(res.n_levels - 1).q_level
+
+
+def test_limits_of_a_batch(Louvain, oracle):
+    """Graphs at and one entry above the steps of the clusters' sizes, and of
+    what a batch gives to clusters."""
+    graphs = [sized(k // 12, k + more) for k in (16 << 10, 48 << 10, 128 << 10, 256 << 10) for more in (0, 1)]
+    with Louvain(arena_bytes=1 << 30) as lv:
+        b = lv.run_batch(graphs)
+    check_sample(oracle, graphs, b.part, b.n_levels, range(len(graphs)))
+
+
+@pytest.mark.parametrize("n", [200, 1000])
+def test_runs_of_more_levels_than_a_launch_takes(Louvain, oracle, n):
+    """A ring merges a few vertices a level: the launch leaves the run open
+    (its levels' partitions, or records, are full) and the level kernels end it."""
+    from test_gpu_batch_edges import cycle
+    n, s, d, w = cycle(n)
+    orun = oracle.Run(n, s, d, w)
+    assert len(orun.levels) > 12
+    with Louvain() as lv:
+        lv.load_edges(s, d, w, n)
+        res, count = run_counted(lv)
+        assert count > 100
+        run_equal(lv, res, orun, n, s, d, w, oracle)
+        b = lv.run_batch([(n, s, d, w), triangles()])
+        np.testing.assert_array_equal(b.part(0), orun.final)
+        assert b.n_levels[0] == len(orun.levels)
