@@ -199,7 +199,7 @@ uint32_t* facts_room(lvg_ctx* c, int32_t V, int64_t E) {
 // built while it streamed in.
 void load_common(lvg_ctx* c, const int32_t* d_src, const int32_t* d_dst, const float* d_w, int64_t E,
                  int32_t V, bool copied, const ListFacts* facts) {
-  // A sorted and symmetric list that one launch can run waits with its level
+  // A sorted and symmetric list that a small run takes waits with its level
   // build until a call needs it -- if the arena has room for any list's build,
   // so that what a load refuses for lack of memory does not depend on the
   // list's order.
@@ -449,7 +449,7 @@ struct RunState {
   bool no_small = false; // a list was found not to be in small_run's form
 };
 
-// Runs the levels from the current one (a list, not built) on in one launch.
+// Runs the levels from the current one (a list, not built) on as a small run.
 // Returns true when that finished the run.  Otherwise the context stands at
 // the level it left open (perhaps the same one), still only a list.
 bool run_small(lvg_ctx* c, RunState& R) {

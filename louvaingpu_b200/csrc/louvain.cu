@@ -2629,6 +2629,11 @@ static void launch_thread(const LevelGraph& g, MoveArgs P, int bucket, cudaStrea
 // done.  Level-0 passes (both, ms) of R-MAT 25 / 24 / 22 at the default
 // thresholds, with 8 and 5 blocks (all that fit) 48.4 / 20.5 / 4.3, 5 and 4
 // 46.9 / 20.3 / 4.3, 4 and 3 45.0 / 20.0 / 4.2, 4 and 2 49.7 / 21.1 / 4.9.
+// Power-law graphs without R-MAT's structure gain nothing and lose nothing by 4
+// and 3 (hashing pass, ms, exponents 2.0 / 2.2 / 2.5 of 49 / 76 / 80 M entries:
+// as many as fit 1.26 / 1.76 / 1.69, 4 and 3 1.27 / 1.76 / 1.69, 4 and 2 1.27 /
+// 2.13 / 2.34, 5 and 4 1.29 / 1.84 / 1.92, 3 and 3 1.25 / 1.79 / 1.69), nor do
+// LFR and block graphs, which do not reach the rule.
 // With fewer block-class rows than a wave of their kernel, or in a batch, whose
 // rows are mostly the tiles', there is little to make room for (128 mixed
 // graphs: 39.4 ms without the limit, 40.5 with it).

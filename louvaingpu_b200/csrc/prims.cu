@@ -205,13 +205,13 @@ __device__ __forceinline__ void rs_publish(unsigned long long* w, unsigned code,
 // tiles by decoupled look-back, and writes its keys out digit run by digit
 // run.  Stable: ranks follow key order inside a tile and tiles in order.
 //
-// Bound by shared memory (the L1 data stage is 70 % busy, DRAM 33 %): a key
-// costs some 40 wavefronts per 32, half of them conflicts on random digits.
-// So nothing is looked up twice: ranks and staged positions are kept in 16
-// bits, a digit's lanes meet in one word (an atomic or, 2.5 cycles a warp and
-// SM; a match instruction costs 62), and what can be packed into the key's
-// free bits comes without values (lists of whole weights, induce.cu).  Three
-// tiles fit an SM (two before); the look-back reads kRsWindow tiles at a time.
+// Bound by shared memory (the coarsening's passes on R-MAT scale 20, 31.4 M
+// keys: the L1 data stage 60 to 69 % busy, DRAM 23 to 25 %).  So nothing is
+// looked up twice: ranks and staged positions are kept in 16 bits, a digit's
+// lanes meet in one word (an atomic or, where a match instruction was the
+// slower), and what can be packed into the key's free bits comes without
+// values (lists of whole weights, induce.cu).  Three tiles fit an SM (two
+// before); the look-back reads kRsWindow tiles at a time.
 // 134 M random keys, three passes: 4.81 -> 3.84 ms, 2.96 ms without values.
 template <bool VALS>
 __global__ void __launch_bounds__(kRsThreads, 3) rs_onesweep_kernel(

@@ -1,4 +1,4 @@
-// Whole dendrograms of small graphs in one launch (small.cu).
+// Whole dendrograms of small graphs inside a few launches (small.cu).
 #pragma once
 #include "louvain.cuh"
 
