@@ -68,6 +68,10 @@ struct lvg_ctx {
   ListFacts facts0;              //   for a call that needs its build after all
   const double* kept = nullptr;  // not built because small_run finished the run on this level: the state
                                  //   it ended in (SmallJob::state), with the last level's labels
+  bool loose = false;            // a small run has left room between what is still needed (tighten):
+  size_t tight_lo = 0;           //   the low mark to which the level's list may move,
+  size_t tight_hi = 0;           //   the high mark below the partitions
+  bool list_moves = false;       //   the list lies above that low mark
   bool timed = false;            // the last level's renumbering is between pev[2] and pev[3]
   bool pristine = false;         // level 0 as loaded: no pass, state change or renumbering since
   bool symmetric0 = false;       // the level-0 list was found sorted and symmetric at load
@@ -226,6 +230,7 @@ void load_common(lvg_ctx* c, const int32_t* d_src, const int32_t* d_dst, const f
   c->small0 = ready;
   if (ready) c->facts0 = *facts;
   c->kept = nullptr;
+  c->loose = false;
   c->built = false;
   if (ready) {
     c->have_state = true;
@@ -254,6 +259,7 @@ void reset_to_level0(lvg_ctx* c, bool build = true) {
   c->g.w = c->w0;
   c->g.pre = &c->pre0;
   c->kept = nullptr;
+  c->loose = false;
   c->built = false;
   c->renumbered = false;
   if (build) prepare_level(c, c->small0 ? &c->facts0 : nullptr);
@@ -423,18 +429,68 @@ void induce_level(lvg_ctx* c) {
   c->level += 1;
   c->built = false;
   c->kept = nullptr;
+  c->loose = false;
   c->renumbered = false;
+}
+
+// Gives up what a small run took and the calls after it do not need: its list
+// buffers, the rest of its partitions' room.  What the level kernels could do
+// in an arena stays possible behind a small run.
+void tighten(lvg_ctx* c) {
+  if (!c->loose) return;
+  c->loose = false;
+  Arena& a = c->arena;
+  cudaStream_t s = c->stream;
+  const int64_t E = c->g.E;
+  auto copy = [&](void* to, const void* from, size_t bytes) {
+    LVG_CUDA(cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToDevice, s));
+  };
+  if (c->list_moves) {   // through scratch: the places may overlap
+    HiScope hs(a);
+    int32_t* ts = a.hi_n<int32_t>(E);
+    int32_t* td = a.hi_n<int32_t>(E);
+    float* tw = a.hi_n<float>(E);
+    copy(ts, c->g.src, sizeof(int32_t) * E);
+    copy(td, c->g.dst, sizeof(int32_t) * E);
+    copy(tw, c->g.w, sizeof(float) * E);
+    a.lo = c->tight_lo;
+    int32_t* src = a.lo_n<int32_t>(E);
+    int32_t* dst = a.lo_n<int32_t>(E);
+    float* w = a.lo_n<float>(E);
+    copy(src, ts, sizeof(int32_t) * E);
+    copy(dst, td, sizeof(int32_t) * E);
+    copy(w, tw, sizeof(float) * E);
+    c->g.src = src;
+    c->g.dst = dst;
+    c->g.w = w;
+  } else {
+    a.lo = c->tight_lo;
+  }
+  if (c->kept) {
+    const size_t bytes = small_state_bytes(c->g.V), from = (size_t)((const char*)c->kept - a.base);
+    const size_t to = c->tight_hi > bytes ? (c->tight_hi - bytes) & ~(Arena::kAlign - 1) : 0;
+    if (to >= from + bytes) {
+      copy(a.base + to, a.base + from, bytes);
+      c->kept = (const double*)(a.base + to);
+      c->run_hi = to;
+    }
+  } else {
+    c->run_hi = c->tight_hi;
+  }
+  a.hi = c->run_hi;
 }
 
 // The level's CSR and state, where a call needs them and only the list exists.
 void ensure_built(lvg_ctx* c) {
   if (c->built) return;
+  tighten(c);
   const bool renumbered = c->renumbered, pristine = c->pristine;
   prepare_level(c, c->small0 && c->level == 0 ? &c->facts0 : nullptr);
   if (c->kept) {
     set_state(c->g, c->st, c->levels.back().d_labels, c->kept, c->kept + c->g.V,
               reinterpret_cast<const int32_t*>(c->kept + 2 * (size_t)c->g.V), c->stream);
     c->kept = nullptr;
+    c->run_hi = c->arena.hi = c->tight_hi;
   }
   c->renumbered = renumbered;
   c->pristine = pristine;
@@ -531,7 +587,7 @@ bool run_small(lvg_ctx* c, RunState& R) {
     const SmallLevel& x = o.lv[l];
     LevelRec r;
     std::memset(&r.info, 0, sizeof r.info);
-    r.d_part = J.parts + x.part_off;
+    r.d_part = J.parts + x.part_off;   // the last level's is the lowest
     r.d_labels = r.d_part + x.V;
     r.info.n_vertices = x.V;
     r.info.n_entries = x.E;
@@ -576,8 +632,13 @@ bool run_small(lvg_ctx* c, RunState& R) {
     c->g.dst = ld;
     c->g.w = lw;
   }
-  c->pre_next = PreCsr();
-  c->g.pre = nullptr;
+  // (a run that ends on the level it began with leaves that level's CSR as it was)
+  if (o.res.buf >= 0) c->pre_next = PreCsr();
+  c->g.pre = c->level == 0 ? &c->pre0 : &c->pre_next;
+  c->loose = true;
+  c->list_moves = o.res.buf >= 0;
+  c->tight_lo = c->list_moves ? c->base_lo : lo0;
+  c->tight_hi = (size_t)((char*)c->d_part_cur - a.base) & ~(Arena::kAlign - 1);
   c->renumbered = !o.res.open;
   c->kept = o.res.open ? nullptr : J.state;
   if (o.res.open) {

@@ -1825,11 +1825,12 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
     }
     if (!T.sync()) return false;
     if (J.parts) {
+      int32_t* part = J.parts + (J.parts_cap - at.part_off - 2 * (int64_t)V);
 #pragma unroll 1
       for (int32_t i = T.gt(); i < V; i += T.stride()) {
         const int32_t c = W.comm[i];
-        J.parts[at.part_off + i] = W.newid[c];
-        J.parts[at.part_off + V + i] = c;
+        part[i] = W.newid[c];
+        part[V + i] = c;
       }
     }
     if constexpr (X::kResident) {
@@ -1871,7 +1872,7 @@ __device__ __forceinline__ bool run_levels(Team<X>& T, const SmallCfg& cfg, At& 
       R.ticks[3] = last ? 0.0f : (float)(clock64() - t3);
       R.pass_ticks[0] = pass_ticks[0];
       R.pass_ticks[1] = pass_ticks[1];
-      R.part_off = at.part_off;
+      R.part_off = J.parts_cap - at.part_off - 2 * (int64_t)V;
     }
     at.part_off += 2 * (int64_t)V;
     at.ncomms = (int32_t)C;

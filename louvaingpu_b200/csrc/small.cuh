@@ -52,7 +52,7 @@ struct SmallJob {
   double mod;               // Q of the level before (level0 > 0)
   char* lists;              // two coarse list buffers of E entries each
   char* work;               // small_work_bytes(V, E, dbl, blocks)
-  int32_t* parts;           // per-level partitions and labels, or nullptr
+  int32_t* parts;           // per-level partitions and labels, the first level's last, or nullptr
   int64_t parts_cap;        // ints
   int32_t* comp;            // [V] composition of the levels' partitions
   double* state;            // small_state_bytes(V), or nullptr: the state the run ends in, over the last

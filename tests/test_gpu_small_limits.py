@@ -368,3 +368,36 @@ def test_runs_of_more_levels_than_a_launch_takes(Louvain, oracle, n):
         b = lv.run_batch([(n, s, d, w), triangles()])
         np.testing.assert_array_equal(b.part(0), orun.final)
         assert b.n_levels[0] == len(orun.levels)
+
+
+def accepted(make, n, s, d, w, arena):
+    """Which of the calls of a session succeed in an arena."""
+    from louvaingpu_b200 import LvgError
+    out = []
+    with make(arena_bytes=arena) as lv:
+        for call in (lambda: lv.load_edges(s, d, w, n), lv.run, lv.modularity, lv.induce, lv.modularity, lv.run,
+                     lambda: lv.modularity_fp64(np.zeros(n, np.int32))):
+            try:
+                call()
+                out.append(True)
+            except LvgError as e:
+                assert e.status == 2 or (e.status == 6 and False in out)   # out of memory, or behind such a call
+                out.append(False)
+                if len(out) == 1:
+                    break
+    return out
+
+
+@pytest.mark.parametrize("kind", ["once", "sorted"])
+def test_tight_arenas_hold_what_the_level_kernels_do_there(Louvain, gen, kind):
+    """Few edges among 200,000 vertices, where a small run's memory differs
+    most: no call that succeeds by the level kernels is refused behind one."""
+    _, s, d, w = listed_once(2000, 8, 2) if kind == "once" else gen.sbm(500, 10, 0.3, 0.01, 1, 4, seed=1)
+    size, held = 30e6, 0
+    while size < 72e6:
+        level = accepted(lambda **kw: Louvain(level_kernels=True, **kw), 200000, s, d, w, int(size))
+        small = accepted(Louvain, 200000, s, d, w, int(size))
+        assert all(small[:len(level)][i] for i, ok in enumerate(level) if ok), (int(size), level, small)
+        held += all(level)
+        size *= 1.008
+    assert held > 10
